@@ -2,11 +2,14 @@
 
 There is no fallback: if the shared library is missing or its ABI version differs, loading raises."""
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import threading
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("FLASHMHF_LIB") or os.path.join(_PKG, "lib", "libflashmhf_b200.so")   # FLASHMHF_LIB: another build of the same ABI
+TORCH_PATH = os.path.join(_PKG, "lib", "_flashmhf_torch.so")
 ABI_VERSION = 3
 
 BF16, F32_CHECK = 0, 1
@@ -127,6 +130,29 @@ def load():
         lib.flashmhf_profile_end.argtypes = [C.POINTER(C.c_float), C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int)]
         _lib = lib
         return lib
+
+
+_native = None
+
+
+def native():
+    """Load (once) and return the torch host module (csrc/torch_host.cpp), bound to the library handle of ``load()``."""
+    global _native
+    if _native is not None:
+        return _native
+    import torch  # noqa: F401  (the module links against torch's libraries, which this import has loaded)
+    lib = load()
+    with _lock:
+        if _native is None:
+            if not os.path.exists(TORCH_PATH):
+                raise ImportError(f"{TORCH_PATH} is not built; run `python -m flashmhf_b200.build`")
+            loader = importlib.machinery.ExtensionFileLoader("_flashmhf_torch", TORCH_PATH)
+            spec = importlib.util.spec_from_file_location("_flashmhf_torch", TORCH_PATH, loader=loader)
+            mod = importlib.util.module_from_spec(spec)
+            loader.exec_module(mod)
+            mod.bind(lib._handle, FlashMHFError)
+            _native = mod
+    return _native
 
 
 def check(status):
