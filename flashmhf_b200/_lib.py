@@ -23,7 +23,8 @@ EXPORTS = ("flashmhf_abi_version", "flashmhf_forward_workspace_bytes", "flashmhf
            "flashmhf_backward_static_scratch", "flashmhf_prologue_forward",
            "flashmhf_prologue_backward_workspace_bytes", "flashmhf_prologue_backward", "flashmhf_lm_rope",
            "flashmhf_lm_rmsnorm_forward", "flashmhf_lm_rmsnorm_backward_workspace_bytes", "flashmhf_lm_rmsnorm_backward",
-           "flashmhf_selftest_bounded_wait")
+           "flashmhf_selftest_bounded_wait", "flashmhf_prologue_forward_dtype", "flashmhf_prologue_backward_dtype",
+           "flashmhf_lm_rmsnorm_forward_dtype", "flashmhf_lm_rmsnorm_backward_dtype")
 
 
 class Tensor(C.Structure):

@@ -272,14 +272,18 @@ int flashmhf_selftest_bounded_wait(long long limit_cycles, void *stream) {
     return rc;
 }
 
-int flashmhf_prologue_forward(const flashmhf_prologue_params *p, void *stream) {
+int flashmhf_prologue_forward_dtype(const flashmhf_prologue_params *p, int32_t param_dtype, void *stream) {
     if (!p) return FLASHMHF_ERR_NULL;
+    if (param_dtype != FLASHMHF_BF16 && param_dtype != FLASHMHF_F32_CHECK) return FLASHMHF_ERR_BAD_DTYPE;
     int rc = check_arch();
     if (rc) return rc;
     int n = 0;
-    rc = prologue_forward(*p, static_cast<cudaStream_t>(stream), &n);
+    rc = prologue_forward(*p, param_dtype == FLASHMHF_BF16, static_cast<cudaStream_t>(stream), &n);
     g_launches += (uint64_t)n;
     return rc;
+}
+int flashmhf_prologue_forward(const flashmhf_prologue_params *p, void *stream) {
+    return flashmhf_prologue_forward_dtype(p, FLASHMHF_F32_CHECK, stream);
 }
 
 size_t flashmhf_prologue_backward_workspace_bytes(const flashmhf_prologue_params *p) {
@@ -287,14 +291,18 @@ size_t flashmhf_prologue_backward_workspace_bytes(const flashmhf_prologue_params
     return prologue_backward_workspace_bytes(*p);
 }
 
-int flashmhf_prologue_backward(const flashmhf_prologue_bwd_params *p, void *stream) {
+int flashmhf_prologue_backward_dtype(const flashmhf_prologue_bwd_params *p, int32_t param_dtype, void *stream) {
     if (!p) return FLASHMHF_ERR_NULL;
+    if (param_dtype != FLASHMHF_BF16 && param_dtype != FLASHMHF_F32_CHECK) return FLASHMHF_ERR_BAD_DTYPE;
     int rc = check_arch();
     if (rc) return rc;
     int n = 0;
-    rc = prologue_backward(*p, static_cast<cudaStream_t>(stream), &n);
+    rc = prologue_backward(*p, param_dtype == FLASHMHF_BF16, static_cast<cudaStream_t>(stream), &n);
     g_launches += (uint64_t)n;
     return rc;
+}
+int flashmhf_prologue_backward(const flashmhf_prologue_bwd_params *p, void *stream) {
+    return flashmhf_prologue_backward_dtype(p, FLASHMHF_F32_CHECK, stream);
 }
 
 int flashmhf_lm_rope(const void *x, void *y, const float *cos_t, const float *sin_t, int64_t tokens, int32_t S,
@@ -309,27 +317,38 @@ int flashmhf_lm_rope(const void *x, void *y, const float *cos_t, const float *si
     return rc;
 }
 
-int flashmhf_lm_rmsnorm_forward(const void *x, const float *w, void *y, int64_t rows, int32_t n, float eps, void *stream) {
+int flashmhf_lm_rmsnorm_forward_dtype(const void *x, const void *w, int32_t w_dtype, void *y, int64_t rows, int32_t n, float eps,
+                                      void *stream) {
+    if (w_dtype != FLASHMHF_BF16 && w_dtype != FLASHMHF_F32_CHECK) return FLASHMHF_ERR_BAD_DTYPE;
     int rc = check_arch();
     if (rc) return rc;
     int nl = 0;
-    rc = lm_rmsnorm_forward(x, w, y, rows, n, eps, static_cast<cudaStream_t>(stream), &nl);
+    rc = lm_rmsnorm_forward(x, w, w_dtype == FLASHMHF_BF16, y, rows, n, eps, static_cast<cudaStream_t>(stream), &nl);
     g_launches += (uint64_t)nl;
     return rc;
+}
+int flashmhf_lm_rmsnorm_forward(const void *x, const float *w, void *y, int64_t rows, int32_t n, float eps, void *stream) {
+    return flashmhf_lm_rmsnorm_forward_dtype(x, w, FLASHMHF_F32_CHECK, y, rows, n, eps, stream);
 }
 
 size_t flashmhf_lm_rmsnorm_backward_workspace_bytes(int64_t rows, int32_t n) {
     return lm_rmsnorm_backward_workspace_bytes(rows, n);
 }
 
-int flashmhf_lm_rmsnorm_backward(const void *x, const float *w, const void *g, void *dx, float *dw, void *workspace,
-                                 size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream) {
+int flashmhf_lm_rmsnorm_backward_dtype(const void *x, const void *w, int32_t w_dtype, const void *g, void *dx, void *dw,
+                                       void *workspace, size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream) {
+    if (w_dtype != FLASHMHF_BF16 && w_dtype != FLASHMHF_F32_CHECK) return FLASHMHF_ERR_BAD_DTYPE;
     int rc = check_arch();
     if (rc) return rc;
     int nl = 0;
-    rc = lm_rmsnorm_backward(x, w, g, dx, dw, workspace, workspace_bytes, rows, n, eps, static_cast<cudaStream_t>(stream), &nl);
+    rc = lm_rmsnorm_backward(x, w, w_dtype == FLASHMHF_BF16, g, dx, dw, workspace, workspace_bytes, rows, n, eps,
+                             static_cast<cudaStream_t>(stream), &nl);
     g_launches += (uint64_t)nl;
     return rc;
+}
+int flashmhf_lm_rmsnorm_backward(const void *x, const float *w, const void *g, void *dx, float *dw, void *workspace,
+                                 size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream) {
+    return flashmhf_lm_rmsnorm_backward_dtype(x, w, FLASHMHF_F32_CHECK, g, dx, dw, workspace, workspace_bytes, rows, n, eps, stream);
 }
 
 int flashmhf_profile_begin(int max_marks) {

@@ -62,14 +62,14 @@ rope_kernel(const __nv_bfloat16 *X, __nv_bfloat16 *Y, const float *cosT, const f
 // ---- RMSNorm over rows of N = 256*CPL elements: one warp per row, lane l holds 16-byte chunks i*32 + l ----
 template <int CPL>
 __global__ void __launch_bounds__(kWarpsAux * 32)
-rmsnorm_fwd_kernel(const __nv_bfloat16 *X, const float *W, __nv_bfloat16 *Y, long long rows, float eps) {
+rmsnorm_fwd_kernel(const __nv_bfloat16 *X, const void *W, bool bf16_w, __nv_bfloat16 *Y, long long rows, float eps) {
     constexpr int N = CPL * 256;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float w[CPL][8];
 #pragma unroll
     for (int i = 0; i < CPL; ++i)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) w[i][k] = W[(i * 32 + lane) * 8 + k];
+        for (int k = 0; k < 8; ++k) w[i][k] = load_param(W, (i * 32 + lane) * 8 + k, bf16_w);
     for (long long r = (long long)blockIdx.x * kWarpsAux + warp; r < rows; r += (long long)gridDim.x * kWarpsAux) {
         const uint4 *xr = reinterpret_cast<const uint4 *>(X + r * N);
         float x[CPL][8], ss = 0.f;
@@ -94,7 +94,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16 *X, const float *W, __nv_bfloat16 *Y, lon
 // dx = rstd w g - rstd^3 x mean(w g x) ;  dw += g x rstd  (per-block partial sums, reduced in a second kernel)
 template <int CPL>
 __global__ void __launch_bounds__(kWarpsAux * 32)
-rmsnorm_bwd_kernel(const __nv_bfloat16 *X, const float *W, const __nv_bfloat16 *G, __nv_bfloat16 *dX, float *part_w,
+rmsnorm_bwd_kernel(const __nv_bfloat16 *X, const void *W, bool bf16_w, const __nv_bfloat16 *G, __nv_bfloat16 *dX, float *part_w,
                    long long rows, float eps) {
     constexpr int N = CPL * 256;
     extern __shared__ float sm_aux[];   // [kWarpsAux][N]
@@ -104,7 +104,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16 *X, const float *W, const __nv_bfloat16 *
     for (int i = 0; i < CPL; ++i)
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            w[i][k] = W[(i * 32 + lane) * 8 + k];
+            w[i][k] = load_param(W, (i * 32 + lane) * 8 + k, bf16_w);
             wacc[i][k] = 0.f;
         }
     for (long long r = (long long)blockIdx.x * kWarpsAux + warp; r < rows; r += (long long)gridDim.x * kWarpsAux) {
@@ -147,12 +147,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16 *X, const float *W, const __nv_bfloat16 *
     }
 }
 
-__global__ void __launch_bounds__(128) aux_reduce_kernel(const float *part, float *out, int n, int nblk) {
+__global__ void __launch_bounds__(128) aux_reduce_kernel(const float *part, void *out, bool bf16_w, int n, int nblk) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float v = 0.f;
     for (int b = 0; b < nblk; ++b) v += part[(long long)b * n + i];
-    out[i] = v;
+    store_param(out, i, v, bf16_w);
 }
 
 int norm_blocks(long long rows) {
@@ -183,16 +183,16 @@ int lm_rope(const void *x, void *y, const float *cos_t, const float *sin_t, long
     return FLASHMHF_OK;
 }
 
-int lm_rmsnorm_forward(const void *x, const float *w, void *y, long long rows, int n, float eps, cudaStream_t st, int *n_launch) {
+int lm_rmsnorm_forward(const void *x, const void *w, bool bf16_w, void *y, long long rows, int n, float eps, cudaStream_t st, int *n_launch) {
     if (!x || !w || !y) return FLASHMHF_ERR_NULL;
     if (!norm_ok(rows, n)) return FLASHMHF_ERR_BAD_SHAPE;
     if (!aligned16(x) || !aligned16(y)) return FLASHMHF_ERR_BAD_STRIDE;
     const int grid = norm_blocks(rows);
     const __nv_bfloat16 *X = static_cast<const __nv_bfloat16 *>(x);
     __nv_bfloat16 *Y = static_cast<__nv_bfloat16 *>(y);
-    if (n == 768) rmsnorm_fwd_kernel<3><<<grid, kWarpsAux * 32, 0, st>>>(X, w, Y, rows, eps);
-    else if (n == 1024) rmsnorm_fwd_kernel<4><<<grid, kWarpsAux * 32, 0, st>>>(X, w, Y, rows, eps);
-    else rmsnorm_fwd_kernel<8><<<grid, kWarpsAux * 32, 0, st>>>(X, w, Y, rows, eps);
+    if (n == 768) rmsnorm_fwd_kernel<3><<<grid, kWarpsAux * 32, 0, st>>>(X, w, bf16_w, Y, rows, eps);
+    else if (n == 1024) rmsnorm_fwd_kernel<4><<<grid, kWarpsAux * 32, 0, st>>>(X, w, bf16_w, Y, rows, eps);
+    else rmsnorm_fwd_kernel<8><<<grid, kWarpsAux * 32, 0, st>>>(X, w, bf16_w, Y, rows, eps);
     *n_launch += 1;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_cuda_error(e, "rmsnorm_fwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
@@ -203,7 +203,7 @@ size_t lm_rmsnorm_backward_workspace_bytes(long long rows, int n) {
     return norm_ok(rows, n) ? (size_t)norm_blocks(rows) * (size_t)n * sizeof(float) : 0;
 }
 
-int lm_rmsnorm_backward(const void *x, const float *w, const void *g, void *dx, float *dw, void *workspace,
+int lm_rmsnorm_backward(const void *x, const void *w, bool bf16_w, const void *g, void *dx, void *dw, void *workspace,
                         size_t workspace_bytes, long long rows, int n, float eps, cudaStream_t st, int *n_launch) {
     if (!x || !w || !g || !dx || !dw) return FLASHMHF_ERR_NULL;
     if (!norm_ok(rows, n)) return FLASHMHF_ERR_BAD_SHAPE;
@@ -217,17 +217,17 @@ int lm_rmsnorm_backward(const void *x, const float *w, const void *g, void *dx, 
     float *part = static_cast<float *>(workspace);
     cudaError_t e = cudaSuccess;
     if (n == 768) {
-        rmsnorm_bwd_kernel<3><<<grid, kWarpsAux * 32, smem, st>>>(X, w, G, dX, part, rows, eps);
+        rmsnorm_bwd_kernel<3><<<grid, kWarpsAux * 32, smem, st>>>(X, w, bf16_w, G, dX, part, rows, eps);
     } else if (n == 1024) {
-        rmsnorm_bwd_kernel<4><<<grid, kWarpsAux * 32, smem, st>>>(X, w, G, dX, part, rows, eps);
+        rmsnorm_bwd_kernel<4><<<grid, kWarpsAux * 32, smem, st>>>(X, w, bf16_w, G, dX, part, rows, eps);
     } else {
         e = cudaFuncSetAttribute(rmsnorm_bwd_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) rmsnorm_bwd_kernel<8><<<grid, kWarpsAux * 32, smem, st>>>(X, w, G, dX, part, rows, eps);
+        if (e == cudaSuccess) rmsnorm_bwd_kernel<8><<<grid, kWarpsAux * 32, smem, st>>>(X, w, bf16_w, G, dX, part, rows, eps);
     }
     *n_launch += 1;
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) { set_cuda_error(e, "rmsnorm_bwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
-    aux_reduce_kernel<<<(n + 127) / 128, 128, 0, st>>>(part, dw, n, grid);
+    aux_reduce_kernel<<<(n + 127) / 128, 128, 0, st>>>(part, dw, bf16_w, n, grid);
     *n_launch += 1;
     if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "aux_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
     return FLASHMHF_OK;

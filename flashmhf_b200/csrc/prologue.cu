@@ -41,8 +41,9 @@ __device__ __forceinline__ long long first_row(int q, int by, int gy, int warp) 
 struct ProArgs {
     const __nv_bfloat16 *X;   // [B,S,H,Dh]
     long long x_tok;          // element stride between tokens (= H*Dh when contiguous)
-    const float *W;           // [H,Dh] or nullptr (no RMSNorm)
-    const float *router;      // [H,Dh,E]
+    const void *W;            // [H,Dh] or nullptr (no RMSNorm)
+    const void *router;       // [H,Dh,E]
+    bool bf16_params;         // W and router are bf16, else fp32
     float eps;
     int T, H, E, S;           // T = B*S tokens
     unsigned s_mul, s_shift;  // t / S == (t * s_mul) >> s_shift for 0 <= t < 2^31
@@ -125,10 +126,10 @@ struct RouterSlice {
     const float *sm;
     int lane;
     // Stages router[h] (Dh*E floats) in shared memory with coalesced loads, then re-orders it.  `stage`: 2*Dh*E floats.
-    __device__ __forceinline__ void init(const float *router_h, float *stage, int E, int lane_) {
+    __device__ __forceinline__ void init(const ProArgs &a, int h, float *stage, int lane_) {
         lane = lane_;
-        const int n = EPL * 32 * E;
-        for (int k = threadIdx.x; k < n; k += blockDim.x) stage[k] = router_h[k];
+        const int E = a.E, n = EPL * 32 * E;
+        for (int k = threadIdx.x; k < n; k += blockDim.x) stage[k] = load_param(a.router, (long long)h * n + k, a.bf16_params);
         __syncthreads();
         float *dst = stage + n;
         for (int k = threadIdx.x; k < n; k += blockDim.x) {
@@ -186,10 +187,10 @@ prologue_fwd_kernel(const ProArgs a, __nv_bfloat16 *Q, float *R) {
     extern __shared__ float sm[];
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RouterSlice<EPL, EP> rt;
-    rt.init(a.router + (long long)h * DH * a.E, sm, a.E, lane);
+    rt.init(a, h, sm, lane);
     float w[EPL];
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) w[i] = NORM ? a.W[h * DH + lane * EPL + i] : 1.f;
+    for (int i = 0; i < EPL; ++i) w[i] = NORM ? load_param(a.W, h * DH + lane * EPL + i, a.bf16_params) : 1.f;
 
     const int by = blockIdx.y, gy = gridDim.y;
     float xn[kNR][EPL];
@@ -241,11 +242,11 @@ prologue_bwd_kernel(const ProArgs a, const ProBwdArgs g) {
     float *acc_r = sm + 2 * DE, *acc_w = acc_r + kWarps * DE;
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RouterSlice<EPL, EP> rt;
-    rt.init(a.router + (long long)h * DE, router_s, E, lane);
+    rt.init(a, h, router_s, lane);
     float w[EPL], wacc[EPL], racc[EPL][EP];
 #pragma unroll
     for (int i = 0; i < EPL; ++i) {
-        w[i] = NORM ? a.W[h * DH + lane * EPL + i] : 1.f;
+        w[i] = NORM ? load_param(a.W, h * DH + lane * EPL + i, a.bf16_params) : 1.f;
         wacc[i] = 0.f;
 #pragma unroll
         for (int e = 0; e < EP; ++e) racc[i][e] = 0.f;
@@ -344,21 +345,30 @@ prologue_bwd_kernel(const ProArgs a, const ProBwdArgs g) {
 
 #include "prologue_mma.cuh"
 
-// out[i] = sum over blocks (in index order) of part[blk][i]
-__global__ void __launch_bounds__(128) prologue_reduce_kernel(const float *part, float *out, long long n, int nblk) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// d router, then d norm weight: out[i] = sum over blocks (in index order) of part[blk][i].  One launch for both.
+struct ProReduceArgs {
+    const float *part_r, *part_w;
+    void *d_router, *d_w;
+    int nr, nw, nblk;   // nw = 0 without RMSNorm
+    bool bf16_params;
+};
+__global__ void __launch_bounds__(128) prologue_reduce_kernel(const ProReduceArgs a) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= a.nr + a.nw) return;
+    const bool is_w = j >= a.nr;
+    const int i = is_w ? j - a.nr : j, n = is_w ? a.nw : a.nr;
+    const float *part = is_w ? a.part_w : a.part_r;
     float v = 0.f;
     int b = 0;
-    for (; b + 8 <= nblk; b += 8) {
+    for (; b + 8 <= a.nblk; b += 8) {
         float u[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) u[k] = part[(long long)(b + k) * n + i];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v += u[k];
     }
-    for (; b < nblk; ++b) v += part[(long long)b * n + i];
-    out[i] = v;
+    for (; b < a.nblk; ++b) v += part[(long long)b * n + i];
+    store_param(is_w ? a.d_w : a.d_router, i, v, a.bf16_params);
 }
 
 int check_pro(const flashmhf_prologue_params &p, bool forward) {
@@ -372,12 +382,12 @@ int check_pro(const flashmhf_prologue_params &p, bool forward) {
         return FLASHMHF_ERR_BAD_STRIDE;
     return FLASHMHF_OK;
 }
-ProArgs pro_args(const flashmhf_prologue_params &p) {
+ProArgs pro_args(const flashmhf_prologue_params &p, bool bf16_params) {
     // l = ceil(log2 S); m = floor(2^(31+l) / S) + 1 < 2^32 gives exact quotients for dividends below 2^31
     unsigned l = 0;
     while ((1ull << l) < (unsigned long long)p.S) ++l;
     const unsigned mul = (unsigned)(((1ull << (31 + l)) / (unsigned long long)p.S) + 1ull);
-    return ProArgs{static_cast<const __nv_bfloat16 *>(p.X), p.x_token_stride, p.norm_weight, p.router, p.eps,
+    return ProArgs{static_cast<const __nv_bfloat16 *>(p.X), p.x_token_stride, p.norm_weight, p.router, bf16_params, p.eps,
                    p.B * p.S, p.H, p.E, p.S, mul, 31 + l};
 }
 // E <= 24 runs the MMA kernels (16-token tiles per warp; the backward's d-router accumulator takes 32 registers per
@@ -440,10 +450,10 @@ cudaError_t launch_bwd(const ProArgs &a, dim3 grid, const ProBwdArgs &g, cudaStr
 
 }  // namespace
 
-int prologue_forward(const flashmhf_prologue_params &p, cudaStream_t st, int *n_launch) {
+int prologue_forward(const flashmhf_prologue_params &p, bool bf16_params, cudaStream_t st, int *n_launch) {
     int rc = check_pro(p, true);
     if (rc) return rc;
-    const ProArgs a = pro_args(p);
+    const ProArgs a = pro_args(p, bf16_params);
     const dim3 grid(p.H, blocks_per_head(p, kFwdBlocksPerSM));
     __nv_bfloat16 *Q = static_cast<__nv_bfloat16 *>(p.Q);
     cudaError_t e = cudaSuccess;
@@ -464,7 +474,7 @@ size_t prologue_backward_workspace_bytes(const flashmhf_prologue_params &p) {
     return (size_t)blocks_per_head(p, 1) * p.H * ((size_t)p.Dh * p.E + p.Dh) * sizeof(float);
 }
 
-int prologue_backward(const flashmhf_prologue_bwd_params &q, cudaStream_t st, int *n_launch) {
+int prologue_backward(const flashmhf_prologue_bwd_params &q, bool bf16_params, cudaStream_t st, int *n_launch) {
     const flashmhf_prologue_params &p = q.fwd;
     int rc = check_pro(p, false);
     if (rc) return rc;
@@ -475,7 +485,7 @@ int prologue_backward(const flashmhf_prologue_bwd_params &q, cudaStream_t st, in
     const size_t need = prologue_backward_workspace_bytes(p);
     if (!q.workspace || q.workspace_bytes < need || (reinterpret_cast<uintptr_t>(q.workspace) & 255u))
         return FLASHMHF_ERR_WORKSPACE;
-    const ProArgs a = pro_args(p);
+    const ProArgs a = pro_args(p, bf16_params);
     const int ny = blocks_per_head(p, 1), DE = p.Dh * p.E;
     float *part_r = static_cast<float *>(q.workspace);
     float *part_w = part_r + (size_t)ny * p.H * DE;
@@ -493,13 +503,9 @@ int prologue_backward(const flashmhf_prologue_bwd_params &q, cudaStream_t st, in
     prof_mark(st, kMarkPrologueBwd);
     *n_launch += 1;
     if (e != cudaSuccess) { set_cuda_error(e, "prologue_bwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
-    const long long nr = (long long)p.H * DE, nw = (long long)p.H * p.Dh;
-    prologue_reduce_kernel<<<(int)((nr + 127) / 128), 128, 0, st>>>(part_r, q.d_router, nr, ny);
+    const ProReduceArgs ra{part_r, part_w, q.d_router, q.d_norm_weight, p.H * DE, p.norm_weight ? p.H * p.Dh : 0, ny, bf16_params};
+    prologue_reduce_kernel<<<(ra.nr + ra.nw + 127) / 128, 128, 0, st>>>(ra);
     *n_launch += 1;
-    if (p.norm_weight) {
-        prologue_reduce_kernel<<<(int)((nw + 127) / 128), 128, 0, st>>>(part_w, q.d_norm_weight, nw, ny);
-        *n_launch += 1;
-    }
     prof_mark(st, kMarkPrologueReduce);
     if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "prologue_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
     return FLASHMHF_OK;

@@ -92,8 +92,10 @@ struct MmaLayout {
 
 // Router fragments of head h.  Bf feeds logits = y . router (k = d), B2f feeds dy += dlogits . router^T (k = e).
 template <int DH, int NT, bool BWD>
-__device__ __forceinline__ void build_router_fragments(const float *router_h, int E, uint8_t *smem) {
+__device__ __forceinline__ void build_router_fragments(const ProArgs &a, int h, uint8_t *smem) {
     using L = MmaLayout<DH, NT>;
+    const int E = a.E;
+    const long long r0 = (long long)h * DH * E;
     uint2 *bf = reinterpret_cast<uint2 *>(smem + L::kOffBf);
     for (int idx = threadIdx.x; idx < L::NKS * NT * 32; idx += blockDim.x) {
         const int ln = idx & 31, nt = (idx >> 5) % NT, ks = (idx >> 5) / NT;
@@ -102,7 +104,7 @@ __device__ __forceinline__ void build_router_fragments(const float *router_h, in
 #pragma unroll
         for (int j = 0; j < 4; ++j) {   // (u0,b0) (u0,b1) (u1,b0) (u1,b1)
             const int d = mma_col(q, 2 * ks + (j >> 1)) + (j & 1);
-            v[j] = e < E ? router_h[d * E + e] : 0.f;
+            v[j] = e < E ? load_param(a.router, r0 + d * E + e, a.bf16_params) : 0.f;
             split3(v[j], s[0][j], s[1][j], s[2][j]);
         }
 #pragma unroll
@@ -119,7 +121,7 @@ __device__ __forceinline__ void build_router_fragments(const float *router_h, in
 #pragma unroll
             for (int j = 0; j < 4; ++j) {   // experts kk*16 + 2q + {0,1}, then + 8
                 const int e = kk * 16 + (j >> 1) * 8 + 2 * q + (j & 1);
-                const float v = e < E ? router_h[d * E + e] : 0.f;
+                const float v = e < E ? load_param(a.router, r0 + d * E + e, a.bf16_params) : 0.f;
                 split3(v, hi[j], mid[j], lo);
             }
             b2[((0 * L::NKK + kk) * L::NU + u) * 32 + ln] = make_uint2(pack_bf16(hi[0], hi[1]), pack_bf16(hi[2], hi[3]));
@@ -237,9 +239,9 @@ prologue_fwd_mma_kernel(const ProArgs a, __nv_bfloat16 *Q, float *R) {
     using L = MmaLayout<DH, NT>;
     extern __shared__ __align__(16) uint8_t smem_mma[];
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    build_router_fragments<DH, NT, false>(a.router + (long long)h * DH * a.E, a.E, smem_mma);
+    build_router_fragments<DH, NT, false>(a, h, smem_mma);
     float *wsm = reinterpret_cast<float *>(smem_mma + L::kOffW);
-    for (int i = threadIdx.x; i < DH; i += blockDim.x) wsm[i] = NORM ? a.W[h * DH + i] : 1.f;
+    for (int i = threadIdx.x; i < DH; i += blockDim.x) wsm[i] = NORM ? load_param(a.W, h * DH + i, a.bf16_params) : 1.f;
     __syncthreads();
     for (int it = 0;; ++it) {
         const long long t0 = mma_tile_row(it, blockIdx.y, gridDim.y, warp);
@@ -275,9 +277,9 @@ prologue_bwd_mma_kernel(const ProArgs a, const ProBwdArgs gp) {
     extern __shared__ __align__(16) uint8_t smem_mma[];
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int E = a.E, DE = DH * E;
-    build_router_fragments<DH, NT, true>(a.router + (long long)h * DE, E, smem_mma);
+    build_router_fragments<DH, NT, true>(a, h, smem_mma);
     float *wsm = reinterpret_cast<float *>(smem_mma + L::kOffW);
-    for (int i = threadIdx.x; i < DH; i += blockDim.x) wsm[i] = NORM ? a.W[h * DH + i] : 1.f;
+    for (int i = threadIdx.x; i < DH; i += blockDim.x) wsm[i] = NORM ? load_param(a.W, h * DH + i, a.bf16_params) : 1.f;
     __syncthreads();
     const uint2 *b2 = reinterpret_cast<const uint2 *>(smem_mma + L::kOffB2f);
 

@@ -346,6 +346,14 @@ __device__ __forceinline__ float fast_tanh(float x) {
 }
 __device__ __forceinline__ float fast_sigmoid(float x) { return fmaf(0.5f, fast_tanh(0.5f * x), 0.5f); }
 
+// Element i of a parameter kept as bf16 or fp32 (read once per block, so the choice is a run-time flag).
+__device__ __forceinline__ float load_param(const void *p, long long i, bool bf16) {
+    return bf16 ? __bfloat162float(static_cast<const __nv_bfloat16 *>(p)[i]) : static_cast<const float *>(p)[i];
+}
+__device__ __forceinline__ void store_param(void *p, long long i, float v, bool bf16) {
+    if (bf16) static_cast<__nv_bfloat16 *>(p)[i] = __float2bfloat16(v);
+    else static_cast<float *>(p)[i] = v;
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));

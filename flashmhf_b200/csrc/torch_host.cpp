@@ -10,6 +10,7 @@
 // The C-ABI library itself stays free of torch types: its entry points are taken from the handle that
 // flashmhf_b200/_lib.py has loaded (bind()), so one copy of the library serves ctypes callers and this module.
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <dlfcn.h>
@@ -33,13 +34,13 @@ struct Api {
     decltype(&flashmhf_backward) backward = nullptr;
     decltype(&flashmhf_forward_workspace_bytes) forward_ws = nullptr;
     decltype(&flashmhf_backward_workspace_bytes) backward_ws = nullptr;
-    decltype(&flashmhf_prologue_forward) prologue_forward = nullptr;
+    decltype(&flashmhf_prologue_forward_dtype) prologue_forward = nullptr;
     decltype(&flashmhf_prologue_backward_workspace_bytes) prologue_backward_ws = nullptr;
-    decltype(&flashmhf_prologue_backward) prologue_backward = nullptr;
+    decltype(&flashmhf_prologue_backward_dtype) prologue_backward = nullptr;
     decltype(&flashmhf_lm_rope) lm_rope = nullptr;
-    decltype(&flashmhf_lm_rmsnorm_forward) rmsnorm_forward = nullptr;
+    decltype(&flashmhf_lm_rmsnorm_forward_dtype) rmsnorm_forward = nullptr;
     decltype(&flashmhf_lm_rmsnorm_backward_workspace_bytes) rmsnorm_backward_ws = nullptr;
-    decltype(&flashmhf_lm_rmsnorm_backward) rmsnorm_backward = nullptr;
+    decltype(&flashmhf_lm_rmsnorm_backward_dtype) rmsnorm_backward = nullptr;
     PyObject *error_type = nullptr;  // flashmhf_b200._lib.FlashMHFError(status, message)
 };
 Api api;
@@ -58,13 +59,13 @@ void bind(uintptr_t handle, py::object error_type) {
     get(api.backward, "flashmhf_backward");
     get(api.forward_ws, "flashmhf_forward_workspace_bytes");
     get(api.backward_ws, "flashmhf_backward_workspace_bytes");
-    get(api.prologue_forward, "flashmhf_prologue_forward");
+    get(api.prologue_forward, "flashmhf_prologue_forward_dtype");
     get(api.prologue_backward_ws, "flashmhf_prologue_backward_workspace_bytes");
-    get(api.prologue_backward, "flashmhf_prologue_backward");
+    get(api.prologue_backward, "flashmhf_prologue_backward_dtype");
     get(api.lm_rope, "flashmhf_lm_rope");
-    get(api.rmsnorm_forward, "flashmhf_lm_rmsnorm_forward");
+    get(api.rmsnorm_forward, "flashmhf_lm_rmsnorm_forward_dtype");
     get(api.rmsnorm_backward_ws, "flashmhf_lm_rmsnorm_backward_workspace_bytes");
-    get(api.rmsnorm_backward, "flashmhf_lm_rmsnorm_backward");
+    get(api.rmsnorm_backward, "flashmhf_lm_rmsnorm_backward_dtype");
     Py_XDECREF(api.error_type);
     api.error_type = error_type.release().ptr();
 }
@@ -173,6 +174,22 @@ Tensor scratch(const std::optional<Tensor> &given, size_t nbytes, const Tensor &
 }
 
 // ------------------------------------------------------------------------------------------------ operator
+// The call itself, from addresses and strides.
+void launch_forward(flashmhf_fwd_params &p, const Tensor &like, bool chained, const std::optional<Tensor> &workspace) {
+    if (p.d.S == 1 && p.d.B > 1) {
+        p.Q = tokens_as_sequence(p.Q); p.R = tokens_as_sequence(p.R); p.O = tokens_as_sequence(p.O);
+        p.d.S = p.d.B;
+        p.d.B = 1;
+    }
+    Tensor ws;
+    p.workspace_bytes = api.forward_ws(&p.d);
+    if (p.workspace_bytes) {
+        ws = scratch(workspace, p.workspace_bytes, like);
+        p.workspace = ws.data_ptr();
+    }
+    check((chained ? api.forward_chained : api.forward)(&p, current_stream(like)));
+}
+
 Tensor forward_checked(const Shape &s, const Tensor &Q0, const Tensor &K0, const Tensor &U0, const Tensor &V0, const Tensor &R0,
                        const std::optional<Tensor> &out, const flashmhf_scaling &sc, bool chained,
                        const std::optional<Tensor> &workspace) {
@@ -183,18 +200,7 @@ Tensor forward_checked(const Shape &s, const Tensor &Q0, const Tensor &K0, const
     p.d = dims_of(s, Q.scalar_type());
     p.Q = view4(Q); p.K = view4(K); p.U = view4(U); p.V = view4(V); p.R = view4(R); p.O = view4(O);
     p.scale = sc;
-    if (s.S == 1 && s.B > 1) {
-        p.Q = tokens_as_sequence(p.Q); p.R = tokens_as_sequence(p.R); p.O = tokens_as_sequence(p.O);
-        p.d.B = 1;
-        p.d.S = (int32_t)s.B;
-    }
-    Tensor ws;
-    p.workspace_bytes = api.forward_ws(&p.d);
-    if (p.workspace_bytes) {
-        ws = scratch(workspace, p.workspace_bytes, Q);
-        p.workspace = ws.data_ptr();
-    }
-    check((chained ? api.forward_chained : api.forward)(&p, current_stream(Q)));
+    launch_forward(p, Q, chained, workspace);
     return O;
 }
 
@@ -298,7 +304,7 @@ Tensor flash_mhf(const Tensor &Q, const Tensor &K, const Tensor &U, const Tensor
 
 // ------------------------------------------------------------------------------------------------ prologue
 struct Prologue {
-    Tensor x, w, r;   // projected activations [B,S,H*d_h]; norm weight and router as contiguous fp32 (w undefined: no RMSNorm)
+    Tensor x, w, r;   // projected activations [B,S,H*d_h]; norm weight (undefined: no RMSNorm) and router, both bf16 or both fp32
     int64_t B, S, H, Dh, E;
     double eps;
 };
@@ -315,8 +321,11 @@ Prologue prologue_args(const Tensor &x_proj, const std::optional<Tensor> &q_norm
         throw py::value_error("fused_prologue supports d_h in {64, 96, 128} and at most 32 sub-networks");
     a.eps = eps;
     a.x = x_proj.contiguous();
-    if (q_norm) a.w = q_norm->detach().to(at::kFloat).contiguous();
-    a.r = router.detach().to(at::kFloat).contiguous();
+    // bf16 parameters are read as they are; any other mix goes in as fp32
+    const bool bf16 = router.scalar_type() == at::kBFloat16 && (!q_norm || q_norm->scalar_type() == at::kBFloat16);
+    const auto dt = bf16 ? at::kBFloat16 : at::kFloat;
+    if (q_norm) a.w = q_norm->detach().to(dt).contiguous();
+    a.r = router.detach().to(dt).contiguous();
     return a;
 }
 flashmhf_prologue_params prologue_params(const Prologue &a) {
@@ -325,10 +334,11 @@ flashmhf_prologue_params prologue_params(const Prologue &a) {
     p.eps = (float)a.eps;
     p.X = a.x.data_ptr();
     p.x_token_stride = a.H * a.Dh;
-    p.norm_weight = a.w.defined() ? a.w.data_ptr<float>() : nullptr;
-    p.router = a.r.data_ptr<float>();
+    p.norm_weight = a.w.defined() ? static_cast<const float *>(a.w.data_ptr()) : nullptr;   // in the type dtype_code(a.r) names
+    p.router = static_cast<const float *>(a.r.data_ptr());
     return p;
 }
+int32_t dtype_code(const Tensor &param) { return param.scalar_type() == at::kBFloat16 ? FLASHMHF_BF16 : FLASHMHF_F32_CHECK; }
 // Q [B,S,H*d_h] in the activations' own layout (the activations themselves without RMSNorm) and R [B,H,S,E]
 std::pair<Tensor, Tensor> run_prologue(const Prologue &a) {
     c10::cuda::CUDAGuard guard(a.x.device());
@@ -337,28 +347,28 @@ std::pair<Tensor, Tensor> run_prologue(const Prologue &a) {
     flashmhf_prologue_params p = prologue_params(a);
     p.Q = q.data_ptr();
     p.R = R.data_ptr<float>();
-    check(api.prologue_forward(&p, current_stream(a.x)));
+    check(api.prologue_forward(&p, dtype_code(a.r), current_stream(a.x)));
     return {q, R};
 }
 struct PrologueGrads {
     Tensor dX, d_router, d_norm;
 };
-// dQ [B,H,S,d_h] with a unit inner stride, dR [B,H,S,E] contiguous fp32
-PrologueGrads run_prologue_backward(const Prologue &a, const Tensor &dQ, const Tensor &dR) {
+// dQ [B,H,S,d_h] bf16 with a unit inner stride, dR [B,H,S,E] contiguous fp32
+PrologueGrads run_prologue_backward(const Prologue &a, const void *dQ, const int64_t *dq_stride, const float *dR) {
     c10::cuda::CUDAGuard guard(a.x.device());
     PrologueGrads g{at::empty_like(a.x), at::empty_like(a.r), a.w.defined() ? at::empty_like(a.w) : Tensor()};
     flashmhf_prologue_bwd_params p{};
     p.fwd = prologue_params(a);
-    p.dQ = dQ.data_ptr();
-    for (int i = 0; i < 3; ++i) p.dq_stride[i] = dQ.stride(i);
-    p.dR = dR.data_ptr<float>();
+    p.dQ = dQ;
+    for (int i = 0; i < 3; ++i) p.dq_stride[i] = dq_stride[i];
+    p.dR = dR;
     p.dX = g.dX.data_ptr();
-    p.d_router = g.d_router.data_ptr<float>();
-    p.d_norm_weight = g.d_norm.defined() ? g.d_norm.data_ptr<float>() : nullptr;
+    p.d_router = static_cast<float *>(g.d_router.data_ptr());
+    p.d_norm_weight = g.d_norm.defined() ? static_cast<float *>(g.d_norm.data_ptr()) : nullptr;
     p.workspace_bytes = api.prologue_backward_ws(&p.fwd);
     Tensor ws = at::empty({(int64_t)p.workspace_bytes}, a.x.options().dtype(at::kByte));
     p.workspace = ws.data_ptr();
-    check(api.prologue_backward(&p, current_stream(a.x)));
+    check(api.prologue_backward(&p, dtype_code(a.r), current_stream(a.x)));
     return g;
 }
 Tensor heads_view(const Tensor &t, int64_t H, int64_t Dh) {   // [B,S,H*d_h] memory as a [B,H,S,d_h] view
@@ -385,7 +395,8 @@ struct PrologueFunction : public torch::autograd::Function<PrologueFunction> {
         if (!dR.defined()) dR = at::zeros({a.B, a.H, a.S, a.E}, a.x.options().dtype(at::kFloat));
         dQ = dQ.to(at::kBFloat16);
         if (dQ.stride(3) != 1) dQ = dQ.contiguous();
-        PrologueGrads g = run_prologue_backward(a, dQ, dR.to(at::kFloat).contiguous());
+        dR = dR.to(at::kFloat).contiguous();
+        PrologueGrads g = run_prologue_backward(a, dQ.data_ptr(), dQ.strides().data(), dR.data_ptr<float>());
         const int64_t nd = ctx->saved_data["norm_dtype"].toInt();
         if (nd >= 0) g.d_norm = g.d_norm.to((at::ScalarType)nd);
         return {g.dX, g.d_norm, g.d_router.to((at::ScalarType)ctx->saved_data["router_dtype"].toInt()), Tensor()};
@@ -402,50 +413,118 @@ Tensor expert_view(const Tensor &w, int64_t Hkuv, int64_t E) {
     const int64_t I = w.size(0), dh = w.size(1) / Hkuv;
     return w.view({E, I / E, Hkuv, dh}).permute({2, 0, 1, 3});
 }
+// The same view, and the [B,H,S,*] views of activations and routing weights, as addresses and strides only: a torch view
+// costs the host about as much as an allocation, and a layer call needs a dozen of them each way.
+flashmhf_tensor expert_address(const Tensor &w, int64_t Dh, int64_t De) {
+    const int64_t ld = w.stride(0);
+    return flashmhf_tensor{w.data_ptr(), {Dh, De * ld, ld}};
+}
+flashmhf_tensor heads_address(void *p, const Prologue &a) { return flashmhf_tensor{p, {a.S * a.H * a.Dh, a.Dh, a.H * a.Dh}}; }
+flashmhf_tensor routing_address(void *p, const Prologue &a) { return flashmhf_tensor{p, {a.H * a.S * a.E, a.S * a.E, a.E}}; }
+// Can the operator read this parameter as it lies? (the rule of in_place_ok for the view above)
+bool expert_ok(const Tensor &w) {
+    return w.dim() == 2 && w.scalar_type() == at::kBFloat16 && w.stride(1) == 1 && w.stride(0) % 8 == 0 && w.stride(0) >= w.size(1) &&
+           !(reinterpret_cast<uintptr_t>(w.data_ptr()) & 15u);
+}
+size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// Prologue and operator as one autograd node: projected activations [B,S,H*d_h] -> O [B,S,H*d_h].
-struct LayerCoreFunction : public torch::autograd::Function<LayerCoreFunction> {
-    static Tensor forward(AutogradContext *ctx, const Tensor &x_proj, const std::optional<Tensor> &q_norm, const Tensor &router,
-                          const Tensor &gate, const Tensor &up, const Tensor &down, int64_t Hkuv, double eps, double hs, double us, double fs) {
-        const Prologue a = prologue_args(x_proj, q_norm, router, eps);
+// The whole layer as one autograd node: projection, prologue, operator, projection.  As separate nodes its backward is a
+// dozen small steps of the autograd engine (views, transposes and products of the two linear maps, the prologue, the
+// operator), which on short inputs take the host longer than their kernels take the GPU.
+Shape layer_shape(const Prologue &a, const Tensor &gate, const Tensor &up, const Tensor &down, int64_t Hkuv) {
+    const int64_t I = gate.size(0);
+    if (Hkuv < 1 || a.H % Hkuv != 0)
+        throw py::value_error("num_heads " + std::to_string(a.H) + " must be a multiple of num_kuv_heads " + std::to_string(Hkuv));
+    if (gate.size(1) != Hkuv * a.Dh || up.sizes() != gate.sizes() || down.sizes() != gate.sizes() || I % a.E != 0)
+        throw py::value_error("gate, up and down weights must be [E*d_e, H_kuv*d_h], got " + dims_text(gate) + ", " + dims_text(up) + ", " +
+                              dims_text(down));
+    if ((I / a.E) % 64 != 0) throw py::value_error("Expert dimension " + std::to_string(I / a.E) + " must be divisible by 64");
+    if (gate.device() != a.x.device() || up.device() != a.x.device() || down.device() != a.x.device())
+        throw py::value_error("flash_mhf runs on CUDA tensors of one device; there is no CPU path");
+    return Shape{a.B, a.H, a.S, a.Dh, Hkuv, a.E, I / a.E};
+}
+struct LayerFunction : public torch::autograd::Function<LayerFunction> {
+    static Tensor forward(AutogradContext *ctx, const Tensor &x, const std::optional<Tensor> &w1, const std::optional<Tensor> &b1,
+                          const std::optional<Tensor> &q_norm, const Tensor &router, const Tensor &gate, const Tensor &up,
+                          const Tensor &down, const std::optional<Tensor> &w2, const std::optional<Tensor> &b2, int64_t Hkuv, double eps,
+                          double hs, double us, double fs) {
+        const Prologue a = prologue_args(w1 ? at::linear(x, *w1, b1) : x, q_norm, router, eps);
+        const Shape s = layer_shape(a, gate, up, down, Hkuv);
+        const flashmhf_scaling sc = scaling_of(hs, us, fs);
         auto [q, R] = run_prologue(a);
-        const Tensor Q = heads_view(q, a.H, a.Dh);
-        const Tensor K = expert_view(gate, Hkuv, a.E), U = expert_view(up, Hkuv, a.E), V = expert_view(down, Hkuv, a.E);
-        const Shape s = validate(Q, K, U, V, R);
-        const Tensor O = forward_checked(s, Q, K, U, V, R, std::nullopt, scaling_of(hs, us, fs), false, std::nullopt);
-        ctx->save_for_backward({a.x, a.w, a.r, q, R, gate, up, down});
+        const Tensor O = at::empty_like(a.x);
+        {
+            c10::cuda::CUDAGuard guard(x.device());
+            flashmhf_fwd_params p{};
+            p.d = dims_of(s, at::kBFloat16);
+            p.Q = heads_address(q.data_ptr(), a); p.O = heads_address(O.data_ptr(), a); p.R = routing_address(R.data_ptr(), a);
+            p.K = expert_address(gate, s.Dh, s.De); p.U = expert_address(up, s.Dh, s.De); p.V = expert_address(down, s.Dh, s.De);
+            p.scale = sc;
+            launch_forward(p, a.x, false, std::nullopt);
+        }
+        ctx->save_for_backward({w1 ? x : Tensor(), w1 ? *w1 : Tensor(), a.x, a.w, a.r, q, R, gate, up, down, w2 ? O : Tensor(),
+                                w2 ? *w2 : Tensor()});
         ctx->saved_data["k"] = std::vector<double>{eps, hs, us, fs};
-        ctx->saved_data["i"] = std::vector<int64_t>{Hkuv, (int64_t)router.scalar_type(), q_norm ? (int64_t)q_norm->scalar_type() : (int64_t)-1};
-        return O.transpose(1, 2).reshape({a.B, a.S, a.H * a.Dh});   // no copy: O has Q's layout
+        ctx->saved_data["i"] = std::vector<int64_t>{Hkuv, (int64_t)router.scalar_type(), q_norm ? (int64_t)q_norm->scalar_type() : (int64_t)-1,
+                                                    (int64_t)b1.has_value(), (int64_t)b2.has_value()};
+        return w2 ? at::linear(O, *w2, b2) : O;
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
-        variable_list out(11);
+        variable_list out(15);
         if (!grads[0].defined()) return out;
         const variable_list sv = ctx->get_saved_variables();
         const std::vector<double> k = ctx->saved_data["k"].toDoubleVector();
         const std::vector<int64_t> n = ctx->saved_data["i"].toIntVector();
-        const Prologue a{sv[0], sv[1], sv[2], sv[0].size(0), sv[0].size(1), sv[2].size(0), sv[2].size(1), sv[2].size(2), k[0]};
-        const Tensor Q = heads_view(sv[3], a.H, a.Dh), &R = sv[4];
-        const Tensor K = expert_view(sv[5], n[0], a.E), U = expert_view(sv[6], n[0], a.E), V = expert_view(sv[7], n[0], a.E);
+        const Tensor &x = sv[0], &w1 = sv[1], &O = sv[10], &w2 = sv[11], &R = sv[6];
+        const Prologue a{sv[2], sv[3], sv[4], sv[2].size(0), sv[2].size(1), sv[4].size(0), sv[4].size(1), sv[4].size(2), k[0]};
+        // which arguments want a gradient (autograd numbers the tensors that were passed)
+        const bool given[10] = {true, w1.defined(), n[3] != 0, a.w.defined(), true, true, true, true, w2.defined(), n[4] != 0};
+        bool need[10];
+        for (int i = 0, edge = 0; i < 10; ++i) need[i] = given[i] && ctx->needs_input_grad(edge++);
+        const int64_t T = a.B * a.S, hid = a.H * a.Dh;
         uint32_t parts = 0;
-        const int nt = a.w.defined() ? 6 : 5;   // tensor arguments present: x, (norm weight), router, then the three weights
-        for (int i = 0; i < nt; ++i)
-            if (ctx->needs_input_grad(i)) parts |= i < nt - 3 ? FLASHMHF_BWD_INPUTS : FLASHMHF_BWD_WEIGHTS;
+        if (need[0] || need[1] || need[2] || need[3] || need[4]) parts |= FLASHMHF_BWD_INPUTS;
+        if (need[5] || need[6] || need[7]) parts |= FLASHMHF_BWD_WEIGHTS;
+
+        Tensor d = grads[0].reshape({T, grads[0].size(2)});
+        if (need[8]) out[8] = d.t().mm(O.view({T, hid}));
+        if (need[9]) out[9] = d.sum(0);
         if (!parts) return out;
-        const Shape s{a.B, a.H, a.S, a.Dh, n[0], a.E, K.size(2)};
-        const Tensor dO = grads[0].reshape({a.B, a.S, a.H, a.Dh}).transpose(1, 2);
-        const Grads g = backward_checked(s, Q, K, U, V, R, dO, flashmhf_scaling{(float)k[1], (float)k[2], (float)k[3]}, parts, nullptr);
-        if (parts & FLASHMHF_BWD_INPUTS) {
-            PrologueGrads pg = run_prologue_backward(a, g.dQ, g.dR);
-            out[0] = pg.dX;
-            if (pg.d_norm.defined()) out[1] = pg.d_norm.to((at::ScalarType)n[2]);
-            out[2] = pg.d_router.to((at::ScalarType)n[1]);
+        if (w2.defined()) d = d.mm(w2);
+        d = d.contiguous();
+        const bool inputs = parts & FLASHMHF_BWD_INPUTS, weights = parts & FLASHMHF_BWD_WEIGHTS;
+        const Tensor &gate = sv[7], &up = sv[8], &down = sv[9];
+        c10::cuda::CUDAGuard guard(d.device());
+        flashmhf_bwd_params p{};
+        p.d = dims_of(Shape{a.B, a.H, a.S, a.Dh, n[0], a.E, gate.size(0) / a.E}, at::kBFloat16);
+        // dQ, dR and the scratch of the operator live until the prologue's backward has run: one allocation for all three
+        const size_t dq_bytes = align256((size_t)T * hid * 2), dr_bytes = align256((size_t)T * a.H * a.E * 4);
+        p.workspace_bytes = api.backward_ws(&p.d);
+        const Tensor tmp = at::empty({(int64_t)(dq_bytes + dr_bytes + p.workspace_bytes + 1)}, d.options().dtype(at::kByte));
+        char *base = static_cast<char *>(tmp.data_ptr());
+        p.Q = heads_address(sv[5].data_ptr(), a); p.dO = heads_address(d.data_ptr(), a); p.R = routing_address(R.data_ptr(), a);
+        p.K = expert_address(gate, a.Dh, p.d.De); p.U = expert_address(up, a.Dh, p.d.De); p.V = expert_address(down, a.Dh, p.d.De);
+        p.dQ = heads_address(base, a); p.dR = routing_address(base + dq_bytes, a);
+        p.workspace = base + dq_bytes + dr_bytes;
+        p.scale = flashmhf_scaling{(float)k[1], (float)k[2], (float)k[3]};
+        p.parts = parts;
+        if (weights) {
+            out[5] = at::empty_like(gate); out[6] = at::empty_like(up); out[7] = at::empty_like(down);
+            p.dK = expert_address(out[5], a.Dh, p.d.De); p.dU = expert_address(out[6], a.Dh, p.d.De); p.dV = expert_address(out[7], a.Dh, p.d.De);
         }
-        if (parts & FLASHMHF_BWD_WEIGHTS) {
-            auto param = [&](const Tensor &d, const Tensor &w) { return d.permute({1, 2, 0, 3}).reshape(w.sizes()); };
-            out[3] = param(g.dK, sv[5]);
-            out[4] = param(g.dU, sv[6]);
-            out[5] = param(g.dV, sv[7]);
+        check(api.backward(&p, current_stream(d)));
+        if (inputs) {
+            const PrologueGrads pg = run_prologue_backward(a, static_cast<char *>(p.dQ.ptr), p.dQ.stride, static_cast<float *>(p.dR.ptr));
+            if (pg.d_norm.defined()) out[3] = pg.d_norm.to((at::ScalarType)n[2]);
+            out[4] = pg.d_router.to((at::ScalarType)n[1]);
+            if (w1.defined()) {
+                const Tensor dp = pg.dX.view({T, hid});
+                if (need[1]) out[1] = dp.t().mm(x.reshape({T, x.size(2)}));
+                if (need[2]) out[2] = dp.sum(0);
+                if (need[0]) out[0] = dp.mm(w1).view(x.sizes());
+            } else {
+                out[0] = pg.dX;
+            }
         }
         return out;
     }
@@ -454,8 +533,14 @@ struct LayerCoreFunction : public torch::autograd::Function<LayerCoreFunction> {
 Tensor mhffn_layer(const Tensor &x, const std::optional<Tensor> &w1, const std::optional<Tensor> &b1, const std::optional<Tensor> &q_norm,
                    const Tensor &router, const Tensor &gate, const Tensor &up, const Tensor &down, const std::optional<Tensor> &w2,
                    const std::optional<Tensor> &b2, int64_t Hkuv, double eps, double hs, double us, double fs) {
-    const Tensor q_lin = w1 ? at::linear(x, *w1, b1) : x;
-    const Tensor O = LayerCoreFunction::apply(q_lin, q_norm, router, gate, up, down, Hkuv, eps, hs, us, fs);
+    auto plain = [](const std::optional<Tensor> &t) { return !t || t->scalar_type() == at::kBFloat16; };
+    if (x.dim() == 3 && expert_ok(gate) && expert_ok(up) && expert_ok(down) && plain(x) && plain(w1) && plain(b1) && plain(w2) && plain(b2) && !at::autocast::is_autocast_enabled(at::kCUDA))
+        return LayerFunction::apply(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs);
+    // other dtypes, autocast, or weights that have to be copied first: torch's own rules for each step
+    auto [Q, R] = fused_prologue(w1 ? at::linear(x, *w1, b1) : x, q_norm, router, eps);
+    const int64_t E = router.size(2);
+    const Tensor O = flash_mhf(Q, expert_view(gate, Hkuv, E), expert_view(up, Hkuv, E), expert_view(down, Hkuv, E), R, hs, us, fs)
+                         .transpose(1, 2).reshape({x.size(0), x.size(1), router.size(0) * router.size(1)});
     return w2 ? at::linear(O, *w2, b2) : O;
 }
 
@@ -482,11 +567,12 @@ Tensor rotary(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t) { retur
 
 struct RMSNormFunction : public torch::autograd::Function<RMSNormFunction> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x0, const Tensor &weight, double eps) {
-        const Tensor x = x0.contiguous(), w = weight.detach().to(at::kFloat).contiguous();
+        const Tensor x = x0.contiguous();
+        const Tensor w = (weight.scalar_type() == at::kBFloat16 ? weight.detach() : weight.detach().to(at::kFloat)).contiguous();
         c10::cuda::CUDAGuard guard(x.device());
         Tensor y = at::empty_like(x);
         const int64_t n = x.size(-1);
-        check(api.rmsnorm_forward(x.data_ptr(), w.data_ptr<float>(), y.data_ptr(), x.numel() / n, (int32_t)n, (float)eps, current_stream(x)));
+        check(api.rmsnorm_forward(x.data_ptr(), w.data_ptr(), dtype_code(w), y.data_ptr(), x.numel() / n, (int32_t)n, (float)eps, current_stream(x)));
         ctx->save_for_backward({x, w});
         ctx->saved_data["eps"] = eps;
         ctx->saved_data["dtype"] = (int64_t)weight.scalar_type();
@@ -501,8 +587,8 @@ struct RMSNormFunction : public torch::autograd::Function<RMSNormFunction> {
         const int64_t n = x.size(-1), rows = x.numel() / n;
         const size_t nbytes = api.rmsnorm_backward_ws(rows, (int32_t)n);
         Tensor ws = at::empty({(int64_t)nbytes}, x.options().dtype(at::kByte));
-        check(api.rmsnorm_backward(x.data_ptr(), w.data_ptr<float>(), g.data_ptr(), dx.data_ptr(), dw.data_ptr<float>(), ws.data_ptr(),
-                                   nbytes, rows, (int32_t)n, (float)ctx->saved_data["eps"].toDouble(), current_stream(x)));
+        check(api.rmsnorm_backward(x.data_ptr(), w.data_ptr(), dtype_code(w), g.data_ptr(), dx.data_ptr(), dw.data_ptr(),
+                                   ws.data_ptr(), nbytes, rows, (int32_t)n, (float)ctx->saved_data["eps"].toDouble(), current_stream(x)));
         return {dx, dw.to((at::ScalarType)ctx->saved_data["dtype"].toInt()), Tensor()};
     }
 };

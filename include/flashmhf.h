@@ -201,6 +201,13 @@ int flashmhf_prologue_forward(const flashmhf_prologue_params *p, void *stream);
 size_t flashmhf_prologue_backward_workspace_bytes(const flashmhf_prologue_params *p);
 int flashmhf_prologue_backward(const flashmhf_prologue_bwd_params *p, void *stream);
 
+/* The same calls for parameters kept in `param_dtype` (a flashmhf_dtype: FLASHMHF_BF16, or FLASHMHF_F32_CHECK for
+ * float32): norm_weight and router are then read, and d_norm_weight and d_router written, in that type, which saves a
+ * bf16 model two conversion kernels each way.  bf16 values are widened exactly, gradients rounded once from their fp32
+ * sums: the same numbers the conversions would give. */
+int flashmhf_prologue_forward_dtype(const flashmhf_prologue_params *p, int32_t param_dtype, void *stream);
+int flashmhf_prologue_backward_dtype(const flashmhf_prologue_bwd_params *p, int32_t param_dtype, void *stream);
+
 /* ---- Helpers for the measurement LM (flashmhf_b200/lm.py), outside the operator -------------------
  * Rotary position embedding on [tokens, heads, head_dim] bf16 (token strides in elements, multiples of 8):
  *   y[..., :h] = x[..., :h] cos - x[..., h:] sin ;  y[..., h:] = x[..., h:] cos + x[..., :h] sin,  h = head_dim/2,
@@ -218,6 +225,11 @@ int flashmhf_lm_rmsnorm_forward(const void *x, const float *w, void *y, int64_t 
 size_t flashmhf_lm_rmsnorm_backward_workspace_bytes(int64_t rows, int32_t n);
 int flashmhf_lm_rmsnorm_backward(const void *x, const float *w, const void *g, void *dx, float *dw, void *workspace,
                                  size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream);
+/* The same with the weight (and dw) in `w_dtype`, FLASHMHF_BF16 or FLASHMHF_F32_CHECK (float32). */
+int flashmhf_lm_rmsnorm_forward_dtype(const void *x, const void *w, int32_t w_dtype, void *y, int64_t rows, int32_t n, float eps,
+                                      void *stream);
+int flashmhf_lm_rmsnorm_backward_dtype(const void *x, const void *w, int32_t w_dtype, const void *g, void *dx, void *dw,
+                                       void *workspace, size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream);
 
 /* SYNCHRONOUS.  Waits for the current device, then reads and clears the status word the kernels
  * write when a bounded wait runs out.  *code = 0 if none did; otherwise a kernel/role identifier
