@@ -88,13 +88,14 @@ struct DqSmem {
     static constexpr uint32_t kQBytes = kChunks * kTile;
     static constexpr uint32_t kKUStage = kChunks * 2 * kWChunk;  // per chunk: [K;U] = 128 rows
     static constexpr uint32_t kVStage = kChunks * kWChunk;
-    static constexpr int kKUStages = 3, kVStages = 2;
+    // d_h = 64: shared memory is plentiful and a block is short, so the way of a stage from L2 takes more stages to hide
+    static constexpr int kKUStages = DH == 64 ? 6 : 3, kVStages = DH == 64 ? 6 : 2;
     static constexpr uint32_t kOffQ = 0;
     static constexpr uint32_t kOffdO = kOffQ + kQBytes;
     static constexpr uint32_t kOffKU = kOffdO + kQBytes;
     static constexpr uint32_t kOffV = kOffKU + kKUStages * kKUStage;
     static constexpr uint32_t kOffCtl = kOffV + kVStages * kVStage;
-    static constexpr uint32_t kCtlBytes = 256 + 2 * (kParts - 1) * 128 * 4;  // barriers + two sets of dR exchange rows
+    static constexpr uint32_t kCtlBytes = 320 + 2 * (kParts - 1) * 128 * 4;  // barriers + two sets of dR exchange rows
     static constexpr uint32_t kTotal = kOffCtl + kCtlBytes + 1024;
 };
 
@@ -103,8 +104,11 @@ struct DqSmem {
 //   SFULL (S and dA of the block computed: one commit from each of their issuers), SEMPTY (both are in the
 //   element-wise warps' registers), PFULL ([dM|dN] written), PEMPTY (the dQ update that read it is done).
 // All of them complete once per block and every waiter waits on every phase, so a one-bit parity is enough.
-enum { DQ_QFULL = 0, DQ_KUFULL = 1, DQ_KUEMPTY = 4, DQ_VFULL = 7, DQ_VEMPTY = 9, DQ_SFULL = 11, DQ_SEMPTY = 12,
-       DQ_PFULL = 13, DQ_PEMPTY = 14, DQ_ACCFULL = 15, DQ_QT = 16, DQ_DRFULL = 18, DQ_DRFREE = 20, DQ_BARS = 22 };
+constexpr int kMaxRing = 6;
+enum { DQ_QFULL = 0, DQ_SFULL = 1, DQ_SEMPTY = 2, DQ_PFULL = 3, DQ_PEMPTY = 4, DQ_ACCFULL = 5, DQ_QT = 6, DQ_DRFULL = 7, DQ_DRFREE = 9,
+       DQ_KUFULL = 11, DQ_KUEMPTY = DQ_KUFULL + kMaxRing, DQ_VFULL = DQ_KUEMPTY + kMaxRing, DQ_VEMPTY = DQ_VFULL + kMaxRing,
+       DQ_BARS = DQ_VEMPTY + kMaxRing };
+static_assert(DQ_BARS * 8 + 8 <= 320, "control area");
 
 struct DqArgs {
     const float *R;
@@ -130,7 +134,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                    sBar = base + L::kOffCtl;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(gbase + L::kOffCtl + DQ_BARS * 8);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(gbase + L::kOffCtl + DQ_BARS * 8 + 4);
-    volatile float *drx = reinterpret_cast<volatile float *>(gbase + L::kOffCtl + 256);  // [2][kParts - 1][128]
+    volatile float *drx = reinterpret_cast<volatile float *>(gbase + L::kOffCtl + 320);  // [2][kParts - 1][128]
     auto bar = [&](int i) { return sBar + 8u * i; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -438,7 +442,8 @@ struct DwSmem {
     static constexpr uint32_t kWBytes = 3 * kChunks * kWChunk;  // [K;U] chunks then V chunks
     static constexpr uint32_t kOffWV = 2 * kChunks * kWChunk;
     static constexpr uint32_t kTokStage = 2 * kChunks * kTile;  // Q chunks then dO chunks
-    static constexpr int kTokStages = 2;
+    // token stages: what is left beside the resident weights and the staged operands (two at 96 and 128 columns)
+    static constexpr int kTokStages = DH == 64 ? 4 : 2;
     static constexpr uint32_t kOffW = 0;
     static constexpr uint32_t kOffTok = kOffW + kWBytes;
     static constexpr uint32_t kOffP = kOffTok + kTokStages * kTokStage;  // [dM | dN] : 2 x 16 KB
@@ -452,8 +457,11 @@ struct DwSmem {
 // load or the next MMA can start earlier shortens the loop load -> recompute -> element-wise -> accumulate.
 // S has two buffers in tensor memory, each with its own full/empty pair, so that every waiter sees every
 // phase of the barrier it waits on (a one-bit parity cannot tell phase k from phase k+2).
-enum { DW_WFULL = 0, DW_QFULL = 1, DW_GFULL = 3, DW_QEMPTY = 5, DW_GEMPTY = 7, DW_SFULL = 9, DW_SEMPTY = 11,
-       DW_PFULL = 13, DW_AFULL = 14, DW_PEMPTY = 15, DW_AEMPTY = 16, DW_ACCFULL = 17, DW_DAEMPTY = 18, DW_BARS = 19 };
+constexpr int kMaxTok = 4;
+enum { DW_WFULL = 0, DW_SFULL = 1, DW_SEMPTY = 3, DW_PFULL = 5, DW_AFULL = 6, DW_PEMPTY = 7, DW_AEMPTY = 8, DW_ACCFULL = 9, DW_DAEMPTY = 10,
+       DW_QFULL = 11, DW_GFULL = DW_QFULL + kMaxTok, DW_QEMPTY = DW_GFULL + kMaxTok, DW_GEMPTY = DW_QEMPTY + kMaxTok,
+       DW_BARS = DW_GEMPTY + kMaxTok };
+static_assert(DW_BARS * 8 + 8 <= 256, "control area");
 
 struct DwArgs {
     const float *R;

@@ -40,12 +40,19 @@ namespace {
 
 constexpr int kBT = 128;  // token rows per tile
 constexpr int kBI = 64;   // intermediate rows per block
-// Shared-memory stages of the [K;U] ring and of the V ring (two Q tiles take the rest).  The [K;U] ring must have an
+// Shared-memory stages of the [K;U] ring and of the V ring.  The [K;U] ring must have an
 // EVEN number of stages: its "full" barriers are waited on by the two S issuers, which own alternate blocks, and a
 // barrier's phase is tracked with one parity bit, so each stage must always be waited on by the same issuer (with an
 // odd ring an issuer would meet a stage only every other time it fills and could take an old phase for the new one).
-constexpr int kKURing = 4, kVRing = 2;
-static_assert(kKURing % 2 == 0, "each [K;U] stage must belong to one S issuer");
+// The depth is what hides a stage's way from L2 (about 1000 clk under load, 32 KB per 64-wide chunk row pair): a stage of
+// the V ring is asked for again only when the O update that read it is done, so two stages cap the loop at two blocks per
+// (load + update + hand-offs).  At d_h = 64 a block is short and shared memory is plentiful; at 96 and 128 the rings
+// take what two Q tiles leave.
+template <int DH>
+struct FwdRings {
+    static constexpr int kKU = DH == 64 ? 6 : 4, kV = DH == 64 ? 6 : 2;
+    static_assert(kKU % 2 == 0, "each [K;U] stage must belong to one S issuer");
+};
 // Activation teams of eight warps (warp % 4 = lane quarter, next bit = which 32 of a block's 64 columns).  With two
 // teams, team t owns the blocks j = t (mod 2) and with them S buffer t and A slot t; the two teams are then in
 // different phases of their loop (wait, load, arithmetic, store), which keeps the arithmetic pipes busy.
@@ -67,8 +74,8 @@ struct FwdSmem {
     // offsets from the 1024-aligned base
     static constexpr uint32_t kOffQ = 0;                        // two Q tiles: work items alternate between them
     static constexpr uint32_t kOffKU = kOffQ + 2 * kQBytes;
-    static constexpr uint32_t kOffV = kOffKU + kKURing * kKUStage;
-    static constexpr uint32_t kOffBar = kOffV + kVRing * kVStage;
+    static constexpr uint32_t kOffV = kOffKU + FwdRings<DH>::kKU * kKUStage;
+    static constexpr uint32_t kOffBar = kOffV + FwdRings<DH>::kV * kVStage;
     static constexpr uint32_t kTotal = kOffBar + 320 + 1024;  // + barriers/control + alignment slack
 };
 
@@ -80,8 +87,11 @@ struct FwdSmem {
 // A CTA walks several work items (token tiles); blocks are counted through all of them (g), buffer and slot of a block
 // are g % 2, Q tile and per-item barriers alternate with the item count, so every barrier has one fixed set of
 // waiters that observes each of its phases and a one-bit phase parity is enough.
-enum { BAR_QFULL = 0, BAR_QFREE = 2, BAR_KUFULL = 4, BAR_KUEMPTY = 8, BAR_VFULL = 12, BAR_VEMPTY = 16, BAR_SFULL = 20,  // rings: up to 4 stages
-       BAR_SEMPTY = 22, BAR_AFULL = 24, BAR_AFREE = 26, BAR_OFULL = 28, BAR_OFREE = 29, BAR_QT = 30, BAR_COUNT = 31 };
+constexpr int kMaxRing = 6;
+enum { BAR_QFULL = 0, BAR_QFREE = 2, BAR_SFULL = 4, BAR_SEMPTY = 6, BAR_AFULL = 8, BAR_AFREE = 10, BAR_OFULL = 12, BAR_OFREE = 13,
+       BAR_QT = 14, BAR_KUFULL = 15, BAR_KUEMPTY = BAR_KUFULL + kMaxRing, BAR_VFULL = BAR_KUEMPTY + kMaxRing,
+       BAR_VEMPTY = BAR_VFULL + kMaxRing, BAR_COUNT = BAR_VEMPTY + kMaxRing };
+static_assert(BAR_COUNT * 8 + 8 <= 320, "control area");
 
 struct FwdArgs {
     const float *R;
@@ -136,7 +146,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
            const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV,
            const __grid_constant__ CUtensorMap tmO, const FwdArgs args) {
     using L = FwdSmem<DH>;
-    constexpr int kTeams = teams_for(DH);
+    constexpr int kTeams = teams_for(DH), kKURing = FwdRings<DH>::kKU, kVRing = FwdRings<DH>::kV;
+    static_assert(kKURing <= kMaxRing && kVRing <= kMaxRing, "barrier slots");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
