@@ -196,6 +196,12 @@ size_t flashmhf_backward_workspace_bytes(const flashmhf_dims *d) {
     return tc_backward_workspace_bytes(*d);
 }
 
+size_t flashmhf_backward_inputs_workspace_bytes(const flashmhf_dims *d) {
+    if (!d || check_dims(*d) != 0) return 0;
+    if (d->dtype == FLASHMHF_F32_CHECK) return 0;
+    return tc_backward_inputs_workspace_bytes(*d);
+}
+
 // Shared argument checks of the two backward entry points.  Tensors of a part that is not asked for are not looked at.
 static int check_bwd(const flashmhf_bwd_params *p, unsigned *parts_out) {
     if (!p) return FLASHMHF_ERR_NULL;
@@ -223,7 +229,7 @@ int flashmhf_backward(const flashmhf_bwd_params *p, void *stream) {
     int rc = check_bwd(p, &parts);
     if (rc) return rc;
     if (parts & FLASHMHF_BWD_WEIGHTS) {
-        const size_t need = flashmhf_backward_workspace_bytes(&p->d);
+        const size_t need = p->d.dtype == FLASHMHF_BF16 ? tc_backward_weights_workspace_bytes(p->d) : 0;
         if (need > 0 && (!p->workspace || p->workspace_bytes < need || (reinterpret_cast<uintptr_t>(p->workspace) & 255u)))
             return FLASHMHF_ERR_WORKSPACE;
     }

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../include/flashmhf.h"
 
 namespace fmhf {
@@ -47,7 +49,14 @@ cudaError_t simt_backward(const flashmhf_bwd_params &p, cudaStream_t st, int *n_
 int tc_forward(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, bool chained);
 size_t tc_forward_workspace_bytes(const flashmhf_dims &d);
 int tc_backward(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch);
-size_t tc_backward_workspace_bytes(const flashmhf_dims &d);
+size_t tc_backward_workspace_bytes(const flashmhf_dims &d);          // all of it
+size_t tc_backward_weights_workspace_bytes(const flashmhf_dims &d);  // what the dK/dU/dV part cannot do without
+size_t tc_backward_inputs_workspace_bytes(const flashmhf_dims &d);   // what a call for dQ and dR alone can use (0: nothing)
+// Sum of `nsplit` fp32 partial planes [B,H,S,Dh], in index order, as bf16 to `out` (strides multiples of 4 elements).
+// kReduceAfterKernel: launched early, runs when the kernel before it is done; kReduceChained: between two chained forward kernels.
+enum ReduceMode { kReduceAfterKernel, kReduceChained };
+cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, ReduceMode mode, int num_sms,
+                            cudaStream_t st);
 int tc_backward_static_scratch(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch);
 
 // ---- fused layer prologue (per-head RMSNorm + router weights), HBM-bound CUDA-core kernels --
@@ -63,6 +72,23 @@ int lm_rmsnorm_forward(const void *x, const void *w, bool bf16_w, void *y, long 
 size_t lm_rmsnorm_backward_workspace_bytes(long long rows, int n);
 int lm_rmsnorm_backward(const void *x, const void *w, bool bf16_w, const void *g, void *dx, void *dw, void *workspace,
                         size_t workspace_bytes, long long rows, int n, float eps, cudaStream_t st, int *n_launch);
+
+// Launch.  `early`: with programmatic stream serialization, so that the kernel may start before the one ahead of it on the
+// stream has ended (as soon as that one's CTAs have all asked for it, or exited).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_kernel(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 void set_cuda_error(cudaError_t e, const char *where);
 int selftest_bounded_wait(long long limit_cycles, cudaStream_t st, int *n_launch);

@@ -116,6 +116,10 @@ struct DqArgs {
     float *dR;
     long long dr_sb, dr_sh, dr_ss;
     int S, E, De, G;
+    // Few token tiles: the sub-networks are split over CTAs, e_per_split each (blockIdx.x = tile * nsplit + split).  A CTA then
+    // writes an fp32 partial dQ to `part` ([nsplit][B][H][S][DH], added by the split reduction) and dR of its own sub-networks.
+    int nsplit, e_per_split, H, B;
+    float *part;
     float s0, c;  // head_scaling; head_scaling * up_scaling * final_scaling
     WaitArgs wait;
 };
@@ -138,8 +142,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     auto bar = [&](int i) { return sBar + 8u * i; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t0 = blockIdx.x * kBT, h = blockIdx.y, b = blockIdx.z, hk = h / args.G;
-    const int bpe = args.De / kBI, nblk = args.E * bpe;
+    const int isplit = blockIdx.x % args.nsplit, e0 = isplit * args.e_per_split, ne = min(args.E - e0, args.e_per_split);
+    const int t0 = (int)(blockIdx.x / args.nsplit) * kBT, h = blockIdx.y, b = blockIdx.z, hk = h / args.G;
+    const int bpe = args.De / kBI, nblk = ne * bpe;
     const WaitCtl ctl{abort_flag, args.wait};
     constexpr int W = kKernelBwdDq * 100;
     // Tensor memory: dQ accumulator, Q and dO as bf16 A operands (64 columns each), S = [M | N], dA, [dM | dN] (bf16).
@@ -183,7 +188,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             int sk = 0, sv = 0;
             uint32_t phk = 1, phv = 1;
             for (int j = 0; j < nblk; ++j) {
-                const int row = j * kBI;
+                const int row = e0 * args.De + j * kBI;
                 if (!mbar_wait(bar(DQ_KUEMPTY + sk), phk, ctl, W + 1)) break;
                 const uint32_t fk = bar(DQ_KUFULL + sk);
                 mbar_arrive_expect_tx(fk, L::kKUStage);
@@ -286,8 +291,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         const int quarter = warp & 3, part = (warp - 4) >> 2, half = part;  // part: which kCols of the block's 64 columns
         const int row = quarter * 32 + lane, t = t0 + row;
         const bool in_range = t < args.S;
-        const float *rrow = args.R + (long long)b * args.r_sb + (long long)h * args.r_sh + (long long)t * args.r_ss;
-        float *drrow = args.dR + (long long)b * args.dr_sb + (long long)h * args.dr_sh + (long long)t * args.dr_ss;
+        const float *rrow = args.R + (long long)b * args.r_sb + (long long)h * args.r_sh + (long long)t * args.r_ss + e0;
+        float *drrow = args.dR + (long long)b * args.dr_sb + (long long)h * args.dr_sh + (long long)t * args.dr_ss + e0;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
         bool ok = true;
         // Q and dO: shared -> tensor memory, once (thread = token row; column part p < 2 copies columns [64p, 64p + 64)
@@ -316,7 +321,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         for (int j = 0; ok && j < nblk; ++j) {
             if (in_e == 0) {
                 r_cur = r_next;
-                r_next = (in_range && e + 1 < args.E) ? __ldg(rrow + e + 1) : 0.f;
+                r_next = (in_range && e + 1 < ne) ? __ldg(rrow + e + 1) : 0.f;
                 dr2 = f2_pack(0.f, 0.f);
             }
             if (!mbar_wait(bar(DQ_SFULL), j & 1, ctl, W + 7)) { ok = false; break; }
@@ -395,10 +400,21 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             tc_fence_after();
             constexpr int kColsPerHalf = DH / 2;
             const int c0 = half * kColsPerHalf;
+            float *pdst = args.part + ((((long long)isplit * args.B + b) * args.H + h) * args.S + t) * DH + c0;
 #pragma unroll
             for (int g = 0; g < kColsPerHalf / 16; ++g) {
                 uint32_t o[16];
                 tmem_ld16_sync(lane_base + kColAcc + c0 + g * 16, o);
+                if (args.nsplit > 1) {
+                    if (in_range) {
+#pragma unroll
+                        for (int v = 0; v < 4; ++v)
+                            *reinterpret_cast<float4 *>(pdst + g * 16 + v * 4) =
+                                make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]),
+                                            __uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3]));
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int v = 0; v < 2; ++v) {
                     const int col = c0 + g * 16 + v * 8;
@@ -413,7 +429,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             fence_async_smem();
         }
         if (part < 2) named_bar_sync(1, kEpiThreads);
-        if (ok && warp == 4 && lane == 0 && !*abort_flag) {
+        if (ok && warp == 4 && lane == 0 && !*abort_flag && args.nsplit == 1) {
             for (int c = 0; c < L::kChunks; ++c) tma_store_4d(&tmdQ, sQ + c * kTile, c * 64, t0, h, b);
             tma_store_commit();
             tma_store_wait_all();
@@ -421,6 +437,9 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     }
 
     __syncwarp();
+    // Launched so that it may start under the tail of the dK/dU/dV kernel, whose results it does not read.  Its own end must
+    // still come after that kernel's, for whatever follows on the stream: one CTA waits.
+    if (blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1) griddep_wait();
     if (*abort_flag) {
         const long long t_end = clock64() + (1LL << 19);
         while (clock64() < t_end) __nanosleep(256);
@@ -466,7 +485,10 @@ static_assert(DW_BARS * 8 + 8 <= 256, "control area");
 struct DwArgs {
     const float *R;
     long long r_sb, r_sh, r_ss;
-    float *ws;  // [nsplit][3][Hkuv][I][DH] fp32 partial sums
+    float *ws;  // [nsplit][3][Hkuv][I][DH] fp32 partial sums (nsplit > 1)
+    // One part per block: its sums are the results and are written as bf16 at once (dK, dU, dV: head and row strides)
+    __nv_bfloat16 *out[3];
+    long long o_head[3], o_row[3];
     int S, E, De, G, B, Hkuv;
     int tiles_per_seq, tiles_total, tiles_per_split;
     // CTA -> (weight block, token-tile range).  Blocks [0, n_mixed) are split unevenly into a long part (launched first)
@@ -557,6 +579,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const bool dead = *abort_flag != 0;
+    griddep_launch_dependents();   // the dQ/dR kernel may take over SMs that this kernel's last CTAs leave idle
 
     if (dead) {
         // nothing: fall through to the teardown
@@ -738,47 +761,65 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (ok) ok = mbar_wait(bar(DW_ACCFULL), 0, ctl, W + 9);
         if (ok) {
             tc_fence_after();
-            // fp32 partial sums -> workspace[split][which][hk][row][DH]
+            // fp32 partial sums -> workspace[split][which][hk][row][DH], or bf16 results
+            const bool direct = args.nsplit == 1;
             const long long I = (long long)args.E * args.De;
             const long long plane = (long long)args.Hkuv * I * DH;
             float *wsb = args.ws + (long long)split * 3 * plane + ((long long)hk * I + (long long)jblk * kBI) * DH;
+            auto out_row = [&](int which, int r) {
+                return args.out[which] + hk * args.o_head[which] + ((long long)jblk * kBI + r) * args.o_row[which];
+            };
             constexpr int kColsPerHalf = DH / 2;
             const int c0 = half * kColsPerHalf;
+            auto store16 = [&](float *dst, __nv_bfloat16 *o16, const uint32_t (&o)[16]) {   // 16 columns of one row
+                if (direct) {
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        *reinterpret_cast<uint2 *>(o16 + v * 4) =
+                            make_uint2(pack_bf16(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1])),
+                                       pack_bf16(__uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3])));
+                } else {
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        *reinterpret_cast<float4 *>(dst + v * 4) =
+                            make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]), __uint_as_float(o[4 * v + 2]),
+                                        __uint_as_float(o[4 * v + 3]));
+                }
+            };
             {   // [dK;dU]: lane = row of the stacked block (0-63 dK, 64-127 dU)
                 float *dst = wsb + (row < kBI ? 0 : plane) + (long long)(row & (kBI - 1)) * DH + c0;
+                __nv_bfloat16 *o16 = out_row(row < kBI ? 0 : 1, row & (kBI - 1)) + c0;
 #pragma unroll
                 for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
                     tmem_ld16_sync(lane_base + kColKU + c0 + g * 16, o);
-#pragma unroll
-                    for (int v = 0; v < 4; ++v)
-                        *reinterpret_cast<float4 *>(dst + g * 16 + v * 4) =
-                            make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]),
-                                        __uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3]));
+                    store16(dst + g * 16, o16 + g * 16, o);
                 }
             }
-            if (kVt) {  // dV^T: lane = column d of dV, tensor-memory column = row of the block; a warp stores 32 consecutive floats per row
+            if (kVt) {  // dV^T: lane = column d of dV, tensor-memory column = row of the block; a warp stores 32 consecutive elements per row
                 float *dst = wsb + 2 * plane + row;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     uint32_t o[16];
                     tmem_ld16_sync(lane_base + kColV + half * 32 + g * 16, o);
+                    const int r0 = half * 32 + g * 16;
+                    if (direct) {
 #pragma unroll
-                    for (int v = 0; v < 16; ++v) dst[(long long)(half * 32 + g * 16 + v) * DH] = __uint_as_float(o[v]);
+                        for (int v = 0; v < 16; ++v) out_row(2, r0 + v)[row] = __float2bfloat16(__uint_as_float(o[v]));
+                    } else {
+#pragma unroll
+                        for (int v = 0; v < 16; ++v) dst[(long long)(r0 + v) * DH] = __uint_as_float(o[v]);
+                    }
                 }
             } else {    // dV (M = 64 accumulator): row r lives in TMEM lane 32*(r/16) + r%16
-                float *dst = wsb + 2 * plane + (long long)(quarter * 16 + (lane & 15)) * DH + c0;
+                const int r = quarter * 16 + (lane & 15);
+                float *dst = wsb + 2 * plane + (long long)r * DH + c0;
+                __nv_bfloat16 *o16 = out_row(2, r) + c0;
 #pragma unroll
                 for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
                     tmem_ld16_sync(lane_base + kColV + c0 + g * 16, o);
-                    if (lane < 16) {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v)
-                            *reinterpret_cast<float4 *>(dst + g * 16 + v * 4) =
-                                make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]),
-                                            __uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3]));
-                    }
+                    if (lane < 16) store16(dst + g * 16, o16 + g * 16, o);
                 }
             }
             tc_fence_before();
@@ -798,7 +839,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     }
 }
 
-// Sum the token-axis splits in index order and write bf16 gradients (4 elements per thread).
+// Sum the token-axis splits in index order and write bf16 gradients (4 elements per thread, blockIdx.y = dK, dU or dV).
 struct ReduceArgs {
     const float *ws;
     __nv_bfloat16 *out[3];
@@ -807,37 +848,27 @@ struct ReduceArgs {
     int nsplit, I, DH;
 };
 __global__ void __launch_bounds__(256) dw_reduce_kernel(const ReduceArgs a) {
-    const long long n4 = 3 * a.plane / 4;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n4;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const long long el = idx * 4;
-        float4 acc = *reinterpret_cast<const float4 *>(a.ws + el);
+    griddep_wait();   // launched early, behind the kernel whose partial sums it adds
+    const int which = blockIdx.y;
+    const unsigned per_row = (unsigned)a.DH / 4;
+    const long long n4 = a.plane / 4;
+    const float4 *src = reinterpret_cast<const float4 *>(a.ws + which * a.plane);
+    const long long split4 = 3 * n4;
+    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n4; idx += (long long)gridDim.x * blockDim.x) {
+        float4 acc = src[idx];
+#pragma unroll 4
         for (int s = 1; s < a.nsplit; ++s) {
-            const float4 v = *reinterpret_cast<const float4 *>(a.ws + (long long)s * 3 * a.plane + el);
+            const float4 v = src[s * split4 + idx];
             acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
-        const int which = (int)(el / a.plane);
-        const long long rem = el - (long long)which * a.plane;
-        const int c = (int)(rem % a.DH);
-        const long long rowi = rem / a.DH;
-        const int r = (int)(rowi % a.I), hk = (int)(rowi / a.I);
-        __nv_bfloat16 *o = a.out[which] + hk * a.s_head[which] + r * a.s_row[which] + c;
-        uint2 packed = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
-        *reinterpret_cast<uint2 *>(o) = packed;
+        long long rowi;
+        unsigned c;
+        if (n4 <= 0x7fffffffLL) { rowi = (unsigned)idx / per_row; c = (unsigned)idx - (unsigned)rowi * per_row; }
+        else { rowi = idx / per_row; c = (unsigned)(idx - rowi * per_row); }
+        const int hk = (int)(rowi / a.I), r = (int)(rowi - (long long)hk * a.I);
+        __nv_bfloat16 *o = a.out[which] + hk * a.s_head[which] + r * a.s_row[which] + c * 4;
+        *reinterpret_cast<uint2 *>(o) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
     }
-}
-
-int choose_nsplit(long long items, int tiles_total, int num_sms) {
-    int best = 1;
-    double best_eff = 0.0;
-    for (int ns = 1; ns <= 16 && ns <= tiles_total; ++ns) {
-        const long long ctas = items * ns;
-        const long long waves = (ctas + num_sms - 1) / num_sms;
-        const double eff = (double)ctas / (double)(waves * num_sms);
-        if (eff > best_eff + 1e-9) { best_eff = eff; best = ns; }
-        if (eff >= 0.9) return ns;
-    }
-    return best;
 }
 
 struct DwPlan {
@@ -859,27 +890,31 @@ double list_schedule(const std::vector<double> &jobs, int num_sms) {
     return end;
 }
 
+// What a CTA costs besides its token tiles (weights in, first tile through the pipeline, accumulators out), in token tiles
+// (about 1.9 us each): the intercept of kernel time over tiles per CTA, 7 us.
+constexpr double kDwFixed = 4.0;
+
 // With a two-way split the CTAs are equal and their last wave is partly empty (704 CTAs on 148 SMs: the fifth wave is
 // 76 % full, 5 % of the kernel).  Splitting some blocks unevenly -- long parts launched first, short parts last, the
 // equal halves of the other blocks in between -- lets the short parts fill the SMs the last wave would leave idle.
-// The split point and the number of such blocks are found by simulating the launch order for a few candidates; a CTA's
-// fixed cost (weights in, accumulators out) is taken as two token tiles.  The partial sums still number two per
-// block, so the reduction and the workspace do not change.
-void plan_uneven(DwPlan &p, long long items, int num_sms) {
+// The split point and the number of such blocks are found by simulating the launch order for a few candidates.
+// The partial sums still number two per block, so the reduction and the workspace do not change.
+// Returns the simulated duration (token tiles).
+double plan_uneven(DwPlan &p, long long items, int num_sms) {
     p.n_mixed = p.small_tiles = 0;
-    if (p.nsplit != 2 || items > 2048 || p.tiles_total < 32) return;
-    const double ovh = 2.0;
     const int T = p.tiles_total, half = p.tiles_per_split;
     auto makespan = [&](int nmix, int small) {
         std::vector<double> jobs;
         jobs.reserve((size_t)(2 * items));
-        for (int i = 0; i < nmix; ++i) jobs.push_back(T - small + ovh);
-        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(half + ovh);
-        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(T - half + ovh);
-        for (int i = 0; i < nmix; ++i) jobs.push_back(small + ovh);
+        for (int i = 0; i < nmix; ++i) jobs.push_back(T - small + kDwFixed);
+        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(half + kDwFixed);
+        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(T - half + kDwFixed);
+        for (int i = 0; i < nmix; ++i) jobs.push_back(small + kDwFixed);
         return list_schedule(jobs, num_sms);
     };
+    if (items > 2048 || T < 2) return (double)((2 * items + num_sms - 1) / num_sms) * (half + kDwFixed);
     const double base = makespan(0, 0);
+    if (T < 32) return base;
     double best = base;
     const int step_small = T / 32 > 1 ? T / 32 : 1, step_mix = num_sms / 4 > 1 ? num_sms / 4 : 1;
     for (int small = step_small; small < half; small += step_small)
@@ -887,32 +922,77 @@ void plan_uneven(DwPlan &p, long long items, int num_sms) {
             const double m = makespan(nmix, small);
             if (m < best - 1e-9) { best = m; p.n_mixed = nmix; p.small_tiles = small; }
         }
-    if (best > 0.985 * base) p.n_mixed = p.small_tiles = 0;   // not worth a different launch order
+    if (best > 0.985 * base) {   // not worth a different launch order
+        p.n_mixed = p.small_tiles = 0;
+        best = base;
+    }
+    return best;
 }
 
+// How many ways to split the token axis: the one whose waves of CTAs (fixed cost + its token tiles each) plus the addition
+// of its partial sums are shortest.  Unsplit blocks write their bf16 results themselves; a split costs the reduction's
+// launch (1.5 tiles) and its fp32 sums, written once and read once through L2 (about 4 TB/s, i.e. 7.5 MB per tile time).
 DwPlan dw_plan(const flashmhf_dims &d, int num_sms) {
-    struct Key { long long items; int tiles_per_seq, tiles_total, num_sms; };
+    struct Key { long long items, dh; int tiles_per_seq, tiles_total, num_sms; };
     struct Entry { Key k; DwPlan p; };
     static std::mutex mu;
     static std::vector<Entry> cache;
     const int G = d.H / d.Hkuv;
     const long long items = (long long)d.Hkuv * ((long long)d.E * d.De / kBI);
-    const Key key{items, (d.S + kBT - 1) / kBT, ((d.S + kBT - 1) / kBT) * G * d.B, num_sms};
+    const Key key{items, (long long)d.Dh, (d.S + kBT - 1) / kBT, ((d.S + kBT - 1) / kBT) * G * d.B, num_sms};
     std::lock_guard<std::mutex> lk(mu);
     for (const Entry &e : cache)
-        if (e.k.items == key.items && e.k.tiles_per_seq == key.tiles_per_seq && e.k.tiles_total == key.tiles_total &&
-            e.k.num_sms == key.num_sms)
+        if (e.k.items == key.items && e.k.dh == key.dh && e.k.tiles_per_seq == key.tiles_per_seq &&
+            e.k.tiles_total == key.tiles_total && e.k.num_sms == key.num_sms)
             return e.p;
-    DwPlan p;
-    p.tiles_per_seq = key.tiles_per_seq;
-    p.tiles_total = key.tiles_total;
-    const int ns = choose_nsplit(items, p.tiles_total, num_sms);
-    p.tiles_per_split = (p.tiles_total + ns - 1) / ns;
-    p.nsplit = (p.tiles_total + p.tiles_per_split - 1) / p.tiles_per_split;  // no empty split
-    plan_uneven(p, items, num_sms);
-    if (cache.size() < 256) cache.push_back(Entry{key, p});
-    return p;
+    const double sum_tiles = (double)items * kBI * 3 * d.Dh * 4 / 7.5e6;   // one set of partial sums, in token-tile times
+    DwPlan best{};
+    double best_cost = 1e300;
+    for (int ns = 1; ns <= 16 && ns <= key.tiles_total; ++ns) {
+        DwPlan p{};
+        p.tiles_per_seq = key.tiles_per_seq;
+        p.tiles_total = key.tiles_total;
+        p.tiles_per_split = (p.tiles_total + ns - 1) / ns;
+        p.nsplit = (p.tiles_total + p.tiles_per_split - 1) / p.tiles_per_split;  // no empty split
+        if (p.nsplit != ns) continue;
+        double cost = ns == 2 ? plan_uneven(p, items, num_sms)
+                              : (double)((items * ns + num_sms - 1) / num_sms) * (p.tiles_per_split + kDwFixed);
+        if (ns > 1) cost += 1.5 + ns * sum_tiles;
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = p; }
+    }
+    if (cache.size() < 256) cache.push_back(Entry{key, best});
+    return best;
 }
+
+// dQ/dR: with few token tiles the sub-networks are split over CTAs.  In 64-row blocks (about 0.8 us): a CTA costs six besides
+// its blocks, the reduction three and its partial sums.  Splits only while the tiles are no more than two waves, and only for
+// a gain of a tenth: the split sums dQ in another order than the unsplit kernel.
+struct DqPlan {
+    int nsplit, e_per_split;
+};
+DqPlan dq_plan(const flashmhf_dims &d, int num_sms) {
+    const long long tiles = (long long)((d.S + kBT - 1) / kBT) * d.H * d.B;
+    const int bpe = d.De / kBI;
+    DqPlan best{1, d.E};
+    if (tiles > 2LL * num_sms) return best;
+    const double plane_blocks = (double)d.B * d.H * d.S * d.Dh * 4 / 3.0e6;
+    auto waves = [&](long long n) { return (double)((n + num_sms - 1) / num_sms); };
+    double best_cost = 0.9 * waves(tiles) * (6.0 + d.E * bpe);
+    for (int eps = d.E - 1; eps >= 1; --eps) {
+        const int ns = (d.E + eps - 1) / eps;
+        const double cost = waves(tiles * ns) * (6.0 + eps * bpe) + 3.0 + ns * plane_blocks;
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = DqPlan{ns, eps}; }
+    }
+    return best;
+}
+
+size_t dw_workspace(const flashmhf_dims &d, const DwPlan &pl) {
+    return (size_t)pl.nsplit * 3 * (size_t)d.Hkuv * (size_t)d.E * d.De * d.Dh * sizeof(float);
+}
+size_t dq_workspace(const flashmhf_dims &d, const DqPlan &pl) {
+    return pl.nsplit > 1 ? (size_t)pl.nsplit * d.B * d.H * d.S * d.Dh * sizeof(float) : 0;
+}
+size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 template <int DH>
 int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
@@ -947,24 +1027,13 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
     const int G = d.H / d.Hkuv;
     const float s0 = p.scale.head_scaling, c = p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling;
 
-    // Weight gradients first: in data-parallel training their all-reduce can then start while dQ/dR still run.
+    // Weight gradients first: in data-parallel training their all-reduce can then start while dQ/dR still run.  In a call for
+    // everything the dQ/dR kernel follows the dK/dU/dV kernel directly, launched so that it may start under its tail, and the
+    // additions of partial sums come last.
+    const DwPlan pl = dw_plan(d, dc->num_sms);
+    ReduceArgs ra{};
+    ra.ws = static_cast<const float *>(p.workspace);
     if (want_weights) {
-        const DwPlan pl = dw_plan(d, dc->num_sms);
-        DwArgs wa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
-                  static_cast<float *>(p.workspace), d.S, d.E, d.De, G, d.B, d.Hkuv,
-                  pl.tiles_per_seq, pl.tiles_total, pl.tiles_per_split,
-                  d.E * d.De / kBI, d.Hkuv * (d.E * d.De / kBI), pl.nsplit, pl.n_mixed, pl.small_tiles, s0, c, wait_args(dc)};
-        const long long ctas = (long long)wa.n_blocks * pl.nsplit;
-        if (ctas > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
-        dim3 gw((unsigned)ctas);
-        prof_mark(st, kMarkStart);
-        bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, wa);
-        prof_mark(st, kMarkBwdDw);
-        *n_launch += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "bwd_dw_kernel launch"); return FLASHMHF_ERR_CUDA; }
-
-        ReduceArgs ra;
-        ra.ws = static_cast<const float *>(p.workspace);
         const flashmhf_tensor *outs[3] = {&p.dK, &p.dU, &p.dV};
         for (int i = 0; i < 3; ++i) {
             ra.out[i] = static_cast<__nv_bfloat16 *>(outs[i]->ptr);
@@ -975,34 +1044,73 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         ra.DH = DH;
         ra.plane = (long long)d.Hkuv * ra.I * DH;
         ra.nsplit = pl.nsplit;
-        const long long n4 = 3 * ra.plane / 4, cap = (long long)dc->num_sms * 8;
-        const int blocks = (int)((n4 + 255) / 256 < cap ? (n4 + 255) / 256 : cap);
-        dw_reduce_kernel<<<blocks, 256, 0, st>>>(ra);
-        prof_mark(st, kMarkBwdReduce);
+        DwArgs wa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
+                  static_cast<float *>(p.workspace), {ra.out[0], ra.out[1], ra.out[2]}, {ra.s_head[0], ra.s_head[1], ra.s_head[2]},
+                  {ra.s_row[0], ra.s_row[1], ra.s_row[2]}, d.S, d.E, d.De, G, d.B, d.Hkuv,
+                  pl.tiles_per_seq, pl.tiles_total, pl.tiles_per_split,
+                  d.E * d.De / kBI, d.Hkuv * (d.E * d.De / kBI), pl.nsplit, pl.n_mixed, pl.small_tiles, s0, c, wait_args(dc)};
+        const long long ctas = (long long)wa.n_blocks * pl.nsplit;
+        if (ctas > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
+        dim3 gw((unsigned)ctas);
+        prof_mark(st, kMarkStart);
+        bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, wa);
+        prof_mark(st, kMarkBwdDw);
         *n_launch += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "dw_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
+        if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "bwd_dw_kernel launch"); return FLASHMHF_ERR_CUDA; }
     }
 
+    DqPlan ql = dq_plan(d, dc->num_sms);
+    float *q_part = nullptr;
     if (want_inputs) {
-        DqArgs qa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
-                  static_cast<float *>(p.dR.ptr), p.dR.stride[0], p.dR.stride[1], p.dR.stride[2],
-                  d.S, d.E, d.De, G, s0, c, wait_args(dc)};
-        dim3 gq((d.S + kBT - 1) / kBT, d.H, d.B);
+        if (ql.nsplit > 1) {   // the split's partial sums lie behind those of dK, dU, dV; without room for them the kernel runs unsplit
+            const size_t off = want_weights ? align256(dw_workspace(d, pl)) : 0;
+            if (p.workspace && p.workspace_bytes >= off + dq_workspace(d, ql))
+                q_part = reinterpret_cast<float *>(static_cast<char *>(p.workspace) + off);
+            else
+                ql = DqPlan{1, d.E};
+        }
+        const DqArgs qa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
+                        static_cast<float *>(p.dR.ptr), p.dR.stride[0], p.dR.stride[1], p.dR.stride[2],
+                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c, wait_args(dc)};
+        const dim3 gq((unsigned)((d.S + kBT - 1) / kBT * ql.nsplit), d.H, d.B);
         prof_mark(st, kMarkStart);
-        bwd_dq_kernel<DH><<<gq, kThreads, DqSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);
+        e = launch_kernel(want_weights, bwd_dq_kernel<DH>, gq, dim3(kThreads), DqSmem<DH>::kTotal, st, tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);
         prof_mark(st, kMarkBwdDq);
         *n_launch += 1;
-        if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "bwd_dq_kernel launch"); return FLASHMHF_ERR_CUDA; }
+        if (e != cudaSuccess) { set_cuda_error(e, "bwd_dq_kernel launch"); return FLASHMHF_ERR_CUDA; }
+    }
+    if (want_weights && pl.nsplit > 1) {
+        const long long n4 = ra.plane / 4, cap = (long long)dc->num_sms * 3;
+        const dim3 blocks((unsigned)((n4 + 255) / 256 < cap ? (n4 + 255) / 256 : cap), 3);
+        prof_mark(st, kMarkStart);
+        e = launch_kernel(true, dw_reduce_kernel, blocks, dim3(256), 0, st, ra);
+        prof_mark(st, kMarkBwdReduce);
+        *n_launch += 1;
+        if (e != cudaSuccess) { set_cuda_error(e, "dw_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
+    }
+    if (want_inputs && ql.nsplit > 1) {
+        prof_mark(st, kMarkStart);
+        e = launch_o_reduce(q_part, p.dQ, d, ql.nsplit, kReduceAfterKernel, dc->num_sms, st);
+        prof_mark(st, kMarkBwdReduce);
+        *n_launch += 1;
+        if (e != cudaSuccess) { set_cuda_error(e, "dQ split reduction launch"); return FLASHMHF_ERR_CUDA; }
     }
     return FLASHMHF_OK;
 }
 
 }  // namespace
 
-size_t tc_backward_workspace_bytes(const flashmhf_dims &d) {
+size_t tc_backward_weights_workspace_bytes(const flashmhf_dims &d) {
     const DeviceCtl *dc = device_ctl();
-    const DwPlan pl = dw_plan(d, dc ? dc->num_sms : 148);
-    return (size_t)pl.nsplit * 3 * (size_t)d.Hkuv * (size_t)d.E * d.De * d.Dh * sizeof(float);
+    return dw_workspace(d, dw_plan(d, dc ? dc->num_sms : 148));
+}
+size_t tc_backward_inputs_workspace_bytes(const flashmhf_dims &d) {
+    const DeviceCtl *dc = device_ctl();
+    return dq_workspace(d, dq_plan(d, dc ? dc->num_sms : 148));
+}
+size_t tc_backward_workspace_bytes(const flashmhf_dims &d) {
+    const size_t w = tc_backward_weights_workspace_bytes(d), q = tc_backward_inputs_workspace_bytes(d);
+    return q ? align256(w) + q : w;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1043,7 +1151,7 @@ int static_scratch_ptr(void **out) {
 }  // namespace
 
 int tc_backward_static_scratch(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
-    if (tc_backward_workspace_bytes(p.d) > kStaticScratchBytes) return FLASHMHF_ERR_SCRATCH_LIMIT;
+    if (tc_backward_weights_workspace_bytes(p.d) > kStaticScratchBytes) return FLASHMHF_ERR_SCRATCH_LIMIT;
     void *ptr = nullptr;
     const int rc = static_scratch_ptr(&ptr);
     if (rc != FLASHMHF_OK) return rc;

@@ -32,7 +32,6 @@
 
 #include "kernels.h"
 #include "tc_common.cuh"
-#include <utility>
 #include "tensormap.cuh"
 
 namespace fmhf {
@@ -191,7 +190,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const bool dead = *abort_flag != 0;
-    if (args.chained) griddep_launch_dependents();   // every CTA of this launch is running: the next call may start
+    griddep_launch_dependents();   // every CTA of this launch is running: what follows (the reduction, a chained call) may start
 
     if (dead) {
         // nothing: fall through to the teardown
@@ -471,19 +470,17 @@ struct OReduceArgs {
     __nv_bfloat16 *O;
     long long s_b, s_h, s_s;
     int nsplit, H, S, DH;
-    int chained;   // launched with programmatic stream serialization, between two chained forward kernels
+    int chained;   // between two chained forward kernels: lets the next one start
 };
 // 128 threads and few registers: its CTAs fit beside the forward kernel's on an SM, so a chained launch is resident (and
 // has let the next forward launch in turn) long before the forward kernel it waits for ends.
 __global__ void __maxnreg__(48) o_reduce_kernel(const OReduceArgs a) {
-    if (a.chained) {
-        griddep_launch_dependents();
-        griddep_wait();
-    }
+    if (a.chained) griddep_launch_dependents();
+    griddep_wait();   // launched early, behind the kernel whose partial sums it adds
     // Every thread takes two 16-byte pieces of O at a time and has the loads of three splits of both in flight at once
     // (the partial sums come from L2 while the next call's weights stream in from HBM: latency is what this kernel is
     // made of); the splits are added in index order.  48 registers: 128 threads of it fit beside the d_h = 128 forward CTA.
-    // (a split call has fewer than SMs / 2 token tiles: every index fits 32 bits)
+    // (a split call has at most a few hundred token tiles: every index fits 32 bits)
     const int n4 = (int)(a.plane / 4), stride = (int)(gridDim.x * blockDim.x);
     auto store = [&](int idx, const float4 &acc) {
         const int per_row = a.DH / 4;
@@ -539,22 +536,6 @@ FwdPlan fwd_plan(const flashmhf_dims &d, int num_sms) {
     return p;
 }
 
-// Launch with programmatic stream serialization: the kernel may start before the one ahead of it on the stream has ended.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 template <int DH>
 int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, bool chained) {
     using L = FwdSmem<DH>;
@@ -594,35 +575,32 @@ int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, boo
     // (a split call has one item per CTA: tiles * splits <= SMs)
     const unsigned grid = (unsigned)(items < dc->num_sms ? items : dc->num_sms);
     prof_mark(st, kMarkStart);
-    cudaError_t e;
-    if (chained) {
-        e = launch_chained(fwd_kernel<DH>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
-    } else {
-        fwd_kernel<DH><<<grid, threads_for(DH), L::kTotal, st>>>(tmQ, tmK, tmU, tmV, tmO, a);
-        e = cudaGetLastError();
-    }
+    cudaError_t e = launch_kernel(chained, fwd_kernel<DH>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
     prof_mark(st, kMarkFwd);
     *n_launch += 1;
     if (e != cudaSuccess) { set_cuda_error(e, "fwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
     if (pl.nsplit > 1) {
-        const long long plane = (long long)p.d.B * p.d.H * p.d.S * DH;
-        OReduceArgs ra{static_cast<const float *>(p.workspace), plane, static_cast<__nv_bfloat16 *>(p.O.ptr),
-                       p.O.stride[0], p.O.stride[1], p.O.stride[2], pl.nsplit, p.d.H, p.d.S, DH, chained ? 1 : 0};
-        const long long n4 = plane / 4;
-        // chained: at most one (small) CTA per SM, so that all of them are resident beside the forward kernel's
-        const long long cap = chained ? (long long)dc->num_sms : (long long)dc->num_sms * 8;
-        const int blocks = (int)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap);
-        if (chained) e = launch_chained(o_reduce_kernel, dim3(blocks), dim3(128), 0, st, ra);
-        else o_reduce_kernel<<<blocks, 128, 0, st>>>(ra);
+        e = launch_o_reduce(static_cast<const float *>(p.workspace), p.O, p.d, pl.nsplit, chained ? kReduceChained : kReduceAfterKernel,
+                            dc->num_sms, st);
         prof_mark(st, kMarkFwdReduce);
         *n_launch += 1;
-        if (!chained) e = cudaGetLastError();
         if (e != cudaSuccess) { set_cuda_error(e, "o_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
     }
     return FLASHMHF_OK;
 }
 
 }  // namespace
+
+cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, ReduceMode mode, int num_sms,
+                            cudaStream_t st) {
+    const long long plane = (long long)d.B * d.H * d.S * d.Dh, n4 = plane / 4;
+    const OReduceArgs ra{part, plane, static_cast<__nv_bfloat16 *>(out.ptr), out.stride[0], out.stride[1], out.stride[2], nsplit, d.H, d.S,
+                         d.Dh, mode == kReduceChained ? 1 : 0};
+    // chained: at most one (small) CTA per SM, so that all of them are resident beside the forward kernel's
+    const long long cap = mode == kReduceChained ? (long long)num_sms : (long long)num_sms * 8;
+    const int blocks = (int)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap);
+    return launch_kernel(true, o_reduce_kernel, dim3(blocks), dim3(128), 0, st, ra);
+}
 
 size_t tc_forward_workspace_bytes(const flashmhf_dims &d) {
     const DeviceCtl *dc = device_ctl();

@@ -33,7 +33,7 @@ struct Api {
     decltype(&flashmhf_forward) forward = nullptr, forward_chained = nullptr;
     decltype(&flashmhf_backward) backward = nullptr;
     decltype(&flashmhf_forward_workspace_bytes) forward_ws = nullptr;
-    decltype(&flashmhf_backward_workspace_bytes) backward_ws = nullptr;
+    decltype(&flashmhf_backward_workspace_bytes) backward_ws = nullptr, backward_inputs_ws = nullptr;
     decltype(&flashmhf_prologue_forward_dtype) prologue_forward = nullptr;
     decltype(&flashmhf_prologue_backward_workspace_bytes) prologue_backward_ws = nullptr;
     decltype(&flashmhf_prologue_backward_dtype) prologue_backward = nullptr;
@@ -59,6 +59,7 @@ void bind(uintptr_t handle, py::object error_type) {
     get(api.backward, "flashmhf_backward");
     get(api.forward_ws, "flashmhf_forward_workspace_bytes");
     get(api.backward_ws, "flashmhf_backward_workspace_bytes");
+    get(api.backward_inputs_ws, "flashmhf_backward_inputs_workspace_bytes");
     get(api.prologue_forward, "flashmhf_prologue_forward_dtype");
     get(api.prologue_backward_ws, "flashmhf_prologue_backward_workspace_bytes");
     get(api.prologue_backward, "flashmhf_prologue_backward_dtype");
@@ -244,8 +245,10 @@ Grads backward_checked(const Shape &s, const Tensor &Q0, const Tensor &K0, const
             g.dV = at::empty_like(V, V.options(), fmt);
         }
         p.dK = view4(g.dK); p.dU = view4(g.dU); p.dV = view4(g.dV);
-        p.workspace_bytes = api.backward_ws(&p.d);
-        ws = at::empty({(int64_t)std::max<size_t>(p.workspace_bytes, 1)}, Q.options().dtype(at::kByte));
+    }
+    p.workspace_bytes = weights ? api.backward_ws(&p.d) : api.backward_inputs_ws(&p.d);
+    if (p.workspace_bytes) {
+        ws = at::empty({(int64_t)p.workspace_bytes}, Q.options().dtype(at::kByte));
         p.workspace = ws.data_ptr();
     }
     check(api.backward(&p, current_stream(Q)));

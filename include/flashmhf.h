@@ -134,6 +134,11 @@ size_t flashmhf_forward_workspace_bytes(const flashmhf_dims *d);
 /* Bytes of scratch flashmhf_backward needs for these dims (0 is possible).  Pure host arithmetic. */
 size_t flashmhf_backward_workspace_bytes(const flashmhf_dims *d);
 
+/* Bytes of scratch a call with parts = FLASHMHF_BWD_INPUTS can use: 0 except for short token counts, where the sub-networks
+ * are split over CTAs and fp32 partial dQ are summed in a fixed order.  Optional: without it the kernel runs unsplit, with the
+ * same results up to the order of that sum.  Pure host arithmetic. */
+size_t flashmhf_backward_inputs_workspace_bytes(const flashmhf_dims *d);
+
 /* Backward: dQ, dK, dU, dV, dR from dO, recomputing the intermediate.  Enqueues on `stream` and
  * returns.  Deterministic (no floating-point atomics).  Replaces flashffn_moe_backward,
  * flash_ffn_moe.cu:1012-1133, and the two launches at kernels/triton/flash_mlp_moe.py:832-866. */
