@@ -48,22 +48,22 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTile = kBT * 128;    // one 128-row x 64-col SW128 chunk: 16 KB
 constexpr uint32_t kWChunk = kBI * 128;  // one 64-row x 64-col chunk: 8 KB
 
-// Element-wise backward math for two neighbouring intermediate columns of one token row, on packed
+// dQ/dR: element-wise backward math for two neighbouring intermediate columns of one token row, on packed
 // fp32 pairs.  m, n are the raw products Q K^T, Q U^T; with the layer's constants s0 (head), s1 (up),
 // s2 (final) the forward is A = silu(s0 m) (s1 n) s2 r.  With t = tanh(s0 m / 2): sg = sigmoid(s0 m) =
 // 0.5 + 0.5 t, s = m*sg (so silu(s0 m) = s0 s), silu'(s0 m) = sg + s * s0 (1 - sg).  All three constants
 // fold into the per-row factor r2 = s0 s1 s2 r and into the two constants below, at no cost per element:
 //   dM = dA r2 n silu'(s0 m),  dN = dA r2 s,  A = s n r2,  dR = s0 s1 s2 * sum dA s n.
-struct BwdConst {
+struct DqConst {
     f32x2 half_s0, p_half_s0, n_half_s0;  // (s0/2), (s0/2), (-s0/2): tanh argument scale and s0 (1 - sg) = s0/2 - (s0/2) t
 };
-__device__ __forceinline__ BwdConst bwd_const(float s0) {
-    return BwdConst{f2_pack(0.5f * s0, 0.5f * s0), f2_pack(0.5f * s0, 0.5f * s0), f2_pack(-0.5f * s0, -0.5f * s0)};
+__device__ __forceinline__ DqConst dq_const(float s0) {
+    return DqConst{f2_pack(0.5f * s0, 0.5f * s0), f2_pack(0.5f * s0, 0.5f * s0), f2_pack(-0.5f * s0, -0.5f * s0)};
 }
-struct BwdPair {
+struct DqPair {
     f32x2 dm, dn, sn, da;  // dM, dN, s*N (times r2 gives A, times dA sums to dR / (s0 s1 s2)), dA
 };
-__device__ __forceinline__ BwdPair bwd_pair(f32x2 m, f32x2 n, f32x2 da, f32x2 r2, const BwdConst &k) {
+__device__ __forceinline__ DqPair dq_pair(f32x2 m, f32x2 n, f32x2 da, f32x2 r2, const DqConst &k) {
     const f32x2 half = f2_pack(0.5f, 0.5f);
     const f32x2 t = f2_tanh(f2_mul(m, k.half_s0));
     const f32x2 sg = f2_fma(t, half, half);
@@ -71,12 +71,33 @@ __device__ __forceinline__ BwdPair bwd_pair(f32x2 m, f32x2 n, f32x2 da, f32x2 r2
     const f32x2 s = f2_mul(m, sg);
     const f32x2 dsilu = f2_fma(s, omsg, sg);
     const f32x2 dar = f2_mul(da, r2);
-    BwdPair o;
+    DqPair o;
     o.sn = f2_mul(s, n);
     o.dn = f2_mul(dar, s);
     o.dm = f2_mul(f2_mul(dar, n), dsilu);
     o.da = da;
     return o;
+}
+
+// dK/dU/dV: the same for that kernel, cut where dA comes in.  With h = s0/2, t = tanh(h m):
+//   silu(s0 m) = h S with S = m + m t,   2 silu'(s0 m) = D = (1 + h m) + t ((1 + h m) - h S)      (sigmoid = (1 + t) / 2)
+// and with the per-row factor rho = h s1 s2 r, carried through (q = rho S, w = n rho D),
+//   A = q n,  dN = dA q,  dM = dA w:
+// 8 operations before dA, which run while the tensor core still computes it, and 2 after.
+struct DwConst {
+    f32x2 h, nh;  // h, -h, twice each
+};
+__device__ __forceinline__ DwConst dw_const(float s0) { return DwConst{f2_pack(0.5f * s0, 0.5f * s0), f2_pack(-0.5f * s0, -0.5f * s0)}; }
+struct DwPair {
+    f32x2 q, w, a;  // dN = dA q, dM = dA w, A
+};
+__device__ __forceinline__ DwPair dw_pair(f32x2 m, f32x2 n, f32x2 rho, const DwConst &k) {
+    const f32x2 t = f2_tanh(f2_mul(m, k.h));
+    const f32x2 mr = f2_mul(m, rho);
+    const f32x2 q = f2_fma(mr, t, mr);
+    const f32x2 d = f2_fma(mr, k.h, rho);
+    const f32x2 e = f2_fma(t, f2_fma(q, k.nh, d), d);
+    return DwPair{q, f2_mul(n, e), f2_mul(q, n)};
 }
 
 // =============================================================================================
@@ -316,7 +337,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         warp_arrive(bar(DQ_QT));
         float r_cur = 0.f, r_next = in_range ? __ldg(rrow) : 0.f;
         f32x2 dr2 = f2_pack(0.f, 0.f);  // running dR_e of this thread's columns (two interleaved partial sums)
-        const BwdConst kc = bwd_const(args.s0);
+        const DqConst kc = dq_const(args.s0);
         int in_e = 0, e = 0;  // block index inside the current sub-network; current sub-network
         for (int j = 0; ok && j < nblk; ++j) {
             if (in_e == 0) {
@@ -337,7 +358,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 warp_arrive(bar(DQ_SEMPTY));
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const BwdPair x = bwd_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
+                    const DqPair x = dq_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
                                                f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
                     dr2 = f2_fma(x.da, x.sn, dr2);
                     pm[i] = f2_to_bf16x2(x.dm);
@@ -350,7 +371,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 warp_arrive(bar(DQ_SEMPTY));
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const BwdPair x = bwd_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
+                    const DqPair x = dq_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
                                                f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
                     dr2 = f2_fma(x.da, x.sn, dr2);
                     pm[i] = f2_to_bf16x2(x.dm);
@@ -476,9 +497,12 @@ struct DwSmem {
 // load or the next MMA can start earlier shortens the loop load -> recompute -> element-wise -> accumulate.
 // S has two buffers in tensor memory, each with its own full/empty pair, so that every waiter sees every
 // phase of the barrier it waits on (a one-bit parity cannot tell phase k from phase k+2).
+// That loop over two stages is what bounds the kernel, so the element-wise step is cut in two: A and the factors of dM, dN need
+// only S; A goes out first and its dV update runs while dA is still being computed.  (One step behind S and dA before: the
+// 370M layer at 32768 tokens 1.07 -> 1.04 ms burst, 1.21 -> 1.18 sustained; 16 x 16 x 192 at d_h = 64, 16384 tokens 0.876 -> 0.794.)
 constexpr int kMaxTok = 4;
-enum { DW_WFULL = 0, DW_SFULL = 1, DW_SEMPTY = 3, DW_PFULL = 5, DW_AFULL = 6, DW_PEMPTY = 7, DW_AEMPTY = 8, DW_ACCFULL = 9, DW_DAEMPTY = 10,
-       DW_QFULL = 11, DW_GFULL = DW_QFULL + kMaxTok, DW_QEMPTY = DW_GFULL + kMaxTok, DW_GEMPTY = DW_QEMPTY + kMaxTok,
+enum { DW_WFULL = 0, DW_SFULL = 1, DW_SEMPTY = 3, DW_PFULL = 5, DW_AFULL = 6, DW_PEMPTY = 7, DW_AEMPTY = 8, DW_ACCFULL = 9, DW_DAFULL = 10,
+       DW_DAEMPTY = 11, DW_QFULL = 12, DW_GFULL = DW_QFULL + kMaxTok, DW_QEMPTY = DW_GFULL + kMaxTok, DW_GEMPTY = DW_QEMPTY + kMaxTok,
        DW_BARS = DW_GEMPTY + kMaxTok };
 static_assert(DW_BARS * 8 + 8 <= 256, "control area");
 
@@ -494,7 +518,7 @@ struct DwArgs {
     // CTA -> (weight block, token-tile range).  Blocks [0, n_mixed) are split unevenly into a long part (launched first)
     // and a short part of `small_tiles` tiles (launched last); the others into `nsplit` equal parts, part by part.
     int nblk_j, n_blocks, nsplit, n_mixed, small_tiles;
-    float s0, c;  // head_scaling; head_scaling * up_scaling * final_scaling
+    float s0, c;  // head_scaling; head_scaling * up_scaling * final_scaling / 2
     WaitArgs wait;
 };
 
@@ -559,12 +583,13 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             mbar_init(bar(DW_QFULL + s), 1);
             mbar_init(bar(DW_GFULL + s), 1);
             mbar_init(bar(DW_QEMPTY + s), 1);
-            mbar_init(bar(DW_GEMPTY + s), 1);
+            mbar_init(bar(DW_GEMPTY + s), 2);   // the dA product and the dV update have read it
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar(DW_SFULL + b), 1);
             mbar_init(bar(DW_SEMPTY + b), arrivals_of(kActThreads));
         }
+        mbar_init(bar(DW_DAFULL), 1);
         mbar_init(bar(DW_DAEMPTY), arrivals_of(kActThreads));
         mbar_init(bar(DW_PFULL), arrivals_of(kActThreads));
         mbar_init(bar(DW_AFULL), arrivals_of(kActThreads));
@@ -641,6 +666,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     umma_ss(tmem + kColS + sb * 2 * kBI, dq + ((c * kTile + kk * 32) >> 4),
                             dKU + ((c * 2 * kWChunk + kk * 32) >> 4), idS, k > 0 ? 1u : 0u);
                 }
+                umma_commit(bar(DW_SFULL + sb));
                 if (!mbar_wait(bar(DW_GFULL + st), ph, ctl, W + 4)) break;
                 if (!mbar_wait(bar(DW_DAEMPTY), (i & 1) ^ 1, ctl, W + 10)) break;
                 tc_fence_after();
@@ -650,7 +676,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     umma_ss(tmem + kColdA, dg + ((c * kTile + kk * 32) >> 4), dV + ((c * kWChunk + kk * 32) >> 4), idA,
                             k > 0 ? 1u : 0u);
                 }
-                umma_commit(bar(DW_SFULL + sb));
+                umma_commit(bar(DW_GEMPTY + st));
+                umma_commit(bar(DW_DAFULL));
                 if (++st == L::kTokStages) { st = 0; ph ^= 1; }
             }
         }
@@ -665,14 +692,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             int st = 0;
             bool ok = true;
             for (int i = 0; i < ntiles; ++i) {
-                if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
-                tc_fence_after();
                 const uint64_t dq = dQmn0 + st * kTokStep, dg = dGmn0 + st * kTokStep;
-#pragma unroll
-                for (int k = 0; k < kBT / 16; ++k)
-                    umma_ss(tmem + kColKU, dPmn + k * 128, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(bar(DW_QEMPTY + st));  // Q of this stage and the [dM|dN] tile are free
-                umma_commit(bar(DW_PEMPTY));
                 if (!mbar_wait(bar(DW_AFULL), i & 1, ctl, W + 6)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
@@ -680,8 +700,15 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     if (kVt) umma_ss(tmem + kColV, dg + k * 128, dAmn + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
                     else umma_ss(tmem + kColV, dAmn + k * 128, dg + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
                 }
-                umma_commit(bar(DW_GEMPTY + st));  // dO of this stage and the A tile are free
+                umma_commit(bar(DW_GEMPTY + st));  // dO of this stage (once its dA is computed too) and the A tile are free
                 umma_commit(bar(DW_AEMPTY));
+                if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < kBT / 16; ++k)
+                    umma_ss(tmem + kColKU, dPmn + k * 128, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(bar(DW_QEMPTY + st));  // Q of this stage and the [dM|dN] tile are free
+                umma_commit(bar(DW_PEMPTY));
                 if (++st == L::kTokStages) st = 0;
             }
             if (ok) umma_commit(bar(DW_ACCFULL));
@@ -691,7 +718,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         const int row = quarter * 32 + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
         bool ok = true;
-        const BwdConst kc = bwd_const(args.s0);
+        const DwConst kc = dw_const(args.s0);
         // This row's routing weight for sub-network e, fetched one tile ahead.  The tile's (sequence tile, head, batch)
         // coordinates advance by counting, with no division in the loop.
         int c_ts, c_hh, c_bb;
@@ -715,14 +742,11 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             const int sb = i % kSB;
             if (!mbar_wait(bar(DW_SFULL + sb), (uint32_t)(i / kSB) & 1u, ctl, W + 7)) { ok = false; break; }
             tc_fence_after();
-            uint32_t pm[kCols / 2], pn[kCols / 2], pa[kCols / 2], da[kCols];
-            // dA first: its single buffer goes straight back
-            if (kCols == 32) tmem_ld32_sync(lane_base + kColdA + part * kCols, da);
-            else tmem_ld16_sync(lane_base + kColdA + part * kCols, da);
-            tc_fence_before();
-            warp_arrive(bar(DW_DAEMPTY));
             const f32x2 r2 = f2_pack(args.c * r, args.c * r);
             const uint32_t colS = kColS + sb * 2 * kBI;
+            // first what needs only S: A goes out, and its dV update runs, while dA is still being computed
+            f32x2 fq[kCols / 2], fw[kCols / 2];
+            uint32_t pa[kCols / 2];
 #pragma unroll
             for (int sub = 0; sub < kSubs; ++sub) {
                 uint32_t m[16], n[16];
@@ -734,12 +758,31 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 }
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const BwdPair x = bwd_pair(f2_pack_bits(m[2 * q], m[2 * q + 1]), f2_pack_bits(n[2 * q], n[2 * q + 1]),
-                                               f2_pack_bits(da[sub * 16 + 2 * q], da[sub * 16 + 2 * q + 1]), r2, kc);
-                    pm[sub * 8 + q] = f2_to_bf16x2(x.dm);
-                    pn[sub * 8 + q] = f2_to_bf16x2(x.dn);
-                    pa[sub * 8 + q] = f2_to_bf16x2(f2_mul(x.sn, r2));
+                    const DwPair x = dw_pair(f2_pack_bits(m[2 * q], m[2 * q + 1]), f2_pack_bits(n[2 * q], n[2 * q + 1]), r2, kc);
+                    fq[sub * 8 + q] = x.q;
+                    fw[sub * 8 + q] = x.w;
+                    pa[sub * 8 + q] = f2_to_bf16x2(x.a);
                 }
+            }
+            if (!mbar_wait(bar(DW_AEMPTY), (i & 1) ^ 1, ctl, W + 8)) { ok = false; break; }
+#pragma unroll
+            for (int q = 0; q < kCols / 8; ++q)
+                st_shared_v4(sA + sw128_offset(row, part * (kCols / 8) + q), pa[4 * q], pa[4 * q + 1], pa[4 * q + 2], pa[4 * q + 3]);
+            fence_async_smem();
+            warp_arrive(bar(DW_AFULL));
+            // then dM and dN
+            uint32_t da[kCols], pm[kCols / 2], pn[kCols / 2];
+            if (!mbar_wait(bar(DW_DAFULL), i & 1, ctl, W + 11)) { ok = false; break; }
+            tc_fence_after();
+            if (kCols == 32) tmem_ld32_sync(lane_base + kColdA + part * kCols, da);
+            else tmem_ld16_sync(lane_base + kColdA + part * kCols, da);
+            tc_fence_before();
+            warp_arrive(bar(DW_DAEMPTY));
+#pragma unroll
+            for (int q = 0; q < kCols / 2; ++q) {
+                const f32x2 da2 = f2_pack_bits(da[2 * q], da[2 * q + 1]);
+                pm[q] = f2_to_bf16x2(f2_mul(da2, fw[q]));
+                pn[q] = f2_to_bf16x2(f2_mul(da2, fq[q]));
             }
             if (!mbar_wait(bar(DW_PEMPTY), (i & 1) ^ 1, ctl, W + 8)) { ok = false; break; }
 #pragma unroll
@@ -750,12 +793,6 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             }
             fence_async_smem();
             warp_arrive(bar(DW_PFULL));
-            if (!mbar_wait(bar(DW_AEMPTY), (i & 1) ^ 1, ctl, W + 8)) { ok = false; break; }
-#pragma unroll
-            for (int q = 0; q < kCols / 8; ++q)
-                st_shared_v4(sA + sw128_offset(row, part * (kCols / 8) + q), pa[4 * q], pa[4 * q + 1], pa[4 * q + 2], pa[4 * q + 3]);
-            fence_async_smem();
-            warp_arrive(bar(DW_AFULL));
         }
         if (part >= 2) ok = false;  // the accumulators are written out by the warps of parts 0 and 1
         if (ok) ok = mbar_wait(bar(DW_ACCFULL), 0, ctl, W + 9);
@@ -1048,7 +1085,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
                   static_cast<float *>(p.workspace), {ra.out[0], ra.out[1], ra.out[2]}, {ra.s_head[0], ra.s_head[1], ra.s_head[2]},
                   {ra.s_row[0], ra.s_row[1], ra.s_row[2]}, d.S, d.E, d.De, G, d.B, d.Hkuv,
                   pl.tiles_per_seq, pl.tiles_total, pl.tiles_per_split,
-                  d.E * d.De / kBI, d.Hkuv * (d.E * d.De / kBI), pl.nsplit, pl.n_mixed, pl.small_tiles, s0, c, wait_args(dc)};
+                  d.E * d.De / kBI, d.Hkuv * (d.E * d.De / kBI), pl.nsplit, pl.n_mixed, pl.small_tiles, s0, 0.5f * c, wait_args(dc)};
         const long long ctas = (long long)wa.n_blocks * pl.nsplit;
         if (ctas > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
         dim3 gw((unsigned)ctas);
