@@ -24,7 +24,8 @@ EXPORTS = ("flashmhf_abi_version", "flashmhf_forward_workspace_bytes", "flashmhf
            "flashmhf_prologue_backward_workspace_bytes", "flashmhf_prologue_backward", "flashmhf_lm_rope",
            "flashmhf_lm_rmsnorm_forward", "flashmhf_lm_rmsnorm_backward_workspace_bytes", "flashmhf_lm_rmsnorm_backward",
            "flashmhf_selftest_bounded_wait", "flashmhf_prologue_forward_dtype", "flashmhf_prologue_backward_dtype",
-           "flashmhf_lm_rmsnorm_forward_dtype", "flashmhf_lm_rmsnorm_backward_dtype")
+           "flashmhf_lm_rmsnorm_forward_dtype", "flashmhf_lm_rmsnorm_backward_dtype", "flashmhf_lm_rope_pair",
+           "flashmhf_lm_add_rmsnorm_forward", "flashmhf_lm_add_rmsnorm_backward")
 
 
 class Tensor(C.Structure):

@@ -329,7 +329,7 @@ int flashmhf_lm_rmsnorm_forward_dtype(const void *x, const void *w, int32_t w_dt
     int rc = check_arch();
     if (rc) return rc;
     int nl = 0;
-    rc = lm_rmsnorm_forward(x, w, w_dtype == FLASHMHF_BF16, y, rows, n, eps, static_cast<cudaStream_t>(stream), &nl);
+    rc = lm_rmsnorm_forward(x, nullptr, nullptr, w, w_dtype == FLASHMHF_BF16, y, rows, n, eps, static_cast<cudaStream_t>(stream), &nl);
     g_launches += (uint64_t)nl;
     return rc;
 }
@@ -347,7 +347,7 @@ int flashmhf_lm_rmsnorm_backward_dtype(const void *x, const void *w, int32_t w_d
     int rc = check_arch();
     if (rc) return rc;
     int nl = 0;
-    rc = lm_rmsnorm_backward(x, w, w_dtype == FLASHMHF_BF16, g, dx, dw, workspace, workspace_bytes, rows, n, eps,
+    rc = lm_rmsnorm_backward(x, w, w_dtype == FLASHMHF_BF16, g, nullptr, dx, dw, workspace, workspace_bytes, rows, n, eps,
                              static_cast<cudaStream_t>(stream), &nl);
     g_launches += (uint64_t)nl;
     return rc;
@@ -355,6 +355,40 @@ int flashmhf_lm_rmsnorm_backward_dtype(const void *x, const void *w, int32_t w_d
 int flashmhf_lm_rmsnorm_backward(const void *x, const float *w, const void *g, void *dx, float *dw, void *workspace,
                                  size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream) {
     return flashmhf_lm_rmsnorm_backward_dtype(x, w, FLASHMHF_F32_CHECK, g, dx, dw, workspace, workspace_bytes, rows, n, eps, stream);
+}
+
+int flashmhf_lm_rope_pair(const void *q, void *yq, int32_t heads_q, const void *k, void *yk, int32_t heads_k, const float *cos_t,
+                          const float *sin_t, int64_t tokens, int32_t S, int32_t head_dim, int32_t transpose, void *stream) {
+    int rc = check_arch();
+    if (rc) return rc;
+    int n = 0;
+    rc = lm_rope_pair(q, yq, heads_q, k, yk, heads_k, cos_t, sin_t, tokens, S, head_dim, transpose, static_cast<cudaStream_t>(stream), &n);
+    g_launches += (uint64_t)n;
+    return rc;
+}
+
+int flashmhf_lm_add_rmsnorm_forward(const void *x, const void *d, const void *w, int32_t w_dtype, void *sum, void *y, int64_t rows,
+                                    int32_t n, float eps, void *stream) {
+    if (w_dtype != FLASHMHF_BF16 && w_dtype != FLASHMHF_F32_CHECK) return FLASHMHF_ERR_BAD_DTYPE;
+    if (!d || !sum) return FLASHMHF_ERR_NULL;
+    int rc = check_arch();
+    if (rc) return rc;
+    int nl = 0;
+    rc = lm_rmsnorm_forward(x, d, sum, w, w_dtype == FLASHMHF_BF16, y, rows, n, eps, static_cast<cudaStream_t>(stream), &nl);
+    g_launches += (uint64_t)nl;
+    return rc;
+}
+
+int flashmhf_lm_add_rmsnorm_backward(const void *sum, const void *w, int32_t w_dtype, const void *g, const void *g_sum, void *dx, void *dw,
+                                     void *workspace, size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream) {
+    if (w_dtype != FLASHMHF_BF16 && w_dtype != FLASHMHF_F32_CHECK) return FLASHMHF_ERR_BAD_DTYPE;
+    int rc = check_arch();
+    if (rc) return rc;
+    int nl = 0;
+    rc = lm_rmsnorm_backward(sum, w, w_dtype == FLASHMHF_BF16, g, g_sum, dx, dw, workspace, workspace_bytes, rows, n, eps,
+                             static_cast<cudaStream_t>(stream), &nl);
+    g_launches += (uint64_t)nl;
+    return rc;
 }
 
 int flashmhf_profile_begin(int max_marks) {

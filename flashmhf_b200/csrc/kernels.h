@@ -68,9 +68,12 @@ int prologue_backward(const flashmhf_prologue_bwd_params &p, bool bf16_params, c
 // ---- helpers for the measurement LM: rotary embedding and hidden-size RMSNorm (lm_aux.cu) ----
 int lm_rope(const void *x, void *y, const float *cos_t, const float *sin_t, long long tokens, int S, int heads, int hd,
             long long x_tok, long long y_tok, int transpose, cudaStream_t st, int *n_launch);
-int lm_rmsnorm_forward(const void *x, const void *w, bool bf16_w, void *y, long long rows, int n, float eps, cudaStream_t st, int *n_launch);
+int lm_rope_pair(const void *q, void *yq, int heads_q, const void *k, void *yk, int heads_k, const float *cos_t, const float *sin_t,
+                 long long tokens, int S, int hd, int transpose, cudaStream_t st, int *n_launch);
+int lm_rmsnorm_forward(const void *x, const void *d, void *sum, const void *w, bool bf16_w, void *y, long long rows, int n, float eps,
+                       cudaStream_t st, int *n_launch);
 size_t lm_rmsnorm_backward_workspace_bytes(long long rows, int n);
-int lm_rmsnorm_backward(const void *x, const void *w, bool bf16_w, const void *g, void *dx, void *dw, void *workspace,
+int lm_rmsnorm_backward(const void *x, const void *w, bool bf16_w, const void *g, const void *gh, void *dx, void *dw, void *workspace,
                         size_t workspace_bytes, long long rows, int n, float eps, cudaStream_t st, int *n_launch);
 
 // Launch.  `early`: with programmatic stream serialization, so that the kernel may start before the one ahead of it on the

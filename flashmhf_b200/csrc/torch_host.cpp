@@ -41,6 +41,9 @@ struct Api {
     decltype(&flashmhf_lm_rmsnorm_forward_dtype) rmsnorm_forward = nullptr;
     decltype(&flashmhf_lm_rmsnorm_backward_workspace_bytes) rmsnorm_backward_ws = nullptr;
     decltype(&flashmhf_lm_rmsnorm_backward_dtype) rmsnorm_backward = nullptr;
+    decltype(&flashmhf_lm_rope_pair) lm_rope_pair = nullptr;
+    decltype(&flashmhf_lm_add_rmsnorm_forward) add_rmsnorm_forward = nullptr;
+    decltype(&flashmhf_lm_add_rmsnorm_backward) add_rmsnorm_backward = nullptr;
     PyObject *error_type = nullptr;  // flashmhf_b200._lib.FlashMHFError(status, message)
 };
 Api api;
@@ -67,6 +70,9 @@ void bind(uintptr_t handle, py::object error_type) {
     get(api.rmsnorm_forward, "flashmhf_lm_rmsnorm_forward_dtype");
     get(api.rmsnorm_backward_ws, "flashmhf_lm_rmsnorm_backward_workspace_bytes");
     get(api.rmsnorm_backward, "flashmhf_lm_rmsnorm_backward_dtype");
+    get(api.lm_rope_pair, "flashmhf_lm_rope_pair");
+    get(api.add_rmsnorm_forward, "flashmhf_lm_add_rmsnorm_forward");
+    get(api.add_rmsnorm_backward, "flashmhf_lm_add_rmsnorm_backward");
     Py_XDECREF(api.error_type);
     api.error_type = error_type.release().ptr();
 }
@@ -597,6 +603,77 @@ struct RMSNormFunction : public torch::autograd::Function<RMSNormFunction> {
 };
 Tensor rmsnorm(const Tensor &x, const Tensor &weight, double eps) { return RMSNormFunction::apply(x, weight, eps); }
 
+// queries [B,S,nq,hd] and keys [B,S,nk,hd], both rotated in one launch
+variable_list run_rope_pair(const Tensor &q, const Tensor &k, const Tensor &cos_t, const Tensor &sin_t, bool transpose) {
+    c10::cuda::CUDAGuard guard(q.device());
+    Tensor yq = at::empty_like(q), yk = at::empty_like(k);
+    const int64_t B = q.size(0), S = q.size(1);
+    check(api.lm_rope_pair(q.data_ptr(), yq.data_ptr(), (int32_t)q.size(2), k.data_ptr(), yk.data_ptr(), (int32_t)k.size(2),
+                           cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), B * S, (int32_t)S, (int32_t)q.size(3), transpose ? 1 : 0,
+                           current_stream(q)));
+    return {yq, yk};
+}
+struct RotaryPairFunction : public torch::autograd::Function<RotaryPairFunction> {
+    static variable_list forward(AutogradContext *ctx, const Tensor &q, const Tensor &k, const Tensor &cos_t, const Tensor &sin_t) {
+        ctx->save_for_backward({cos_t, sin_t});
+        ctx->saved_data["shape"] = std::vector<int64_t>{q.size(2), k.size(2)};
+        return run_rope_pair(q.contiguous(), k.contiguous(), cos_t, sin_t, false);
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        const variable_list sv = ctx->get_saved_variables();
+        variable_list out(4);
+        if (grads[0].defined() && grads[1].defined()) {
+            variable_list d = run_rope_pair(grads[0].contiguous(), grads[1].contiguous(), sv[0], sv[1], true);
+            out[0] = d[0];
+            out[1] = d[1];
+        } else {
+            for (int i = 0; i < 2; ++i)
+                if (grads[i].defined()) out[i] = run_rope(grads[i].contiguous(), sv[0], sv[1], true);
+        }
+        return out;
+    }
+};
+std::pair<Tensor, Tensor> rotary_pair(const Tensor &q, const Tensor &k, const Tensor &cos_t, const Tensor &sin_t) {
+    variable_list o = RotaryPairFunction::apply(q, k, cos_t, sin_t);
+    return {o[0], o[1]};
+}
+
+// (h + d, RMSNorm(h + d) * weight)
+struct AddRMSNormFunction : public torch::autograd::Function<AddRMSNormFunction> {
+    static variable_list forward(AutogradContext *ctx, const Tensor &h0, const Tensor &d0, const Tensor &weight, double eps) {
+        const Tensor h = h0.contiguous(), d = d0.contiguous();
+        const Tensor w = (weight.scalar_type() == at::kBFloat16 ? weight.detach() : weight.detach().to(at::kFloat)).contiguous();
+        c10::cuda::CUDAGuard guard(h.device());
+        Tensor sum = at::empty_like(h), y = at::empty_like(h);
+        const int64_t n = h.size(-1);
+        check(api.add_rmsnorm_forward(h.data_ptr(), d.data_ptr(), w.data_ptr(), dtype_code(w), sum.data_ptr(), y.data_ptr(), h.numel() / n,
+                                      (int32_t)n, (float)eps, current_stream(h)));
+        ctx->save_for_backward({sum, w});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["dtype"] = (int64_t)weight.scalar_type();
+        return {sum, y};
+    }
+    static variable_list backward(AutogradContext *ctx, variable_list grads) {
+        const variable_list sv = ctx->get_saved_variables();
+        const Tensor &sum = sv[0], &w = sv[1];
+        if (!grads[1].defined()) return {grads[0], grads[0], Tensor(), Tensor()};
+        const Tensor g = grads[1].contiguous(), gh = grads[0].defined() ? grads[0].contiguous() : Tensor();
+        c10::cuda::CUDAGuard guard(sum.device());
+        Tensor dx = at::empty_like(sum), dw = at::empty_like(w);
+        const int64_t n = sum.size(-1), rows = sum.numel() / n;
+        const size_t nbytes = api.rmsnorm_backward_ws(rows, (int32_t)n);
+        Tensor ws = at::empty({(int64_t)nbytes}, sum.options().dtype(at::kByte));
+        check(api.add_rmsnorm_backward(sum.data_ptr(), w.data_ptr(), dtype_code(w), g.data_ptr(), gh.defined() ? gh.data_ptr() : nullptr,
+                                       dx.data_ptr(), dw.data_ptr(), ws.data_ptr(), nbytes, rows, (int32_t)n,
+                                       (float)ctx->saved_data["eps"].toDouble(), current_stream(sum)));
+        return {dx, dx, dw.to((at::ScalarType)ctx->saved_data["dtype"].toInt()), Tensor()};
+    }
+};
+std::pair<Tensor, Tensor> add_rmsnorm(const Tensor &h, const Tensor &d, const Tensor &weight, double eps) {
+    variable_list o = AddRMSNormFunction::apply(h, d, weight, eps);
+    return {o[0], o[1]};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -607,5 +684,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("fused_prologue", torch::wrap_pybind_function(fused_prologue));
     m.def("mhffn_layer", torch::wrap_pybind_function(mhffn_layer));
     m.def("rotary", torch::wrap_pybind_function(rotary));
+    m.def("rotary_pair", torch::wrap_pybind_function(rotary_pair));
+    m.def("add_rmsnorm", torch::wrap_pybind_function(add_rmsnorm));
     m.def("rmsnorm", torch::wrap_pybind_function(rmsnorm));
 }

@@ -79,6 +79,19 @@ class RMSNorm(nn.Module):
         return self.weight * x.to(dt)
 
 
+def add_norm(norm, h, d):
+    """(h + d, norm(h + d)): the residual addition and the RMSNorm behind it; one kernel on CUDA bf16 tensors.  ``d`` may be
+    None (nothing to add)."""
+    if d is None:
+        return h, norm(h)
+    if h.is_cuda and h.dtype == torch.bfloat16 and d.dtype == torch.bfloat16:
+        from . import lm_ops
+        if h.shape[-1] in lm_ops.NORM_SIZES:
+            return lm_ops.add_rmsnorm(h, d, norm.weight, norm.eps)
+    h = h + d
+    return h, norm(h)
+
+
 def rotary_tables(S, head_dim, theta, device, dtype, first=0):
     """cos/sin [S, head_dim] of positions first .. first+S-1 as the reference builds them (fp32 angles, duplicated
     halves, cast to the activations' dtype)."""
@@ -142,8 +155,9 @@ class Attention(nn.Module):
         self.v_proj = nn.Linear(cfg.hidden_size, self.nkv * self.hd, bias=False)
         self.o_proj = nn.Linear(self.nh * self.hd, cfg.hidden_size, bias=False)
 
-    def forward(self, x, cos, sin, kv_out=None, link=None):
-        """``kv_out``: optional (k_cache, v_cache) of one layer, [B, n_kv, T_max, hd]; the keys (rotated) and values of
+    def forward(self, x, cos, sin, kv_out=None, link=None, tables=None):
+        """``tables``: optional fp32 halves of cos and sin (lm_ops.rotary_tables_f32), made once for all layers.
+        ``kv_out``: optional (k_cache, v_cache) of one layer, [B, n_kv, T_max, hd]; the keys (rotated) and values of
         the S positions are stored at [0, S) for later ``decode`` calls.
         ``link``: optional SequenceLink when a sequence is split over two ranks: the rank with the earlier part sends
         its keys and values on, the rank with the later part receives them and attends over both parts."""
@@ -153,9 +167,9 @@ class Attention(nn.Module):
         v = self.v_proj(x).view(B, S, self.nkv, self.hd).transpose(1, 2)
         if x.is_cuda and x.dtype == torch.bfloat16 and self.hd % 16 == 0:
             from . import lm_ops
-            ct, st = lm_ops.rotary_tables_f32(cos, sin)
-            q = lm_ops.RotaryFunction.apply(q, ct, st).transpose(1, 2)
-            k = lm_ops.RotaryFunction.apply(k, ct, st).transpose(1, 2)
+            ct, st = lm_ops.rotary_tables_f32(cos, sin) if tables is None else tables
+            q, k = lm_ops.rotary_pair(q, k, ct, st)
+            q, k = q.transpose(1, 2), k.transpose(1, 2)
         else:
             q, k = _Rotary.apply(q.transpose(1, 2), cos, sin), _Rotary.apply(k.transpose(1, 2), cos, sin)
         if kv_out is not None:
@@ -234,8 +248,15 @@ class DecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(cfg.hidden_size, cfg.rms_norm_eps)
 
     def forward(self, h, cos, sin, kv_out=None, link=None):
-        h = h + self.self_attn(self.input_layernorm(h), cos, sin, kv_out, link)
-        return h + self.mlp(self.post_attention_layernorm(h))
+        h, d = self.step(h, None, cos, sin, kv_out, link)
+        return h + d
+
+    def step(self, h, d, cos, sin, kv_out=None, link=None, tables=None):
+        """The layer on h + d (the residual stream and what the layer before has yet to add to it); returns the new pair, so
+        that every addition happens in the norm that follows it, across layers too."""
+        h, x = add_norm(self.input_layernorm, h, d)
+        h, x = add_norm(self.post_attention_layernorm, h, self.self_attn(x, cos, sin, kv_out, link, tables))
+        return h, self.mlp(x)
 
     def decode(self, h, cos_p, sin_p, k_cache, v_cache, pos):
         h = h + self.self_attn.decode(self.input_layernorm(h), cos_p, sin_p, k_cache, v_cache, pos)
@@ -356,11 +377,15 @@ class DecoderLM(nn.Module):
         cos, sin = rotary_tables(S, hd, self.cfg.rope_theta, ids.device, h.dtype, first=0 if link is None else link.first)
         if link is not None:
             link.start(self.cfg, B, ids.device, h.dtype)
+        tables, d = None, None
+        if h.is_cuda and h.dtype == torch.bfloat16:
+            from . import lm_ops
+            tables = lm_ops.rotary_tables_f32(cos, sin)
         for i, layer in enumerate(self.model.layers):
-            h = layer(h, cos, sin, None if cache is None else (cache.k[i], cache.v[i]), link)
+            h, d = layer.step(h, d, cos, sin, None if cache is None else (cache.k[i], cache.v[i]), link, tables)
         if link is not None:
             link.finish()
-        return self.model.norm(h)
+        return add_norm(self.model.norm, h, d)[1]
 
     def decode_step(self, ids, cache, pos):
         """ids [B,1], the token at position ``pos`` of every sequence; the cache holds positions [0, pos).  Returns the

@@ -24,6 +24,16 @@ class RMSNormFunction:
         return _lib.native().rmsnorm(x, weight, eps)
 
 
+def rotary_pair(q, k, cos_t, sin_t):
+    """(q, k) [B,S,heads,head_dim] bf16, rotated in one launch."""
+    return _lib.native().rotary_pair(q, k, cos_t, sin_t)
+
+
+def add_rmsnorm(h, d, weight, eps):
+    """(h + d, RMSNorm(h + d) * weight) for bf16 [..., n], n in NORM_SIZES, in one pass."""
+    return _lib.native().add_rmsnorm(h, d, weight, eps)
+
+
 def rotary_tables_f32(cos, sin):
     """The first half of the reference's (duplicated) cos/sin tables, as the fp32 values of their bf16 roundings."""
     h = cos.shape[-1] // 2

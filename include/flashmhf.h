@@ -236,6 +236,18 @@ int flashmhf_lm_rmsnorm_forward_dtype(const void *x, const void *w, int32_t w_dt
 int flashmhf_lm_rmsnorm_backward_dtype(const void *x, const void *w, int32_t w_dtype, const void *g, void *dx, void *dw,
                                        void *workspace, size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream);
 
+/* Rotary embedding of two contiguous tensors [tokens, heads_q | heads_k, head_dim] (the queries and keys of a layer) in one
+ * launch; otherwise as flashmhf_lm_rope. */
+int flashmhf_lm_rope_pair(const void *q, void *yq, int32_t heads_q, const void *k, void *yk, int32_t heads_k, const float *cos_t,
+                          const float *sin_t, int64_t tokens, int32_t S, int32_t head_dim, int32_t transpose, void *stream);
+
+/* The residual addition and the RMSNorm behind it in one pass: sum = bf16(x + d), y = RMSNorm(sum) w.  Backward: dx, the gradient
+ * of both x and d, from the gradients of y (g) and of sum (g_sum, may be NULL); the rest as in the calls without the addition. */
+int flashmhf_lm_add_rmsnorm_forward(const void *x, const void *d, const void *w, int32_t w_dtype, void *sum, void *y, int64_t rows,
+                                    int32_t n, float eps, void *stream);
+int flashmhf_lm_add_rmsnorm_backward(const void *sum, const void *w, int32_t w_dtype, const void *g, const void *g_sum, void *dx, void *dw,
+                                     void *workspace, size_t workspace_bytes, int64_t rows, int32_t n, float eps, void *stream);
+
 /* SYNCHRONOUS.  Waits for the current device, then reads and clears the status word the kernels
  * write when a bounded wait runs out.  *code = 0 if none did; otherwise a kernel/role identifier
  * (kernel * 100 + wait), and the call returns FLASHMHF_ERR_DEVICE_TIMEOUT.
