@@ -49,7 +49,7 @@ constexpr int kBI = 64;   // intermediate rows per block
 // take what two Q tiles leave.
 template <int DH>
 struct FwdRings {
-    static constexpr int kKU = DH == 64 ? 6 : 4, kV = DH == 64 ? 6 : 2;
+    static constexpr int kKU = DH == 64 ? 6 : 4, kV = DH == 64 ? 6 : 4;
     static_assert(kKU % 2 == 0, "each [K;U] stage must belong to one S issuer");
 };
 // Activation teams of eight warps (warp % 4 = lane quarter, next bit = which 32 of a block's 64 columns).  With two
@@ -71,20 +71,22 @@ struct FwdSmem {
     static constexpr uint32_t kKUStage = 2 * kChunks * kWChunk; // per chunk: K rows then U rows = one 128-row K-major tile
     static constexpr uint32_t kVStage = kChunks * kWChunk;
     // offsets from the 1024-aligned base
-    static constexpr uint32_t kOffQ = 0;                        // two Q tiles: work items alternate between them
-    static constexpr uint32_t kOffKU = kOffQ + 2 * kQBytes;
+    // ONE Q tile: an item's Q is copied to tensor memory before the item ahead of it is written out, so the tile is Q first and
+    // that item's O staging tile next.  (A second tile would cost the V ring two of its stages.)
+    static constexpr uint32_t kOffQ = 0;
+    static constexpr uint32_t kOffKU = kOffQ + kQBytes;
     static constexpr uint32_t kOffV = kOffKU + FwdRings<DH>::kKU * kKUStage;
     static constexpr uint32_t kOffBar = kOffV + FwdRings<DH>::kV * kVStage;
     static constexpr uint32_t kTotal = kOffBar + 320 + 1024;  // + barriers/control + alignment slack
 };
 
 // barrier slots (8 bytes each) inside the control area
-// QFULL[q]: Q tile q has landed; QFREE[q]: the O tile staged over it has been read by its TMA store;
+// QFULL: an item's Q has landed; QFREE: an item's O, staged over the Q of the item after it, has been read by its TMA store;
 // SFULL[b]: S computed into buffer b; SEMPTY[b]: every warp of the team working on it has its part in registers;
 // AFULL[s]: A written to slot s; AFREE[s]: the O update that read slot s is done; QT: Q copied to tensor memory;
 // OFULL: the last O update of a work item is done; OFREE: its accumulator has been read out.
 // A CTA walks several work items (token tiles); blocks are counted through all of them (g), buffer and slot of a block
-// are g % 2, Q tile and per-item barriers alternate with the item count, so every barrier has one fixed set of
+// are g % 2, so every barrier has one fixed set of
 // waiters that observes each of its phases and a one-bit phase parity is enough.
 constexpr int kMaxRing = 6;
 enum { BAR_QFULL = 0, BAR_QFREE = 2, BAR_SFULL = 4, BAR_SEMPTY = 6, BAR_AFULL = 8, BAR_AFREE = 10, BAR_OFULL = 12, BAR_OFREE = 13,
@@ -164,8 +166,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     if (threadIdx.x == 0) {
         *abort_flag = launch_aborted(args.wait);  // a CTA of this launch gave up: drain fast
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar(BAR_QFULL + i), 1);
-            mbar_init(bar(BAR_QFREE + i), 1);
             mbar_init(bar(BAR_SFULL + i), 1);
             mbar_init(bar(BAR_SEMPTY + i), arrivals_of(kTeamThreads));
             mbar_init(bar(BAR_AFULL + i), arrivals_of(kTeamThreads));
@@ -179,6 +179,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             mbar_init(bar(BAR_VFULL + i), 1);
             mbar_init(bar(BAR_VEMPTY + i), 1);
         }
+        mbar_init(bar(BAR_QFULL), 1);
+        mbar_init(bar(BAR_QFREE), 1);
         mbar_init(bar(BAR_OFULL), 1);
         mbar_init(bar(BAR_OFREE), arrivals_of(kTeamThreads));
         mbar_init(bar(BAR_QT), arrivals_of(kTeamThreads));
@@ -207,15 +209,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             int n = 0;  // work items of this CTA so far
             for (int item = blockIdx.x; ok && item < args.n_items; item += gridDim.x, ++n) {
                 const FwdItem w = fwd_item(args, item, nblk_total);
-                const int hk = w.h / args.G, q = n & 1;
-                // the Q tile of item n - 2 doubled as its O staging tile: wait until its store has read it
-                if (n >= 2 && !mbar_wait(bar(BAR_QFREE + q), ((n >> 1) - 1) & 1, ctl, W + 12)) break;
+                const int hk = w.h / args.G;
+                // the tile's last use: Q of item 0 (until it is in tensor memory), then O of item n - 2
+                if (n == 1 && !mbar_wait(bar(BAR_QT), 0, ctl, W + 12)) break;
+                if (n >= 2 && !mbar_wait(bar(BAR_QFREE), n & 1, ctl, W + 12)) break;
                 // (the first Q of a chained call is asked for by the activation warps, once the kernel before this one has
                 // completed: this thread touches only the weights and never waits for that)
                 if (!(args.chained && n == 0)) {
-                    mbar_arrive_expect_tx(bar(BAR_QFULL + q), L::kQBytes);
+                    mbar_arrive_expect_tx(bar(BAR_QFULL), L::kQBytes);
                     for (int c = 0; c < L::kChunks; ++c)
-                        tma_load_4d(sQ + q * L::kQBytes + c * (kBT * 128), &tmQ, bar(BAR_QFULL + q), c * 64, w.t0, w.h, w.b);
+                        tma_load_4d(sQ + c * (kBT * 128), &tmQ, bar(BAR_QFULL), c * 64, w.t0, w.h, w.b);
                 }
                 // [K;U] of block j, then V of block j-2: V is consumed about two blocks later than K and U of
                 // the same block, so with this lag the producer never waits on the V ring while a [K;U]
@@ -332,10 +335,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         // copy columns [0, 64) of d_h, the upper four [64, 128)).  Done as soon as the previous item's last S has been
         // read, i.e. before that item's epilogue, so that the first S of the new item is computed under the epilogue.
         auto copy_q = [&](int nn) -> bool {
-            if (!mbar_wait(bar(BAR_QFULL + (nn & 1)), (nn >> 1) & 1, ctl, W + 11)) return false;
+            if (!mbar_wait(bar(BAR_QFULL), nn & 1, ctl, W + 11)) return false;
             if (group * 64 < DH) {
                 uint32_t qv[32];
-                const uint8_t *src = gbase + L::kOffQ + (nn & 1) * L::kQBytes + group * (kBT * 128);
+                const uint8_t *src = gbase + L::kOffQ + group * (kBT * 128);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
@@ -399,7 +402,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             tc_fence_after();
             constexpr int kColsPerGroup = DH / 2;  // 64, 48 or 32 columns per thread
             const int c0 = group * kColsPerGroup;
-            const uint32_t sO = sQ + (n & 1) * L::kQBytes;
+            const uint32_t sO = sQ;
             if (args.nsplit > 1) {
                 // partial O of this item's blocks, fp32, straight from tensor memory to the workspace
                 float *dst = args.part + ((((long long)w.isplit * args.B + w.b) * args.H + w.h) * args.S + t) * DH + c0;
@@ -418,6 +421,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 tc_fence_before();
                 warp_arrive(bar(BAR_OFREE));
             } else {
+                named_bar_sync(2, kTeamThreads);   // the next item's Q has been copied out of the tile by all of the team
 #pragma unroll
                 for (int gg = 0; gg < kColsPerGroup / 16; ++gg) {
                     uint32_t o[16];
@@ -440,7 +444,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     for (int c = 0; c < L::kChunks; ++c) tma_store_4d(&tmO, sO + c * (kBT * 128), c * 64, w.t0, w.h, w.b);
                     tma_store_commit();
                     tma_store_wait_read();          // the tile has been read: it may take the Q of the item after next
-                    mbar_arrive(bar(BAR_QFREE + (n & 1)));
+                    mbar_arrive(bar(BAR_QFREE));
                 }
             }
         }
