@@ -109,14 +109,16 @@ struct DqSmem {
     static constexpr uint32_t kQBytes = kChunks * kTile;
     static constexpr uint32_t kKUStage = kChunks * 2 * kWChunk;  // per chunk: [K;U] = 128 rows
     static constexpr uint32_t kVStage = kChunks * kWChunk;
-    // d_h = 64: shared memory is plentiful and a block is short, so the way of a stage from L2 takes more stages to hide
-    static constexpr int kKUStages = DH == 64 ? 6 : 3, kVStages = DH == 64 ? 6 : 2;
-    static constexpr uint32_t kOffQ = 0;
-    static constexpr uint32_t kOffdO = kOffQ + kQBytes;
-    static constexpr uint32_t kOffKU = kOffdO + kQBytes;
+    // Q and dO are needed in shared memory only until they are copied to tensor memory: they arrive in the last two stages of
+    // the [K;U] ring, which joins the ring after that (the ring's first lap waits for it there), and dQ leaves through one of them.
+    // With tiles of their own the rings had three and two stages, too few for the way of a stage from L2.
+    static constexpr int kKUStages = DH == 64 ? 8 : 5, kVStages = DH == 64 ? 8 : 4;
+    static_assert(kQBytes == kKUStage, "a token tile takes one [K;U] stage");
+    static constexpr uint32_t kOffKU = 0;
+    static constexpr uint32_t kOffQ = kOffKU + (kKUStages - 2) * kKUStage, kOffdO = kOffQ + kQBytes;
     static constexpr uint32_t kOffV = kOffKU + kKUStages * kKUStage;
     static constexpr uint32_t kOffCtl = kOffV + kVStages * kVStage;
-    static constexpr uint32_t kCtlBytes = 320 + 2 * (kParts - 1) * 128 * 4;  // barriers + two sets of dR exchange rows
+    static constexpr uint32_t kCtlBytes = 384 + 2 * (kParts - 1) * 128 * 4;  // barriers + two sets of dR exchange rows
     static constexpr uint32_t kTotal = kOffCtl + kCtlBytes + 1024;
 };
 
@@ -125,11 +127,11 @@ struct DqSmem {
 //   SFULL (S and dA of the block computed: one commit from each of their issuers), SEMPTY (both are in the
 //   element-wise warps' registers), PFULL ([dM|dN] written), PEMPTY (the dQ update that read it is done).
 // All of them complete once per block and every waiter waits on every phase, so a one-bit parity is enough.
-constexpr int kMaxRing = 6;
+constexpr int kMaxRing = 8;
 enum { DQ_QFULL = 0, DQ_SFULL = 1, DQ_SEMPTY = 2, DQ_PFULL = 3, DQ_PEMPTY = 4, DQ_ACCFULL = 5, DQ_QT = 6, DQ_DRFULL = 7, DQ_DRFREE = 9,
        DQ_KUFULL = 11, DQ_KUEMPTY = DQ_KUFULL + kMaxRing, DQ_VFULL = DQ_KUEMPTY + kMaxRing, DQ_VEMPTY = DQ_VFULL + kMaxRing,
        DQ_BARS = DQ_VEMPTY + kMaxRing };
-static_assert(DQ_BARS * 8 + 8 <= 320, "control area");
+static_assert(DQ_BARS * 8 + 8 <= 384, "control area");
 
 struct DqArgs {
     const float *R;
@@ -159,7 +161,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                    sBar = base + L::kOffCtl;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(gbase + L::kOffCtl + DQ_BARS * 8);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(gbase + L::kOffCtl + DQ_BARS * 8 + 4);
-    volatile float *drx = reinterpret_cast<volatile float *>(gbase + L::kOffCtl + 320);  // [2][kParts - 1][128]
+    volatile float *drx = reinterpret_cast<volatile float *>(gbase + L::kOffCtl + 384);  // [2][kParts - 1][128]
     auto bar = [&](int i) { return sBar + 8u * i; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -210,6 +212,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             uint32_t phk = 1, phv = 1;
             for (int j = 0; j < nblk; ++j) {
                 const int row = e0 * args.De + j * kBI;
+                // Q and dO are in tensor memory: their tiles join the ring
+                if (j == L::kKUStages - 2 && !mbar_wait(bar(DQ_QT), 0, ctl, W + 14)) break;
                 if (!mbar_wait(bar(DQ_KUEMPTY + sk), phk, ctl, W + 1)) break;
                 const uint32_t fk = bar(DQ_KUFULL + sk);
                 mbar_arrive_expect_tx(fk, L::kKUStage);
