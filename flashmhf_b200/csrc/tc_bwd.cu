@@ -526,6 +526,37 @@ struct DwArgs {
     WaitArgs wait;
 };
 
+// This CTA's weight block and token tiles.
+__device__ __forceinline__ void dw_range(const DwArgs &args, int &blk, int &split, int &tile_begin, int &tile_end) {
+    const int cta = blockIdx.x, n_even = args.n_blocks - args.n_mixed;
+    if (cta < args.n_mixed) {                               // long part of an unevenly split block
+        blk = cta; split = 0; tile_begin = 0; tile_end = args.tiles_total - args.small_tiles;
+    } else if (cta < args.n_mixed + n_even * args.nsplit) { // equal parts, part by part
+        const int r = cta - args.n_mixed;
+        split = r / n_even;
+        blk = args.n_mixed + (r - split * n_even);
+        tile_begin = split * args.tiles_per_split;
+        tile_end = min(tile_begin + args.tiles_per_split, args.tiles_total);
+    } else {                                                // short part of an unevenly split block
+        blk = cta - (args.n_mixed + n_even * args.nsplit); split = 1;
+        tile_begin = args.tiles_total - args.small_tiles; tile_end = args.tiles_total;
+    }
+}
+// 16 columns of one row of an accumulator: fp32 to the workspace, or the bf16 result.
+__device__ __forceinline__ void dw_store16(bool direct, float *dst, __nv_bfloat16 *o16, const uint32_t (&o)[16]) {
+    if (direct) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            *reinterpret_cast<uint2 *>(o16 + v * 4) = make_uint2(pack_bf16(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1])),
+                                                                 pack_bf16(__uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3])));
+    } else {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            *reinterpret_cast<float4 *>(dst + v * 4) = make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]),
+                                                                   __uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3]));
+    }
+}
+
 template <int DH>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
@@ -544,21 +575,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int blk, split, tile_begin, tile_end;
-    {
-        const int cta = blockIdx.x, n_even = args.n_blocks - args.n_mixed;
-        if (cta < args.n_mixed) {                               // long part of an unevenly split block
-            blk = cta; split = 0; tile_begin = 0; tile_end = args.tiles_total - args.small_tiles;
-        } else if (cta < args.n_mixed + n_even * args.nsplit) { // equal parts, part by part
-            const int r = cta - args.n_mixed;
-            split = r / n_even;
-            blk = args.n_mixed + (r - split * n_even);
-            tile_begin = split * args.tiles_per_split;
-            tile_end = min(tile_begin + args.tiles_per_split, args.tiles_total);
-        } else {                                                // short part of an unevenly split block
-            blk = cta - (args.n_mixed + n_even * args.nsplit); split = 1;
-            tile_begin = args.tiles_total - args.small_tiles; tile_end = args.tiles_total;
-        }
-    }
+    dw_range(args, blk, split, tile_begin, tile_end);
     const int hk = blk / args.nblk_j, jblk = blk - hk * args.nblk_j;
     const int e = (jblk * kBI) / args.De;
     const int ntiles = tile_end - tile_begin;  // >= 1 by construction of the plan
@@ -812,21 +829,6 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             };
             constexpr int kColsPerHalf = DH / 2;
             const int c0 = half * kColsPerHalf;
-            auto store16 = [&](float *dst, __nv_bfloat16 *o16, const uint32_t (&o)[16]) {   // 16 columns of one row
-                if (direct) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v)
-                        *reinterpret_cast<uint2 *>(o16 + v * 4) =
-                            make_uint2(pack_bf16(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1])),
-                                       pack_bf16(__uint_as_float(o[4 * v + 2]), __uint_as_float(o[4 * v + 3])));
-                } else {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v)
-                        *reinterpret_cast<float4 *>(dst + v * 4) =
-                            make_float4(__uint_as_float(o[4 * v]), __uint_as_float(o[4 * v + 1]), __uint_as_float(o[4 * v + 2]),
-                                        __uint_as_float(o[4 * v + 3]));
-                }
-            };
             {   // [dK;dU]: lane = row of the stacked block (0-63 dK, 64-127 dU)
                 float *dst = wsb + (row < kBI ? 0 : plane) + (long long)(row & (kBI - 1)) * DH + c0;
                 __nv_bfloat16 *o16 = out_row(row < kBI ? 0 : 1, row & (kBI - 1)) + c0;
@@ -834,7 +836,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
                     tmem_ld16_sync(lane_base + kColKU + c0 + g * 16, o);
-                    store16(dst + g * 16, o16 + g * 16, o);
+                    dw_store16(direct, dst + g * 16, o16 + g * 16, o);
                 }
             }
             if (kVt) {  // dV^T: lane = column d of dV, tensor-memory column = row of the block; a warp stores 32 consecutive elements per row
@@ -860,7 +862,358 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
                     tmem_ld16_sync(lane_base + kColV + c0 + g * 16, o);
-                    if (lane < 16) store16(dst + g * 16, o16 + g * 16, o);
+                    if (lane < 16) dw_store16(direct, dst + g * 16, o16 + g * 16, o);
+                }
+            }
+            tc_fence_before();
+        }
+    }
+
+    __syncwarp();
+    if (*abort_flag) {
+        const long long t_end = clock64() + (1LL << 19);
+        while (clock64() < t_end) __nanosleep(256);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kTmemCols);
+    }
+}
+
+// =============================================================================================
+//                        dK / dU / dV kernel, transposed (d_h = 64 and 96)
+// =============================================================================================
+// The kernel above is bound by shared memory: every operand of its four products comes from there, the staged [dM|dN] and A
+// tiles included (ncu at d_h = 64: 142 KB read and 89 KB written per 128-token x 64-row block, 1800 of 2330 clk).  Where the
+// accumulators are narrow enough, the recompute is done transposed instead: a CTA owns 128 weight rows, and
+//     M^T = K Q^T,  N^T = U Q^T,  dA^T = V dO^T      (128 weight rows x 64 tokens each, lane = weight row)
+// come out such that dM^T, dN^T and A^T, written back to tensor memory as bf16, are the A operands of
+//     dK += dM^T Q,  dU += dN^T Q,  dV += A^T dO     (128 x d_h each).
+// Nothing is staged in shared memory, the accumulating products read only their B operand there, and a token tile serves twice as
+// many weight rows: 112 KB (d_h = 64) instead of 231 KB per block.
+// Tensor memory: three accumulators of d_h columns; d_h = 64: two buffers of [M^T | N^T] (128 columns), whose columns A^T, dM^T and
+// dN^T later take, and dA^T; d_h = 96: one [M^T | N^T], given back as soon as it is in registers, dA^T, over which dM^T and dN^T
+// are written, and 32 columns for A^T.  (d_h = 128 would need 576 columns.)
+// The routing weight now goes with the column: warp 2 fetches the 64 tokens' weights of a tile (of the two sub-networks that
+// 128 rows can touch) into a small ring in shared memory, from where the element-wise warps read them as pairs.
+constexpr int kTT = 64;    // tokens per tile
+constexpr int kTI = 128;   // weight rows per CTA
+
+template <int DH>
+struct DwtSmem {
+    static constexpr int kChunks = (DH + 63) / 64;
+    static constexpr uint32_t kWMat = kChunks * 2 * kWChunk;      // one of K, U, V: 128 rows
+    static constexpr uint32_t kTok = kChunks * kWChunk;           // Q or dO of a tile: 64 rows
+    static constexpr int kStages = DH == 64 ? 8 : 3;
+    static constexpr int kRSlots = 4;
+    static constexpr uint32_t kOffW = 0;
+    static constexpr uint32_t kOffTok = 3 * kWMat;
+    static constexpr uint32_t kOffR = kOffTok + kStages * 2 * kTok;
+    static constexpr uint32_t kOffCtl = kOffR + kRSlots * 2 * kTT * 4;
+    static constexpr uint32_t kTotal = kOffCtl + 512 + 1024;
+};
+
+// Barriers: as in the kernel above, with S = [M^T | N^T] (buffer b = tile % kSB).  SEMPTY[b], DAEMPTY: the buffer may be computed
+// into again (d_h = 64: the updates that read [dM|dN] and A from S are done / dA is in registers; d_h = 96: S is in registers /
+// the updates that read dM and dN over dA are done).  AEMPTY (d_h = 96): the dV update has read A.  RFULL, REMPTY: routing weights.
+constexpr int kMaxTokT = 8;
+enum { DT_WFULL = 0, DT_SFULL = 1, DT_SEMPTY = 3, DT_AFULL = 5, DT_PFULL = 7, DT_AEMPTY = 9, DT_DAFULL = 10, DT_DAEMPTY = 11, DT_ACCFULL = 12,
+       DT_RFULL = 13, DT_REMPTY = 17, DT_QFULL = 21, DT_GFULL = DT_QFULL + kMaxTokT, DT_QEMPTY = DT_GFULL + kMaxTokT,
+       DT_GEMPTY = DT_QEMPTY + kMaxTokT, DT_BARS = DT_GEMPTY + kMaxTokT };
+static_assert(DT_BARS * 8 + 8 <= 512, "control area");
+
+template <int DH>
+__global__ void __launch_bounds__(kThreads, 1)
+bwd_dwt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
+               const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
+               const __grid_constant__ CUtensorMap tmV, const DwArgs args) {
+    static_assert(kParts == 2, "a thread holds 32 of a tile's 64 tokens");
+    using L = DwtSmem<DH>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t *gbase = smem_raw + (base - raw);
+    const uint32_t sW = base + L::kOffW, sTok = base + L::kOffTok, sBar = base + L::kOffCtl;
+    float *rbuf = reinterpret_cast<float *>(gbase + L::kOffR);   // [kRSlots][2][kTT]
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(gbase + L::kOffCtl + DT_BARS * 8);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(gbase + L::kOffCtl + DT_BARS * 8 + 4);
+    auto bar = [&](int i) { return sBar + 8u * i; };
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int blk, split, tile_begin, tile_end;
+    dw_range(args, blk, split, tile_begin, tile_end);
+    const int hk = blk / args.nblk_j, row0 = (blk - hk * args.nblk_j) * kTI;
+    const int I = args.E * args.De;
+    const int ntiles = tile_end - tile_begin;  // >= 1 by construction of the plan
+    const WaitCtl ctl{abort_flag, args.wait};
+    constexpr int W = kKernelBwdDw * 100 + 50;
+    constexpr int kSB = DH == 64 ? 2 : 1;
+    constexpr uint32_t kColAcc = 0, kColS = 3 * DH, kColdA = kColS + kSB * 128, kColA = kColdA + 64;   // kColA: d_h = 96
+    static_assert(kColdA + 64 + (kSB == 1 ? 32 : 0) <= kTmemCols, "tensor memory");
+
+    auto tile_coords = [&](int i, int &ts, int &hh, int &bb) {  // token tile i of this CTA -> (seq tile, head, batch)
+        const int ti = tile_begin + i;
+        ts = ti % args.tiles_per_seq;
+        const int rest = ti / args.tiles_per_seq;
+        hh = hk * args.G + rest % args.G;
+        bb = rest / args.G;
+    };
+
+    if (threadIdx.x == 0) {
+        *abort_flag = launch_aborted(args.wait);  // a CTA of this launch gave up: drain fast
+        for (int i : {DT_WFULL, DT_AEMPTY, DT_DAFULL, DT_ACCFULL}) mbar_init(bar(i), 1);
+        mbar_init(bar(DT_DAEMPTY), kSB == 2 ? arrivals_of(kActThreads) : 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar(DT_SFULL + b), 1);
+            mbar_init(bar(DT_SEMPTY + b), kSB == 2 ? 1 : arrivals_of(kActThreads));
+            mbar_init(bar(DT_AFULL + b), arrivals_of(kActThreads));
+            mbar_init(bar(DT_PFULL + b), arrivals_of(kActThreads));
+        }
+        for (int s = 0; s < L::kRSlots; ++s) {
+            mbar_init(bar(DT_RFULL + s), arrivals_of(32));
+            mbar_init(bar(DT_REMPTY + s), arrivals_of(kActThreads));
+        }
+        for (int s = 0; s < L::kStages; ++s) {
+            mbar_init(bar(DT_QFULL + s), 1);
+            mbar_init(bar(DT_GFULL + s), 1);
+            mbar_init(bar(DT_QEMPTY + s), 1);
+            mbar_init(bar(DT_GEMPTY + s), 2);   // the dA product and the dV update have read it
+        }
+        fence_mbar_init();
+    }
+    if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kTmemCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const bool dead = *abort_flag != 0;
+    griddep_launch_dependents();   // the dQ/dR kernel may take over SMs that this kernel's last CTAs leave idle
+
+    if (dead) {
+        // nothing: fall through to the teardown
+    } else if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer
+        if (lane == 0) {
+            tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK);
+            tma_prefetch_desc(&tmU); tma_prefetch_desc(&tmV);
+            mbar_arrive_expect_tx(bar(DT_WFULL), 3 * L::kWMat);
+            for (int c = 0; c < L::kChunks; ++c)
+                for (int hf = 0; hf < 2; ++hf) {   // rows beyond the last (an odd number of 64-row blocks) read as zero
+                    const uint32_t d = sW + c * 2 * kWChunk + hf * kWChunk;
+                    tma_load_3d(d, &tmK, bar(DT_WFULL), c * 64, row0 + hf * 64, hk);
+                    tma_load_3d(d + L::kWMat, &tmU, bar(DT_WFULL), c * 64, row0 + hf * 64, hk);
+                    tma_load_3d(d + 2 * L::kWMat, &tmV, bar(DT_WFULL), c * 64, row0 + hf * 64, hk);
+                }
+            int st = 0;
+            uint32_t ph = 1;
+            for (int i = 0; i < ntiles; ++i) {
+                int ts, hh, bb;
+                tile_coords(i, ts, hh, bb);
+                const uint32_t d = sTok + st * 2 * L::kTok;
+                if (!mbar_wait(bar(DT_QEMPTY + st), ph, ctl, W + 1)) break;
+                mbar_arrive_expect_tx(bar(DT_QFULL + st), L::kTok);
+#pragma unroll
+                for (int c = 0; c < L::kChunks; ++c) tma_load_4d(d + c * kWChunk, &tmQ, bar(DT_QFULL + st), c * 64, ts * kTT, hh, bb);
+                if (!mbar_wait(bar(DT_GEMPTY + st), ph, ctl, W + 2)) break;
+                mbar_arrive_expect_tx(bar(DT_GFULL + st), L::kTok);
+#pragma unroll
+                for (int c = 0; c < L::kChunks; ++c)
+                    tma_load_4d(d + L::kTok + c * kWChunk, &tmdO, bar(DT_GFULL + st), c * 64, ts * kTT, hh, bb);
+                if (++st == L::kStages) { st = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer 1: M^T, N^T, dA^T
+        if (lane == 0) {
+            constexpr uint32_t idS = umma_idesc(128, kTT, false, false);
+            const uint64_t dK = desc_kmajor(sW), dU = desc_kmajor(sW + L::kWMat), dV = desc_kmajor(sW + 2 * L::kWMat),
+                           dQ0 = desc_kmajor(sTok), dG0 = desc_kmajor(sTok + L::kTok);
+            constexpr uint64_t kTokStep = (2 * L::kTok) >> 4;
+            bool ok = mbar_wait(bar(DT_WFULL), 0, ctl, W + 3);
+            int st = 0;
+            uint32_t ph = 0;
+            for (int i = 0; ok && i < ntiles; ++i) {
+                const int sb = i % kSB;
+                if (!mbar_wait(bar(DT_QFULL + st), ph, ctl, W + 4)) break;
+                if (!mbar_wait(bar(DT_SEMPTY + sb), ((uint32_t)(i / kSB) & 1u) ^ 1u, ctl, W + 5)) break;
+                tc_fence_after();
+                const uint64_t dq = dQ0 + st * kTokStep, dg = dG0 + st * kTokStep;
+                const uint32_t tS = tmem + kColS + sb * 128;
+#pragma unroll
+                for (int which = 0; which < 2; ++which)
+#pragma unroll
+                    for (int k = 0; k < DH / 16; ++k) {
+                        const int c = k >> 2, kk = k & 3;
+                        umma_ss(tS + which * kTT, (which ? dU : dK) + ((c * 2 * kWChunk + kk * 32) >> 4), dq + ((c * kWChunk + kk * 32) >> 4),
+                                idS, k > 0 ? 1u : 0u);
+                    }
+                umma_commit(bar(DT_SFULL + sb));
+                if (!mbar_wait(bar(DT_GFULL + st), ph, ctl, W + 4)) break;
+                if (!mbar_wait(bar(DT_DAEMPTY), (i & 1) ^ 1, ctl, W + 10)) break;
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < DH / 16; ++k) {
+                    const int c = k >> 2, kk = k & 3;
+                    umma_ss(tmem + kColdA, dV + ((c * 2 * kWChunk + kk * 32) >> 4), dg + ((c * kWChunk + kk * 32) >> 4), idS, k > 0 ? 1u : 0u);
+                }
+                umma_commit(bar(DT_GEMPTY + st));
+                umma_commit(bar(DT_DAFULL));
+                if (++st == L::kStages) { st = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------------------------ routing weights of each tile, times args.c
+        const int e_lo = row0 / args.De, e_hi = min((row0 + 64) / args.De, args.E - 1);
+        for (int i = 0; i < ntiles; ++i) {
+            int ts, hh, bb;
+            tile_coords(i, ts, hh, bb);
+            const float *src = args.R + (long long)bb * args.r_sb + (long long)hh * args.r_sh;
+            float v[2][2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int t = ts * kTT + k * 32 + lane;
+                v[0][k] = t < args.S ? args.c * __ldg(src + (long long)t * args.r_ss + e_lo) : 0.f;
+                v[1][k] = t < args.S ? args.c * __ldg(src + (long long)t * args.r_ss + e_hi) : 0.f;
+            }
+            const int slot = i % L::kRSlots;
+            if (!mbar_wait(bar(DT_REMPTY + slot), ((uint32_t)(i / L::kRSlots) & 1u) ^ 1u, ctl, W + 12)) break;
+            float *dst = rbuf + slot * 2 * kTT;
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int k = 0; k < 2; ++k) dst[x * kTT + k * 32 + lane] = v[x][k];
+            warp_arrive(bar(DT_RFULL + slot));
+        }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ MMA issuer 2: dV, dK, dU, their A operands in tensor memory
+        if (lane == 0) {
+            constexpr uint32_t idA = umma_idesc(128, DH, false, true);
+            const uint64_t dQ0 = desc_mnmajor(sTok, kWChunk), dG0 = desc_mnmajor(sTok + L::kTok, kWChunk);
+            constexpr uint64_t kTokStep = (2 * L::kTok) >> 4;
+            int st = 0;
+            bool ok = true;
+            for (int i = 0; i < ntiles; ++i) {
+                const int sb = i % kSB;
+                const uint32_t sph = (uint32_t)(i / kSB) & 1u;
+                const uint64_t dq = dQ0 + st * kTokStep, dg = dG0 + st * kTokStep;
+                const uint32_t tS = tmem + kColS + sb * 128;
+                // k step of 16 tokens = 8 columns; a thread's 32 tokens (two steps) lie together: see the element-wise warps
+                if (!mbar_wait(bar(DT_AFULL + sb), sph, ctl, W + 6)) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < kTT / 16; ++k) {
+                    const uint32_t a = kSB == 2 ? tS + (k >> 1) * 32 + (k & 1) * 8 : tmem + kColA + k * 8;
+                    umma_ts(tmem + kColAcc + 2 * DH, a, dg + k * 128, idA, (i > 0 || k > 0) ? 1u : 0u);
+                }
+                umma_commit(bar(DT_GEMPTY + st));
+                if (kSB == 1) umma_commit(bar(DT_AEMPTY));
+                if (!mbar_wait(bar(DT_PFULL + sb), sph, ctl, W + 6)) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < kTT / 16; ++k) {
+                    const uint32_t off = (k >> 1) * 32 + (k & 1) * 8;
+                    umma_ts(tmem + kColAcc, (kSB == 2 ? tS : tmem + kColdA) + off + (kSB == 2 ? 16 : 0), dq + k * 128, idA,
+                            (i > 0 || k > 0) ? 1u : 0u);
+                }
+#pragma unroll
+                for (int k = 0; k < kTT / 16; ++k) {
+                    const uint32_t off = (k >> 1) * 32 + (k & 1) * 8;
+                    umma_ts(tmem + kColAcc + DH, (kSB == 2 ? tS + kTT : tmem + kColdA + 16) + off, dq + k * 128, idA, (i > 0 || k > 0) ? 1u : 0u);
+                }
+                umma_commit(bar(DT_QEMPTY + st));
+                umma_commit(bar(kSB == 2 ? DT_SEMPTY + sb : (int)DT_DAEMPTY));
+                if (++st == L::kStages) st = 0;
+            }
+            if (ok) umma_commit(bar(DT_ACCFULL));
+        }
+    } else if (warp >= 4) {
+        // ------------------------------------------------------------------ element-wise math: lane = weight row, 32 tokens a thread
+        const int quarter = warp & 3, part = (warp - 4) >> 2;
+        const int row = quarter * 32 + lane;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+        const float *rsrc = rbuf + (quarter >> 1) * kTT + part * 32;
+        bool ok = true;
+        const DwConst kc = dw_const(args.s0);
+        for (int i = 0; i < ntiles; ++i) {
+            const int sb = i % kSB, slot = i % L::kRSlots;
+            if (!mbar_wait(bar(DT_RFULL + slot), (uint32_t)(i / L::kRSlots) & 1u, ctl, W + 13)) { ok = false; break; }
+            if (!mbar_wait(bar(DT_SFULL + sb), (uint32_t)(i / kSB) & 1u, ctl, W + 7)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t tS = lane_base + kColS + sb * 128 + part * 32, tA = lane_base + kColdA + part * 32;
+            const float *rs = rsrc + slot * 2 * kTT;
+            // first what needs only S: A goes out, and its dV update runs, while dA is still being computed
+            f32x2 fq[16], fw[16];
+            uint32_t pa[16];
+#pragma unroll
+            for (int sub = 0; sub < 2; ++sub) {
+                uint32_t m[16], n[16];
+                tmem_ld16x2_sync(tS + sub * 16, tS + kTT + sub * 16, m, n);
+                if (kSB == 1 && sub == 1) {   // S is in registers: the buffer can take the next tile
+                    tc_fence_before();
+                    warp_arrive(bar(DT_SEMPTY));
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 r4 = *reinterpret_cast<const float4 *>(rs + sub * 16 + q * 4);   // the same address in all lanes
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int x = q * 2 + u;
+                        const DwPair d = dw_pair(f2_pack_bits(m[2 * x], m[2 * x + 1]), f2_pack_bits(n[2 * x], n[2 * x + 1]),
+                                                 u ? f2_pack(r4.z, r4.w) : f2_pack(r4.x, r4.y), kc);
+                        fq[sub * 8 + x] = d.q;
+                        fw[sub * 8 + x] = d.w;
+                        pa[sub * 8 + x] = f2_to_bf16x2(d.a);
+                    }
+                }
+            }
+            warp_arrive(bar(DT_REMPTY + slot));
+            if (kSB == 1 && i >= 1) {
+                if (!mbar_wait(bar(DT_AEMPTY), (i - 1) & 1, ctl, W + 8)) { ok = false; break; }
+                tc_fence_after();
+            }
+            tmem_st16(kSB == 2 ? tS : lane_base + kColA + part * 16, pa);
+            tmem_st_wait();
+            tc_fence_before();
+            warp_arrive(bar(DT_AFULL + sb));
+            // then dM and dN
+            uint32_t da[32], pm[16], pn[16];
+            if (!mbar_wait(bar(DT_DAFULL), i & 1, ctl, W + 11)) { ok = false; break; }
+            tc_fence_after();
+            tmem_ld32_sync(tA, da);
+            if (kSB == 2) {
+                tc_fence_before();
+                warp_arrive(bar(DT_DAEMPTY));
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const f32x2 da2 = f2_pack_bits(da[2 * q], da[2 * q + 1]);
+                pm[q] = f2_to_bf16x2(f2_mul(da2, fw[q]));
+                pn[q] = f2_to_bf16x2(f2_mul(da2, fq[q]));
+            }
+            tmem_st16(kSB == 2 ? tS + 16 : tA, pm);
+            tmem_st16(kSB == 2 ? tS + kTT : tA + 16, pn);
+            tmem_st_wait();
+            tc_fence_before();
+            warp_arrive(bar(DT_PFULL + sb));
+        }
+        if (ok) ok = mbar_wait(bar(DT_ACCFULL), 0, ctl, W + 9);
+        if (ok) {
+            tc_fence_after();
+            const bool in_range = row0 + row < I;
+            const long long plane = (long long)args.Hkuv * I * DH;
+            constexpr int kColsPerHalf = DH / 2;
+            const int c0 = part * kColsPerHalf;
+#pragma unroll
+            for (int which = 0; which < 3; ++which) {
+                float *dst = args.ws + ((long long)split * 3 + which) * plane + ((long long)hk * I + row0 + row) * DH + c0;
+                __nv_bfloat16 *o16 = args.out[which] + hk * args.o_head[which] + (long long)(row0 + row) * args.o_row[which] + c0;
+#pragma unroll
+                for (int g = 0; g < kColsPerHalf / 16; ++g) {
+                    uint32_t o[16];
+                    tmem_ld16_sync(lane_base + kColAcc + which * DH + c0 + g * 16, o);
+                    if (in_range) dw_store16(args.nsplit == 1, dst + g * 16, o16 + g * 16, o);
                 }
             }
             tc_fence_before();
@@ -931,9 +1284,17 @@ double list_schedule(const std::vector<double> &jobs, int num_sms) {
     return end;
 }
 
-// What a CTA costs besides its token tiles (weights in, first tile through the pipeline, accumulators out), in token tiles
-// (about 1.9 us each): the intercept of kernel time over tiles per CTA, 7 us.
-constexpr double kDwFixed = 4.0;
+// How the weight-gradient kernel of a head dimension cuts its work, and what a CTA costs besides its token tiles (weights in,
+// first tile through the pipeline, accumulators out: the intercept of kernel time over tiles per CTA, about 7 us), a split's
+// extra launch (2.8 us) and a byte of partial sums (written once, read once, about 4 TB/s), all in units of one token tile.
+struct DwShape {
+    int rows, tokens;
+    double tile_us;
+    double fixed() const { return 7.0 / tile_us; }
+    double launch() const { return 2.8 / tile_us; }
+    double sums(double bytes) const { return bytes / 4.0e6 / tile_us; }
+};
+DwShape dw_shape(int dh) { return dh == 128 ? DwShape{kBI, kBT, 1.8} : DwShape{kTI, kTT, dh == 64 ? 0.8 : 1.0}; }
 
 // With a two-way split the CTAs are equal and their last wave is partly empty (704 CTAs on 148 SMs: the fifth wave is
 // 76 % full, 5 % of the kernel).  Splitting some blocks unevenly -- long parts launched first, short parts last, the
@@ -941,19 +1302,19 @@ constexpr double kDwFixed = 4.0;
 // The split point and the number of such blocks are found by simulating the launch order for a few candidates.
 // The partial sums still number two per block, so the reduction and the workspace do not change.
 // Returns the simulated duration (token tiles).
-double plan_uneven(DwPlan &p, long long items, int num_sms) {
+double plan_uneven(DwPlan &p, long long items, int num_sms, double fixed) {
     p.n_mixed = p.small_tiles = 0;
     const int T = p.tiles_total, half = p.tiles_per_split;
     auto makespan = [&](int nmix, int small) {
         std::vector<double> jobs;
         jobs.reserve((size_t)(2 * items));
-        for (int i = 0; i < nmix; ++i) jobs.push_back(T - small + kDwFixed);
-        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(half + kDwFixed);
-        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(T - half + kDwFixed);
-        for (int i = 0; i < nmix; ++i) jobs.push_back(small + kDwFixed);
+        for (int i = 0; i < nmix; ++i) jobs.push_back(T - small + fixed);
+        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(half + fixed);
+        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(T - half + fixed);
+        for (int i = 0; i < nmix; ++i) jobs.push_back(small + fixed);
         return list_schedule(jobs, num_sms);
     };
-    if (items > 2048 || T < 2) return (double)((2 * items + num_sms - 1) / num_sms) * (half + kDwFixed);
+    if (items > 2048 || T < 2) return (double)((2 * items + num_sms - 1) / num_sms) * (half + fixed);
     const double base = makespan(0, 0);
     if (T < 32) return base;
     double best = base;
@@ -971,22 +1332,23 @@ double plan_uneven(DwPlan &p, long long items, int num_sms) {
 }
 
 // How many ways to split the token axis: the one whose waves of CTAs (fixed cost + its token tiles each) plus the addition
-// of its partial sums are shortest.  Unsplit blocks write their bf16 results themselves; a split costs the reduction's
-// launch (1.5 tiles) and its fp32 sums, written once and read once through L2 (about 4 TB/s, i.e. 7.5 MB per tile time).
+// of its partial sums are shortest.  Unsplit blocks write their bf16 results themselves.
 DwPlan dw_plan(const flashmhf_dims &d, int num_sms) {
     struct Key { long long items, dh; int tiles_per_seq, tiles_total, num_sms; };
     struct Entry { Key k; DwPlan p; };
     static std::mutex mu;
     static std::vector<Entry> cache;
     const int G = d.H / d.Hkuv;
-    const long long items = (long long)d.Hkuv * ((long long)d.E * d.De / kBI);
-    const Key key{items, (long long)d.Dh, (d.S + kBT - 1) / kBT, ((d.S + kBT - 1) / kBT) * G * d.B, num_sms};
+    const DwShape sh = dw_shape(d.Dh);
+    const long long items = (long long)d.Hkuv * (((long long)d.E * d.De + sh.rows - 1) / sh.rows);
+    const int tps = (d.S + sh.tokens - 1) / sh.tokens;
+    const Key key{items, (long long)d.Dh, tps, tps * G * d.B, num_sms};
     std::lock_guard<std::mutex> lk(mu);
     for (const Entry &e : cache)
         if (e.k.items == key.items && e.k.dh == key.dh && e.k.tiles_per_seq == key.tiles_per_seq &&
             e.k.tiles_total == key.tiles_total && e.k.num_sms == key.num_sms)
             return e.p;
-    const double sum_tiles = (double)items * kBI * 3 * d.Dh * 4 / 7.5e6;   // one set of partial sums, in token-tile times
+    const double sum_tiles = sh.sums((double)d.Hkuv * d.E * d.De * 3 * d.Dh * 4);   // one set of partial sums
     DwPlan best{};
     double best_cost = 1e300;
     for (int ns = 1; ns <= 16 && ns <= key.tiles_total; ++ns) {
@@ -996,9 +1358,9 @@ DwPlan dw_plan(const flashmhf_dims &d, int num_sms) {
         p.tiles_per_split = (p.tiles_total + ns - 1) / ns;
         p.nsplit = (p.tiles_total + p.tiles_per_split - 1) / p.tiles_per_split;  // no empty split
         if (p.nsplit != ns) continue;
-        double cost = ns == 2 ? plan_uneven(p, items, num_sms)
-                              : (double)((items * ns + num_sms - 1) / num_sms) * (p.tiles_per_split + kDwFixed);
-        if (ns > 1) cost += 1.5 + ns * sum_tiles;
+        double cost = ns == 2 ? plan_uneven(p, items, num_sms, sh.fixed())
+                              : (double)((items * ns + num_sms - 1) / num_sms) * (p.tiles_per_split + sh.fixed());
+        if (ns > 1) cost += sh.launch() + ns * sum_tiles;
         if (cost < best_cost - 1e-9) { best_cost = cost; best = p; }
     }
     if (cache.size() < 256) cache.push_back(Entry{key, best});
@@ -1060,7 +1422,10 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         if (!done[dc->device].load(std::memory_order_acquire)) {
             e = cudaFuncSetAttribute(bwd_dq_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DqSmem<DH>::kTotal);
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(bwd_dw_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DwSmem<DH>::kTotal);
+                if constexpr (DH == 128)
+                    e = cudaFuncSetAttribute(bwd_dw_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DwSmem<DH>::kTotal);
+                else
+                    e = cudaFuncSetAttribute(bwd_dwt_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DwtSmem<DH>::kTotal);
             if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(bwd kernels)"); return FLASHMHF_ERR_CUDA; }
             done[dc->device].store(true, std::memory_order_release);
         }
@@ -1085,16 +1450,24 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         ra.DH = DH;
         ra.plane = (long long)d.Hkuv * ra.I * DH;
         ra.nsplit = pl.nsplit;
+        const int nblk_j = (d.E * d.De + dw_shape(DH).rows - 1) / dw_shape(DH).rows;
         DwArgs wa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
                   static_cast<float *>(p.workspace), {ra.out[0], ra.out[1], ra.out[2]}, {ra.s_head[0], ra.s_head[1], ra.s_head[2]},
                   {ra.s_row[0], ra.s_row[1], ra.s_row[2]}, d.S, d.E, d.De, G, d.B, d.Hkuv,
                   pl.tiles_per_seq, pl.tiles_total, pl.tiles_per_split,
-                  d.E * d.De / kBI, d.Hkuv * (d.E * d.De / kBI), pl.nsplit, pl.n_mixed, pl.small_tiles, s0, 0.5f * c, wait_args(dc)};
+                  nblk_j, d.Hkuv * nblk_j, pl.nsplit, pl.n_mixed, pl.small_tiles, s0, 0.5f * c, wait_args(dc)};
         const long long ctas = (long long)wa.n_blocks * pl.nsplit;
         if (ctas > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
         dim3 gw((unsigned)ctas);
         prof_mark(st, kMarkStart);
-        bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, wa);
+        if constexpr (DH == 128) {
+            bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, wa);
+        } else {
+            CUtensorMap tmQt, tmdOt;
+            if ((rc = encode_act_map(&tmQt, p.Q, d, kTT)) != 0) return rc;
+            if ((rc = encode_act_map(&tmdOt, p.dO, d, kTT)) != 0) return rc;
+            bwd_dwt_kernel<DH><<<gw, kThreads, DwtSmem<DH>::kTotal, st>>>(tmQt, tmdOt, tmK, tmU, tmV, wa);
+        }
         prof_mark(st, kMarkBwdDw);
         *n_launch += 1;
         if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "bwd_dw_kernel launch"); return FLASHMHF_ERR_CUDA; }
