@@ -4,25 +4,26 @@
 //   dR_e = rowsum(dA*s*N), dM = dA*(r*N)*(sg + s*(1-sg)), dN = dA*s*r, A = s*N*r
 //   dQ += dM K + dN U ;  dK = sum_t dM^T Q ;  dU = sum_t dN^T Q ;  dV = sum_t A^T dO
 //
-// Two kernels, each the sole owner of its accumulators (no floating-point atomics, bit-reproducible):
+// Three kernels, each the sole owner of its accumulators (no floating-point atomics, bit-reproducible):
 //
 // bwd_dq_kernel  -- token-stationary.  One CTA owns 128 token rows of one (batch, head): its Q and dO
 //   tiles are copied once into tensor memory and all three MMA chains read their A operand from there,
-//   the head's weights stream through shared memory (K/U ring of 3, V ring of 2).
+//   the head's weights stream through shared-memory rings (the first lap shares them with the Q and dO tiles).
 //   Tensor memory: dQ accumulator (128 cols), Q and dO as bf16 (64 + 64), S = [M|N] (128), dA (64), and the
 //   bf16 [dM|dN] operand of the dQ update (64).  Produces dQ (TMA store) and dR (direct stores).
 //
-// bwd_dw_kernel  -- weight-stationary.  One CTA owns one 64-row block of K, U and V of one K/U/V
+// bwd_dw_kernel (d_h = 128)  -- weight-stationary.  One CTA owns one 64-row block of K, U and V of one K/U/V
 //   head and a contiguous range of token tiles (the token axis is split `nsplit` ways to fill the
 //   machine).  Weights stay in shared memory, {Q, dO} tiles stream through a ring of 2.
-//   Tensor memory: [dK;dU] accumulator (128 lanes), dV accumulator (transposed, d_h x 64, when d_h = 128; else
-//   M = 64), two S buffers and one dA buffer (the element-wise warps copy dA to registers first and hand it
-//   back at once), so that the recompute of tile i+1 runs under the element-wise math of tile i.
-//   Each CTA writes fp32 partial sums to the workspace; dw_reduce_kernel adds the splits in a fixed
-//   order and writes bf16 dK, dU, dV.
+//   Tensor memory: [dK;dU] accumulator (128 lanes), dV accumulator (transposed, d_h x 64), two S buffers and one dA
+//   buffer, so that the recompute of tile i+1 runs under the element-wise math of tile i.
+// bwd_dwt_kernel (d_h = 64, 96)  -- the same with 128 weight rows per CTA and the recompute transposed.
+//   With more than one split each CTA writes fp32 partial sums to the workspace; dw_reduce_kernel adds the splits in a
+//   fixed order and writes bf16 dK, dU, dV.
 //
-// Both use 384 threads: warp 0 TMA producer, warps 1 and 3 MMA issuers (one per MMA chain; warp 1 owns
-// tensor memory), warps 4-11 element-wise math (warp % 4 = TMEM lane quarter, (warp-4)/4 = which 32 of the 64 block columns).
+// All use 384 threads: warp 0 TMA producer, warps 1 to 3 MMA issuers (one per MMA chain; warp 1 owns tensor memory; warp 2
+// of bwd_dwt_kernel fetches routing weights), warps 4-11 element-wise math (warp % 4 = TMEM lane quarter, (warp-4)/4 =
+// which half of the columns).
 #include <atomic>
 #include <mutex>
 #include <queue>
@@ -35,13 +36,10 @@
 namespace fmhf {
 namespace {
 
-#ifndef FMHF_BWD_PARTS
-#define FMHF_BWD_PARTS 2
-#endif
 // Element-wise warps: 4 lane quarters x kParts column parts of a 64-column block (a thread = one token row x
 // kCols columns).  More, narrower threads shorten the arithmetic phase of a block; the fixed part of a block's
-// element-wise step (barrier waits, tensor-memory load and store latencies) does not shrink.
-constexpr int kParts = FMHF_BWD_PARTS, kCols = 64 / kParts, kSubs = kCols / 16;
+// element-wise step (barrier waits, tensor-memory load and store latencies) does not shrink: four parts are 2-4 % slower.
+constexpr int kParts = 2, kCols = 64 / kParts, kSubs = kCols / 16;
 constexpr int kBT = 128, kBI = 64, kActThreads = 128 * kParts, kThreads = 128 + kActThreads;
 constexpr int kEpiThreads = 256;  // the warps of column parts 0 and 1 write the accumulators out
 constexpr uint32_t kTmemCols = 512;
@@ -486,8 +484,7 @@ struct DwSmem {
     static constexpr uint32_t kWBytes = 3 * kChunks * kWChunk;  // [K;U] chunks then V chunks
     static constexpr uint32_t kOffWV = 2 * kChunks * kWChunk;
     static constexpr uint32_t kTokStage = 2 * kChunks * kTile;  // Q chunks then dO chunks
-    // token stages: what is left beside the resident weights and the staged operands (two at 96 and 128 columns)
-    static constexpr int kTokStages = DH == 64 ? 4 : 2;
+    static constexpr int kTokStages = 2;   // what is left beside the resident weights and the staged operands
     static constexpr uint32_t kOffW = 0;
     static constexpr uint32_t kOffTok = kOffW + kWBytes;
     static constexpr uint32_t kOffP = kOffTok + kTokStages * kTokStage;  // [dM | dN] : 2 x 16 KB
@@ -503,8 +500,8 @@ struct DwSmem {
 // phase of the barrier it waits on (a one-bit parity cannot tell phase k from phase k+2).
 // That loop over two stages is what bounds the kernel, so the element-wise step is cut in two: A and the factors of dM, dN need
 // only S; A goes out first and its dV update runs while dA is still being computed.  (One step behind S and dA before: the
-// 370M layer at 32768 tokens 1.07 -> 1.04 ms burst, 1.21 -> 1.18 sustained; 16 x 16 x 192 at d_h = 64, 16384 tokens 0.876 -> 0.794.)
-constexpr int kMaxTok = 4;
+// 370M layer at 32768 tokens 1.07 -> 1.04 ms burst, 1.21 -> 1.18 sustained.)
+constexpr int kMaxTok = 2;
 enum { DW_WFULL = 0, DW_SFULL = 1, DW_SEMPTY = 3, DW_PFULL = 5, DW_AFULL = 6, DW_PEMPTY = 7, DW_AEMPTY = 8, DW_ACCFULL = 9, DW_DAFULL = 10,
        DW_DAEMPTY = 11, DW_QFULL = 12, DW_GFULL = DW_QFULL + kMaxTok, DW_QEMPTY = DW_GFULL + kMaxTok, DW_GEMPTY = DW_QEMPTY + kMaxTok,
        DW_BARS = DW_GEMPTY + kMaxTok };
@@ -581,13 +578,12 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const int ntiles = tile_end - tile_begin;  // >= 1 by construction of the plan
     const WaitCtl ctl{abort_flag, args.wait};
     constexpr int W = kKernelBwdDw * 100;
-    // dV^T = sum_t dO^T A (d_h x 64, M = 128, N = 64) needs half the columns and three quarters of the tensor-pipe
-    // time of dV = sum_t A^T dO (M = 64 runs at the M = 128 rate); it needs M = d_h = 128.
-    constexpr bool kVt = DH == 128;
-    // Columns: [dK;dU] at 0 (d_h wide), dV at 128 (64 wide transposed, else d_h wide), S buffers at 256 and 384, dA in
-    // the gap at 192.  d_h = 96 leaves no gap (dV reaches column 224): it keeps one S buffer, with dA at 384.
-    constexpr int kSB = DH == 96 ? 1 : 2;
-    constexpr uint32_t kColKU = 0, kColV = 128, kColS = 256, kColdA = kSB == 2 ? 192 : 384;
+    // dV is accumulated transposed, dV^T = sum_t dO^T A (d_h x 64: M = 128, N = 64): half the columns and three quarters of the
+    // tensor-pipe time of dV = sum_t A^T dO (M = 64 runs at the M = 128 rate).
+    static_assert(DH == 128, "the narrower head dimensions have a kernel of their own");
+    constexpr int kSB = 2;
+    // Columns: [dK;dU] at 0, dV^T at 128 (64 wide), dA at 192, S buffers at 256 and 384.
+    constexpr uint32_t kColKU = 0, kColV = 128, kColS = 256, kColdA = 192;
 
     auto tile_coords = [&](int i, int &ts, int &hh, int &bb) {  // token tile i of this CTA -> (seq tile, head, batch)
         const int ti = tile_begin + i;
@@ -706,7 +702,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         // MMA issuer 2: the accumulation chain [dK;dU] += [dM|dN]^T Q, dV += A^T dO.
         if (lane == 0) {
             constexpr uint32_t idKU = umma_idesc(128, DH, true, true);
-            constexpr uint32_t idV = kVt ? umma_idesc(128, kBI, true, true) : umma_idesc(64, DH, true, true);
+            constexpr uint32_t idV = umma_idesc(128, kBI, true, true);
             const uint64_t dQmn0 = desc_mnmajor(sTok, kTile), dGmn0 = desc_mnmajor(sTok + L::kChunks * kTile, kTile),
                            dPmn = desc_mnmajor(sP, kTile), dAmn = desc_mnmajor(sA, kTile);
             constexpr uint64_t kTokStep = L::kTokStage >> 4;
@@ -717,10 +713,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 if (!mbar_wait(bar(DW_AFULL), i & 1, ctl, W + 6)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < kBT / 16; ++k) {
-                    if (kVt) umma_ss(tmem + kColV, dg + k * 128, dAmn + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
-                    else umma_ss(tmem + kColV, dAmn + k * 128, dg + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
-                }
+                for (int k = 0; k < kBT / 16; ++k)
+                    umma_ss(tmem + kColV, dg + k * 128, dAmn + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
                 umma_commit(bar(DW_GEMPTY + st));  // dO of this stage (once its dA is computed too) and the A tile are free
                 umma_commit(bar(DW_AEMPTY));
                 if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
@@ -839,7 +833,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     dw_store16(direct, dst + g * 16, o16 + g * 16, o);
                 }
             }
-            if (kVt) {  // dV^T: lane = column d of dV, tensor-memory column = row of the block; a warp stores 32 consecutive elements per row
+            {   // dV^T: lane = column d of dV, tensor-memory column = row of the block; a warp stores 32 consecutive elements per row
                 float *dst = wsb + 2 * plane + row;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
@@ -853,16 +847,6 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
                         for (int v = 0; v < 16; ++v) dst[(long long)(r0 + v) * DH] = __uint_as_float(o[v]);
                     }
-                }
-            } else {    // dV (M = 64 accumulator): row r lives in TMEM lane 32*(r/16) + r%16
-                const int r = quarter * 16 + (lane & 15);
-                float *dst = wsb + 2 * plane + (long long)r * DH + c0;
-                __nv_bfloat16 *o16 = out_row(2, r) + c0;
-#pragma unroll
-                for (int g = 0; g < kColsPerHalf / 16; ++g) {
-                    uint32_t o[16];
-                    tmem_ld16_sync(lane_base + kColV + c0 + g * 16, o);
-                    if (lane < 16) dw_store16(direct, dst + g * 16, o16 + g * 16, o);
                 }
             }
             tc_fence_before();
@@ -892,7 +876,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // come out such that dM^T, dN^T and A^T, written back to tensor memory as bf16, are the A operands of
 //     dK += dM^T Q,  dU += dN^T Q,  dV += A^T dO     (128 x d_h each).
 // Nothing is staged in shared memory, the accumulating products read only their B operand there, and a token tile serves twice as
-// many weight rows: 112 KB (d_h = 64) instead of 231 KB per block.
+// many weight rows: 112 KB (d_h = 64) instead of 231 KB per block.  Measured against the other form: 16 x 16 x 192 at d_h = 64,
+// 16384 tokens, 0.795 -> 0.697 ms; 128M layer (d_h = 96), 16384 tokens, 0.377 -> 0.342 ms.
 // Tensor memory: three accumulators of d_h columns; d_h = 64: two buffers of [M^T | N^T] (128 columns), whose columns A^T, dM^T and
 // dN^T later take, and dA^T; d_h = 96: one [M^T | N^T], given back as soon as it is in registers, dA^T, over which dM^T and dN^T
 // are written, and 32 columns for A^T.  (d_h = 128 would need 576 columns.)
