@@ -141,8 +141,10 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdArgs &a, int item, int nblk
     return w;
 }
 
+// Registers: d_h = 128 at most 152, so that a 128-thread CTA of the split reduction (48 registers) fits beside this one on an SM and is
+// resident when it ends; at 154 (allocated as 160) it is not, and a chained 1.3B decode step takes 23.0 instead of 21.9 us.
 template <int DH>
-__global__ void __launch_bounds__(threads_for(DH), 1)
+__global__ void __maxnreg__(DH == 128 ? 152 : 96)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV,
            const __grid_constant__ CUtensorMap tmO, const FwdArgs args) {
@@ -192,7 +194,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const bool dead = *abort_flag != 0;
-    griddep_launch_dependents();   // every CTA of this launch is running: what follows (the reduction, a chained call) may start
+    griddep_launch_dependents();   // every CTA of this launch is running: what follows (the reduction, the next call) may start
+    // Every launch may start under the end of the kernel before it (a decode step of 8 tokens of the 370M layer 12.3 -> 9.6 us a call);
+    // until that kernel has ended only a chained call's producer touches global memory (weight tiles), the others wait below.
 
     if (dead) {
         // nothing: fall through to the teardown
@@ -203,6 +207,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             tma_prefetch_desc(&tmK);
             tma_prefetch_desc(&tmU);
             tma_prefetch_desc(&tmV);
+            if (!args.chained) griddep_wait();
             RingPos<kKURing> pk;
             RingPos<kVRing> pv;
             bool ok = true;
@@ -321,8 +326,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         const f32x2 half_s0 = f2_pack(args.half_s0, args.half_s0);
         bool ok = true;
         int g0 = 0, n = 0;   // blocks before this work item; work items so far
+        griddep_wait();   // these warps read R and write O
         if (args.chained) {
-            griddep_wait();   // these warps read R and write O
             if (warp == 4 && lane == 0 && blockIdx.x < args.n_items) {   // the first item's Q (q.v. the producer)
                 const FwdItem w = fwd_item(args, blockIdx.x, nblk_total);
                 mbar_arrive_expect_tx(bar(BAR_QFULL), L::kQBytes);
@@ -474,14 +479,13 @@ struct OReduceArgs {
     __nv_bfloat16 *O;
     long long s_b, s_h, s_s;
     int nsplit, H, S, DH;
-    int chained;   // between two chained forward kernels: lets the next one start
 };
 // Measured (one B200): a decode step of 8 tokens of the 370M layer 14.4 -> 12.3 us, of 64 chained tokens 12.0 -> 10.0, against a loop
 // that had three splits of two pieces in flight whatever the grid.
 // 128 threads and few registers: its CTAs fit beside the forward kernel's on an SM, so a chained launch is resident (and
 // has let the next forward launch in turn) long before the forward kernel it waits for ends.
 __global__ void __maxnreg__(48) o_reduce_kernel(const OReduceArgs a) {
-    if (a.chained) griddep_launch_dependents();
+    griddep_launch_dependents();
     griddep_wait();   // launched early, behind the kernel whose partial sums it adds
     // Eight 16-byte loads of a thread are in flight (the partial sums come from L2 while the next call's weights stream in from
     // HBM: latency is what this kernel is made of): eight splits of one piece of O, or, where the grid is too small to give every
@@ -490,7 +494,7 @@ __global__ void __maxnreg__(48) o_reduce_kernel(const OReduceArgs a) {
     const int n4 = (int)(a.plane / 4), stride = (int)(gridDim.x * blockDim.x);
     const float4 *part4 = reinterpret_cast<const float4 *>(a.part);
     auto add = [](float4 &acc, const float4 &v) { acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; };
-    auto at = [&](int s, int idx) { return __ldcg(part4 + (long long)min(s, a.nsplit - 1) * n4 + idx); };
+    auto at = [&](int s, int idx) { return __ldcg(part4 + (unsigned)(min(s, a.nsplit - 1) * n4 + idx)); };
     auto store = [&](int idx, const float4 &acc) {
         const int per_row = a.DH / 4;
         const int r1 = idx / per_row, c = (idx - r1 * per_row) * 4;
@@ -585,7 +589,7 @@ int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, boo
     // (a split call has one item per CTA: tiles * splits <= SMs)
     const unsigned grid = (unsigned)(items < dc->num_sms ? items : dc->num_sms);
     prof_mark(st, kMarkStart);
-    cudaError_t e = launch_kernel(chained, fwd_kernel<DH>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
+    cudaError_t e = launch_kernel(true, fwd_kernel<DH>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
     prof_mark(st, kMarkFwd);
     *n_launch += 1;
     if (e != cudaSuccess) { set_cuda_error(e, "fwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
@@ -605,7 +609,7 @@ cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const
                             cudaStream_t st) {
     const long long plane = (long long)d.B * d.H * d.S * d.Dh, n4 = plane / 4;
     const OReduceArgs ra{part, plane, static_cast<__nv_bfloat16 *>(out.ptr), out.stride[0], out.stride[1], out.stride[2], nsplit, d.H, d.S,
-                         d.Dh, mode == kReduceChained ? 1 : 0};
+                         d.Dh};
     // chained: at most one (small) CTA per SM, so that all of them are resident beside the forward kernel's
     const long long cap = mode == kReduceChained ? (long long)num_sms : (long long)num_sms * 8;
     const int blocks = (int)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap);
