@@ -12,6 +12,7 @@
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <dlfcn.h>
 #include <torch/extension.h>
@@ -181,15 +182,18 @@ Tensor scratch(const std::optional<Tensor> &given, size_t nbytes, const Tensor &
 }
 
 // ------------------------------------------------------------------------------------------------ operator
-// The call itself, from addresses and strides.
-void launch_forward(flashmhf_fwd_params &p, const Tensor &like, bool chained, const std::optional<Tensor> &workspace) {
+// The call itself, from addresses and strides: how much scratch it needs, and the launch.
+void as_sequence(flashmhf_fwd_params &p) {
     if (p.d.S == 1 && p.d.B > 1) {
         p.Q = tokens_as_sequence(p.Q); p.R = tokens_as_sequence(p.R); p.O = tokens_as_sequence(p.O);
         p.d.S = p.d.B;
         p.d.B = 1;
     }
-    Tensor ws;
     p.workspace_bytes = api.forward_ws(&p.d);
+}
+void launch_forward(flashmhf_fwd_params &p, const Tensor &like, bool chained, const std::optional<Tensor> &workspace) {
+    as_sequence(p);
+    Tensor ws;
     if (p.workspace_bytes) {
         ws = scratch(workspace, p.workspace_bytes, like);
         p.workspace = ws.data_ptr();
@@ -349,14 +353,17 @@ flashmhf_prologue_params prologue_params(const Prologue &a) {
 }
 int32_t dtype_code(const Tensor &param) { return param.scalar_type() == at::kBFloat16 ? FLASHMHF_BF16 : FLASHMHF_F32_CHECK; }
 // Q [B,S,H*d_h] in the activations' own layout (the activations themselves without RMSNorm) and R [B,H,S,E]
+void launch_prologue(const Prologue &a, void *q, void *R) {
+    flashmhf_prologue_params p = prologue_params(a);
+    p.Q = q;
+    p.R = static_cast<float *>(R);
+    check(api.prologue_forward(&p, dtype_code(a.r), current_stream(a.x)));
+}
 std::pair<Tensor, Tensor> run_prologue(const Prologue &a) {
     c10::cuda::CUDAGuard guard(a.x.device());
     Tensor q = a.w.defined() ? at::empty_like(a.x) : a.x;
     Tensor R = at::empty({a.B, a.H, a.S, a.E}, a.x.options().dtype(at::kFloat));
-    flashmhf_prologue_params p = prologue_params(a);
-    p.Q = q.data_ptr();
-    p.R = R.data_ptr<float>();
-    check(api.prologue_forward(&p, dtype_code(a.r), current_stream(a.x)));
+    launch_prologue(a, q.data_ptr(), R.data_ptr());
     return {q, R};
 }
 struct PrologueGrads {
@@ -452,35 +459,71 @@ Shape layer_shape(const Prologue &a, const Tensor &gate, const Tensor &up, const
         throw py::value_error("flash_mhf runs on CUDA tensors of one device; there is no CPU path");
     return Shape{a.B, a.H, a.S, a.Dh, Hkuv, a.E, I / a.E};
 }
+// x [B,S,n] times w^T: one product on the flattened rows (at::linear takes more steps to the same call)
+Tensor project(const Tensor &x, const Tensor &w, const std::optional<Tensor> &b) {
+    if (b || !x.is_contiguous()) return at::linear(x, w, b);
+    return at::mm(x.view({x.size(0) * x.size(1), x.size(2)}), w.t()).view({x.size(0), x.size(1), w.size(0)});
+}
+struct LayerForward {
+    Prologue a;
+    Tensor q, R, O, y;   // q and R only where they are to be kept for a backward
+};
+LayerForward layer_forward(const Tensor &x, const std::optional<Tensor> &w1, const std::optional<Tensor> &b1,
+                           const std::optional<Tensor> &q_norm, const Tensor &router, const Tensor &gate, const Tensor &up,
+                           const Tensor &down, const std::optional<Tensor> &w2, const std::optional<Tensor> &b2, int64_t Hkuv, double eps,
+                           double hs, double us, double fs, bool keep) {
+    at::AutoDispatchBelowADInplaceOrView below;   // nothing in here is recorded: the caller is the autograd node, or there is none
+    c10::cuda::CUDAGuard guard(x.device());
+    LayerForward f{prologue_args(w1 ? project(x, *w1, b1) : x, q_norm, router, eps)};
+    const Prologue &a = f.a;
+    const Shape s = layer_shape(a, gate, up, down, Hkuv);
+    f.O = at::empty_like(a.x);
+    flashmhf_fwd_params p{};
+    p.d = dims_of(s, at::kBFloat16);
+    p.scale = scaling_of(hs, us, fs);
+    p.K = expert_address(gate, s.Dh, s.De); p.U = expert_address(up, s.Dh, s.De); p.V = expert_address(down, s.Dh, s.De);
+    p.O = heads_address(f.O.data_ptr(), a);
+    if (keep) {
+        std::tie(f.q, f.R) = run_prologue(a);
+        p.Q = heads_address(f.q.data_ptr(), a); p.R = routing_address(f.R.data_ptr(), a);
+        launch_forward(p, a.x, false, std::nullopt);
+    } else {   // Q, R and the operator's scratch in one allocation
+        flashmhf_fwd_params need = p;
+        as_sequence(need);
+        const size_t q_bytes = a.w.defined() ? align256((size_t)a.B * a.S * a.H * a.Dh * 2) : 0, r_bytes = align256((size_t)a.B * a.S * a.H * a.E * 4);
+        const Tensor tmp = at::empty({(int64_t)(q_bytes + r_bytes + need.workspace_bytes)}, a.x.options().dtype(at::kByte));
+        char *base = static_cast<char *>(tmp.data_ptr());
+        void *q = q_bytes ? base : a.x.data_ptr();
+        launch_prologue(a, q, base + q_bytes);
+        p.Q = heads_address(q, a); p.R = routing_address(base + q_bytes, a);
+        as_sequence(p);
+        p.workspace = p.workspace_bytes ? base + q_bytes + r_bytes : nullptr;
+        check(api.forward(&p, current_stream(a.x)));
+    }
+    f.y = w2 ? project(f.O, *w2, b2) : f.O;
+    return f;
+}
+
 struct LayerFunction : public torch::autograd::Function<LayerFunction> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x, const std::optional<Tensor> &w1, const std::optional<Tensor> &b1,
                           const std::optional<Tensor> &q_norm, const Tensor &router, const Tensor &gate, const Tensor &up,
                           const Tensor &down, const std::optional<Tensor> &w2, const std::optional<Tensor> &b2, int64_t Hkuv, double eps,
                           double hs, double us, double fs) {
-        const Prologue a = prologue_args(w1 ? at::linear(x, *w1, b1) : x, q_norm, router, eps);
-        const Shape s = layer_shape(a, gate, up, down, Hkuv);
-        const flashmhf_scaling sc = scaling_of(hs, us, fs);
-        auto [q, R] = run_prologue(a);
-        const Tensor O = at::empty_like(a.x);
-        {
-            c10::cuda::CUDAGuard guard(x.device());
-            flashmhf_fwd_params p{};
-            p.d = dims_of(s, at::kBFloat16);
-            p.Q = heads_address(q.data_ptr(), a); p.O = heads_address(O.data_ptr(), a); p.R = routing_address(R.data_ptr(), a);
-            p.K = expert_address(gate, s.Dh, s.De); p.U = expert_address(up, s.Dh, s.De); p.V = expert_address(down, s.Dh, s.De);
-            p.scale = sc;
-            launch_forward(p, a.x, false, std::nullopt);
-        }
+        const LayerForward f = layer_forward(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs, true);
+        const Prologue &a = f.a;
+        const Tensor &q = f.q, &R = f.R, &O = f.O;
         ctx->save_for_backward({w1 ? x : Tensor(), w1 ? *w1 : Tensor(), a.x, a.w, a.r, q, R, gate, up, down, w2 ? O : Tensor(),
                                 w2 ? *w2 : Tensor()});
         ctx->saved_data["k"] = std::vector<double>{eps, hs, us, fs};
         ctx->saved_data["i"] = std::vector<int64_t>{Hkuv, (int64_t)router.scalar_type(), q_norm ? (int64_t)q_norm->scalar_type() : (int64_t)-1,
                                                     (int64_t)b1.has_value(), (int64_t)b2.has_value()};
-        return w2 ? at::linear(O, *w2, b2) : O;
+        return f.y;
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         variable_list out(15);
         if (!grads[0].defined()) return out;
+        std::optional<at::AutoDispatchBelowADInplaceOrView> below;
+        if (!at::GradMode::is_enabled()) below.emplace();
         const variable_list sv = ctx->get_saved_variables();
         const std::vector<double> k = ctx->saved_data["k"].toDoubleVector();
         const std::vector<int64_t> n = ctx->saved_data["i"].toIntVector();
@@ -544,7 +587,13 @@ Tensor mhffn_layer(const Tensor &x, const std::optional<Tensor> &w1, const std::
                    const std::optional<Tensor> &b2, int64_t Hkuv, double eps, double hs, double us, double fs) {
     auto plain = [](const std::optional<Tensor> &t) { return !t || t->scalar_type() == at::kBFloat16; };
     if (x.dim() == 3 && expert_ok(gate) && expert_ok(up) && expert_ok(down) && plain(x) && plain(w1) && plain(b1) && plain(w2) && plain(b2) && !at::autocast::is_autocast_enabled(at::kCUDA))
-        return LayerFunction::apply(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs);
+    {
+        auto wants = [](const std::optional<Tensor> &t) { return t && t->requires_grad(); };
+        if (at::GradMode::is_enabled() && (wants(x) || wants(w1) || wants(b1) || wants(q_norm) || wants(router) || wants(gate) || wants(up) ||
+                                           wants(down) || wants(w2) || wants(b2)))
+            return LayerFunction::apply(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs);
+        return layer_forward(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs, false).y;
+    }
     // other dtypes, autocast, or weights that have to be copied first: torch's own rules for each step
     auto [Q, R] = fused_prologue(w1 ? at::linear(x, *w1, b1) : x, q_norm, router, eps);
     const int64_t E = router.size(2);
