@@ -238,6 +238,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 prologue_fwd_mma_kernel(const ProArgs a, __nv_bfloat16 *Q, float *R) {
     using L = MmaLayout<DH, NT>;
     extern __shared__ __align__(16) uint8_t smem_mma[];
+    // the operator's forward kernel behind this one may start where SMs are free, and stream weights, which nothing here writes
+    griddep_launch_dependents();
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     build_router_fragments<DH, NT, false>(a, h, smem_mma);
     float *wsm = reinterpret_cast<float *>(smem_mma + L::kOffW);

@@ -483,10 +483,11 @@ LayerForward layer_forward(const Tensor &x, const std::optional<Tensor> &w1, con
     p.scale = scaling_of(hs, us, fs);
     p.K = expert_address(gate, s.Dh, s.De); p.U = expert_address(up, s.Dh, s.De); p.V = expert_address(down, s.Dh, s.De);
     p.O = heads_address(f.O.data_ptr(), a);
+    // (chained: the operation directly before the operator is this layer's prologue, which does not write the weights)
     if (keep) {
         std::tie(f.q, f.R) = run_prologue(a);
         p.Q = heads_address(f.q.data_ptr(), a); p.R = routing_address(f.R.data_ptr(), a);
-        launch_forward(p, a.x, false, std::nullopt);
+        launch_forward(p, a.x, true, std::nullopt);
     } else {   // Q, R and the operator's scratch in one allocation
         flashmhf_fwd_params need = p;
         as_sequence(need);
@@ -498,7 +499,7 @@ LayerForward layer_forward(const Tensor &x, const std::optional<Tensor> &w1, con
         p.Q = heads_address(q, a); p.R = routing_address(base + q_bytes, a);
         as_sequence(p);
         p.workspace = p.workspace_bytes ? base + q_bytes + r_bytes : nullptr;
-        check(api.forward(&p, current_stream(a.x)));
+        check(api.forward_chained(&p, current_stream(a.x)));
     }
     f.y = w2 ? project(f.O, *w2, b2) : f.O;
     return f;
