@@ -688,6 +688,20 @@ std::pair<Tensor, Tensor> rotary_pair(const Tensor &q, const Tensor &k, const Te
     return {o[0], o[1]};
 }
 
+// Self-attention of the LM without gradients: projections, rotary embedding, library attention, projection (the steps of
+// lm.Attention.forward; a forward pass over a short input waits for the interpreter, not for the GPU).
+Tensor lm_attention(const Tensor &x, const Tensor &wq, const Tensor &wk, const Tensor &wv, const Tensor &wo, int64_t nh, int64_t nkv,
+                    const Tensor &cos_t, const Tensor &sin_t) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const int64_t B = x.size(0), S = x.size(1), hd = wq.size(0) / nh;
+    auto heads = [&](const Tensor &w, int64_t n) { return project(x, w, std::nullopt).view({B, S, n, hd}); };
+    const Tensor q = heads(wq, nh), k = heads(wk, nkv), v = heads(wv, nkv).transpose(1, 2);
+    const variable_list r = run_rope_pair(q, k, cos_t, sin_t, false);
+    const Tensor o = at::scaled_dot_product_attention(r[0].transpose(1, 2), r[1].transpose(1, 2), v, std::nullopt, 0.0, /*is_causal=*/true,
+                                                      std::nullopt, /*enable_gqa=*/nkv != nh);
+    return project(o.transpose(1, 2).reshape({B, S, nh * hd}), wo, std::nullopt);
+}
+
 // (h + d, RMSNorm(h + d) * weight)
 struct AddRMSNormFunction : public torch::autograd::Function<AddRMSNormFunction> {
     static variable_list forward(AutogradContext *ctx, const Tensor &h0, const Tensor &d0, const Tensor &weight, double eps) {
@@ -734,6 +748,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("fused_prologue", torch::wrap_pybind_function(fused_prologue));
     m.def("mhffn_layer", torch::wrap_pybind_function(mhffn_layer));
     m.def("rotary", torch::wrap_pybind_function(rotary));
+    m.def("lm_attention", torch::wrap_pybind_function(lm_attention));
     m.def("rotary_pair", torch::wrap_pybind_function(rotary_pair));
     m.def("add_rmsnorm", torch::wrap_pybind_function(add_rmsnorm));
     m.def("rmsnorm", torch::wrap_pybind_function(rmsnorm));

@@ -29,6 +29,11 @@ def rotary_pair(q, k, cos_t, sin_t):
     return _lib.native().rotary_pair(q, k, cos_t, sin_t)
 
 
+def attention(x, wq, wk, wv, wo, num_heads, num_kv_heads, cos_t, sin_t):
+    """Causal self-attention of x [B,S,hidden] bf16 with rotary embedding, without gradients (lm.Attention.forward's steps)."""
+    return _lib.native().lm_attention(x, wq, wk, wv, wo, num_heads, num_kv_heads, cos_t, sin_t)
+
+
 def add_rmsnorm(h, d, weight, eps):
     """(h + d, RMSNorm(h + d) * weight) for bf16 [..., n], n in NORM_SIZES, in one pass."""
     return _lib.native().add_rmsnorm(h, d, weight, eps)

@@ -48,3 +48,19 @@ def test_add_rmsnorm_equals_addition_then_norm(rows, n, wdt, use_sum):
     for p, q in zip(a, b):
         assert orc.rel_l2(p.grad.float(), q.grad.float()) < 4e-3
     assert torch.equal(a[2].grad, b[2].grad)
+
+
+@pytest.mark.parametrize("B,S,kv", [(1, 33, 4), (2, 130, 2)])
+def test_attention_without_gradients_equals_the_module_path(B, S, kv):
+    """lm.Attention takes one native call under no_grad and its own steps otherwise."""
+    from flashmhf_b200 import lm, lm_ops
+    torch.manual_seed(S)
+    cfg = lm.LMConfig(hidden_size=256, num_attention_heads=4, num_key_value_heads=kv)
+    att = lm.Attention(cfg).cuda().bfloat16()
+    x = torch.randn(B, S, 256, device="cuda").bfloat16()
+    cos, sin = lm.rotary_tables(S, 64, 10000.0, x.device, torch.bfloat16)
+    tables = lm_ops.rotary_tables_f32(cos, sin)
+    want = att(x, cos, sin, tables=tables).detach()
+    with torch.no_grad():
+        got = att(x, cos, sin, tables=tables)
+    assert orc.rel_l2(got.float(), want.float()) < 1e-2
