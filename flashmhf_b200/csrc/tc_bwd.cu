@@ -146,7 +146,7 @@ struct DqArgs {
 };
 
 template <int DH>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __maxnreg__(152)
 bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
               const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdQ, const DqArgs args) {
@@ -510,7 +510,9 @@ static_assert(DW_BARS * 8 + 8 <= 256, "control area");
 struct DwArgs {
     const float *R;
     long long r_sb, r_sh, r_ss;
-    float *ws;  // [nsplit][3][Hkuv][I][DH] fp32 partial sums (nsplit > 1)
+    // fp32 partial sums of the split blocks: [nsplit][3][ws_plane], a plane being the elements of [Hkuv][I][DH] from ws_first on
+    float *ws;
+    long long ws_plane, ws_first;
     // One part per block: its sums are the results and are written as bf16 at once (dK, dU, dV: head and row strides)
     __nv_bfloat16 *out[3];
     long long o_head[3], o_row[3];
@@ -518,24 +520,28 @@ struct DwArgs {
     int tiles_per_seq, tiles_total, tiles_per_split;
     // CTA -> (weight block, token-tile range).  Blocks [0, n_mixed) are split unevenly into a long part (launched first)
     // and a short part of `small_tiles` tiles (launched last); the others into `nsplit` equal parts, part by part.
-    int nblk_j, n_blocks, nsplit, n_mixed, small_tiles;
+    // Blocks [0, n_direct) are whole and written as bf16 results.
+    int nblk_j, n_blocks, nsplit, n_direct, n_mixed, small_tiles;
     float s0, c;  // head_scaling; head_scaling * up_scaling * final_scaling / 2
     WaitArgs wait;
 };
 
 // This CTA's weight block and token tiles.
 __device__ __forceinline__ void dw_range(const DwArgs &args, int &blk, int &split, int &tile_begin, int &tile_end) {
-    const int cta = blockIdx.x, n_even = args.n_blocks - args.n_mixed;
-    if (cta < args.n_mixed) {                               // long part of an unevenly split block
-        blk = cta; split = 0; tile_begin = 0; tile_end = args.tiles_total - args.small_tiles;
+    // in launch order: whole blocks (n_direct), long parts (n_mixed), equal parts part by part, short parts (n_mixed)
+    const int cta = (int)blockIdx.x - args.n_direct, first = args.n_direct + args.n_mixed, n_even = args.n_blocks - first;
+    if (cta < 0) {
+        blk = blockIdx.x; split = 0; tile_begin = 0; tile_end = args.tiles_total;
+    } else if (cta < args.n_mixed) {                        // long part of an unevenly split block
+        blk = args.n_direct + cta; split = 0; tile_begin = 0; tile_end = args.tiles_total - args.small_tiles;
     } else if (cta < args.n_mixed + n_even * args.nsplit) { // equal parts, part by part
         const int r = cta - args.n_mixed;
         split = r / n_even;
-        blk = args.n_mixed + (r - split * n_even);
+        blk = first + (r - split * n_even);
         tile_begin = split * args.tiles_per_split;
         tile_end = min(tile_begin + args.tiles_per_split, args.tiles_total);
     } else {                                                // short part of an unevenly split block
-        blk = cta - (args.n_mixed + n_even * args.nsplit); split = 1;
+        blk = args.n_direct + cta - (args.n_mixed + n_even * args.nsplit); split = 1;
         tile_begin = args.tiles_total - args.small_tiles; tile_end = args.tiles_total;
     }
 }
@@ -814,10 +820,10 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (ok) {
             tc_fence_after();
             // fp32 partial sums -> workspace[split][which][hk][row][DH], or bf16 results
-            const bool direct = args.nsplit == 1;
+            const bool direct = args.nsplit == 1 || blk < args.n_direct;
             const long long I = (long long)args.E * args.De;
-            const long long plane = (long long)args.Hkuv * I * DH;
-            float *wsb = args.ws + (long long)split * 3 * plane + ((long long)hk * I + (long long)jblk * kBI) * DH;
+            const long long plane = args.ws_plane;
+            float *wsb = args.ws + (long long)split * 3 * plane + ((long long)hk * I + (long long)jblk * kBI) * DH - args.ws_first;
             auto out_row = [&](int which, int r) {
                 return args.out[which] + hk * args.o_head[which] + ((long long)jblk * kBI + r) * args.o_row[which];
             };
@@ -1187,18 +1193,17 @@ bwd_dwt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (ok) {
             tc_fence_after();
             const bool in_range = row0 + row < I;
-            const long long plane = (long long)args.Hkuv * I * DH;
             constexpr int kColsPerHalf = DH / 2;
             const int c0 = part * kColsPerHalf;
 #pragma unroll
             for (int which = 0; which < 3; ++which) {
-                float *dst = args.ws + ((long long)split * 3 + which) * plane + ((long long)hk * I + row0 + row) * DH + c0;
+                float *dst = args.ws + ((long long)split * 3 + which) * args.ws_plane + ((long long)hk * I + row0 + row) * DH - args.ws_first + c0;
                 __nv_bfloat16 *o16 = args.out[which] + hk * args.o_head[which] + (long long)(row0 + row) * args.o_row[which] + c0;
 #pragma unroll
                 for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
                     tmem_ld16_sync(lane_base + kColAcc + which * DH + c0 + g * 16, o);
-                    if (in_range) dw_store16(args.nsplit == 1, dst + g * 16, o16 + g * 16, o);
+                    if (in_range) dw_store16(args.nsplit == 1 || blk < args.n_direct, dst + g * 16, o16 + g * 16, o);
                 }
             }
             tc_fence_before();
@@ -1224,16 +1229,21 @@ struct ReduceArgs {
     __nv_bfloat16 *out[3];
     long long s_head[3], s_row[3];
     long long plane;  // Hkuv * I * DH
+    long long first;  // element of a plane where the split blocks begin (those before are written by their CTAs)
     int nsplit, I, DH;
 };
-__global__ void __launch_bounds__(256) dw_reduce_kernel(const ReduceArgs a) {
-    griddep_wait();   // launched early, behind the kernel whose partial sums it adds
+// 128 threads and 48 registers: a CTA fits beside one of the dK/dU/dV kernel, waits there for that kernel to end, and then beside one
+// of the dQ/dR kernel, under which the addition runs.
+__global__ void __maxnreg__(48) dw_reduce_kernel(const ReduceArgs a) {
+    griddep_launch_dependents();
+    griddep_wait();
     const int which = blockIdx.y;
     const unsigned per_row = (unsigned)a.DH / 4;
     const long long n4 = a.plane / 4;
-    const float4 *src = reinterpret_cast<const float4 *>(a.ws + which * a.plane);
-    const long long split4 = 3 * n4;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n4; idx += (long long)gridDim.x * blockDim.x) {
+    const long long split4 = 3 * (n4 - a.first / 4);
+    const float4 *src = reinterpret_cast<const float4 *>(a.ws) + which * (n4 - a.first / 4) - a.first / 4;
+    for (long long idx = a.first / 4 + (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n4;
+         idx += (long long)gridDim.x * blockDim.x) {
         float4 acc = src[idx];
 #pragma unroll 4
         for (int s = 1; s < a.nsplit; ++s) {
@@ -1252,6 +1262,7 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const ReduceArgs a) {
 
 struct DwPlan {
     int tiles_per_seq, tiles_total, nsplit, tiles_per_split;
+    int n_direct;               // blocks that are not split at all
     int n_mixed, small_tiles;   // uneven split of the first n_mixed blocks (two-way splits only), else 0
 };
 
@@ -1271,12 +1282,12 @@ double list_schedule(const std::vector<double> &jobs, int num_sms) {
 
 // How the weight-gradient kernel of a head dimension cuts its work, and what a CTA costs besides its token tiles (weights in,
 // first tile through the pipeline, accumulators out: the intercept of kernel time over tiles per CTA, about 7 us), a split's
-// extra launch (2.8 us) and a byte of partial sums (written once, read once, about 4 TB/s), all in units of one token tile.
+// extra launch (4 us) and a byte of partial sums (written once, read once, about 4 TB/s), all in units of one token tile.
 struct DwShape {
     int rows, tokens;
     double tile_us;
     double fixed() const { return 7.0 / tile_us; }
-    double launch() const { return 2.8 / tile_us; }
+    double launch() const { return 4.0 / tile_us; }
     double sums(double bytes) const { return bytes / 4.0e6 / tile_us; }
 };
 DwShape dw_shape(int dh) { return dh == 128 ? DwShape{kBI, kBT, 1.8} : DwShape{kTI, kTT, dh == 64 ? 0.8 : 1.0}; }
@@ -1316,10 +1327,39 @@ double plan_uneven(DwPlan &p, long long items, int num_sms, double fixed) {
     return best;
 }
 
+// Whole blocks for as many full waves as there are, and the rest split k ways to fill the last one: only the rest has partial sums.
+// `sums`: the time to add one set of partial sums of all blocks.  Returns the duration, addition included.
+double plan_rest(DwPlan &p, long long items, int num_sms, double fixed, double launch, double sums) {
+    const int T = p.tiles_total;
+    double best = 1e300;
+    DwPlan b = p;
+    if (items > 2048 || T < 8) return best;
+    for (int k = 2; k <= 6; ++k) {
+        const int tiles = (T + k - 1) / k;
+        if ((T + tiles - 1) / tiles != k) continue;
+        for (int q = 2; q * (long long)num_sms / 4 < items; ++q) {   // quarter waves
+            const int nd = (int)(q * (long long)num_sms / 4);
+            std::vector<double> jobs((size_t)nd, T + fixed);
+            for (int part = 0; part < k; ++part)
+                jobs.insert(jobs.end(), (size_t)(items - nd), (part + 1 < k ? tiles : T - (k - 1) * tiles) + fixed);
+            const double m = list_schedule(jobs, num_sms) + launch + k * sums * (double)(items - nd) / (double)items;
+            if (m < best - 1e-9) {
+                best = m;
+                b.n_direct = nd;
+                b.nsplit = k;
+                b.tiles_per_split = tiles;
+            }
+        }
+    }
+    p = b;
+    return best;
+}
+
 // How many ways to split the token axis: the one whose waves of CTAs (fixed cost + its token tiles each) plus the addition
 // of its partial sums are shortest.  Unsplit blocks write their bf16 results themselves.
-DwPlan dw_plan(const flashmhf_dims &d, int num_sms) {
-    struct Key { long long items, dh; int tiles_per_seq, tiles_total, num_sms; };
+// `followed`: the dQ/dR kernel comes next and fills the last wave, so an unsplit plan loses less there.
+DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed) {
+    struct Key { long long items, dh; int tiles_per_seq, tiles_total, num_sms; bool followed; };
     struct Entry { Key k; DwPlan p; };
     static std::mutex mu;
     static std::vector<Entry> cache;
@@ -1327,11 +1367,11 @@ DwPlan dw_plan(const flashmhf_dims &d, int num_sms) {
     const DwShape sh = dw_shape(d.Dh);
     const long long items = (long long)d.Hkuv * (((long long)d.E * d.De + sh.rows - 1) / sh.rows);
     const int tps = (d.S + sh.tokens - 1) / sh.tokens;
-    const Key key{items, (long long)d.Dh, tps, tps * G * d.B, num_sms};
+    const Key key{items, (long long)d.Dh, tps, tps * G * d.B, num_sms, followed};
     std::lock_guard<std::mutex> lk(mu);
     for (const Entry &e : cache)
         if (e.k.items == key.items && e.k.dh == key.dh && e.k.tiles_per_seq == key.tiles_per_seq &&
-            e.k.tiles_total == key.tiles_total && e.k.num_sms == key.num_sms)
+            e.k.tiles_total == key.tiles_total && e.k.num_sms == key.num_sms && e.k.followed == followed)
             return e.p;
     const double sum_tiles = sh.sums((double)d.Hkuv * d.E * d.De * 3 * d.Dh * 4);   // one set of partial sums
     DwPlan best{};
@@ -1346,8 +1386,13 @@ DwPlan dw_plan(const flashmhf_dims &d, int num_sms) {
         double cost = ns == 2 ? plan_uneven(p, items, num_sms, sh.fixed())
                               : (double)((items * ns + num_sms - 1) / num_sms) * (p.tiles_per_split + sh.fixed());
         if (ns > 1) cost += sh.launch() + ns * sum_tiles;
+        else if (followed) cost *= 0.9;   // (of d_h = 64, 16384 tokens, 16 x 16 x 192: 1356 -> 1328 us for the whole backward)
         if (cost < best_cost - 1e-9) { best_cost = cost; best = p; }
     }
+    DwPlan rest{};
+    rest.tiles_per_seq = key.tiles_per_seq;
+    rest.tiles_total = key.tiles_total;
+    if (plan_rest(rest, items, num_sms, sh.fixed(), sh.launch(), sum_tiles) < best_cost - 1e-9) best = rest;
     if (cache.size() < 256) cache.push_back(Entry{key, best});
     return best;
 }
@@ -1374,8 +1419,15 @@ DqPlan dq_plan(const flashmhf_dims &d, int num_sms) {
     return best;
 }
 
+// First element of [Hkuv][I][DH] that belongs to a split block.
+long long dw_first(const flashmhf_dims &d, const DwPlan &pl) {
+    const int I = d.E * d.De, rows = dw_shape(d.Dh).rows, nblk_j = (I + rows - 1) / rows;
+    return pl.nsplit > 1 ? ((long long)(pl.n_direct / nblk_j) * I + (long long)(pl.n_direct % nblk_j) * rows) * d.Dh : 0;
+}
+// Whole sets of partial sums, one at least.
 size_t dw_workspace(const flashmhf_dims &d, const DwPlan &pl) {
-    return (size_t)pl.nsplit * 3 * (size_t)d.Hkuv * (size_t)d.E * d.De * d.Dh * sizeof(float);
+    const size_t plane = (size_t)d.Hkuv * (size_t)d.E * d.De * d.Dh, need = (size_t)pl.nsplit * (plane - (size_t)dw_first(d, pl));
+    return (need + plane - 1) / plane * 3 * plane * sizeof(float);
 }
 size_t dq_workspace(const flashmhf_dims &d, const DqPlan &pl) {
     return pl.nsplit > 1 ? (size_t)pl.nsplit * d.B * d.H * d.S * d.Dh * sizeof(float) : 0;
@@ -1419,9 +1471,8 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
     const float s0 = p.scale.head_scaling, c = p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling;
 
     // Weight gradients first: in data-parallel training their all-reduce can then start while dQ/dR still run.  In a call for
-    // everything the dQ/dR kernel follows the dK/dU/dV kernel directly, launched so that it may start under its tail, and the
-    // additions of partial sums come last.
-    const DwPlan pl = dw_plan(d, dc->num_sms);
+    // everything the dQ/dR kernel is launched so that it may start under the tail of the dK/dU/dV kernel.
+    const DwPlan pl = dw_plan(d, dc->num_sms, want_inputs);
     ReduceArgs ra{};
     ra.ws = static_cast<const float *>(p.workspace);
     if (want_weights) {
@@ -1435,13 +1486,14 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         ra.DH = DH;
         ra.plane = (long long)d.Hkuv * ra.I * DH;
         ra.nsplit = pl.nsplit;
+        ra.first = dw_first(d, pl);
         const int nblk_j = (d.E * d.De + dw_shape(DH).rows - 1) / dw_shape(DH).rows;
         DwArgs wa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
-                  static_cast<float *>(p.workspace), {ra.out[0], ra.out[1], ra.out[2]}, {ra.s_head[0], ra.s_head[1], ra.s_head[2]},
+                  static_cast<float *>(p.workspace), ra.plane - ra.first, ra.first, {ra.out[0], ra.out[1], ra.out[2]}, {ra.s_head[0], ra.s_head[1], ra.s_head[2]},
                   {ra.s_row[0], ra.s_row[1], ra.s_row[2]}, d.S, d.E, d.De, G, d.B, d.Hkuv,
                   pl.tiles_per_seq, pl.tiles_total, pl.tiles_per_split,
-                  nblk_j, d.Hkuv * nblk_j, pl.nsplit, pl.n_mixed, pl.small_tiles, s0, 0.5f * c, wait_args(dc)};
-        const long long ctas = (long long)wa.n_blocks * pl.nsplit;
+                  nblk_j, d.Hkuv * nblk_j, pl.nsplit, pl.n_direct, pl.n_mixed, pl.small_tiles, s0, 0.5f * c, wait_args(dc)};
+        const long long ctas = pl.n_direct + (long long)(wa.n_blocks - pl.n_direct) * pl.nsplit;
         if (ctas > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
         dim3 gw((unsigned)ctas);
         prof_mark(st, kMarkStart);
@@ -1457,6 +1509,22 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         *n_launch += 1;
         if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "bwd_dw_kernel launch"); return FLASHMHF_ERR_CUDA; }
     }
+
+    // The addition of the split blocks' partial sums: beside the dQ/dR kernel where they are few (one CTA per SM adds about 1 TB/s),
+    // else after it at full width.  (3 x 333 tokens, shared heads: backward 51 -> 44 us; 40 MB of sums beside dQ/dR: 586 -> 605.)
+    auto add_splits = [&](bool beside) -> int {
+        const long long n4 = (ra.plane - ra.first) / 4, cap = beside ? dc->num_sms / 3 : dc->num_sms * 6;   // per gradient
+        const dim3 blocks((unsigned)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap), 3);
+        prof_mark(st, kMarkStart);
+        const cudaError_t err = launch_kernel(true, dw_reduce_kernel, blocks, dim3(128), 0, st, ra);
+        prof_mark(st, kMarkBwdReduce);
+        *n_launch += 1;
+        if (err != cudaSuccess) { set_cuda_error(err, "dw_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
+        return FLASHMHF_OK;
+    };
+    const bool split = want_weights && pl.nsplit > 1;
+    const bool beside = split && want_inputs && 3.0 * (double)(ra.plane - ra.first) * 4 * pl.nsplit <= 24e6;
+    if (beside && (rc = add_splits(true)) != 0) return rc;
 
     DqPlan ql = dq_plan(d, dc->num_sms);
     float *q_part = nullptr;
@@ -1478,15 +1546,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         *n_launch += 1;
         if (e != cudaSuccess) { set_cuda_error(e, "bwd_dq_kernel launch"); return FLASHMHF_ERR_CUDA; }
     }
-    if (want_weights && pl.nsplit > 1) {
-        const long long n4 = ra.plane / 4, cap = (long long)dc->num_sms * 3;
-        const dim3 blocks((unsigned)((n4 + 255) / 256 < cap ? (n4 + 255) / 256 : cap), 3);
-        prof_mark(st, kMarkStart);
-        e = launch_kernel(true, dw_reduce_kernel, blocks, dim3(256), 0, st, ra);
-        prof_mark(st, kMarkBwdReduce);
-        *n_launch += 1;
-        if (e != cudaSuccess) { set_cuda_error(e, "dw_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
-    }
+    if (split && !beside && (rc = add_splits(false)) != 0) return rc;
     if (want_inputs && ql.nsplit > 1) {
         prof_mark(st, kMarkStart);
         e = launch_o_reduce(q_part, p.dQ, d, ql.nsplit, kReduceAfterKernel, dc->num_sms, st);
@@ -1501,7 +1561,9 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
 
 size_t tc_backward_weights_workspace_bytes(const flashmhf_dims &d) {
     const DeviceCtl *dc = device_ctl();
-    return dw_workspace(d, dw_plan(d, dc ? dc->num_sms : 148));
+    const int sms = dc ? dc->num_sms : 148;
+    const size_t a = dw_workspace(d, dw_plan(d, sms, true)), b = dw_workspace(d, dw_plan(d, sms, false));
+    return a > b ? a : b;
 }
 size_t tc_backward_inputs_workspace_bytes(const flashmhf_dims &d) {
     const DeviceCtl *dc = device_ctl();
