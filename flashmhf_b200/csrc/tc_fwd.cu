@@ -46,7 +46,7 @@ constexpr int kBI = 64;   // intermediate rows per block
 // The depth is what hides a stage's way from L2 (about 1000 clk under load, 32 KB per 64-wide chunk row pair): a stage of
 // the V ring is asked for again only when the O update that read it is done, so two stages cap the loop at two blocks per
 // (load + update + hand-offs).  At d_h = 64 a block is short and shared memory is plentiful; at 96 and 128 the rings
-// take what two Q tiles leave.
+// take what the Q tile leaves.
 template <int DH>
 struct FwdRings {
     static constexpr int kKU = DH == 64 ? 6 : 4, kV = DH == 64 ? 6 : 4;

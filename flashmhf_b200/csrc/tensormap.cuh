@@ -98,9 +98,22 @@ inline int encode_bf16_map_uncached(CUtensorMap *out, const void *base, int rank
         if (s <= 0 || (s % 8) != 0 || (uint64_t)s * 2 >= (1ull << 40)) return FLASHMHF_ERR_BAD_STRIDE;
         gstr[i] = (cuuint64_t)s * 2;
     }
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void *>(base), gdim, gstr, gbox,
-                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&] {
+        return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void *>(base), gdim, gstr, gbox,
+                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {
+        // A thread on which the runtime has not yet bound a context, such as an autograd thread whose allocations all came
+        // from torch's cache: this is then the first call there that needs one.  Selecting the thread's device again binds it
+        // (and, unlike an allocation or a free, is allowed while a stream is captured).
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaSetDevice(dev);
+        if (e != cudaSuccess) { set_cuda_error(e, "cudaSetDevice before cuTensorMapEncodeTiled"); return FLASHMHF_ERR_CUDA; }
+        r = encode();
+    }
     if (r != CUDA_SUCCESS) {
         set_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled rejected the tensor");
         return FLASHMHF_ERR_BAD_STRIDE;
