@@ -713,9 +713,12 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                            dPmn = desc_mnmajor(sP, kTile), dAmn = desc_mnmajor(sA, kTile);
             constexpr uint64_t kTokStep = L::kTokStage >> 4;
             int st = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int i = 0; i < ntiles; ++i) {
                 const uint64_t dq = dQmn0 + st * kTokStep, dg = dGmn0 + st * kTokStep;
+                // A needs only Q: that it is there does not say that dO is.  (The dA product, which waits for dO too, may still be ahead.)
+                if (!mbar_wait(bar(DW_GFULL + st), ph, ctl, W + 12)) { ok = false; break; }
                 if (!mbar_wait(bar(DW_AFULL), i & 1, ctl, W + 6)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
@@ -730,7 +733,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     umma_ss(tmem + kColKU, dPmn + k * 128, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
                 umma_commit(bar(DW_QEMPTY + st));  // Q of this stage and the [dM|dN] tile are free
                 umma_commit(bar(DW_PEMPTY));
-                if (++st == L::kTokStages) st = 0;
+                if (++st == L::kTokStages) { st = 0; ph ^= 1; }
             }
             if (ok) umma_commit(bar(DW_ACCFULL));
         }
@@ -1086,12 +1089,14 @@ bwd_dwt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             const uint64_t dQ0 = desc_mnmajor(sTok, kWChunk), dG0 = desc_mnmajor(sTok + L::kTok, kWChunk);
             constexpr uint64_t kTokStep = (2 * L::kTok) >> 4;
             int st = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int i = 0; i < ntiles; ++i) {
                 const int sb = i % kSB;
                 const uint32_t sph = (uint32_t)(i / kSB) & 1u;
                 const uint64_t dq = dQ0 + st * kTokStep, dg = dG0 + st * kTokStep;
                 const uint32_t tS = tmem + kColS + sb * 128;
+                if (!mbar_wait(bar(DT_GFULL + st), ph, ctl, W + 14)) { ok = false; break; }   // (A^T does not imply that dO is there)
                 // k step of 16 tokens = 8 columns; a thread's 32 tokens (two steps) lie together: see the element-wise warps
                 if (!mbar_wait(bar(DT_AFULL + sb), sph, ctl, W + 6)) { ok = false; break; }
                 tc_fence_after();
@@ -1117,7 +1122,7 @@ bwd_dwt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                 }
                 umma_commit(bar(DT_QEMPTY + st));
                 umma_commit(bar(kSB == 2 ? DT_SEMPTY + sb : (int)DT_DAEMPTY));
-                if (++st == L::kStages) st = 0;
+                if (++st == L::kStages) { st = 0; ph ^= 1; }
             }
             if (ok) umma_commit(bar(DT_ACCFULL));
         }

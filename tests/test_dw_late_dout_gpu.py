@@ -1,0 +1,44 @@
+"""GPU: dK, dU, dV element by element when the upstream gradient is the last of the inputs to arrive.
+
+A = silu(M) N R needs Q alone, so the update dV += A^T dO must wait for its dO tile by itself.  Each pass here runs on a dO that lies
+in DRAM while the other inputs lie in L2, with more than one wave of CTAs and a ragged last token tile.  A tile of dO read too early
+is one of many terms of a block: relative error of the whole tensor about 1e-3, of the block's elements a third of the rms -- so the
+bound is per element, and every pass must equal the first bit for bit."""
+import pytest
+import torch
+
+from oracle import mhffn_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _worst(a, b):
+    """Largest |a - b| over the rms of b, or over |b| where that is larger."""
+    d, rms = (a.double() - b.double()).abs(), b.double().square().mean().sqrt()
+    return float((d / torch.maximum(rms, b.double().abs())).max())
+
+
+@pytest.mark.parametrize("B,H,Hk,S,dh,E,de", [(5, 8, 8, 1645, 128, 6, 256), (3, 8, 4, 1031, 128, 5, 320), (5, 8, 8, 1645, 96, 8, 256),
+                                              (4, 8, 8, 2050, 64, 6, 192), (3, 8, 4, 1031, 64, 5, 320)])
+def test_weight_gradients_with_a_cold_upstream_gradient(B, H, Hk, S, dh, E, de):
+    import flashmhf_b200 as fm
+    g = torch.Generator(device="cuda").manual_seed(S + dh)
+    rnd = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=g).mul_(std).bfloat16()
+    Q, dO = rnd(B, H, S, dh), rnd(B, H, S, dh)
+    K, U, V = (rnd(Hk, E, de, dh, std=0.02) for _ in range(3))
+    R = torch.rand(B, H, S, E, device="cuda", generator=g)
+    evict = torch.empty(512 << 20, dtype=torch.uint8, device="cuda")
+    first = None
+    for _ in range(12):
+        evict.zero_()                                   # all of L2
+        sum(float(t.float().sum()) for t in (Q, K, U, V, R))   # every input but dO back into it
+        got = fm.backward_raw(Q, K, U, V, R, dO)
+        if first is None:
+            first = got
+        for name, a, b in zip("dQ dK dU dV dR".split(), got, first):
+            assert torch.equal(a, b), name
+    ref = orc.mhffn_backward(*(t.double() for t in (Q, K, U, V, R, dO)))
+    # bf16 operands of fp32 sums and a bf16 result: 2^-9 per term, random signs, about 2^-9 of the rms; 0.05 is 25 of these
+    for name, a, b in zip("dQ dK dU dV dR".split(), first, ref):
+        assert _worst(a, b) < 0.05, name
+    fm.check_device_status()
