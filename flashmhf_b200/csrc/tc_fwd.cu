@@ -84,13 +84,14 @@ struct FwdSmem {
 // QFULL: an item's Q has landed; QFREE: an item's O, staged over the Q of the item after it, has been read by its TMA store;
 // SFULL[b]: S computed into buffer b; SEMPTY[b]: every warp of the team working on it has its part in registers;
 // AFULL[s]: A written to slot s; AFREE[s]: the O update that read slot s is done; QT: Q copied to tensor memory;
+// SLAST: every S of a work item is computed (one commit from each S issuer; two teams only);
 // OFULL: the last O update of a work item is done; OFREE: its accumulator has been read out.
 // A CTA walks several work items (token tiles); blocks are counted through all of them (g), buffer and slot of a block
 // are g % 2, so every barrier has one fixed set of
 // waiters that observes each of its phases and a one-bit phase parity is enough.
 constexpr int kMaxRing = 6;
-enum { BAR_QFULL = 0, BAR_QFREE = 2, BAR_SFULL = 4, BAR_SEMPTY = 6, BAR_AFULL = 8, BAR_AFREE = 10, BAR_OFULL = 12, BAR_OFREE = 13,
-       BAR_QT = 14, BAR_KUFULL = 15, BAR_KUEMPTY = BAR_KUFULL + kMaxRing, BAR_VFULL = BAR_KUEMPTY + kMaxRing,
+enum { BAR_QFULL = 0, BAR_QFREE = 1, BAR_QT = 2, BAR_SLAST = 3, BAR_SFULL = 4, BAR_SEMPTY = 6, BAR_AFULL = 8, BAR_AFREE = 10, BAR_OFULL = 12,
+       BAR_OFREE = 13, BAR_KUFULL = 14, BAR_KUEMPTY = BAR_KUFULL + kMaxRing, BAR_VFULL = BAR_KUEMPTY + kMaxRing,
        BAR_VEMPTY = BAR_VFULL + kMaxRing, BAR_COUNT = BAR_VEMPTY + kMaxRing };
 static_assert(BAR_COUNT * 8 + 8 <= 320, "control area");
 
@@ -183,6 +184,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         }
         mbar_init(bar(BAR_QFULL), 1);
         mbar_init(bar(BAR_QFREE), 1);
+        mbar_init(bar(BAR_SLAST), 2);
         mbar_init(bar(BAR_OFULL), 1);
         mbar_init(bar(BAR_OFREE), arrivals_of(kTeamThreads));
         mbar_init(bar(BAR_QT), arrivals_of(kTeamThreads));
@@ -285,6 +287,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     umma_commit(bar(BAR_KUEMPTY + slot));
                     umma_commit(bar(BAR_SFULL + sb));
                 }
+                if (kTeams == 2 && ok) umma_commit(bar(BAR_SLAST));
                 g0 += w.nblk;
             }
         }
@@ -338,7 +341,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         }
         // Copy of a work item's Q tile from shared into tensor memory, by team 0 (thread = token row; its lower four warps
         // copy columns [0, 64) of d_h, the upper four [64, 128)).  Done as soon as the previous item's last S has been
-        // read, i.e. before that item's epilogue, so that the first S of the new item is computed under the epilogue.
+        // computed, i.e. before that item's epilogue, so that the first S of the new item is computed under the epilogue.
         auto copy_q = [&](int nn) -> bool {
             if (!mbar_wait(bar(BAR_QFULL), nn & 1, ctl, W + 11)) return false;
             if (group * 64 < DH) {
@@ -410,8 +413,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             }
             g0 += w.nblk;
             if (!ok || team != 0) continue;   // the rest of the item is team 0's
-            // every S of this item has been read: the next item's Q may replace it in tensor memory
-            if (item + (int)gridDim.x < args.n_items && !copy_q(n + 1)) { ok = false; break; }
+            // The next item's Q may replace this one's in tensor memory once every S of this item is computed.  One team has read
+            // them all by now; of two, team 0 knows of its own blocks only and waits for the others'.  (An issuer begins an item
+            // after its Q is there, so it is never a phase ahead of this wait.)
+            if (item + (int)gridDim.x < args.n_items) {
+                if (kTeams == 2) {
+                    if (!mbar_wait(bar(BAR_SLAST), n & 1, ctl, W + 14)) { ok = false; break; }
+                    tc_fence_after();
+                }
+                if (!copy_q(n + 1)) { ok = false; break; }
+            }
             // epilogue: O (fp32, tensor memory) -> bf16 -> shared (over this item's Q tile) -> TMA store
             if (!mbar_wait(bar(BAR_OFULL), n & 1, ctl, W + 10)) { ok = false; break; }
             tc_fence_after();
