@@ -366,10 +366,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             const bool in_range = t < args.S;
             const float *rrow = args.R + (long long)w.b * args.r_sb + (long long)w.h * args.r_sh + (long long)t * args.r_ss;
             // this team's first block of the item, its sub-network and position inside it; routing weight fetched one ahead
+            // (plain loads: the kernel before this one, under which this one may have started, can be the one that wrote R, and a
+            // non-coherent load is only for memory that nobody writes while the grid runs)
             const int jfirst = kTeams == 1 ? 0 : ((g0 + team) & 1);
             int e = (w.j0 + jfirst) / blocks_per_e, in_e = (w.j0 + jfirst) - e * blocks_per_e;
-            float r_cur = (in_range && e < args.E) ? __ldg(rrow + e) : 0.f;
-            float r_next = (in_range && e + 1 < args.E) ? __ldg(rrow + e + 1) : 0.f;
+            float r_cur = (in_range && e < args.E) ? rrow[e] : 0.f;
+            float r_next = (in_range && e + 1 < args.E) ? rrow[e + 1] : 0.f;
             for (int j = jfirst; j < w.nblk; j += kTeams) {
                 const int g = g0 + j, sb = g & 1;   // S buffer and A slot of this block
                 const float hr = 0.5f * args.c * r_cur;
@@ -408,7 +410,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         in_e = 0;
                         ++e;
                         r_cur = r_next;
-                        r_next = (in_range && e + 1 < args.E) ? __ldg(rrow + e + 1) : 0.f;
+                        r_next = (in_range && e + 1 < args.E) ? rrow[e + 1] : 0.f;
                     }
             }
             g0 += w.nblk;
