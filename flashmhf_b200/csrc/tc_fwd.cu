@@ -196,7 +196,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const bool dead = *abort_flag != 0;
-    griddep_launch_dependents();   // every CTA of this launch is running: what follows (the reduction, the next call) may start
     // Every launch may start under the end of the kernel before it (a decode step of 8 tokens of the 370M layer 12.3 -> 9.6 us a call);
     // until that kernel has ended only a chained call's producer touches global memory (weight tiles), the others wait below.
 
@@ -330,6 +329,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         bool ok = true;
         int g0 = 0, n = 0;   // blocks before this work item; work items so far
         griddep_wait();   // these warps read R and write O
+        // What follows (the reduction, the next call) may start now, and not before: a chained call reads its weights without waiting
+        // and is promised only that the operation directly before it does not write them, so whatever came before this launch
+        // must be complete when it starts.  (64 chained tokens of the 1.3B layer 21.5 -> 20.5 us against a trigger before the wait.)
+        griddep_launch_dependents();
         if (args.chained) {
             if (warp == 4 && lane == 0 && blockIdx.x < args.n_items) {   // the first item's Q (q.v. the producer)
                 const FwdItem w = fwd_item(args, blockIdx.x, nblk_total);
