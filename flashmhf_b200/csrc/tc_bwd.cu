@@ -1366,7 +1366,7 @@ double plan_rest(DwPlan &p, long long items, int num_sms, double fixed, double l
 // of its partial sums are shortest.  Unsplit blocks write their bf16 results themselves.
 // `followed`: the dQ/dR kernel comes next and fills the last wave, so an unsplit plan loses less there.
 DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed) {
-    struct Key { long long items, dh; int tiles_per_seq, tiles_total, num_sms; bool followed; };
+    struct Key { long long items, rows, dh; int tiles_per_seq, tiles_total, num_sms; bool followed; };   // rows: of all heads, for the sums
     struct Entry { Key k; DwPlan p; };
     static std::mutex mu;
     static std::vector<Entry> cache;
@@ -1374,10 +1374,10 @@ DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed) {
     const DwShape sh = dw_shape(d.Dh);
     const long long items = (long long)d.Hkuv * (((long long)d.E * d.De + sh.rows - 1) / sh.rows);
     const int tps = (d.S + sh.tokens - 1) / sh.tokens;
-    const Key key{items, (long long)d.Dh, tps, tps * G * d.B, num_sms, followed};
+    const Key key{items, (long long)d.Hkuv * d.E * d.De, (long long)d.Dh, tps, tps * G * d.B, num_sms, followed};
     std::lock_guard<std::mutex> lk(mu);
     for (const Entry &e : cache)
-        if (e.k.items == key.items && e.k.dh == key.dh && e.k.tiles_per_seq == key.tiles_per_seq &&
+        if (e.k.items == key.items && e.k.rows == key.rows && e.k.dh == key.dh && e.k.tiles_per_seq == key.tiles_per_seq &&
             e.k.tiles_total == key.tiles_total && e.k.num_sms == key.num_sms && e.k.followed == followed)
             return e.p;
     const double sum_tiles = sh.sums((double)d.Hkuv * d.E * d.De * 3 * d.Dh * 4);   // one set of partial sums
