@@ -25,7 +25,8 @@ EXPORTS = ("flashmhf_abi_version", "flashmhf_forward_workspace_bytes", "flashmhf
            "flashmhf_lm_rmsnorm_forward", "flashmhf_lm_rmsnorm_backward_workspace_bytes", "flashmhf_lm_rmsnorm_backward",
            "flashmhf_selftest_bounded_wait", "flashmhf_prologue_forward_dtype", "flashmhf_prologue_backward_dtype",
            "flashmhf_lm_rmsnorm_forward_dtype", "flashmhf_lm_rmsnorm_backward_dtype", "flashmhf_lm_rope_pair",
-           "flashmhf_lm_add_rmsnorm_forward", "flashmhf_lm_add_rmsnorm_backward")
+           "flashmhf_lm_add_rmsnorm_forward", "flashmhf_lm_add_rmsnorm_backward",
+           "flashmhf_backward_plan")
 
 
 class Tensor(C.Structure):
@@ -53,6 +54,11 @@ class BwdParams(C.Structure):
     _fields_ = [("d", Dims), ("Q", Tensor), ("K", Tensor), ("U", Tensor), ("V", Tensor), ("R", Tensor),
                 ("dO", Tensor), ("dQ", Tensor), ("dK", Tensor), ("dU", Tensor), ("dV", Tensor), ("dR", Tensor),
                 ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("scale", Scaling), ("parts", C.c_uint32)]
+
+
+class BackwardPlan(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("token_tiles", "splits", "tiles_per_split", "whole_blocks", "uneven_blocks", "small_tiles",
+                                         "dq_splits", "reserved")] + [("predicted_tiles", C.c_double)]
 
 
 class PrologueParams(C.Structure):
@@ -101,6 +107,8 @@ def load():
         lib.flashmhf_forward_workspace_bytes.argtypes = [C.POINTER(Dims)]
         lib.flashmhf_backward_workspace_bytes.restype = C.c_size_t
         lib.flashmhf_backward_workspace_bytes.argtypes = [C.POINTER(Dims)]
+        lib.flashmhf_backward_plan.restype = C.c_int
+        lib.flashmhf_backward_plan.argtypes = [C.POINTER(Dims), C.c_uint32, C.POINTER(BackwardPlan)]
         lib.flashmhf_backward.restype = C.c_int
         lib.flashmhf_backward.argtypes = [C.POINTER(BwdParams), C.c_void_p]
         lib.flashmhf_backward_static_scratch.restype = C.c_int

@@ -202,6 +202,16 @@ size_t flashmhf_backward_inputs_workspace_bytes(const flashmhf_dims *d) {
     return tc_backward_inputs_workspace_bytes(*d);
 }
 
+int flashmhf_backward_plan(const flashmhf_dims *d, uint32_t parts, flashmhf_backward_plan_info *out) {
+    if (!d || !out) return FLASHMHF_ERR_NULL;
+    const int rc = check_dims(*d);
+    if (rc) return rc;
+    if (d->dtype != FLASHMHF_BF16) return FLASHMHF_ERR_BAD_DTYPE;
+    if (parts & ~(FLASHMHF_BWD_INPUTS | FLASHMHF_BWD_WEIGHTS)) return FLASHMHF_ERR_BAD_SHAPE;
+    tc_backward_plan(*d, parts ? parts : (FLASHMHF_BWD_INPUTS | FLASHMHF_BWD_WEIGHTS), out);
+    return FLASHMHF_OK;
+}
+
 // Shared argument checks of the two backward entry points.  Tensors of a part that is not asked for are not looked at.
 static int check_bwd(const flashmhf_bwd_params *p, unsigned *parts_out) {
     if (!p) return FLASHMHF_ERR_NULL;

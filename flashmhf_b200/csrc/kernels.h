@@ -57,6 +57,7 @@ size_t tc_backward_inputs_workspace_bytes(const flashmhf_dims &d);   // what a c
 enum ReduceMode { kReduceAfterKernel, kReduceChained };
 cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, ReduceMode mode, int num_sms,
                             cudaStream_t st);
+void tc_backward_plan(const flashmhf_dims &d, uint32_t parts, flashmhf_backward_plan_info *out);
 int tc_backward_static_scratch(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch);
 
 // ---- fused layer prologue (per-head RMSNorm + router weights), HBM-bound CUDA-core kernels --

@@ -26,9 +26,8 @@
 // which half of the columns).
 #include <atomic>
 #include <mutex>
-#include <queue>
-#include <vector>
 
+#include "dw_plan.h"
 #include "kernels.h"
 #include "tc_common.cuh"
 #include "tensormap.cuh"
@@ -1267,143 +1266,6 @@ __global__ void __maxnreg__(48) dw_reduce_kernel(const ReduceArgs a) {
     }
 }
 
-struct DwPlan {
-    int tiles_per_seq, tiles_total, nsplit, tiles_per_split;
-    int n_direct;               // blocks that are not split at all
-    int n_mixed, small_tiles;   // uneven split of the first n_mixed blocks (two-way splits only), else 0
-};
-
-// Time at which the last of `jobs` (durations, in launch order) ends when each goes to the SM that frees up first.
-double list_schedule(const std::vector<double> &jobs, int num_sms) {
-    std::priority_queue<double, std::vector<double>, std::greater<double>> sm;
-    for (int i = 0; i < num_sms; ++i) sm.push(0.0);
-    double end = 0.0;
-    for (double j : jobs) {
-        const double t = sm.top() + j;
-        sm.pop();
-        sm.push(t);
-        if (t > end) end = t;
-    }
-    return end;
-}
-
-// How the weight-gradient kernel of a head dimension cuts its work, and what a CTA costs besides its token tiles (weights in,
-// first tile through the pipeline, accumulators out: the intercept of kernel time over tiles per CTA, about 7 us), a split's
-// extra launch (4 us) and a byte of partial sums (written once, read once, about 4 TB/s), all in units of one token tile.
-struct DwShape {
-    int rows, tokens;
-    double tile_us;
-    double fixed() const { return 7.0 / tile_us; }
-    double launch() const { return 4.0 / tile_us; }
-    double sums(double bytes) const { return bytes / 4.0e6 / tile_us; }
-};
-DwShape dw_shape(int dh) { return dh == 128 ? DwShape{kBI, kBT, 1.8} : DwShape{kTI, kTT, dh == 64 ? 0.8 : 1.0}; }
-
-// With a two-way split the CTAs are equal and their last wave is partly empty (704 CTAs on 148 SMs: the fifth wave is
-// 76 % full, 5 % of the kernel).  Splitting some blocks unevenly -- long parts launched first, short parts last, the
-// equal halves of the other blocks in between -- lets the short parts fill the SMs the last wave would leave idle.
-// The split point and the number of such blocks are found by simulating the launch order for a few candidates.
-// The partial sums still number two per block, so the reduction and the workspace do not change.
-// Returns the simulated duration (token tiles).
-double plan_uneven(DwPlan &p, long long items, int num_sms, double fixed) {
-    p.n_mixed = p.small_tiles = 0;
-    const int T = p.tiles_total, half = p.tiles_per_split;
-    auto makespan = [&](int nmix, int small) {
-        std::vector<double> jobs;
-        jobs.reserve((size_t)(2 * items));
-        for (int i = 0; i < nmix; ++i) jobs.push_back(T - small + fixed);
-        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(half + fixed);
-        for (long long i = 0; i < items - nmix; ++i) jobs.push_back(T - half + fixed);
-        for (int i = 0; i < nmix; ++i) jobs.push_back(small + fixed);
-        return list_schedule(jobs, num_sms);
-    };
-    if (items > 2048 || T < 2) return (double)((2 * items + num_sms - 1) / num_sms) * (half + fixed);
-    const double base = makespan(0, 0);
-    if (T < 32) return base;
-    double best = base;
-    const int step_small = T / 32 > 1 ? T / 32 : 1, step_mix = num_sms / 4 > 1 ? num_sms / 4 : 1;
-    for (int small = step_small; small < half; small += step_small)
-        for (int nmix = step_mix; nmix <= items; nmix += step_mix) {
-            const double m = makespan(nmix, small);
-            if (m < best - 1e-9) { best = m; p.n_mixed = nmix; p.small_tiles = small; }
-        }
-    if (best > 0.985 * base) {   // not worth a different launch order
-        p.n_mixed = p.small_tiles = 0;
-        best = base;
-    }
-    return best;
-}
-
-// Whole blocks for as many full waves as there are, and the rest split k ways to fill the last one: only the rest has partial sums.
-// `sums`: the time to add one set of partial sums of all blocks.  Returns the duration, addition included.
-double plan_rest(DwPlan &p, long long items, int num_sms, double fixed, double launch, double sums) {
-    const int T = p.tiles_total;
-    double best = 1e300;
-    DwPlan b = p;
-    if (items > 2048 || T < 8) return best;
-    for (int k = 2; k <= 6; ++k) {
-        const int tiles = (T + k - 1) / k;
-        if ((T + tiles - 1) / tiles != k) continue;
-        for (int q = 2; q * (long long)num_sms / 4 < items; ++q) {   // quarter waves
-            const int nd = (int)(q * (long long)num_sms / 4);
-            std::vector<double> jobs((size_t)nd, T + fixed);
-            for (int part = 0; part < k; ++part)
-                jobs.insert(jobs.end(), (size_t)(items - nd), (part + 1 < k ? tiles : T - (k - 1) * tiles) + fixed);
-            const double m = list_schedule(jobs, num_sms) + launch + k * sums * (double)(items - nd) / (double)items;
-            if (m < best - 1e-9) {
-                best = m;
-                b.n_direct = nd;
-                b.nsplit = k;
-                b.tiles_per_split = tiles;
-            }
-        }
-    }
-    p = b;
-    return best;
-}
-
-// How many ways to split the token axis: the one whose waves of CTAs (fixed cost + its token tiles each) plus the addition
-// of its partial sums are shortest.  Unsplit blocks write their bf16 results themselves.
-// `followed`: the dQ/dR kernel comes next and fills the last wave, so an unsplit plan loses less there.
-DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed) {
-    struct Key { long long items, rows, dh; int tiles_per_seq, tiles_total, num_sms; bool followed; };   // rows: of all heads, for the sums
-    struct Entry { Key k; DwPlan p; };
-    static std::mutex mu;
-    static std::vector<Entry> cache;
-    const int G = d.H / d.Hkuv;
-    const DwShape sh = dw_shape(d.Dh);
-    const long long items = (long long)d.Hkuv * (((long long)d.E * d.De + sh.rows - 1) / sh.rows);
-    const int tps = (d.S + sh.tokens - 1) / sh.tokens;
-    const Key key{items, (long long)d.Hkuv * d.E * d.De, (long long)d.Dh, tps, tps * G * d.B, num_sms, followed};
-    std::lock_guard<std::mutex> lk(mu);
-    for (const Entry &e : cache)
-        if (e.k.items == key.items && e.k.rows == key.rows && e.k.dh == key.dh && e.k.tiles_per_seq == key.tiles_per_seq &&
-            e.k.tiles_total == key.tiles_total && e.k.num_sms == key.num_sms && e.k.followed == followed)
-            return e.p;
-    const double sum_tiles = sh.sums((double)d.Hkuv * d.E * d.De * 3 * d.Dh * 4);   // one set of partial sums
-    DwPlan best{};
-    double best_cost = 1e300;
-    for (int ns = 1; ns <= 16 && ns <= key.tiles_total; ++ns) {
-        DwPlan p{};
-        p.tiles_per_seq = key.tiles_per_seq;
-        p.tiles_total = key.tiles_total;
-        p.tiles_per_split = (p.tiles_total + ns - 1) / ns;
-        p.nsplit = (p.tiles_total + p.tiles_per_split - 1) / p.tiles_per_split;  // no empty split
-        if (p.nsplit != ns) continue;
-        double cost = ns == 2 ? plan_uneven(p, items, num_sms, sh.fixed())
-                              : (double)((items * ns + num_sms - 1) / num_sms) * (p.tiles_per_split + sh.fixed());
-        if (ns > 1) cost += sh.launch() + ns * sum_tiles;
-        else if (followed) cost *= 0.9;   // (of d_h = 64, 16384 tokens, 16 x 16 x 192: 1356 -> 1328 us for the whole backward)
-        if (cost < best_cost - 1e-9) { best_cost = cost; best = p; }
-    }
-    DwPlan rest{};
-    rest.tiles_per_seq = key.tiles_per_seq;
-    rest.tiles_total = key.tiles_total;
-    if (plan_rest(rest, items, num_sms, sh.fixed(), sh.launch(), sum_tiles) < best_cost - 1e-9) best = rest;
-    if (cache.size() < 256) cache.push_back(Entry{key, best});
-    return best;
-}
-
 // dQ/dR: with few token tiles the sub-networks are split over CTAs.  In 64-row blocks (about 0.8 us): a CTA costs six besides
 // its blocks, the reduction three and its partial sums.  Splits only while the tiles are no more than two waves, and only for
 // a gain of a tenth: the split sums dQ in another order than the unsplit kernel.
@@ -1426,6 +1288,7 @@ DqPlan dq_plan(const flashmhf_dims &d, int num_sms) {
     return best;
 }
 
+static_assert(kBI == 64 && kBT == 128 && kTI == 128 && kTT == 64, "dw_shape");
 // First element of [Hkuv][I][DH] that belongs to a split block.
 long long dw_first(const flashmhf_dims &d, const DwPlan &pl) {
     const int I = d.E * d.De, rows = dw_shape(d.Dh).rows, nblk_j = (I + rows - 1) / rows;
@@ -1479,7 +1342,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
 
     // Weight gradients first: in data-parallel training their all-reduce can then start while dQ/dR still run.  In a call for
     // everything the dQ/dR kernel is launched so that it may start under the tail of the dK/dU/dV kernel.
-    const DwPlan pl = dw_plan(d, dc->num_sms, want_inputs);
+    const DwPlan pl = want_weights ? dw_plan(d, dc->num_sms, want_inputs) : DwPlan{};
     ReduceArgs ra{};
     ra.ws = static_cast<const float *>(p.workspace);
     if (want_weights) {
@@ -1579,6 +1442,23 @@ size_t tc_backward_inputs_workspace_bytes(const flashmhf_dims &d) {
 size_t tc_backward_workspace_bytes(const flashmhf_dims &d) {
     const size_t w = tc_backward_weights_workspace_bytes(d), q = tc_backward_inputs_workspace_bytes(d);
     return q ? align256(w) + q : w;
+}
+
+void tc_backward_plan(const flashmhf_dims &d, uint32_t parts, flashmhf_backward_plan_info *out) {
+    const DeviceCtl *dc = device_ctl();
+    const int sms = dc ? dc->num_sms : 148;
+    *out = flashmhf_backward_plan_info{};
+    if (parts & FLASHMHF_BWD_WEIGHTS) {
+        const DwPlan p = dw_plan(d, sms, (parts & FLASHMHF_BWD_INPUTS) != 0);
+        out->token_tiles = p.tiles_total;
+        out->splits = p.nsplit;
+        out->tiles_per_split = p.tiles_per_split;
+        out->whole_blocks = p.nsplit > 1 ? p.n_direct : 0;
+        out->uneven_blocks = p.n_mixed;
+        out->small_tiles = p.small_tiles;
+        out->predicted_tiles = p.tiles;
+    }
+    if (parts & FLASHMHF_BWD_INPUTS) out->dq_splits = dq_plan(d, sms).nsplit;
 }
 
 // ---------------------------------------------------------------------------------------------

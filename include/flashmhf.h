@@ -139,6 +139,20 @@ size_t flashmhf_backward_workspace_bytes(const flashmhf_dims *d);
  * same results up to the order of that sum.  Pure host arithmetic. */
 size_t flashmhf_backward_inputs_workspace_bytes(const flashmhf_dims *d);
 
+/* How flashmhf_backward cuts its work for these dims and parts (a mask as in flashmhf_bwd_params, 0: everything; bf16 only).  Pure
+ * host arithmetic; a pure function of its arguments and the SM count, which the results' bits may depend on. */
+typedef struct {
+    int32_t token_tiles;       /* dK/dU/dV: tiles the token axis is cut into, all heads of a K/U/V head together */
+    int32_t splits;            /* parts a split block of weight rows is summed in */
+    int32_t tiles_per_split;
+    int32_t whole_blocks;      /* blocks that are not split while others are */
+    int32_t uneven_blocks, small_tiles;   /* two parts: blocks cut unevenly, and the tiles of their short part */
+    int32_t dq_splits;         /* dQ/dR: parts the sub-networks are split into */
+    int32_t reserved;
+    double predicted_tiles;    /* dK/dU/dV and the addition of its parts, in token tiles */
+} flashmhf_backward_plan_info;
+int flashmhf_backward_plan(const flashmhf_dims *d, uint32_t parts, flashmhf_backward_plan_info *out);
+
 /* Backward: dQ, dK, dU, dV, dR from dO, recomputing the intermediate.  Enqueues on `stream` and
  * returns.  Deterministic (no floating-point atomics).  Replaces flashffn_moe_backward,
  * flash_ffn_moe.cu:1012-1133, and the two launches at kernels/triton/flash_mlp_moe.py:832-866. */
