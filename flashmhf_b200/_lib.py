@@ -18,7 +18,7 @@ SELFTEST_CODE = 9901                # status code of flashmhf_selftest_bounded_w
 STATIC_SCRATCH_BYTES = 72 << 20
 
 EXPORTS = ("flashmhf_abi_version", "flashmhf_forward_workspace_bytes", "flashmhf_strerror", "flashmhf_last_cuda_error", "flashmhf_forward", "flashmhf_forward_chained",
-           "flashmhf_backward_workspace_bytes", "flashmhf_backward_inputs_workspace_bytes", "flashmhf_backward", "flashmhf_device_status",
+           "flashmhf_backward_workspace_bytes", "flashmhf_backward_inputs_workspace_bytes", "flashmhf_backward", "flashmhf_backward_inputs", "flashmhf_device_status",
            "flashmhf_launch_count", "flashmhf_profile_begin", "flashmhf_profile_end",
            "flashmhf_backward_static_scratch", "flashmhf_prologue_forward",
            "flashmhf_prologue_backward_workspace_bytes", "flashmhf_prologue_backward", "flashmhf_lm_rope",
@@ -111,6 +111,10 @@ def load():
         lib.flashmhf_backward_plan.argtypes = [C.POINTER(Dims), C.c_uint32, C.POINTER(BackwardPlan)]
         lib.flashmhf_backward.restype = C.c_int
         lib.flashmhf_backward.argtypes = [C.POINTER(BwdParams), C.c_void_p]
+        lib.flashmhf_backward_inputs_workspace_bytes.restype = C.c_size_t
+        lib.flashmhf_backward_inputs_workspace_bytes.argtypes = [C.POINTER(Dims)]
+        lib.flashmhf_backward_inputs.restype = C.c_int
+        lib.flashmhf_backward_inputs.argtypes = [C.POINTER(BwdParams), C.c_void_p]
         lib.flashmhf_backward_static_scratch.restype = C.c_int
         lib.flashmhf_backward_static_scratch.argtypes = [C.POINTER(BwdParams), C.c_void_p]
         lib.flashmhf_prologue_forward.restype = C.c_int

@@ -234,6 +234,22 @@ static int check_bwd(const flashmhf_bwd_params *p, unsigned *parts_out) {
     return FLASHMHF_OK;
 }
 
+// A checked call: parts set, workspace null or what the parts need.
+static int run_bwd(const flashmhf_bwd_params &p, cudaStream_t st) {
+    int n = 0, rc = FLASHMHF_OK;
+    if (p.d.dtype == FLASHMHF_F32_CHECK) {
+        cudaError_t e = simt_backward(p, st, &n);
+        if (e != cudaSuccess) {
+            set_cuda_error(e, "check backward launch");
+            rc = FLASHMHF_ERR_CUDA;
+        }
+    } else {
+        rc = tc_backward(p, st, &n);
+    }
+    g_launches += (uint64_t)n;
+    return rc;
+}
+
 int flashmhf_backward(const flashmhf_bwd_params *p, void *stream) {
     unsigned parts = 0;
     int rc = check_bwd(p, &parts);
@@ -245,21 +261,26 @@ int flashmhf_backward(const flashmhf_bwd_params *p, void *stream) {
     }
     if ((rc = check_arch()) != 0) return rc;
     if (!device_ctl()) return FLASHMHF_ERR_CUDA;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int n = 0;
     flashmhf_bwd_params q = *p;
     q.parts = parts;
-    if (p->d.dtype == FLASHMHF_F32_CHECK) {
-        cudaError_t e = simt_backward(q, st, &n);
-        if (e != cudaSuccess) {
-            set_cuda_error(e, "check backward launch");
-            rc = FLASHMHF_ERR_CUDA;
-        }
-    } else {
-        rc = tc_backward(q, st, &n);
+    if (!(parts & FLASHMHF_BWD_WEIGHTS)) {   // the caller may have left them unset
+        q.workspace = nullptr;
+        q.workspace_bytes = 0;
     }
-    g_launches += (uint64_t)n;
-    return rc;
+    return run_bwd(q, static_cast<cudaStream_t>(stream));
+}
+
+int flashmhf_backward_inputs(const flashmhf_bwd_params *p, void *stream) {
+    if (!p) return FLASHMHF_ERR_NULL;
+    flashmhf_bwd_params q = *p;
+    q.parts = FLASHMHF_BWD_INPUTS;
+    unsigned parts = 0;
+    int rc = check_bwd(&q, &parts);
+    if (rc) return rc;
+    if (reinterpret_cast<uintptr_t>(q.workspace) & 255u) return FLASHMHF_ERR_WORKSPACE;
+    if ((rc = check_arch()) != 0) return rc;
+    if (!device_ctl()) return FLASHMHF_ERR_CUDA;
+    return run_bwd(q, static_cast<cudaStream_t>(stream));
 }
 
 int flashmhf_backward_static_scratch(const flashmhf_bwd_params *p, void *stream) {

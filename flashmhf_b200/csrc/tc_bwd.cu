@@ -1504,8 +1504,13 @@ int tc_backward_static_scratch(const flashmhf_bwd_params &p, cudaStream_t st, in
     const int rc = static_scratch_ptr(&ptr);
     if (rc != FLASHMHF_OK) return rc;
     flashmhf_bwd_params q = p;
-    q.workspace = ptr;
-    q.workspace_bytes = kStaticScratchBytes;
+    if (p.parts & FLASHMHF_BWD_WEIGHTS) {   // (a call for dQ and dR alone leaves the array to others)
+        q.workspace = ptr;
+        q.workspace_bytes = kStaticScratchBytes;
+    } else {
+        q.workspace = nullptr;
+        q.workspace_bytes = 0;
+    }
     return tc_backward(q, st, n_launch);
 }
 

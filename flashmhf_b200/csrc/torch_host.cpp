@@ -32,7 +32,7 @@ struct Api {
     decltype(&flashmhf_strerror) strerror = nullptr;
     decltype(&flashmhf_last_cuda_error) last_cuda_error = nullptr;
     decltype(&flashmhf_forward) forward = nullptr, forward_chained = nullptr;
-    decltype(&flashmhf_backward) backward = nullptr;
+    decltype(&flashmhf_backward) backward = nullptr, backward_inputs = nullptr;
     decltype(&flashmhf_forward_workspace_bytes) forward_ws = nullptr;
     decltype(&flashmhf_backward_workspace_bytes) backward_ws = nullptr, backward_inputs_ws = nullptr;
     decltype(&flashmhf_prologue_forward_dtype) prologue_forward = nullptr;
@@ -61,6 +61,7 @@ void bind(uintptr_t handle, py::object error_type) {
     get(api.forward, "flashmhf_forward");
     get(api.forward_chained, "flashmhf_forward_chained");
     get(api.backward, "flashmhf_backward");
+    get(api.backward_inputs, "flashmhf_backward_inputs");
     get(api.forward_ws, "flashmhf_forward_workspace_bytes");
     get(api.backward_ws, "flashmhf_backward_workspace_bytes");
     get(api.backward_inputs_ws, "flashmhf_backward_inputs_workspace_bytes");
@@ -261,7 +262,7 @@ Grads backward_checked(const Shape &s, const Tensor &Q0, const Tensor &K0, const
         ws = at::empty({(int64_t)p.workspace_bytes}, Q.options().dtype(at::kByte));
         p.workspace = ws.data_ptr();
     }
-    check(api.backward(&p, current_stream(Q)));
+    check((weights ? api.backward : api.backward_inputs)(&p, current_stream(Q)));
     return g;
 }
 
@@ -552,7 +553,7 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
         p.d = dims_of(Shape{a.B, a.H, a.S, a.Dh, n[0], a.E, gate.size(0) / a.E}, at::kBFloat16);
         // dQ, dR and the scratch of the operator live until the prologue's backward has run: one allocation for all three
         const size_t dq_bytes = align256((size_t)T * hid * 2), dr_bytes = align256((size_t)T * a.H * a.E * 4);
-        p.workspace_bytes = api.backward_ws(&p.d);
+        p.workspace_bytes = weights ? api.backward_ws(&p.d) : api.backward_inputs_ws(&p.d);
         const Tensor tmp = at::empty({(int64_t)(dq_bytes + dr_bytes + p.workspace_bytes + 1)}, d.options().dtype(at::kByte));
         char *base = static_cast<char *>(tmp.data_ptr());
         p.Q = heads_address(sv[5].data_ptr(), a); p.dO = heads_address(d.data_ptr(), a); p.R = routing_address(R.data_ptr(), a);
@@ -565,7 +566,7 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
             out[5] = at::empty_like(gate); out[6] = at::empty_like(up); out[7] = at::empty_like(down);
             p.dK = expert_address(out[5], a.Dh, p.d.De); p.dU = expert_address(out[6], a.Dh, p.d.De); p.dV = expert_address(out[7], a.Dh, p.d.De);
         }
-        check(api.backward(&p, current_stream(d)));
+        check((weights ? api.backward : api.backward_inputs)(&p, current_stream(d)));
         if (inputs) {
             const PrologueGrads pg = run_prologue_backward(a, static_cast<char *>(p.dQ.ptr), p.dQ.stride, static_cast<float *>(p.dR.ptr));
             if (pg.d_norm.defined()) out[3] = pg.d_norm.to((at::ScalarType)n[2]);

@@ -134,9 +134,8 @@ size_t flashmhf_forward_workspace_bytes(const flashmhf_dims *d);
 /* Bytes of scratch flashmhf_backward needs for these dims (0 is possible).  Pure host arithmetic. */
 size_t flashmhf_backward_workspace_bytes(const flashmhf_dims *d);
 
-/* Bytes of scratch a call with parts = FLASHMHF_BWD_INPUTS can use: 0 except for short token counts, where the sub-networks
- * are split over CTAs and fp32 partial dQ are summed in a fixed order.  Optional: without it the kernel runs unsplit, with the
- * same results up to the order of that sum.  Pure host arithmetic. */
+/* Bytes of scratch flashmhf_backward_inputs can use: 0 except for short token counts, where the sub-networks are split over
+ * CTAs and fp32 partial dQ are summed in a fixed order.  Pure host arithmetic. */
 size_t flashmhf_backward_inputs_workspace_bytes(const flashmhf_dims *d);
 
 /* How flashmhf_backward cuts its work for these dims and parts (a mask as in flashmhf_bwd_params, 0: everything; bf16 only).  Pure
@@ -157,6 +156,12 @@ int flashmhf_backward_plan(const flashmhf_dims *d, uint32_t parts, flashmhf_back
  * returns.  Deterministic (no floating-point atomics).  Replaces flashffn_moe_backward,
  * flash_ffn_moe.cu:1012-1133, and the two launches at kernels/triton/flash_mlp_moe.py:832-866. */
 int flashmhf_backward(const flashmhf_bwd_params *p, void *stream);
+
+/* dQ and dR alone (p->parts is not looked at), with scratch: `workspace` is NULL, or 256-byte aligned with `workspace_bytes` bytes
+ * that no call on another stream uses meanwhile.  With flashmhf_backward_inputs_workspace_bytes() of them short inputs are split over
+ * more CTAs; with fewer the kernel runs unsplit, as flashmhf_backward(parts = FLASHMHF_BWD_INPUTS) does, which ignores both fields:
+ * the same results up to the order of the fp32 sum of dQ. */
+int flashmhf_backward_inputs(const flashmhf_bwd_params *p, void *stream);
 
 /* Size of the scratch array built into the library for flashmhf_backward_static_scratch: 72 MiB
  * (enough for the 370M layer shape, H_kuv=8, E*d_e=2816, d_h=128, with its two-way token split). */
