@@ -74,6 +74,17 @@ class SmTimes {
     int c_[8];
 };
 
+// First element of [Hkuv][I][DH] that belongs to a split block.
+inline long long dw_first(const flashmhf_dims &d, const DwPlan &pl) {
+    const int I = d.E * d.De, rows = dw_shape(d.Dh).rows, nblk_j = (I + rows - 1) / rows;
+    return pl.nsplit > 1 ? ((long long)(pl.n_direct / nblk_j) * I + (long long)(pl.n_direct % nblk_j) * rows) * d.Dh : 0;
+}
+// Whole sets of partial sums, one at least.
+inline size_t dw_workspace(const flashmhf_dims &d, const DwPlan &pl) {
+    const size_t plane = (size_t)d.Hkuv * (size_t)d.E * d.De * d.Dh, need = (size_t)pl.nsplit * (plane - (size_t)dw_first(d, pl));
+    return (need + plane - 1) / plane * 3 * plane * sizeof(float);
+}
+
 namespace dw_detail {
 
 // With a two-way split the CTAs are equal and their last wave is partly empty (704 CTAs on 148 SMs: the fifth wave is
@@ -114,9 +125,10 @@ inline double plan_uneven(DwPlan &p, long long items, int num_sms, double fixed)
 }
 
 // Whole blocks for as many full waves as there are, and the rest split k ways to fill the last one: only the rest has partial sums.
-// `sums`: the time to add one set of partial sums of all blocks.  Returns the duration, addition included, of a plan that takes less
-// than `best`, or `best`.
-inline double plan_rest(DwPlan &p, long long items, int num_sms, double fixed, double launch, double sums, double best) {
+// `sums`: the time to add one set of partial sums of all blocks.  `fits`: whether there is room for a plan's partial sums.  Returns the
+// duration, addition included, of a plan that takes less than `best`, or `best`.
+template <typename Fits>
+double plan_rest(DwPlan &p, long long items, int num_sms, double fixed, double launch, double sums, double best, const Fits &fits) {
     const int T = p.tiles_total;
     DwPlan b = p;
     if (items > 2048 || T < 8) return best;
@@ -134,25 +146,26 @@ inline double plan_rest(DwPlan &p, long long items, int num_sms, double fixed, d
             sm.run((k - 1) * split, tiles + fixed);
             sm.run(split, T - (k - 1) * tiles + fixed);
             const double m = sm.end() + add;
-            if (m < best - 1e-9) {
-                best = m;
-                b.n_direct = (int)nd;
-                b.nsplit = k;
-                b.tiles_per_split = tiles;
-            }
+            DwPlan c = p;
+            c.n_direct = (int)nd;
+            c.nsplit = k;
+            c.tiles_per_split = tiles;
+            if (m < best - 1e-9 && fits(c)) { best = m; b = c; }
         }
     }
     p = b;
     return best;
 }
 
-inline DwPlan make_plan(const flashmhf_dims &d, int num_sms, bool followed) {
+// `room`: bytes there are for partial sums.  (A plan without any always fits.)
+inline DwPlan make_plan(const flashmhf_dims &d, int num_sms, bool followed, size_t room) {
     const DwShape sh = dw_shape(d.Dh);
     const long long items = (long long)d.Hkuv * (((long long)d.E * d.De + sh.rows - 1) / sh.rows);
     const double sums = sh.sums((double)d.Hkuv * d.E * d.De * 3 * d.Dh * 4);   // one set of partial sums
     DwPlan p0{};
     p0.tiles_per_seq = (d.S + sh.tokens - 1) / sh.tokens;
     p0.tiles_total = p0.tiles_per_seq * (d.H / d.Hkuv) * d.B;
+    auto fits = [&](const DwPlan &p) { return room == SIZE_MAX || dw_workspace(d, p) <= room; };
     // whole, then the rest split, then equal (or two uneven) parts; each family only where it can still be the shortest
     DwPlan best = p0;
     best.nsplit = 1;
@@ -160,13 +173,13 @@ inline DwPlan make_plan(const flashmhf_dims &d, int num_sms, bool followed) {
     double best_cost = (double)((items + num_sms - 1) / num_sms) * (p0.tiles_total + sh.fixed());
     if (followed) best_cost *= 0.9;   // (of d_h = 64, 16384 tokens, 16 x 16 x 192: 1356 -> 1328 us for the whole backward)
     DwPlan rest = p0;
-    const double rest_cost = plan_rest(rest, items, num_sms, sh.fixed(), sh.launch(), sums, best_cost);
+    const double rest_cost = plan_rest(rest, items, num_sms, sh.fixed(), sh.launch(), sums, best_cost, fits);
     if (rest_cost < best_cost) { best = rest; best_cost = rest_cost; }
     for (int ns = 2; ns <= 16 && ns <= p0.tiles_total; ++ns) {
         DwPlan p = p0;
         p.tiles_per_split = (p.tiles_total + ns - 1) / ns;
         p.nsplit = (p.tiles_total + p.tiles_per_split - 1) / p.tiles_per_split;  // no empty split
-        if (p.nsplit != ns) continue;
+        if (p.nsplit != ns || !fits(p)) continue;
         const double add = sh.launch() + ns * sums;
         if ((double)items * (p.tiles_total + ns * sh.fixed()) / num_sms + add >= best_cost - 1e-9) continue;   // as in plan_rest
         const double cost = add + (ns == 2 ? plan_uneven(p, items, num_sms, sh.fixed())
@@ -181,9 +194,10 @@ inline DwPlan make_plan(const flashmhf_dims &d, int num_sms, bool followed) {
 
 // The plan of a call: a pure function of its arguments, kept in a small table per thread (no lock; a shape that comes back late is
 // planned again).  `followed`: the dQ/dR kernel comes next and fills the last wave, so an unsplit plan loses less there.
-inline DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed) {
+inline DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed, size_t room = SIZE_MAX) {
     struct Entry {
         int32_t B, H, S, Dh, Hkuv, E, De, num_sms, followed;
+        size_t room;
         DwPlan p;
     };
     constexpr int kEntries = 256;
@@ -192,8 +206,8 @@ inline DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed) {
     for (int32_t v : {d.B, d.H, d.S, d.Dh, d.Hkuv, d.E, d.De, (int32_t)followed}) h = (h ^ (uint32_t)v) * 16777619u;
     Entry &e = table[(h ^ (h >> 15)) % kEntries];
     if (e.num_sms != num_sms || e.followed != (int32_t)followed || e.B != d.B || e.H != d.H || e.S != d.S || e.Dh != d.Dh || e.Hkuv != d.Hkuv ||
-        e.E != d.E || e.De != d.De)
-        e = Entry{d.B, d.H, d.S, d.Dh, d.Hkuv, d.E, d.De, num_sms, (int32_t)followed, dw_detail::make_plan(d, num_sms, followed)};
+        e.E != d.E || e.De != d.De || e.room != room)
+        e = Entry{d.B, d.H, d.S, d.Dh, d.Hkuv, d.E, d.De, num_sms, (int32_t)followed, room, dw_detail::make_plan(d, num_sms, followed, room)};
     return e.p;
 }
 

@@ -1289,16 +1289,6 @@ DqPlan dq_plan(const flashmhf_dims &d, int num_sms) {
 }
 
 static_assert(kBI == 64 && kBT == 128 && kTI == 128 && kTT == 64, "dw_shape");
-// First element of [Hkuv][I][DH] that belongs to a split block.
-long long dw_first(const flashmhf_dims &d, const DwPlan &pl) {
-    const int I = d.E * d.De, rows = dw_shape(d.Dh).rows, nblk_j = (I + rows - 1) / rows;
-    return pl.nsplit > 1 ? ((long long)(pl.n_direct / nblk_j) * I + (long long)(pl.n_direct % nblk_j) * rows) * d.Dh : 0;
-}
-// Whole sets of partial sums, one at least.
-size_t dw_workspace(const flashmhf_dims &d, const DwPlan &pl) {
-    const size_t plane = (size_t)d.Hkuv * (size_t)d.E * d.De * d.Dh, need = (size_t)pl.nsplit * (plane - (size_t)dw_first(d, pl));
-    return (need + plane - 1) / plane * 3 * plane * sizeof(float);
-}
 size_t dq_workspace(const flashmhf_dims &d, const DqPlan &pl) {
     return pl.nsplit > 1 ? (size_t)pl.nsplit * d.B * d.H * d.S * d.Dh * sizeof(float) : 0;
 }
@@ -1342,7 +1332,11 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
 
     // Weight gradients first: in data-parallel training their all-reduce can then start while dQ/dR still run.  In a call for
     // everything the dQ/dR kernel is launched so that it may start under the tail of the dK/dU/dV kernel.
-    const DwPlan pl = want_weights ? dw_plan(d, dc->num_sms, want_inputs) : DwPlan{};
+    DwPlan pl{};
+    if (want_weights) {
+        pl = dw_plan(d, dc->num_sms, want_inputs);
+        if (dw_workspace(d, pl) > p.workspace_bytes) pl = dw_plan(d, dc->num_sms, want_inputs, p.workspace_bytes);   // (the static array)
+    }
     ReduceArgs ra{};
     ra.ws = static_cast<const float *>(p.workspace);
     if (want_weights) {
@@ -1499,7 +1493,8 @@ int static_scratch_ptr(void **out) {
 }  // namespace
 
 int tc_backward_static_scratch(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
-    if (tc_backward_weights_workspace_bytes(p.d) > kStaticScratchBytes) return FLASHMHF_ERR_SCRATCH_LIMIT;
+    // one set of partial sums has to fit; a plan that wants more of them than fit gives way to one that does not
+    if ((size_t)p.d.Hkuv * p.d.E * p.d.De * p.d.Dh * 3 * sizeof(float) > kStaticScratchBytes) return FLASHMHF_ERR_SCRATCH_LIMIT;
     void *ptr = nullptr;
     const int rc = static_scratch_ptr(&ptr);
     if (rc != FLASHMHF_OK) return rc;

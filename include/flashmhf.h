@@ -42,7 +42,7 @@ typedef enum flashmhf_status {
     FLASHMHF_ERR_ARCH = -7,          /* current device is not compute capability 10.x */
     FLASHMHF_ERR_CUDA = -8,          /* a CUDA runtime/driver call failed (see flashmhf_last_cuda_error) */
     FLASHMHF_ERR_DEVICE_TIMEOUT = -9, /* a kernel gave up on a bounded wait and returned early (flashmhf_device_status) */
-    FLASHMHF_ERR_SCRATCH_LIMIT = -10  /* flashmhf_backward_static_scratch: these dims need more than FLASHMHF_STATIC_SCRATCH_BYTES */
+    FLASHMHF_ERR_SCRATCH_LIMIT = -10  /* flashmhf_backward_static_scratch: dK, dU, dV in fp32 exceed FLASHMHF_STATIC_SCRATCH_BYTES */
 } flashmhf_status;
 
 typedef enum flashmhf_dtype {
@@ -174,8 +174,9 @@ int flashmhf_backward_inputs(const flashmhf_bwd_params *p, void *stream);
  * as flashmhf_backward, but `workspace` / `workspace_bytes` are ignored: the partial sums of dK, dU
  * and dV go to a static array inside the library (FLASHMHF_STATIC_SCRATCH_BYTES per GPU that loads
  * the library, held until the process exits).  The caller still passes every input and output.
- *   - bf16 only.  Dims whose flashmhf_backward_workspace_bytes() exceeds the array are refused
- *     with FLASHMHF_ERR_SCRATCH_LIMIT; nothing is launched.
+ *   - bf16 only.  Dims whose dK, dU and dV in fp32 (12 * H_kuv * E * d_e * d_h bytes) exceed the array are refused
+ *     with FLASHMHF_ERR_SCRATCH_LIMIT; nothing is launched.  Where flashmhf_backward_workspace_bytes() exceeds it, the
+ *     token axis is cut into fewer parts than flashmhf_backward would: the same results up to the order of the fp32 sums.
  *   - The call makes no cudaMalloc, cudaFree or other allocating call.  Its FIRST call on a device
  *     looks up the array's device address (once per device, with that device current).
  *   - All calls on a device share the one array and it keeps the previous call's contents.  The
