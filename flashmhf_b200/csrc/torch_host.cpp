@@ -588,8 +588,8 @@ Tensor mhffn_layer(const Tensor &x, const std::optional<Tensor> &w1, const std::
                    const Tensor &router, const Tensor &gate, const Tensor &up, const Tensor &down, const std::optional<Tensor> &w2,
                    const std::optional<Tensor> &b2, int64_t Hkuv, double eps, double hs, double us, double fs) {
     auto plain = [](const std::optional<Tensor> &t) { return !t || t->scalar_type() == at::kBFloat16; };
-    if (x.dim() == 3 && expert_ok(gate) && expert_ok(up) && expert_ok(down) && plain(x) && plain(w1) && plain(b1) && plain(w2) && plain(b2) && !at::autocast::is_autocast_enabled(at::kCUDA))
-    {
+    if (x.is_cuda() && x.dim() == 3 && expert_ok(gate) && expert_ok(up) && expert_ok(down) && plain(x) && plain(w1) && plain(b1) && plain(w2) &&
+        plain(b2) && !at::autocast::is_autocast_enabled(at::kCUDA)) {
         auto wants = [](const std::optional<Tensor> &t) { return t && t->requires_grad(); };
         if (at::GradMode::is_enabled() && (wants(x) || wants(w1) || wants(b1) || wants(q_norm) || wants(router) || wants(gate) || wants(up) ||
                                            wants(down) || wants(w2) || wants(b2)))
