@@ -53,6 +53,8 @@ def mhffn_layer(x, p, *, H, Hkuv, E, apply_rmsnorm, eps=1e-5, head_scaling=1.0, 
     b1 = p.get("w_self_bias") if w1 is not None else None
     b2 = p.get("w_self_2_bias") if w2 is not None else None
     q_norm = p["q_norm"] if apply_rmsnorm else None
+    if p["router"].shape[-1] != E:
+        raise ValueError(f"router must be [H, d_h, {E}], got {tuple(p['router'].shape)}")
     if E <= 32:
         return _lib.native().mhffn_layer(x, w1, b1, q_norm, p["router"], p["gate_weight"], p["up_weight"], p["down_weight"], w2, b2,
                                          Hkuv, eps, head_scaling, up_scaling, final_scaling)
