@@ -524,9 +524,9 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         variable_list out(15);
         if (!grads[0].defined()) return out;
+        const variable_list sv = ctx->get_saved_variables();   // (may run the caller's hooks, and a checkpointed region again)
         std::optional<at::AutoDispatchBelowADInplaceOrView> below;
         if (!at::GradMode::is_enabled()) below.emplace();
-        const variable_list sv = ctx->get_saved_variables();
         const std::vector<double> k = ctx->saved_data["k"].toDoubleVector();
         const std::vector<int64_t> n = ctx->saved_data["i"].toIntVector();
         const Tensor &x = sv[0], &w1 = sv[1], &O = sv[10], &w2 = sv[11], &R = sv[6];
