@@ -405,7 +405,8 @@ struct PrologueFunction : public torch::autograd::Function<PrologueFunction> {
     }
     static variable_list backward(AutogradContext *ctx, variable_list grads) {
         const variable_list sv = ctx->get_saved_variables();
-        Prologue a{sv[0], sv[1], sv[2], sv[0].size(0), sv[0].size(1), sv[2].size(0), sv[2].size(1), sv[2].size(2),
+        auto rows = [](const Tensor &t) { return t.defined() ? t.contiguous() : t; };   // (a hook may have given back another layout)
+        Prologue a{rows(sv[0]), rows(sv[1]), rows(sv[2]), sv[0].size(0), sv[0].size(1), sv[2].size(0), sv[2].size(1), sv[2].size(2),
                    ctx->saved_data["eps"].toDouble()};
         Tensor dQ = grads[0], dR = grads[1];
         if (!dQ.defined()) dQ = at::zeros({a.B, a.H, a.S, a.Dh}, a.x.options());
@@ -529,8 +530,12 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
         if (!at::GradMode::is_enabled()) below.emplace();
         const std::vector<double> k = ctx->saved_data["k"].toDoubleVector();
         const std::vector<int64_t> n = ctx->saved_data["i"].toIntVector();
-        const Tensor &x = sv[0], &w1 = sv[1], &O = sv[10], &w2 = sv[11], &R = sv[6];
-        const Prologue a{sv[2], sv[3], sv[4], sv[2].size(0), sv[2].size(1), sv[4].size(0), sv[4].size(1), sv[4].size(2), k[0]};
+        // The kernels take these by address, in the layout in which they were saved; what a hook gave back may have another.
+        const Tensor &x = sv[0], &w1 = sv[1], &w2 = sv[11];
+        auto rows = [](const Tensor &t) { return t.defined() ? t.contiguous() : t; };
+        auto weight = [](const Tensor &t) { return expert_ok(t) ? t : t.contiguous(); };
+        const Tensor q = rows(sv[5]), R = rows(sv[6]), O = rows(sv[10]);
+        const Prologue a{rows(sv[2]), rows(sv[3]), rows(sv[4]), sv[2].size(0), sv[2].size(1), sv[4].size(0), sv[4].size(1), sv[4].size(2), k[0]};
         // which arguments want a gradient (autograd numbers the tensors that were passed)
         const bool given[10] = {true, w1.defined(), n[3] != 0, a.w.defined(), true, true, true, true, w2.defined(), n[4] != 0};
         bool need[10];
@@ -547,7 +552,7 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
         if (w2.defined()) d = d.mm(w2);
         d = d.contiguous();
         const bool inputs = parts & FLASHMHF_BWD_INPUTS, weights = parts & FLASHMHF_BWD_WEIGHTS;
-        const Tensor &gate = sv[7], &up = sv[8], &down = sv[9];
+        const Tensor gate = weight(sv[7]), up = weight(sv[8]), down = weight(sv[9]);
         c10::cuda::CUDAGuard guard(d.device());
         flashmhf_bwd_params p{};
         p.d = dims_of(Shape{a.B, a.H, a.S, a.Dh, n[0], a.E, gate.size(0) / a.E}, at::kBFloat16);
@@ -556,7 +561,7 @@ struct LayerFunction : public torch::autograd::Function<LayerFunction> {
         p.workspace_bytes = weights ? api.backward_ws(&p.d) : api.backward_inputs_ws(&p.d);
         const Tensor tmp = at::empty({(int64_t)(dq_bytes + dr_bytes + p.workspace_bytes + 1)}, d.options().dtype(at::kByte));
         char *base = static_cast<char *>(tmp.data_ptr());
-        p.Q = heads_address(sv[5].data_ptr(), a); p.dO = heads_address(d.data_ptr(), a); p.R = routing_address(R.data_ptr(), a);
+        p.Q = heads_address(q.data_ptr(), a); p.dO = heads_address(d.data_ptr(), a); p.R = routing_address(R.data_ptr(), a);
         p.K = expert_address(gate, a.Dh, p.d.De); p.U = expert_address(up, a.Dh, p.d.De); p.V = expert_address(down, a.Dh, p.d.De);
         p.dQ = heads_address(base, a); p.dR = routing_address(base + dq_bytes, a);
         p.workspace = base + dq_bytes + dr_bytes;

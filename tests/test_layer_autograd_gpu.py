@@ -1,8 +1,10 @@
-"""GPU: the layer's native call under the parts of autograd that look inside it: recomputation."""
+"""GPU: the layer's native call under the parts of autograd that look inside it: recomputation and saved-tensor hooks."""
 import pytest
 import torch
 import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint
+
+from oracle import mhffn_oracle as orc
 
 pytestmark = pytest.mark.gpu
 KW = dict(H=4, Hkuv=2, E=3, apply_rmsnorm=True)
@@ -27,3 +29,17 @@ def test_recomputed_in_backward():
     got = torch.autograd.grad(checkpoint(fn, x, use_reentrant=False), leaves, dy)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def test_saved_tensors_come_back_in_another_layout():
+    """What an unpack hook returns has the values and the shape of what was saved; its strides may be others."""
+    import flashmhf_b200 as fm
+    x, _, p, dy = _inputs()
+    leaves = [x, *p.values()]
+    want = torch.autograd.grad(fm.mhffn_layer(x, p, **KW), leaves, dy)
+    turn = lambda t: t.transpose(-1, -2).contiguous().transpose(-1, -2) if t.dim() > 1 else t
+    with torch.autograd.graph.saved_tensors_hooks(turn, lambda t: t):
+        y = fm.mhffn_layer(x, p, **KW)
+    got = torch.autograd.grad(y, leaves, dy)
+    for a, b in zip(got, want):
+        assert orc.rel_l2(a, b) < 1e-3   # (a library product may round otherwise for another layout)
