@@ -99,6 +99,8 @@ void check(int status) {
 
 void *current_stream(const Tensor &t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
+bool has_tangent(const Tensor &t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
 struct Shape {
     int64_t B, H, S, Dh, Hk, E, De;
 };
@@ -595,9 +597,10 @@ Tensor mhffn_layer(const Tensor &x, const std::optional<Tensor> &w1, const std::
     auto plain = [](const std::optional<Tensor> &t) { return !t || t->scalar_type() == at::kBFloat16; };
     if (x.is_cuda() && x.dim() == 3 && expert_ok(gate) && expert_ok(up) && expert_ok(down) && plain(x) && plain(w1) && plain(b1) && plain(w2) &&
         plain(b2) && !at::autocast::is_autocast_enabled(at::kCUDA)) {
-        auto wants = [](const std::optional<Tensor> &t) { return t && t->requires_grad(); };
-        if (at::GradMode::is_enabled() && (wants(x) || wants(w1) || wants(b1) || wants(q_norm) || wants(router) || wants(gate) || wants(up) ||
-                                           wants(down) || wants(w2) || wants(b2)))
+        // (a tangent goes through the node as well, which refuses it: there is no forward-mode derivative)
+        const bool grad = at::GradMode::is_enabled();
+        auto wants = [grad](const std::optional<Tensor> &t) { return t && ((grad && t->requires_grad()) || has_tangent(*t)); };
+        if (wants(x) || wants(w1) || wants(b1) || wants(q_norm) || wants(router) || wants(gate) || wants(up) || wants(down) || wants(w2) || wants(b2))
             return LayerFunction::apply(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs);
         return layer_forward(x, w1, b1, q_norm, router, gate, up, down, w2, b2, Hkuv, eps, hs, us, fs, false).y;
     }
@@ -698,6 +701,7 @@ std::pair<Tensor, Tensor> rotary_pair(const Tensor &q, const Tensor &k, const Te
 // lm.Attention.forward; a forward pass over a short input waits for the interpreter, not for the GPU).
 Tensor lm_attention(const Tensor &x, const Tensor &wq, const Tensor &wk, const Tensor &wv, const Tensor &wo, int64_t nh, int64_t nkv,
                     const Tensor &cos_t, const Tensor &sin_t) {
+    for (const Tensor &t : {x, wq, wk, wv, wo}) TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(t), "attention in one call has no forward-mode derivative");
     at::AutoDispatchBelowADInplaceOrView below;
     const int64_t B = x.size(0), S = x.size(1), hd = wq.size(0) / nh;
     auto heads = [&](const Tensor &w, int64_t n) { return project(x, w, std::nullopt).view({B, S, n, hd}); };

@@ -1,7 +1,8 @@
-"""GPU: the layer's native call under the parts of autograd that look inside it: recomputation and saved-tensor hooks."""
+"""GPU: the layer's native call under the parts of autograd that look inside it: recomputation, saved-tensor hooks and forward mode."""
 import pytest
 import torch
 import torch.nn.functional as F
+import torch.autograd.forward_ad as fwAD
 from torch.utils.checkpoint import checkpoint
 
 from oracle import mhffn_oracle as orc
@@ -43,3 +44,26 @@ def test_saved_tensors_come_back_in_another_layout():
     got = torch.autograd.grad(y, leaves, dy)
     for a, b in zip(got, want):
         assert orc.rel_l2(a, b) < 1e-3   # (a library product may round otherwise for another layout)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_forward_mode_is_refused(grad):
+    """There is no forward-mode derivative: an input that carries a tangent is an error, not a result without one."""
+    import flashmhf_b200 as fm
+    from flashmhf_b200 import lm, lm_ops
+    x, _, p, _ = _inputs(False)
+    with torch.set_grad_enabled(grad), fwAD.dual_level():
+        for name in ("x", "router", "gate_weight"):
+            q = dict(p)
+            t = x if name == "x" else p[name]
+            dual = fwAD.make_dual(t, torch.ones_like(t))
+            if name != "x":
+                q[name] = dual
+            with pytest.raises((RuntimeError, NotImplementedError)):
+                fm.mhffn_layer(dual if name == "x" else x, q, **KW)
+    cfg = lm.LMConfig(hidden_size=256, num_attention_heads=4, num_key_value_heads=4)
+    att = lm.Attention(cfg).cuda().bfloat16()
+    cos, sin = lm.rotary_tables(75, 64, 10000.0, x.device, torch.bfloat16)
+    with torch.set_grad_enabled(grad), fwAD.dual_level():
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            att(fwAD.make_dual(x, torch.ones_like(x)), cos, sin, tables=lm_ops.rotary_tables_f32(cos, sin))
