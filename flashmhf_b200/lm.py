@@ -17,6 +17,16 @@ from dataclasses import dataclass
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules import module as _nn_module
+
+
+def _as_written(m, cls):
+    """May the steps of module ``m`` be taken without calling it?  Only where it is a plain ``cls``: not a wrapper or a subclass in its
+    place (LoRA, quantised, sharded, checkpointed, compiled), its ``forward`` not replaced, and nothing hooked to it."""
+    return (type(m) is cls and "forward" not in m.__dict__ and m._compiled_call_impl is None and
+            not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or
+                 _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or
+                 _nn_module._global_backward_hooks or _nn_module._global_backward_pre_hooks))
 
 
 @dataclass
@@ -387,7 +397,11 @@ class DecoderLM(nn.Module):
             from . import lm_ops
             tables = lm_ops.rotary_tables_f32(cos, sin)
         for i, layer in enumerate(self.model.layers):
-            h, d = layer.step(h, d, cos, sin, None if cache is None else (cache.k[i], cache.v[i]), link, tables)
+            kv = None if cache is None else (cache.k[i], cache.v[i])
+            if _as_written(layer, DecoderLayer):
+                h, d = layer.step(h, d, cos, sin, kv, link, tables)
+            else:
+                h, d = layer(h if d is None else h + d, cos, sin, kv, link), None
         if link is not None:
             link.finish()
         return add_norm(self.model.norm, h, d)[1]
