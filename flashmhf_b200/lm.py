@@ -90,11 +90,11 @@ class RMSNorm(nn.Module):
 
 
 def add_norm(norm, h, d):
-    """(h + d, norm(h + d)): the residual addition and the RMSNorm behind it; one kernel on CUDA bf16 tensors.  ``d`` may be
-    None (nothing to add)."""
+    """(h + d, norm(h + d)): the residual addition and the norm behind it; one kernel on CUDA bf16 tensors where it is a plain
+    RMSNorm.  ``d`` may be None (nothing to add)."""
     if d is None:
         return h, norm(h)
-    if h.is_cuda and h.dtype == torch.bfloat16 and d.dtype == torch.bfloat16:
+    if _as_written(norm, RMSNorm) and h.is_cuda and h.dtype == torch.bfloat16 and d.dtype == torch.bfloat16:
         from . import lm_ops
         if h.shape[-1] in lm_ops.NORM_SIZES:
             return lm_ops.add_rmsnorm(h, d, norm.weight, norm.eps)

@@ -1,0 +1,44 @@
+"""GPU: norms and projections of the LM that are hooked, wrapped or replaced take part in the forward pass, which takes the plain ones'
+steps in joined native calls."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle import mhffn_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _model():
+    from flashmhf_b200 import lm
+    cfg = lm.LMConfig(vocab_size=97, hidden_size=768, num_hidden_layers=2, num_attention_heads=12, num_key_value_heads=12, intermediate_size=128,
+                      mhffnmoe_num_heads=8, mhffnmoe_num_kuv_heads=8, mhffnmoe_num_experts=2, mhffnmoe_apply_rmsnorm=False)
+    m = lm.DecoderLM(cfg).cuda().bfloat16().init_weights(seed=1)
+    return m, torch.randint(0, 97, (2, 40), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+
+
+class _Shifted(torch.nn.Module):
+    """Another norm in the place of an RMSNorm, with the same attributes."""
+
+    def __init__(self, norm):
+        super().__init__()
+        self.weight, self.eps = norm.weight, norm.eps
+
+    def forward(self, x):
+        return F.layer_norm(x, (x.shape[-1],), self.weight, None, self.eps) + 1
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_norms(grad):
+    m, ids = _model()
+    with torch.set_grad_enabled(grad):
+        want, seen = m(ids), []
+        norms = [m.model.layers[0].post_attention_layernorm, m.model.layers[1].input_layernorm, m.model.norm]
+        hooks = [n.register_forward_hook(lambda mod, a, out: seen.append(mod)) for n in norms]
+        assert orc.rel_l2(m(ids), want) < 2e-2 and seen == norms
+        for h in hooks:
+            h.remove()
+        m.model.norm = _Shifted(m.model.norm)
+        shifted = m(ids)
+        m.model.norm, last = torch.nn.Identity(), m.model.norm
+        assert orc.rel_l2(shifted, m.lm_head(last(m.hidden(ids)))) < 2e-2
