@@ -172,11 +172,12 @@ class Attention(nn.Module):
         ``link``: optional SequenceLink when a sequence is split over two ranks: the rank with the earlier part sends
         its keys and values on, the rank with the later part receives them and attends over both parts."""
         B, S, _ = x.shape
-        if tables is not None and kv_out is None and link is None and self.hd % 16 == 0 and x.dtype == self.q_proj.weight.dtype and \
-                not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda"):
-            from . import lm_ops   # the steps below in one native call
-            return lm_ops.attention(x, self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.o_proj.weight, self.nh, self.nkv,
-                                    *tables)
+        if tables is not None and kv_out is None and link is None and self.hd % 16 == 0 and not torch.is_grad_enabled() and \
+                not torch.is_autocast_enabled("cuda"):
+            proj = (self.q_proj, self.k_proj, self.v_proj, self.o_proj)
+            if all(_as_written(p, nn.Linear) and p.bias is None and p.weight.dtype == x.dtype for p in proj):
+                from . import lm_ops   # the steps below in one native call
+                return lm_ops.attention(x, *(p.weight for p in proj), self.nh, self.nkv, *tables)
         q = self.q_proj(x).view(B, S, self.nh, self.hd)
         k = self.k_proj(x).view(B, S, self.nkv, self.hd)
         v = self.v_proj(x).view(B, S, self.nkv, self.hd).transpose(1, 2)

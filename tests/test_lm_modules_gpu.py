@@ -42,3 +42,40 @@ def test_norms(grad):
         shifted = m(ids)
         m.model.norm, last = torch.nn.Identity(), m.model.norm
         assert orc.rel_l2(shifted, m.lm_head(last(m.hidden(ids)))) < 2e-2
+
+
+class _LowRank(torch.nn.Module):
+    """A projection with an addition of its own, as an adapter puts it in place."""
+
+    def __init__(self, lin):
+        super().__init__()
+        self.base, self.weight = lin, lin.weight
+        self.down = torch.nn.Parameter(torch.full((4, lin.in_features), 0.02, device="cuda", dtype=torch.bfloat16))
+        self.up = torch.nn.Parameter(torch.full((lin.out_features, 4), 0.05, device="cuda", dtype=torch.bfloat16))
+
+    def forward(self, x):
+        return self.base(x) + F.linear(F.linear(x, self.down), self.up)
+
+
+@pytest.mark.parametrize("name", ["q_proj", "k_proj", "v_proj", "o_proj"])
+def test_projections(name):
+    m, ids = _model()
+    att = m.model.layers[0].self_attn
+    with torch.no_grad():
+        plain, seen = m(ids), []
+        h = getattr(att, name).register_forward_hook(lambda mod, a, out: seen.append(out.shape))
+        assert orc.rel_l2(m(ids), plain) < 2e-2 and len(seen) == 1
+        h.remove()
+        setattr(att, name, _LowRank(getattr(att, name)))
+        got = m(ids)
+        lin = getattr(att, name)
+        bias = torch.nn.Linear(768, 768, device="cuda", dtype=torch.bfloat16)
+        bias.weight.copy_(lin.weight)
+        bias.bias.fill_(0.5)
+        setattr(att, name, bias)
+        biased = m(ids)
+    with torch.enable_grad():        # every module is called here
+        setattr(att, name, lin)
+        assert orc.rel_l2(got, m(ids).detach()) < 2e-2
+        setattr(att, name, bias)
+        assert orc.rel_l2(biased, m(ids).detach()) < 2e-2
