@@ -613,6 +613,14 @@ Tensor mhffn_layer(const Tensor &x, const std::optional<Tensor> &w1, const std::
 }
 
 // ------------------------------------------------------------------------------------------------ LM helpers
+// The kernels take addresses and trust the sizes: bf16 [B,S,heads,hd] with tables of at least S rows of hd/2, all on one GPU.
+void check_rope(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t) {
+    if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 4) throw py::value_error("rotary embedding expects CUDA bf16 [B,S,heads,head_dim]");
+    for (const Tensor &t : {cos_t, sin_t})
+        if (t.device() != x.device() || t.scalar_type() != at::kFloat || t.dim() != 2 || !t.is_contiguous() || t.size(0) < x.size(1) ||
+            t.size(1) * 2 != x.size(3))
+            throw py::value_error("rotary tables must be contiguous fp32 [S or more, head_dim/2] on the activations' device");
+}
 Tensor run_rope(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t, bool transpose) {
     c10::cuda::CUDAGuard guard(x.device());
     Tensor y = at::empty_like(x);
@@ -623,6 +631,7 @@ Tensor run_rope(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t, bool 
 }
 struct RotaryFunction : public torch::autograd::Function<RotaryFunction> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x, const Tensor &cos_t, const Tensor &sin_t) {
+        check_rope(x, cos_t, sin_t);
         ctx->save_for_backward({cos_t, sin_t});
         return run_rope(x.contiguous(), cos_t, sin_t, false);
     }
@@ -633,8 +642,15 @@ struct RotaryFunction : public torch::autograd::Function<RotaryFunction> {
 };
 Tensor rotary(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t) { return RotaryFunction::apply(x, cos_t, sin_t); }
 
+// bf16 [..., n] and a weight of n values on the same GPU
+void check_norm(const Tensor &x, const Tensor &weight) {
+    if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() < 1) throw py::value_error("RMSNorm expects a CUDA bf16 tensor");
+    if (weight.device() != x.device() || weight.numel() != x.size(-1))
+        throw py::value_error("RMSNorm weight must have " + std::to_string(x.size(-1)) + " values on " + x.device().str() + ", got " + dims_text(weight));
+}
 struct RMSNormFunction : public torch::autograd::Function<RMSNormFunction> {
     static Tensor forward(AutogradContext *ctx, const Tensor &x0, const Tensor &weight, double eps) {
+        check_norm(x0, weight);
         const Tensor x = x0.contiguous();
         const Tensor w = (weight.scalar_type() == at::kBFloat16 ? weight.detach() : weight.detach().to(at::kFloat)).contiguous();
         c10::cuda::CUDAGuard guard(x.device());
@@ -662,6 +678,11 @@ struct RMSNormFunction : public torch::autograd::Function<RMSNormFunction> {
 };
 Tensor rmsnorm(const Tensor &x, const Tensor &weight, double eps) { return RMSNormFunction::apply(x, weight, eps); }
 
+void check_rope_pair(const Tensor &q, const Tensor &k, const Tensor &cos_t, const Tensor &sin_t) {
+    check_rope(q, cos_t, sin_t);
+    check_rope(k, cos_t, sin_t);
+    if (k.device() != q.device() || k.size(0) != q.size(0) || k.size(1) != q.size(1)) throw py::value_error("queries and keys must have the same B and S");
+}
 // queries [B,S,nq,hd] and keys [B,S,nk,hd], both rotated in one launch
 variable_list run_rope_pair(const Tensor &q, const Tensor &k, const Tensor &cos_t, const Tensor &sin_t, bool transpose) {
     c10::cuda::CUDAGuard guard(q.device());
@@ -674,6 +695,7 @@ variable_list run_rope_pair(const Tensor &q, const Tensor &k, const Tensor &cos_
 }
 struct RotaryPairFunction : public torch::autograd::Function<RotaryPairFunction> {
     static variable_list forward(AutogradContext *ctx, const Tensor &q, const Tensor &k, const Tensor &cos_t, const Tensor &sin_t) {
+        check_rope_pair(q, k, cos_t, sin_t);
         ctx->save_for_backward({cos_t, sin_t});
         ctx->saved_data["shape"] = std::vector<int64_t>{q.size(2), k.size(2)};
         return run_rope_pair(q.contiguous(), k.contiguous(), cos_t, sin_t, false);
@@ -706,6 +728,7 @@ Tensor lm_attention(const Tensor &x, const Tensor &wq, const Tensor &wk, const T
     const int64_t B = x.size(0), S = x.size(1), hd = wq.size(0) / nh;
     auto heads = [&](const Tensor &w, int64_t n) { return project(x, w, std::nullopt).view({B, S, n, hd}); };
     const Tensor q = heads(wq, nh), k = heads(wk, nkv), v = heads(wv, nkv).transpose(1, 2);
+    check_rope_pair(q, k, cos_t, sin_t);
     const variable_list r = run_rope_pair(q, k, cos_t, sin_t, false);
     const Tensor o = at::scaled_dot_product_attention(r[0].transpose(1, 2), r[1].transpose(1, 2), v, std::nullopt, 0.0, /*is_causal=*/true,
                                                       std::nullopt, /*enable_gqa=*/nkv != nh);
@@ -715,6 +738,9 @@ Tensor lm_attention(const Tensor &x, const Tensor &wq, const Tensor &wk, const T
 // (h + d, RMSNorm(h + d) * weight)
 struct AddRMSNormFunction : public torch::autograd::Function<AddRMSNormFunction> {
     static variable_list forward(AutogradContext *ctx, const Tensor &h0, const Tensor &d0, const Tensor &weight, double eps) {
+        check_norm(h0, weight);
+        if (d0.sizes() != h0.sizes() || d0.scalar_type() != h0.scalar_type() || d0.device() != h0.device())
+            throw py::value_error("add_rmsnorm expects two tensors alike, got " + dims_text(h0) + " and " + dims_text(d0));
         const Tensor h = h0.contiguous(), d = d0.contiguous();
         const Tensor w = (weight.scalar_type() == at::kBFloat16 ? weight.detach() : weight.detach().to(at::kFloat)).contiguous();
         c10::cuda::CUDAGuard guard(h.device());

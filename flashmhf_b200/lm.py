@@ -94,7 +94,7 @@ def add_norm(norm, h, d):
     RMSNorm.  ``d`` may be None (nothing to add)."""
     if d is None:
         return h, norm(h)
-    if _as_written(norm, RMSNorm) and h.is_cuda and h.dtype == torch.bfloat16 and d.dtype == torch.bfloat16:
+    if _as_written(norm, RMSNorm) and h.is_cuda and h.dtype == torch.bfloat16 and d.dtype == torch.bfloat16 and d.shape == h.shape:
         from . import lm_ops
         if h.shape[-1] in lm_ops.NORM_SIZES:
             return lm_ops.add_rmsnorm(h, d, norm.weight, norm.eps)
@@ -172,8 +172,8 @@ class Attention(nn.Module):
         ``link``: optional SequenceLink when a sequence is split over two ranks: the rank with the earlier part sends
         its keys and values on, the rank with the later part receives them and attends over both parts."""
         B, S, _ = x.shape
-        if tables is not None and kv_out is None and link is None and self.hd % 16 == 0 and not torch.is_grad_enabled() and \
-                not torch.is_autocast_enabled("cuda"):
+        if tables is not None and kv_out is None and link is None and x.is_cuda and x.dtype == torch.bfloat16 and self.hd % 16 == 0 and \
+                not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda"):
             proj = (self.q_proj, self.k_proj, self.v_proj, self.o_proj)
             if all(_as_written(p, nn.Linear) and p.bias is None and p.weight.dtype == x.dtype for p in proj):
                 from . import lm_ops   # the steps below in one native call

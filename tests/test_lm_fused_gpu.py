@@ -64,3 +64,27 @@ def test_attention_without_gradients_equals_the_module_path(B, S, kv):
     with torch.no_grad():
         got = att(x, cos, sin, tables=tables)
     assert orc.rel_l2(got.float(), want.float()) < 1e-2
+
+
+def test_sizes_that_do_not_fit_are_refused():
+    """Before an address goes to a kernel; an addend that would have to be broadcast takes the separate steps."""
+    from flashmhf_b200 import lm, lm_ops
+    rnd = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    x, w = rnd(4, 6, 768), torch.ones(768, device="cuda", dtype=torch.bfloat16)
+    for d in (rnd(1, 6, 768), rnd(4, 6, 767), rnd(4, 6, 768).float(), rnd(4, 6, 768).cpu()):
+        with pytest.raises(ValueError):
+            lm_ops.add_rmsnorm(x, d, w, 1e-5)
+    for weight in (w[:512], w[:1], w.cpu()):
+        with pytest.raises(ValueError):
+            lm_ops.add_rmsnorm(x, x, weight, 1e-5)
+        with pytest.raises(ValueError):
+            lm_ops.RMSNormFunction.apply(x, weight, 1e-5)
+    q, k = rnd(2, 9, 4, 32), rnd(2, 9, 2, 32)
+    ct, st = lm_ops.rotary_tables_f32(*lm.rotary_tables(9, 32, 10000.0, q.device, torch.bfloat16))
+    for args in ((q, k, ct[:8], st), (q, k, ct, st[:, :8]), (q, k[:, :8], ct, st), (q, k[:1], ct, st), (q, k.float(), ct, st), (q, k, ct.cpu(), st)):
+        with pytest.raises(ValueError):
+            lm_ops.rotary_pair(*args)
+    norm = lm.RMSNorm(768, 1e-5).cuda().bfloat16()
+    d = rnd(1, 6, 768)
+    s, y = lm.add_norm(norm, x, d)
+    assert torch.equal(s, x + d) and torch.equal(y, norm(x + d))
