@@ -335,6 +335,10 @@ Prologue prologue_args(const Tensor &x_proj, const std::optional<Tensor> &q_norm
         throw py::value_error("hidden size " + std::to_string(x_proj.size(2)) + " != H*d_h = " + std::to_string(a.H) + "*" + std::to_string(a.Dh));
     if ((a.Dh != 64 && a.Dh != 96 && a.Dh != 128) || a.E > 32)
         throw py::value_error("fused_prologue supports d_h in {64, 96, 128} and at most 32 sub-networks");
+    for (const Tensor *t : {&router, q_norm ? &*q_norm : &router})
+        if (t->device() != x_proj.device()) throw py::value_error("router and norm weight must be on the activations' device, " + x_proj.device().str());
+    if (q_norm && q_norm->numel() != a.H * a.Dh)
+        throw py::value_error("norm weight must have " + std::to_string(a.H) + "*" + std::to_string(a.Dh) + " values, got " + dims_text(*q_norm));
     a.eps = eps;
     a.x = x_proj.contiguous();
     // bf16 parameters are read as they are; any other mix goes in as fp32
@@ -617,8 +621,8 @@ Tensor mhffn_layer(const Tensor &x, const std::optional<Tensor> &w1, const std::
 void check_rope(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t) {
     if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 4) throw py::value_error("rotary embedding expects CUDA bf16 [B,S,heads,head_dim]");
     for (const Tensor &t : {cos_t, sin_t})
-        if (t.device() != x.device() || t.scalar_type() != at::kFloat || t.dim() != 2 || !t.is_contiguous() || t.size(0) < x.size(1) ||
-            t.size(1) * 2 != x.size(3))
+        if (t.device() != x.device() || t.scalar_type() != at::kFloat || t.dim() < 1 || !t.is_contiguous() || t.size(-1) * 2 != x.size(3) ||
+            t.numel() < x.size(1) * t.size(-1))
             throw py::value_error("rotary tables must be contiguous fp32 [S or more, head_dim/2] on the activations' device");
 }
 Tensor run_rope(const Tensor &x, const Tensor &cos_t, const Tensor &sin_t, bool transpose) {

@@ -47,3 +47,13 @@ def test_layer_node_equals_its_parts(norm, proj, bias, fp32_router, frozen):
         assert a.dtype == b.dtype and a.shape == b.shape, name
         assert _rel(a, b) < 5e-3, name
     fm.check_device_status()
+
+
+def test_parameters_that_do_not_fit_are_refused():
+    """Before their addresses go to a kernel."""
+    import flashmhf_b200 as fm
+    x = torch.zeros(1, 4, 256, device="cuda", dtype=torch.bfloat16)
+    router, norm = torch.zeros(4, 64, 2, device="cuda"), torch.ones(4, 64, device="cuda")
+    for r, n in ((router.cpu(), norm), (router, norm.cpu()), (router, norm[:2])):
+        with pytest.raises(ValueError):
+            fm.fused_prologue(x, n, r)
