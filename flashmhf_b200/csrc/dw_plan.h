@@ -9,6 +9,7 @@
 #include "kernels.h"
 
 namespace fmhf {
+namespace {   // (a table shared by two builds of the library in one process would mix their plans)
 
 struct DwPlan {
     int tiles_per_seq, tiles_total, nsplit, tiles_per_split;
@@ -211,4 +212,5 @@ inline DwPlan dw_plan(const flashmhf_dims &d, int num_sms, bool followed, size_t
     return e.p;
 }
 
+}  // namespace
 }  // namespace fmhf
