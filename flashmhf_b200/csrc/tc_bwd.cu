@@ -1238,8 +1238,7 @@ struct ReduceArgs {
     long long first;  // element of a plane where the split blocks begin (those before are written by their CTAs)
     int nsplit, I, DH;
 };
-// 128 threads and 48 registers: a CTA fits beside one of the dK/dU/dV kernel, waits there for that kernel to end, and then beside one
-// of the dQ/dR kernel, under which the addition runs.
+// Launched early: what its CTAs have to set up is done when the kernel before it ends.
 __global__ void __maxnreg__(48) dw_reduce_kernel(const ReduceArgs a) {
     griddep_launch_dependents();
     griddep_wait();
@@ -1268,7 +1267,9 @@ __global__ void __maxnreg__(48) dw_reduce_kernel(const ReduceArgs a) {
 
 // dQ/dR: with few token tiles the sub-networks are split over CTAs.  In 64-row blocks (about 0.8 us): a CTA costs six besides
 // its blocks, the reduction three and its partial sums.  Splits only while the tiles are no more than two waves, and only for
-// a gain of a tenth: the split sums dQ in another order than the unsplit kernel.
+// a gain of a tenth: the split sums dQ in another order than the unsplit kernel.  (The whole backward of 14 shapes of each head
+// dimension that split, against never: 1.34x faster at d_h = 64, 1.22x at 96, 1.19x at 128; the rule does not know that unsplit CTAs may fit
+// beside a small dK/dU/dV launch: 2 x 125 tokens, 16 heads, d_h = 96, 23 sub-networks of 64, 41 against 31 us.)
 struct DqPlan {
     int nsplit, e_per_split;
 };
@@ -1374,22 +1375,6 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         if ((e = cudaGetLastError()) != cudaSuccess) { set_cuda_error(e, "bwd_dw_kernel launch"); return FLASHMHF_ERR_CUDA; }
     }
 
-    // The addition of the split blocks' partial sums: beside the dQ/dR kernel where they are few (one CTA per SM adds about 1 TB/s),
-    // else after it at full width.  (3 x 333 tokens, shared heads: backward 51 -> 44 us; 40 MB of sums beside dQ/dR: 586 -> 605.)
-    auto add_splits = [&](bool beside) -> int {
-        const long long n4 = (ra.plane - ra.first) / 4, cap = beside ? dc->num_sms / 3 : dc->num_sms * 6;   // per gradient
-        const dim3 blocks((unsigned)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap), 3);
-        prof_mark(st, kMarkStart);
-        const cudaError_t err = launch_kernel(true, dw_reduce_kernel, blocks, dim3(128), 0, st, ra);
-        prof_mark(st, kMarkBwdReduce);
-        *n_launch += 1;
-        if (err != cudaSuccess) { set_cuda_error(err, "dw_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
-        return FLASHMHF_OK;
-    };
-    const bool split = want_weights && pl.nsplit > 1;
-    const bool beside = split && want_inputs && 3.0 * (double)(ra.plane - ra.first) * 4 * pl.nsplit <= 24e6;
-    if (beside && (rc = add_splits(true)) != 0) return rc;
-
     DqPlan ql = dq_plan(d, dc->num_sms);
     float *q_part = nullptr;
     if (want_inputs) {
@@ -1410,7 +1395,19 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         *n_launch += 1;
         if (e != cudaSuccess) { set_cuda_error(e, "bwd_dq_kernel launch"); return FLASHMHF_ERR_CUDA; }
     }
-    if (split && !beside && (rc = add_splits(false)) != 0) return rc;
+    if (want_weights && pl.nsplit > 1) {
+        // The addition of the split blocks' partial sums comes last, at full width.  (In front of the dQ/dR kernel, so as to run beside
+        // it, its waiting CTAs keep that kernel's off their SMs: over 122 shapes of all head dimensions with up to 45 MB of sums the
+        // backward took 5 % longer, up to 40 % where the weights are small: 16 x 1268 tokens, one sub-network of 64 at d_h = 96,
+        // 118 against 84 us; 72 token tiles of d_h = 128 won most, 42 against 48 us.)
+        const long long n4 = (ra.plane - ra.first) / 4, cap = dc->num_sms * 6;   // per gradient
+        const dim3 blocks((unsigned)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap), 3);
+        prof_mark(st, kMarkStart);
+        e = launch_kernel(true, dw_reduce_kernel, blocks, dim3(128), 0, st, ra);
+        prof_mark(st, kMarkBwdReduce);
+        *n_launch += 1;
+        if (e != cudaSuccess) { set_cuda_error(e, "dw_reduce_kernel launch"); return FLASHMHF_ERR_CUDA; }
+    }
     if (want_inputs && ql.nsplit > 1) {
         prof_mark(st, kMarkStart);
         e = launch_o_reduce(q_part, p.dQ, d, ql.nsplit, kReduceAfterKernel, dc->num_sms, st);
