@@ -53,9 +53,8 @@ size_t tc_backward_workspace_bytes(const flashmhf_dims &d);          // all of i
 size_t tc_backward_weights_workspace_bytes(const flashmhf_dims &d);  // what the dK/dU/dV part cannot do without
 size_t tc_backward_inputs_workspace_bytes(const flashmhf_dims &d);   // what a call for dQ and dR alone can use (0: nothing)
 // Sum of `nsplit` fp32 partial planes [B,H,S,Dh], in index order, as bf16 to `out` (strides multiples of 4 elements).
-// kReduceAfterKernel: launched early, runs when the kernel before it is done; kReduceChained: between two chained forward kernels.
-enum ReduceMode { kReduceAfterKernel, kReduceChained };
-cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, ReduceMode mode, int num_sms,
+// Launched early; adds when the kernel before it is done.  `chained`: between two chained forward kernels.
+cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, bool chained, int num_sms,
                             cudaStream_t st);
 void tc_backward_plan(const flashmhf_dims &d, uint32_t parts, flashmhf_backward_plan_info *out);
 int tc_backward_static_scratch(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch);

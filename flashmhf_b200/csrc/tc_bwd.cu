@@ -35,12 +35,11 @@
 namespace fmhf {
 namespace {
 
-// Element-wise warps: 4 lane quarters x kParts column parts of a 64-column block (a thread = one token row x
-// kCols columns).  More, narrower threads shorten the arithmetic phase of a block; the fixed part of a block's
-// element-wise step (barrier waits, tensor-memory load and store latencies) does not shrink: four parts are 2-4 % slower.
-constexpr int kParts = 2, kCols = 64 / kParts, kSubs = kCols / 16;
-constexpr int kBT = 128, kBI = 64, kActThreads = 128 * kParts, kThreads = 128 + kActThreads;
-constexpr int kEpiThreads = 256;  // the warps of column parts 0 and 1 write the accumulators out
+// Element-wise warps: 4 lane quarters x two column parts of a 64-column block (a thread = one token row x kCols columns).  The fixed part
+// of a block's element-wise step (barrier waits, tensor-memory load and store latencies) does not shrink with narrower threads:
+// four parts are 2-4 % slower.
+constexpr int kCols = 32;
+constexpr int kBT = 128, kBI = 64, kActThreads = 256, kThreads = 128 + kActThreads;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTile = kBT * 128;    // one 128-row x 64-col SW128 chunk: 16 KB
 constexpr uint32_t kWChunk = kBI * 128;  // one 64-row x 64-col chunk: 8 KB
@@ -115,7 +114,7 @@ struct DqSmem {
     static constexpr uint32_t kOffQ = kOffKU + (kKUStages - 2) * kKUStage, kOffdO = kOffQ + kQBytes;
     static constexpr uint32_t kOffV = kOffKU + kKUStages * kKUStage;
     static constexpr uint32_t kOffCtl = kOffV + kVStages * kVStage;
-    static constexpr uint32_t kCtlBytes = 384 + 2 * (kParts - 1) * 128 * 4;  // barriers + two sets of dR exchange rows
+    static constexpr uint32_t kCtlBytes = 384 + 2 * 128 * 4;  // barriers + two sets of dR exchange rows
     static constexpr uint32_t kTotal = kOffCtl + kCtlBytes + 1024;
 };
 
@@ -158,7 +157,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                    sBar = base + L::kOffCtl;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(gbase + L::kOffCtl + DQ_BARS * 8);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(gbase + L::kOffCtl + DQ_BARS * 8 + 4);
-    volatile float *drx = reinterpret_cast<volatile float *>(gbase + L::kOffCtl + 384);  // [2][kParts - 1][128]
+    volatile float *drx = reinterpret_cast<volatile float *>(gbase + L::kOffCtl + 384);  // [2][128]
     auto bar = [&](int i) { return sBar + 8u * i; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -181,7 +180,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         mbar_init(bar(DQ_PEMPTY), 1);                         // the dQ update that read [dM|dN] is done
         mbar_init(bar(DQ_QT), arrivals_of(kActThreads));      // Q and dO copied to tensor memory
         for (int i = 0; i < 2; ++i) {
-            mbar_init(bar(DQ_DRFULL + i), arrivals_of(kActThreads - 128));  // column parts 1.. have written their dR_e partials
+            mbar_init(bar(DQ_DRFULL + i), arrivals_of(128));  // column part 1 has written its dR_e partial sums
             mbar_init(bar(DQ_DRFREE + i), arrivals_of(128));                 // part 0 has read them: the rows may be reused
         }
         mbar_init(bar(DQ_ACCFULL), 1);
@@ -310,17 +309,17 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             if (ok) umma_commit(bar(DQ_ACCFULL));
         }
     } else if (warp >= 4) {
-        const int quarter = warp & 3, part = (warp - 4) >> 2, half = part;  // part: which kCols of the block's 64 columns
+        const int quarter = warp & 3, part = (warp - 4) >> 2;  // part: which kCols of the block's 64 columns
         const int row = quarter * 32 + lane, t = t0 + row;
         const bool in_range = t < args.S;
         const float *rrow = args.R + (long long)b * args.r_sb + (long long)h * args.r_sh + (long long)t * args.r_ss + e0;
         float *drrow = args.dR + (long long)b * args.dr_sb + (long long)h * args.dr_sh + (long long)t * args.dr_ss + e0;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
         bool ok = true;
-        // Q and dO: shared -> tensor memory, once (thread = token row; column part p < 2 copies columns [64p, 64p + 64)
+        // Q and dO: shared -> tensor memory, once (thread = token row; column part p copies columns [64p, 64p + 64)
         // of d_h of both tiles).
         if (!mbar_wait(bar(DQ_QFULL), 0, ctl, W + 12)) ok = false;
-        if (ok && part < 2 && part * 64 < DH) {
+        if (ok && part * 64 < DH) {
 #pragma unroll
             for (int which = 0; which < 2; ++which) {
                 uint32_t v32[32];
@@ -351,45 +350,25 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             const uint32_t tS = lane_base + kColS + part * kCols, tA = lane_base + kColdA + part * kCols;
             uint32_t pm[kCols / 2], pn[kCols / 2];  // packed bf16 pairs of dM, dN for this thread's columns
             const f32x2 r2 = f2_pack(args.c * r_cur, args.c * r_cur);
-            if (kCols == 32) {
-                // the whole part at once, so that S and dA are free for the next block before any arithmetic
-                uint32_t m[32], n[32], da[32];
-                tmem_ld32x3_sync(tS, tS + kBI, tA, m, n, da);
-                tc_fence_before();
-                warp_arrive(bar(DQ_SEMPTY));
+            // the whole part at once, so that S and dA are free for the next block before any arithmetic
+            uint32_t m[kCols], n[kCols], da[kCols];
+            tmem_ld32x3_sync(tS, tS + kBI, tA, m, n, da);
+            tc_fence_before();
+            warp_arrive(bar(DQ_SEMPTY));
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const DqPair x = dq_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
-                                               f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
-                    dr2 = f2_fma(x.da, x.sn, dr2);
-                    pm[i] = f2_to_bf16x2(x.dm);
-                    pn[i] = f2_to_bf16x2(x.dn);
-                }
-            } else {
-                uint32_t m[16], n[16], da[16];
-                tmem_ld16x3_sync(tS, tS + kBI, tA, m, n, da);
-                tc_fence_before();
-                warp_arrive(bar(DQ_SEMPTY));
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const DqPair x = dq_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
-                                               f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
-                    dr2 = f2_fma(x.da, x.sn, dr2);
-                    pm[i] = f2_to_bf16x2(x.dm);
-                    pn[i] = f2_to_bf16x2(x.dn);
-                }
+            for (int i = 0; i < kCols / 2; ++i) {
+                const DqPair x = dq_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
+                                         f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
+                dr2 = f2_fma(x.da, x.sn, dr2);
+                pm[i] = f2_to_bf16x2(x.dm);
+                pn[i] = f2_to_bf16x2(x.dn);
             }
             // the dQ update of the previous block has read the [dM|dN] buffer
             if (j >= 1 && !mbar_wait(bar(DQ_PEMPTY), (j - 1) & 1, ctl, W + 8)) { ok = false; break; }
             tc_fence_after();
             const uint32_t tP = lane_base + kColP + part * kCols;
-            if (kCols == 32) {
-                tmem_st16(tP, pm);
-                tmem_st16(tP + 16, pn);
-            } else {
-                tmem_st8(tP, pm);
-                tmem_st8(tP + 8, pn);
-            }
+            tmem_st16(tP, pm);
+            tmem_st16(tP + kCols / 2, pn);
             tmem_st_wait();
             tc_fence_before();
             warp_arrive(bar(DQ_PFULL));
@@ -398,17 +377,15 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 float dr_lo, dr_hi;
                 f2_unpack(dr2, dr_lo, dr_hi);
                 const float dr_acc = (dr_lo + dr_hi) * args.c;
-                volatile float *xrow = drx + (xb * (kParts - 1)) * 128 + row;
+                volatile float *xrow = drx + xb * 128 + row;
                 if (part != 0) {
                     // the exchange rows of sub-network e were last used by e - 2: wait until those values have been read
                     if (e >= 2 && !mbar_wait(bar(DQ_DRFREE + xb), ((e >> 1) - 1) & 1, ctl, W + 11)) { ok = false; break; }
-                    xrow[(part - 1) * 128] = dr_acc;
+                    *xrow = dr_acc;
                     warp_arrive(bar(DQ_DRFULL + xb));
                 } else {
                     if (!mbar_wait(bar(DQ_DRFULL + xb), (e >> 1) & 1, ctl, W + 9)) { ok = false; break; }
-                    float sum = dr_acc;
-#pragma unroll
-                    for (int q = 0; q < kParts - 1; ++q) sum += xrow[q * 128];
+                    const float sum = dr_acc + *xrow;
                     warp_arrive(bar(DQ_DRFREE + xb));
                     if (in_range) drrow[e] = sum;
                 }
@@ -416,12 +393,11 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 ++e;
             }
         }
-        if (part >= 2) ok = false;  // the accumulator is written out by the warps of parts 0 and 1
         if (ok) ok = mbar_wait(bar(DQ_ACCFULL), 0, ctl, W + 10);
         if (ok) {
             tc_fence_after();
             constexpr int kColsPerHalf = DH / 2;
-            const int c0 = half * kColsPerHalf;
+            const int c0 = part * kColsPerHalf;
             float *pdst = args.part + ((((long long)isplit * args.B + b) * args.H + h) * args.S + t) * DH + c0;
 #pragma unroll
             for (int g = 0; g < kColsPerHalf / 16; ++g) {
@@ -450,7 +426,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             tc_fence_before();
             fence_async_smem();
         }
-        if (part < 2) named_bar_sync(1, kEpiThreads);
+        named_bar_sync(1, kActThreads);
         if (ok && warp == 4 && lane == 0 && !*abort_flag && args.nsplit == 1) {
             for (int c = 0; c < L::kChunks; ++c) tma_store_4d(&tmdQ, sQ + c * kTile, c * 64, t0, h, b);
             tma_store_commit();
@@ -737,7 +713,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             if (ok) umma_commit(bar(DW_ACCFULL));
         }
     } else if (warp >= 4) {
-        const int quarter = warp & 3, part = (warp - 4) >> 2, half = part;  // part: which kCols of the block's 64 columns
+        const int quarter = warp & 3, part = (warp - 4) >> 2;  // part: which kCols of the block's 64 columns
         const int row = quarter * 32 + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
         bool ok = true;
@@ -771,11 +747,11 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             f32x2 fq[kCols / 2], fw[kCols / 2];
             uint32_t pa[kCols / 2];
 #pragma unroll
-            for (int sub = 0; sub < kSubs; ++sub) {
+            for (int sub = 0; sub < kCols / 16; ++sub) {
                 uint32_t m[16], n[16];
                 const uint32_t c = part * kCols + sub * 16;
                 tmem_ld16x2_sync(lane_base + colS + c, lane_base + colS + kBI + c, m, n);
-                if (sub == kSubs - 1) {   // S is in registers: the buffer can take the tile after next
+                if (sub == kCols / 16 - 1) {   // S is in registers: the buffer can take the tile after next
                     tc_fence_before();
                     warp_arrive(bar(DW_SEMPTY + sb));
                 }
@@ -797,8 +773,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             uint32_t da[kCols], pm[kCols / 2], pn[kCols / 2];
             if (!mbar_wait(bar(DW_DAFULL), i & 1, ctl, W + 11)) { ok = false; break; }
             tc_fence_after();
-            if (kCols == 32) tmem_ld32_sync(lane_base + kColdA + part * kCols, da);
-            else tmem_ld16_sync(lane_base + kColdA + part * kCols, da);
+            tmem_ld32_sync(lane_base + kColdA + part * kCols, da);
             tc_fence_before();
             warp_arrive(bar(DW_DAEMPTY));
 #pragma unroll
@@ -817,7 +792,6 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             fence_async_smem();
             warp_arrive(bar(DW_PFULL));
         }
-        if (part >= 2) ok = false;  // the accumulators are written out by the warps of parts 0 and 1
         if (ok) ok = mbar_wait(bar(DW_ACCFULL), 0, ctl, W + 9);
         if (ok) {
             tc_fence_after();
@@ -830,7 +804,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 return args.out[which] + hk * args.o_head[which] + ((long long)jblk * kBI + r) * args.o_row[which];
             };
             constexpr int kColsPerHalf = DH / 2;
-            const int c0 = half * kColsPerHalf;
+            const int c0 = part * kColsPerHalf;
             {   // [dK;dU]: lane = row of the stacked block (0-63 dK, 64-127 dU)
                 float *dst = wsb + (row < kBI ? 0 : plane) + (long long)(row & (kBI - 1)) * DH + c0;
                 __nv_bfloat16 *o16 = out_row(row < kBI ? 0 : 1, row & (kBI - 1)) + c0;
@@ -846,8 +820,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     uint32_t o[16];
-                    tmem_ld16_sync(lane_base + kColV + half * 32 + g * 16, o);
-                    const int r0 = half * 32 + g * 16;
+                    tmem_ld16_sync(lane_base + kColV + part * 32 + g * 16, o);
+                    const int r0 = part * 32 + g * 16;
                     if (direct) {
 #pragma unroll
                         for (int v = 0; v < 16; ++v) out_row(2, r0 + v)[row] = __float2bfloat16(__uint_as_float(o[v]));
@@ -924,7 +898,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 bwd_dwt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
                const __grid_constant__ CUtensorMap tmV, const DwArgs args) {
-    static_assert(kParts == 2, "a thread holds 32 of a tile's 64 tokens");
     using L = DwtSmem<DH>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -1410,7 +1383,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
     }
     if (want_inputs && ql.nsplit > 1) {
         prof_mark(st, kMarkStart);
-        e = launch_o_reduce(q_part, p.dQ, d, ql.nsplit, kReduceAfterKernel, dc->num_sms, st);
+        e = launch_o_reduce(q_part, p.dQ, d, ql.nsplit, /*chained=*/false, dc->num_sms, st);
         prof_mark(st, kMarkBwdReduce);
         *n_launch += 1;
         if (e != cudaSuccess) { set_cuda_error(e, "dQ split reduction launch"); return FLASHMHF_ERR_CUDA; }

@@ -38,20 +38,11 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 // One arrival on behalf of a whole warp whose 32 lanes have all finished the work the barrier guards: the lanes meet
 // first, so everything each of them did (and fenced) is ordered before the one arrival.  Barriers signalled this way
-// are initialised with the number of WARPS (kWarpArrive = 1) -- 32 times fewer arrivals on the same shared-memory word.
-#ifndef FMHF_LANE_ARRIVE
-constexpr int kWarpArrive = 1;
-#else
-constexpr int kWarpArrive = 0;
-#endif
-__host__ __device__ constexpr int arrivals_of(int threads) { return kWarpArrive ? threads / 32 : threads; }
+// are initialised with the number of WARPS -- 32 times fewer arrivals on the same shared-memory word.
+__host__ __device__ constexpr int arrivals_of(int threads) { return threads / 32; }
 __device__ __forceinline__ void warp_arrive(uint32_t bar) {
-    if (kWarpArrive) {
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
-    } else {
-        mbar_arrive(bar);
-    }
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar),
@@ -200,11 +191,6 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Register reallocation between warpgroups (whole warpgroups of 4 warps execute these together): the control warps give
-// registers back, the element-wise warps take them.  `N` is a multiple of 8.
-template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-
 // ------------------------------------------------------------------------------------ tensor memory
 // Whole-warp operations.  `slot` is a shared-memory word that receives the base address.
 __device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t ncols) {
@@ -246,17 +232,6 @@ __device__ __forceinline__ void tmem_ld32x2_sync(uint32_t ta, uint32_t tb, uint3
         : "r"(ta), "r"(tb)
         : "memory");
 }
-// 64 + 64 consecutive fp32 columns (e.g. a thread's whole row of M and of N of a 64-column block) in one statement.
-__device__ __forceinline__ void tmem_ld64x2_sync(uint32_t ta, uint32_t tb, uint32_t *a, uint32_t *b) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%128];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%64,%65,%66,%67,%68,%69,%70,%71,%72,%73,%74,%75,%76,%77,%78,%79,%80,%81,%82,%83,%84,%85,%86,%87,%88,%89,%90,%91,%92,%93,%94,%95,%96,%97,%98,%99,%100,%101,%102,%103,%104,%105,%106,%107,%108,%109,%110,%111,%112,%113,%114,%115,%116,%117,%118,%119,%120,%121,%122,%123,%124,%125,%126,%127}, [%129];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]), "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]), "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]), "=r"(a[16]), "=r"(a[17]), "=r"(a[18]), "=r"(a[19]), "=r"(a[20]), "=r"(a[21]), "=r"(a[22]), "=r"(a[23]), "=r"(a[24]), "=r"(a[25]), "=r"(a[26]), "=r"(a[27]), "=r"(a[28]), "=r"(a[29]), "=r"(a[30]), "=r"(a[31]), "=r"(a[32]), "=r"(a[33]), "=r"(a[34]), "=r"(a[35]), "=r"(a[36]), "=r"(a[37]), "=r"(a[38]), "=r"(a[39]), "=r"(a[40]), "=r"(a[41]), "=r"(a[42]), "=r"(a[43]), "=r"(a[44]), "=r"(a[45]), "=r"(a[46]), "=r"(a[47]), "=r"(a[48]), "=r"(a[49]), "=r"(a[50]), "=r"(a[51]), "=r"(a[52]), "=r"(a[53]), "=r"(a[54]), "=r"(a[55]), "=r"(a[56]), "=r"(a[57]), "=r"(a[58]), "=r"(a[59]), "=r"(a[60]), "=r"(a[61]), "=r"(a[62]), "=r"(a[63]),
-          "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]), "=r"(b[8]), "=r"(b[9]), "=r"(b[10]), "=r"(b[11]), "=r"(b[12]), "=r"(b[13]), "=r"(b[14]), "=r"(b[15]), "=r"(b[16]), "=r"(b[17]), "=r"(b[18]), "=r"(b[19]), "=r"(b[20]), "=r"(b[21]), "=r"(b[22]), "=r"(b[23]), "=r"(b[24]), "=r"(b[25]), "=r"(b[26]), "=r"(b[27]), "=r"(b[28]), "=r"(b[29]), "=r"(b[30]), "=r"(b[31]), "=r"(b[32]), "=r"(b[33]), "=r"(b[34]), "=r"(b[35]), "=r"(b[36]), "=r"(b[37]), "=r"(b[38]), "=r"(b[39]), "=r"(b[40]), "=r"(b[41]), "=r"(b[42]), "=r"(b[43]), "=r"(b[44]), "=r"(b[45]), "=r"(b[46]), "=r"(b[47]), "=r"(b[48]), "=r"(b[49]), "=r"(b[50]), "=r"(b[51]), "=r"(b[52]), "=r"(b[53]), "=r"(b[54]), "=r"(b[55]), "=r"(b[56]), "=r"(b[57]), "=r"(b[58]), "=r"(b[59]), "=r"(b[60]), "=r"(b[61]), "=r"(b[62]), "=r"(b[63])
-        : "r"(ta), "r"(tb)
-        : "memory");
-}
 // Three runs of 32 consecutive fp32 columns (a thread's part of M, N and dA of a block) in one statement.
 __device__ __forceinline__ void tmem_ld32x3_sync(uint32_t ta, uint32_t tb, uint32_t tc, uint32_t *a, uint32_t *b, uint32_t *c) {
     asm volatile(
@@ -293,21 +268,6 @@ __device__ __forceinline__ void tmem_ld16x2_sync(uint32_t ta, uint32_t tb, uint3
         : "r"(ta), "r"(tb)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld16x3_sync(uint32_t ta, uint32_t tb, uint32_t tc, uint32_t *a, uint32_t *b, uint32_t *c) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%48];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%49];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47}, [%50];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]),
-          "=r"(a[8]), "=r"(a[9]), "=r"(a[10]), "=r"(a[11]), "=r"(a[12]), "=r"(a[13]), "=r"(a[14]), "=r"(a[15]),
-          "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7]),
-          "=r"(b[8]), "=r"(b[9]), "=r"(b[10]), "=r"(b[11]), "=r"(b[12]), "=r"(b[13]), "=r"(b[14]), "=r"(b[15]),
-          "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7]),
-          "=r"(c[8]), "=r"(c[9]), "=r"(c[10]), "=r"(c[11]), "=r"(c[12]), "=r"(c[13]), "=r"(c[14]), "=r"(c[15])
-        : "r"(ta), "r"(tb), "r"(tc)
-        : "memory");
-}
 
 // Each lane of the warp writes 32 consecutive 32-bit columns of its own TMEM lane.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t *r) {
@@ -329,22 +289,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t *r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------------ arithmetic
-// sigmoid(x) = 0.5 * tanh(0.5 x) + 0.5 with the hardware tanh approximation (one MUFU op,
+// Hardware tanh approximation, of which the kernels make sigmoid(x) = 0.5 * tanh(0.5 x) + 0.5 (one MUFU op,
 // max relative error about 2^-11 -- below bf16 rounding of the value it feeds).
 __device__ __forceinline__ float fast_tanh(float x) {
     float y;
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float fast_sigmoid(float x) { return fmaf(0.5f, fast_tanh(0.5f * x), 0.5f); }
 
 // Element i of a parameter kept as bf16 or fp32 (read once per block, so the choice is a run-time flag).
 __device__ __forceinline__ float load_param(const void *p, long long i, bool bf16) {
@@ -383,11 +337,6 @@ __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
 __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
     f32x2 d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 __device__ __forceinline__ f32x2 f2_tanh(f32x2 v) {

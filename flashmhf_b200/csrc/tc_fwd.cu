@@ -515,7 +515,8 @@ __global__ void __maxnreg__(48) o_reduce_kernel(const OReduceArgs a) {
     griddep_wait();   // launched early, behind the kernel whose partial sums it adds
     // Eight 16-byte loads of a thread are in flight (the partial sums come from L2 while the next call's weights stream in from
     // HBM: latency is what this kernel is made of): eight splits of one piece of O, or, where the grid is too small to give every
-    // thread one piece, four splits of two; the splits are added in index order.  48 registers: 128 threads of it fit beside
+    // thread one piece, of two pieces the first split and then three more at a time; the splits are added in index order.  48
+    // registers: 128 threads of it fit beside
     // the d_h = 128 forward CTA.  (a split call has at most a few hundred token tiles: every index fits 32 bits)
     const int n4 = (int)(a.plane / 4), stride = (int)(gridDim.x * blockDim.x);
     const float4 *part4 = reinterpret_cast<const float4 *>(a.part);
@@ -620,7 +621,7 @@ int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, boo
     *n_launch += 1;
     if (e != cudaSuccess) { set_cuda_error(e, "fwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
     if (pl.nsplit > 1) {
-        e = launch_o_reduce(static_cast<const float *>(p.workspace), p.O, p.d, pl.nsplit, chained ? kReduceChained : kReduceAfterKernel,
+        e = launch_o_reduce(static_cast<const float *>(p.workspace), p.O, p.d, pl.nsplit, chained,
                             dc->num_sms, st);
         prof_mark(st, kMarkFwdReduce);
         *n_launch += 1;
@@ -631,13 +632,13 @@ int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, boo
 
 }  // namespace
 
-cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, ReduceMode mode, int num_sms,
+cudaError_t launch_o_reduce(const float *part, const flashmhf_tensor &out, const flashmhf_dims &d, int nsplit, bool chained, int num_sms,
                             cudaStream_t st) {
     const long long plane = (long long)d.B * d.H * d.S * d.Dh, n4 = plane / 4;
     const OReduceArgs ra{part, plane, static_cast<__nv_bfloat16 *>(out.ptr), out.stride[0], out.stride[1], out.stride[2], nsplit, d.H, d.S,
                          d.Dh};
     // chained: at most one (small) CTA per SM, so that all of them are resident beside the forward kernel's
-    const long long cap = mode == kReduceChained ? (long long)num_sms : (long long)num_sms * 8;
+    const long long cap = chained ? (long long)num_sms : (long long)num_sms * 8;
     const int blocks = (int)((n4 + 127) / 128 < cap ? (n4 + 127) / 128 : cap);
     return launch_kernel(true, o_reduce_kernel, dim3(blocks), dim3(128), 0, st, ra);
 }
