@@ -19,6 +19,7 @@ def test_weight_gradients(dh, B, H, Hk, S, E, de):
     ref = orc.mhffn_backward(*(t.cpu().double() for t in ins))[1:4]
     for name, a, b in zip("dK dU dV".split(), got, ref):
         assert orc.rel_l2(a.cpu().double(), b) < 1e-2, name
+        assert orc.worst_element(a.cpu(), b) < 0.05, name
     again = [torch.full_like(t, float("nan")) for t in ins[1:4]]
     fm.backward_raw(*ins, parts="weights", weight_grads=again)
     for a, b in zip(got, again):

@@ -26,7 +26,6 @@ def test_forward_over_several_items_per_cta(dh, B, H, Hk, S, E, de):
             evict.zero_()
         assert torch.equal(fm.forward_raw(Q, K, U, V, R), first)
     ref = orc.mhffn_forward(*(t.double() for t in (Q, K, U, V, R)))
-    d, rms = (first.double() - ref).abs(), ref.square().mean().sqrt()
     # bf16 operands and result (2^-9 of each term, about 2^-9 of the rms together); a tile of the wrong Q is off by the rms itself
-    assert float((d / torch.maximum(rms, ref.abs())).max()) < 0.05
+    assert orc.worst_element(first, ref) < 0.05
     fm.check_device_status()

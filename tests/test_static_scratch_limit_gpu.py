@@ -6,6 +6,7 @@ import ctypes as C
 import pytest
 import torch
 
+from oracle import mhffn_oracle as orc
 from tests.test_zz_no_alloc import _static_backward
 
 pytestmark = pytest.mark.gpu
@@ -24,5 +25,4 @@ def test_fewer_parts_where_the_sums_do_not_fit(B, H, S, dh, Hk, E, de):
     want = fm.backward_raw(Q, K, U, V, R, dO)
     got, _ = _static_backward(Q, K, U, V, R, dO)
     for name, a, b in zip("dQ dK dU dV dR".split(), got, want):
-        b = b.double()
-        assert float(((a.double() - b).abs() / torch.maximum(b.square().mean().sqrt(), b.abs())).max()) < 0.02, name
+        assert orc.worst_element(a, b) < 0.02, name
