@@ -33,7 +33,7 @@ import torch  # noqa: E402
 
 WORKLOAD = dict(name="flashmhf_370m_layer_op_fwd_bwd", B=16, S=2048, H=8, Hkuv=8, Dh=128, E=11, De=256)
 NOMINAL_BF16_TFLOPS = 2250.0
-KERNEL_SOURCES = ("tc_common.cuh", "tc_fwd.cu", "tc_bwd.cu")
+KERNEL_SOURCES = ("tc_common.cuh", "tc_fwd.cu", "tc_bwd.cu", "dw_plan.h")
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "ncu_dram_traffic.json")
 CPU_CHUNK_ROWS = 4          # the CPU legs walk the batch in chunks of this many rows to bound host memory
 
