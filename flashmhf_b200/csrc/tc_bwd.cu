@@ -14,15 +14,14 @@
 //
 // bwd_dw_kernel (d_h = 128)  -- weight-stationary.  One CTA owns one 64-row block of K, U and V of one K/U/V
 //   head and a contiguous range of token tiles (the token axis is split `nsplit` ways to fill the
-//   machine).  Weights stay in shared memory, {Q, dO} tiles stream through a ring of 2.
-//   Tensor memory: [dK;dU] accumulator (128 lanes), dV accumulator (transposed, d_h x 64), two S buffers and one dA
-//   buffer, so that the recompute of tile i+1 runs under the element-wise math of tile i.
-// bwd_dwt_kernel (d_h = 64, 96)  -- the same with 128 weight rows per CTA and the recompute transposed.
+//   machine).  The recompute is transposed (lane = weight row), with K and U stacked in the 128 lanes; {Q, dO} tiles stream
+//   through rings of 3.
+// bwd_dwt_kernel (d_h = 64, 96)  -- the same with 128 weight rows per CTA, K and U side by side.
 //   With more than one split each CTA writes fp32 partial sums to the workspace; dw_reduce_kernel adds the splits in a
 //   fixed order and writes bf16 dK, dU, dV.
 //
 // All use 384 threads: warp 0 TMA producer, warps 1 to 3 MMA issuers (one per MMA chain; warp 1 owns tensor memory; warp 2
-// of bwd_dwt_kernel fetches routing weights), warps 4-11 element-wise math (warp % 4 = TMEM lane quarter, (warp-4)/4 =
+// of bwd_dwt_kernel and warp 3 of bwd_dw_kernel fetch routing weights), warps 4-11 element-wise math (warp % 4 = TMEM lane quarter, (warp-4)/4 =
 // which half of the columns).
 #include <atomic>
 #include <mutex>
@@ -453,33 +452,40 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // =============================================================================================
 //                                    dK / dU / dV kernel
 // =============================================================================================
+// A CTA owns 64 weight rows.  The rows of K and U lie in the 128 lanes of one operand, sixteen of K, sixteen of U and so on, so that
+//     S^T = [K;U] Q^T        (128 lanes x 128 tokens: M in lanes 0-15 of each 32, N of the same weight rows in lanes 16-31)
+//     dA^T = V dO^T          (64 rows x 128 tokens: an M = 64 product fills lanes 0-15 of each 32)
+// put M, N and dA of a weight row under one warp, which reads sixteen lanes at a time, and what it writes back over dA, [dM;dN] as
+// bf16, is the A operand of
+//     [dK;dU] += [dM;dN] Q   (128 x d_h).
+// Only A^T goes through shared memory, as the B operand of dV^T += dO^T A.  [K;U] are copied to tensor memory once.
+// Bound: shared memory (160 KB of operand reads, 64 KB of fills and 16 KB of A a tile: 1875 clk at 128 B/clk) and the tensor pipe
+// (1940 clk) alike, and power.  The other orientation (lane = token) moved 336 KB, since [dM|dN] had to be staged too and S read both its
+// operands there.  370M layer's operator, 32768 tokens, this kernel in a loop at the power limit: 1146 -> 1062 us (2.00 -> 1.70 M cycles);
+// ten passes 1035 -> 926.  Ordering matters as much as traffic: see the issuers.
 template <int DH>
 struct DwSmem {
     static constexpr int kChunks = (DH + 63) / 64;
-    static constexpr uint32_t kWBytes = 3 * kChunks * kWChunk;  // [K;U] chunks then V chunks
-    static constexpr uint32_t kOffWV = 2 * kChunks * kWChunk;
-    static constexpr uint32_t kTokStage = 2 * kChunks * kTile;  // Q chunks then dO chunks
-    static constexpr int kTokStages = 2;   // what is left beside the resident weights and the staged operands
-    static constexpr uint32_t kOffW = 0;
-    static constexpr uint32_t kOffTok = kOffW + kWBytes;
-    static constexpr uint32_t kOffP = kOffTok + kTokStages * kTokStage;  // [dM | dN] : 2 x 16 KB
-    static constexpr uint32_t kOffA = kOffP + 2 * kTile;                 // A : 16 KB
-    static constexpr uint32_t kOffCtl = kOffA + kTile;
+    static constexpr uint32_t kTok = kChunks * kTile;      // Q or dO of a tile: 128 rows
+    static constexpr uint32_t kVBytes = kChunks * kWChunk;
+    // [K;U] are needed in shared memory only until they are copied to tensor memory: they arrive in the last stage of the dO ring.
+    static constexpr int kQStages = 3, kGStages = 3, kRSlots = 2;
+    static constexpr uint32_t kOffQ = 0;
+    static constexpr uint32_t kOffG = kOffQ + kQStages * kTok;
+    static constexpr uint32_t kOffKU = kOffG + (kGStages - 1) * kTok;
+    static constexpr uint32_t kOffV = kOffG + kGStages * kTok;
+    static constexpr uint32_t kOffA = kOffV + kVBytes;            // A^T of a tile: 64 weight rows x 128 tokens
+    static constexpr uint32_t kOffR = kOffA + 2 * kWChunk;
+    static constexpr uint32_t kOffCtl = kOffR + kRSlots * kBT * 4;
     static constexpr uint32_t kTotal = kOffCtl + 256 + 1024;
 };
 
-// The Q half and the dO half of a token stage, and the [dM|dN] tile and the A tile, have barriers of their
-// own: each is needed by, and released after, a different MMA chain, and every cycle by which the next
-// load or the next MMA can start earlier shortens the loop load -> recompute -> element-wise -> accumulate.
-// S has two buffers in tensor memory, each with its own full/empty pair, so that every waiter sees every
-// phase of the barrier it waits on (a one-bit parity cannot tell phase k from phase k+2).
-// That loop over two stages is what bounds the kernel, so the element-wise step is cut in two: A and the factors of dM, dN need
-// only S; A goes out first and its dV update runs while dA is still being computed.  (One step behind S and dA before: the
-// 370M layer at 32768 tokens 1.07 -> 1.04 ms burst, 1.21 -> 1.18 sustained.)
-constexpr int kMaxTok = 2;
-enum { DW_WFULL = 0, DW_SFULL = 1, DW_SEMPTY = 3, DW_PFULL = 5, DW_AFULL = 6, DW_PEMPTY = 7, DW_AEMPTY = 8, DW_ACCFULL = 9, DW_DAFULL = 10,
-       DW_DAEMPTY = 11, DW_QFULL = 12, DW_GFULL = DW_QFULL + kMaxTok, DW_QEMPTY = DW_GFULL + kMaxTok, DW_GEMPTY = DW_QEMPTY + kMaxTok,
-       DW_BARS = DW_GEMPTY + kMaxTok };
+// Barriers.  Each is waited on by one fixed thread (or all element-wise warps) in every phase, so a one-bit parity is enough.
+//   KUT: [K;U] copied to tensor memory;  SFULL / SEMPTY: S computed / in registers;  DAFULL: dA computed, and with it, because the
+//   same thread issues it behind the [dK;dU] update of the tile before, that update is done, whose operand lies over dA;
+//   AFULL / AEMPTY: A staged / its dV update done;  PFULL: [dM;dN] written;  RFULL, REMPTY: routing weights;  DAISSUED (tile % 2): dA issued.
+enum { DW_WFULL = 0, DW_KUT = 1, DW_SFULL = 2, DW_SEMPTY = 3, DW_DAFULL = 4, DW_AFULL = 5, DW_AEMPTY = 6, DW_PFULL = 7, DW_ACCFULL = 8,
+       DW_RFULL = 9, DW_REMPTY = 11, DW_DAISSUED = 13, DW_QFULL = 15, DW_QEMPTY = 18, DW_GFULL = 21, DW_GEMPTY = 24, DW_BARS = 27 };
 static_assert(DW_BARS * 8 + 8 <= 256, "control area");
 
 struct DwArgs {
@@ -541,12 +547,14 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
               const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
               const __grid_constant__ CUtensorMap tmV, const DwArgs args) {
     using L = DwSmem<DH>;
+    static_assert(DH == 128, "the narrower head dimensions have a kernel of their own");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *gbase = smem_raw + (base - raw);
-    const uint32_t sW = base + L::kOffW, sTok = base + L::kOffTok, sP = base + L::kOffP, sA = base + L::kOffA,
+    const uint32_t sQ = base + L::kOffQ, sG = base + L::kOffG, sKU = base + L::kOffKU, sV = base + L::kOffV, sA = base + L::kOffA,
                    sBar = base + L::kOffCtl;
+    float *rbuf = reinterpret_cast<float *>(gbase + L::kOffR);   // [kRSlots][kBT]
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(gbase + L::kOffCtl + DW_BARS * 8);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(gbase + L::kOffCtl + DW_BARS * 8 + 4);
     auto bar = [&](int i) { return sBar + 8u * i; };
@@ -559,12 +567,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const int ntiles = tile_end - tile_begin;  // >= 1 by construction of the plan
     const WaitCtl ctl{abort_flag, args.wait};
     constexpr int W = kKernelBwdDw * 100;
-    // dV is accumulated transposed, dV^T = sum_t dO^T A (d_h x 64: M = 128, N = 64): half the columns and three quarters of the
-    // tensor-pipe time of dV = sum_t A^T dO (M = 64 runs at the M = 128 rate).
-    static_assert(DH == 128, "the narrower head dimensions have a kernel of their own");
-    constexpr int kSB = 2;
-    // Columns: [dK;dU] at 0, dV^T at 128 (64 wide), dA at 192, S buffers at 256 and 384.
-    constexpr uint32_t kColKU = 0, kColV = 128, kColS = 256, kColdA = 192;
+    // Columns: [dK;dU] (d_h wide), dV^T (lane = column of dV, 64 wide), [K;U] as bf16 operand, S^T, dA^T (over which [dM;dN] is written).
+    constexpr uint32_t kColKU = 0, kColV = 128, kColW = 192, kColS = 256, kColdA = 384;
 
     auto tile_coords = [&](int i, int &ts, int &hh, int &bb) {  // token tile i of this CTA -> (seq tile, head, batch)
         const int ti = tile_begin + i;
@@ -576,24 +580,21 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 
     if (threadIdx.x == 0) {
         *abort_flag = launch_aborted(args.wait);  // a CTA of this launch gave up: drain fast
-        mbar_init(bar(DW_WFULL), 1);
-        for (int s = 0; s < L::kTokStages; ++s) {
+        for (int i : {DW_WFULL, DW_SFULL, DW_DAFULL, DW_AEMPTY, DW_ACCFULL}) mbar_init(bar(i), 1);
+        for (int i = 0; i < 2; ++i) mbar_init(bar(DW_DAISSUED + i), 1);
+        for (int i : {DW_KUT, DW_SEMPTY, DW_AFULL, DW_PFULL}) mbar_init(bar(i), arrivals_of(kActThreads));
+        for (int s = 0; s < L::kRSlots; ++s) {
+            mbar_init(bar(DW_RFULL + s), arrivals_of(32));
+            mbar_init(bar(DW_REMPTY + s), arrivals_of(kActThreads));
+        }
+        for (int s = 0; s < L::kQStages; ++s) {
             mbar_init(bar(DW_QFULL + s), 1);
-            mbar_init(bar(DW_GFULL + s), 1);
             mbar_init(bar(DW_QEMPTY + s), 1);
+        }
+        for (int s = 0; s < L::kGStages; ++s) {
+            mbar_init(bar(DW_GFULL + s), 1);
             mbar_init(bar(DW_GEMPTY + s), 2);   // the dA product and the dV update have read it
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(bar(DW_SFULL + b), 1);
-            mbar_init(bar(DW_SEMPTY + b), arrivals_of(kActThreads));
-        }
-        mbar_init(bar(DW_DAFULL), 1);
-        mbar_init(bar(DW_DAEMPTY), arrivals_of(kActThreads));
-        mbar_init(bar(DW_PFULL), arrivals_of(kActThreads));
-        mbar_init(bar(DW_AFULL), arrivals_of(kActThreads));
-        mbar_init(bar(DW_PEMPTY), 1);
-        mbar_init(bar(DW_AEMPTY), 1);
-        mbar_init(bar(DW_ACCFULL), 1);
         fence_mbar_init();
     }
     if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kTmemCols);
@@ -607,192 +608,225 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     if (dead) {
         // nothing: fall through to the teardown
     } else if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK);
             tma_prefetch_desc(&tmU); tma_prefetch_desc(&tmV);
-            mbar_arrive_expect_tx(bar(DW_WFULL), L::kWBytes);
+            mbar_arrive_expect_tx(bar(DW_WFULL), L::kChunks * kTile + L::kVBytes);
             const int row = jblk * kBI;
             for (int c = 0; c < L::kChunks; ++c) {
-                tma_load_3d(sW + c * 2 * kWChunk, &tmK, bar(DW_WFULL), c * 64, row, hk);
-                tma_load_3d(sW + c * 2 * kWChunk + kWChunk, &tmU, bar(DW_WFULL), c * 64, row, hk);
-                tma_load_3d(sW + L::kOffWV + c * kWChunk, &tmV, bar(DW_WFULL), c * 64, row, hk);
+                for (int g = 0; g < 4; ++g) {   // sixteen rows of K, sixteen of U, ...
+                    tma_load_3d(sKU + c * kTile + g * 32 * 128, &tmK, bar(DW_WFULL), c * 64, row + g * 16, hk);
+                    tma_load_3d(sKU + c * kTile + (g * 32 + 16) * 128, &tmU, bar(DW_WFULL), c * 64, row + g * 16, hk);
+                }
+                tma_load_3d(sV + c * kWChunk, &tmV, bar(DW_WFULL), c * 64, row, hk);
             }
-            int st = 0;
-            uint32_t ph = 1;
+            int sq = 0, sg = 0;
+            uint32_t phq = 1, phg = 1;
             for (int i = 0; i < ntiles; ++i) {
                 int ts, hh, bb;
                 tile_coords(i, ts, hh, bb);
-                const uint32_t d = sTok + st * L::kTokStage;
-                if (!mbar_wait(bar(DW_QEMPTY + st), ph, ctl, W + 1)) break;
-                const uint32_t fq = bar(DW_QFULL + st);
-                mbar_arrive_expect_tx(fq, L::kTokStage / 2);
-#pragma unroll
-                for (int c = 0; c < L::kChunks; ++c) tma_load_4d(d + c * kTile, &tmQ, fq, c * 64, ts * kBT, hh, bb);
-                if (!mbar_wait(bar(DW_GEMPTY + st), ph, ctl, W + 2)) break;
-                const uint32_t fg = bar(DW_GFULL + st);
-                mbar_arrive_expect_tx(fg, L::kTokStage / 2);
+                if (!mbar_wait(bar(DW_QEMPTY + sq), phq, ctl, W + 1)) break;
+                mbar_arrive_expect_tx(bar(DW_QFULL + sq), L::kTok);
 #pragma unroll
                 for (int c = 0; c < L::kChunks; ++c)
-                    tma_load_4d(d + (L::kChunks + c) * kTile, &tmdO, fg, c * 64, ts * kBT, hh, bb);
-                if (++st == L::kTokStages) { st = 0; ph ^= 1; }
+                    tma_load_4d(sQ + sq * L::kTok + c * kTile, &tmQ, bar(DW_QFULL + sq), c * 64, ts * kBT, hh, bb);
+                if (i == L::kGStages - 1 && !mbar_wait(bar(DW_KUT), 0, ctl, W + 17)) break;   // [K;U] are in tensor memory
+                if (!mbar_wait(bar(DW_GEMPTY + sg), phg, ctl, W + 2)) break;
+                mbar_arrive_expect_tx(bar(DW_GFULL + sg), L::kTok);
+#pragma unroll
+                for (int c = 0; c < L::kChunks; ++c)
+                    tma_load_4d(sG + sg * L::kTok + c * kTile, &tmdO, bar(DW_GFULL + sg), c * 64, ts * kBT, hh, bb);
+                if (++sq == L::kQStages) { sq = 0; phq ^= 1; }
+                if (++sg == L::kGStages) { sg = 0; phg ^= 1; }
             }
         }
     } else if (warp == 1) {
-        // MMA issuer 1: the recompute chain S = Q [K;U]^T, dA = dO V^T of each token tile.  The two
-        // chains have their own issuing threads so that neither waits on the other's barriers and the
-        // tensor pipe, which accepts MMAs only a few ahead of execution, is fed by whichever is ready.
-        // Descriptors are built once and advanced by constants (16-byte units).
+        // ------------------------------------------------------------------ MMA issuer 1: S^T of the next tile, dV^T += dO^T A of this one
         if (lane == 0) {
-            constexpr uint32_t idS = umma_idesc(128, 2 * kBI, false, false);
-            constexpr uint32_t idA = umma_idesc(128, kBI, false, false);
-            const uint64_t dQk0 = desc_kmajor(sTok), dGk0 = desc_kmajor(sTok + L::kChunks * kTile),
-                           dKU = desc_kmajor(sW), dV = desc_kmajor(sW + L::kOffWV);
-            constexpr uint64_t kTokStep = L::kTokStage >> 4;
-            bool ok = mbar_wait(bar(DW_WFULL), 0, ctl, W + 3);
-            int st = 0;
-            uint32_t ph = 0;
-            for (int i = 0; ok && i < ntiles; ++i) {
-                if (!mbar_wait(bar(DW_QFULL + st), ph, ctl, W + 4)) break;
-                const int sb = i % kSB;
-                const uint32_t sph = (uint32_t)(i / kSB) & 1u;
-                if (!mbar_wait(bar(DW_SEMPTY + sb), sph ^ 1, ctl, W + 5)) break;
-                tc_fence_after();
-                const uint64_t dq = dQk0 + st * kTokStep, dg = dGk0 + st * kTokStep;
+            constexpr uint32_t idS = umma_idesc(128, kBT, false, false);
+            constexpr uint32_t idV = umma_idesc(128, kBI, true, false);
+            const uint64_t dQ0 = desc_kmajor(sQ), dG0 = desc_mnmajor(sG, kTile), dA0 = desc_kmajor(sA);
+            constexpr uint64_t kTokStep = L::kTok >> 4;
+            bool ok = mbar_wait(bar(DW_KUT), 0, ctl, W + 3);
+            int sq = 0, sg = 0;
+            uint32_t phq = 0;
+            for (int i = -1; ok && i < ntiles; ++i) {
+                // S of the next tile goes behind dA of this one, which is needed first.  That dA is issued says, too, that dO is there.
+                const bool more = i + 1 < ntiles;
+                if (more && !mbar_wait(bar(DW_QFULL + sq), phq, ctl, W + 4)) break;
+                if (more && i >= 0 && !mbar_wait(bar(DW_SEMPTY), i & 1, ctl, W + 5)) break;
+                // S of the next tile goes behind dA of this one, which is needed first (any order: 1091 instead of 1062 us).  That dA is
+                // issued says, too, that dO is there.  Two barriers in turn: issuer 2 can be one tile ahead of this wait, not two, since
+                // its dA after next needs S of the next tile.
+                if (i >= 0 && !mbar_wait(bar(DW_DAISSUED + (i & 1)), (i >> 1) & 1, ctl, W + 10)) break;
+                if (more) {
+                    tc_fence_after();
+                    const uint64_t dq = dQ0 + sq * kTokStep;
 #pragma unroll
-                for (int k = 0; k < DH / 16; ++k) {
-                    const int c = k >> 2, kk = k & 3;
-                    umma_ss(tmem + kColS + sb * 2 * kBI, dq + ((c * kTile + kk * 32) >> 4),
-                            dKU + ((c * 2 * kWChunk + kk * 32) >> 4), idS, k > 0 ? 1u : 0u);
+                    for (int k = 0; k < DH / 16; ++k) {
+                        const int c = k >> 2, kk = k & 3;
+                        umma_ts(tmem + kColS, tmem + kColW + k * 8, dq + ((c * kTile + kk * 32) >> 4), idS, k > 0 ? 1u : 0u);
+                    }
+                    umma_commit(bar(DW_SFULL));
+                    if (++sq == L::kQStages) { sq = 0; phq ^= 1; }
                 }
-                umma_commit(bar(DW_SFULL + sb));
-                if (!mbar_wait(bar(DW_GFULL + st), ph, ctl, W + 4)) break;
-                if (!mbar_wait(bar(DW_DAEMPTY), (i & 1) ^ 1, ctl, W + 10)) break;
+                if (i < 0) continue;
+                if (!mbar_wait(bar(DW_AFULL), i & 1, ctl, W + 6)) break;
                 tc_fence_after();
+                const uint64_t dg = dG0 + sg * kTokStep;
 #pragma unroll
-                for (int k = 0; k < DH / 16; ++k) {
-                    const int c = k >> 2, kk = k & 3;
-                    umma_ss(tmem + kColdA, dg + ((c * kTile + kk * 32) >> 4), dV + ((c * kWChunk + kk * 32) >> 4), idA,
-                            k > 0 ? 1u : 0u);
-                }
-                umma_commit(bar(DW_GEMPTY + st));
-                umma_commit(bar(DW_DAFULL));
-                if (++st == L::kTokStages) { st = 0; ph ^= 1; }
+                for (int k = 0; k < kBT / 16; ++k)
+                    umma_ss(tmem + kColV, dg + k * 128, dA0 + (((k >> 2) * kWChunk + (k & 3) * 32) >> 4), idV, (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(bar(DW_GEMPTY + sg));
+                umma_commit(bar(DW_AEMPTY));
+                if (++sg == L::kGStages) sg = 0;
             }
         }
-    } else if (warp == 3) {
-        // MMA issuer 2: the accumulation chain [dK;dU] += [dM|dN]^T Q, dV += A^T dO.
+    } else if (warp == 2) {
+        // ------------------------------------------------------------------ MMA issuer 2: dA^T, [dK;dU] += [dM;dN] Q
+        // One thread for both: a tile's dA overwrites the columns that the update of the tile before reads, and MMAs of one thread
+        // execute in order.
         if (lane == 0) {
-            constexpr uint32_t idKU = umma_idesc(128, DH, true, true);
-            constexpr uint32_t idV = umma_idesc(128, kBI, true, true);
-            const uint64_t dQmn0 = desc_mnmajor(sTok, kTile), dGmn0 = desc_mnmajor(sTok + L::kChunks * kTile, kTile),
-                           dPmn = desc_mnmajor(sP, kTile), dAmn = desc_mnmajor(sA, kTile);
-            constexpr uint64_t kTokStep = L::kTokStage >> 4;
-            int st = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int i = 0; i < ntiles; ++i) {
-                const uint64_t dq = dQmn0 + st * kTokStep, dg = dGmn0 + st * kTokStep;
-                // A needs only Q: that it is there does not say that dO is.  (The dA product, which waits for dO too, may still be ahead.)
-                if (!mbar_wait(bar(DW_GFULL + st), ph, ctl, W + 12)) { ok = false; break; }
-                if (!mbar_wait(bar(DW_AFULL), i & 1, ctl, W + 6)) { ok = false; break; }
-                tc_fence_after();
+            constexpr uint32_t idA = umma_idesc(64, kBT, false, false);
+            constexpr uint32_t idKU = umma_idesc(128, DH, false, true);
+            const uint64_t dV = desc_kmajor(sV), dG0 = desc_kmajor(sG), dQ0 = desc_mnmajor(sQ, kTile);
+            constexpr uint64_t kTokStep = L::kTok >> 4;
+            bool ok = mbar_wait(bar(DW_WFULL), 0, ctl, W + 3);
+            int sq = 0, sg = 0;
+            uint32_t phg = 0;
+            // No wait between the update of tile i and dA of tile i + 1: after a batch of MMAs a wait returns only when they have gone
+            // into the pipe, which is then empty.
+            for (int i = -1; ok && i < ntiles; ++i) {
+                const bool more = i + 1 < ntiles;
+                if (more && !mbar_wait(bar(DW_GFULL + sg), phg, ctl, W + 4)) { ok = false; break; }
+                if (i >= 0) {
+                    if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t dq = dQ0 + sq * kTokStep;
 #pragma unroll
-                for (int k = 0; k < kBT / 16; ++k)
-                    umma_ss(tmem + kColV, dg + k * 128, dAmn + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(bar(DW_GEMPTY + st));  // dO of this stage (once its dA is computed too) and the A tile are free
-                umma_commit(bar(DW_AEMPTY));
-                if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
+                    for (int k = 0; k < kBT / 16; ++k)
+                        umma_ts(tmem + kColKU, tmem + kColdA + (k >> 2) * 64 + (k & 3) * 8, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(bar(DW_QEMPTY + sq));
+                    if (++sq == L::kQStages) sq = 0;
+                }
+                if (!more) break;
                 tc_fence_after();
+                const uint64_t dg = dG0 + sg * kTokStep;
 #pragma unroll
-                for (int k = 0; k < kBT / 16; ++k)
-                    umma_ss(tmem + kColKU, dPmn + k * 128, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(bar(DW_QEMPTY + st));  // Q of this stage and the [dM|dN] tile are free
-                umma_commit(bar(DW_PEMPTY));
-                if (++st == L::kTokStages) { st = 0; ph ^= 1; }
+                for (int k = 0; k < DH / 16; ++k) {
+                    const int c = k >> 2, kk = k & 3;
+                    umma_ss(tmem + kColdA, dV + ((c * kWChunk + kk * 32) >> 4), dg + ((c * kTile + kk * 32) >> 4), idA, k > 0 ? 1u : 0u);
+                }
+                umma_commit(bar(DW_DAFULL));
+                umma_commit(bar(DW_GEMPTY + sg));
+                mbar_arrive(bar(DW_DAISSUED + ((i + 1) & 1)));
+                if (++sg == L::kGStages) { sg = 0; phg ^= 1; }
             }
             if (ok) umma_commit(bar(DW_ACCFULL));
         }
-    } else if (warp >= 4) {
-        const int quarter = warp & 3, part = (warp - 4) >> 2;  // part: which kCols of the block's 64 columns
-        const int row = quarter * 32 + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
-        bool ok = true;
-        const DwConst kc = dw_const(args.s0);
-        // This row's routing weight for sub-network e, fetched one tile ahead.  The tile's (sequence tile, head, batch)
-        // coordinates advance by counting, with no division in the loop.
-        int c_ts, c_hh, c_bb;
-        tile_coords(0, c_ts, c_hh, c_bb);
-        int c_g = c_hh - hk * args.G;
-        auto r_of_tile = [&]() {
-            const int t = c_ts * kBT + row;
-            return (t < args.S) ? __ldg(args.R + (long long)c_bb * args.r_sb + (long long)(hk * args.G + c_g) * args.r_sh +
-                                        (long long)t * args.r_ss + e) : 0.f;
-        };
-        float r_next = r_of_tile();
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ routing weights of each tile, times args.c
         for (int i = 0; i < ntiles; ++i) {
-            const float r = r_next;
-            if (i + 1 < ntiles) {
-                if (++c_ts == args.tiles_per_seq) {
-                    c_ts = 0;
-                    if (++c_g == args.G) { c_g = 0; ++c_bb; }
-                }
-                r_next = r_of_tile();
+            int ts, hh, bb;
+            tile_coords(i, ts, hh, bb);
+            const float *src = args.R + (long long)bb * args.r_sb + (long long)hh * args.r_sh + e;
+            float v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int t = ts * kBT + k * 32 + lane;
+                v[k] = t < args.S ? args.c * __ldg(src + (long long)t * args.r_ss) : 0.f;
             }
-            const int sb = i % kSB;
-            if (!mbar_wait(bar(DW_SFULL + sb), (uint32_t)(i / kSB) & 1u, ctl, W + 7)) { ok = false; break; }
+            const int slot = i % L::kRSlots;
+            if (!mbar_wait(bar(DW_REMPTY + slot), ((uint32_t)(i / L::kRSlots) & 1u) ^ 1u, ctl, W + 13)) break;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) rbuf[slot * kBT + k * 32 + lane] = v[k];
+            warp_arrive(bar(DW_RFULL + slot));
+        }
+    } else if (warp >= 4) {
+        // ------------------------------------------------------------------ element-wise math
+        // A warp has sixteen weight rows (M, dA in lanes 0-15 of its quarter, N in lanes 16-31) and 64 tokens; a thread rows lane / 4
+        // and lane / 4 + 8 and of each eight tokens the two at 2 (lane % 4).  Pair 2x + rr: tokens 8x.., row lane / 4 + 8 rr.
+        const int quarter = warp & 3, part = (warp - 4) >> 2;
+        const int row = quarter * 32 + lane;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), lane_up = lane_base + (16u << 16);
+        bool ok = mbar_wait(bar(DW_WFULL), 0, ctl, W + 14);
+        if (ok) {   // [K;U]: shared -> tensor memory, once (thread = stacked row; column part p copies columns [64p, 64p + 64) of d_h)
+            uint32_t v32[32];
+            const uint8_t *src = gbase + L::kOffKU + part * kTile;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
+                v32[4 * c] = v.x; v32[4 * c + 1] = v.y; v32[4 * c + 2] = v.z; v32[4 * c + 3] = v.w;
+            }
+            tmem_st32(lane_base + kColW + part * 32, v32);
+            tmem_st_wait();
+        }
+        tc_fence_before();
+        warp_arrive(bar(DW_KUT));
+        const DwConst kc = dw_const(args.s0);
+        // stmatrix: lane l gives the row address of matrix l / 8: token group x + l / 16, row (l % 8) + 8 ((l / 8) % 2)
+        const int arow = quarter * 16 + (lane & 15);
+        const uint32_t a_row = sA + part * kWChunk + arow * 128, a_x = lane >> 4;
+        const float *rsrc = rbuf + part * 64 + 2 * (lane & 3);
+        for (int i = 0; ok && i < ntiles; ++i) {
+            const int slot = i % L::kRSlots;
+            const bool r_there = mbar_test(bar(DW_RFULL + slot), (uint32_t)(i / L::kRSlots) & 1u);
+            if (!mbar_wait(bar(DW_SFULL), i & 1, ctl, W + 7)) { ok = false; break; }
+            if (!r_there && !mbar_wait(bar(DW_RFULL + slot), (uint32_t)(i / L::kRSlots) & 1u, ctl, W + 15)) { ok = false; break; }
             tc_fence_after();
-            const f32x2 r2 = f2_pack(args.c * r, args.c * r);
-            const uint32_t colS = kColS + sb * 2 * kBI;
             // first what needs only S: A goes out, and its dV update runs, while dA is still being computed
-            f32x2 fq[kCols / 2], fw[kCols / 2];
-            uint32_t pa[kCols / 2];
+            f32x2 fq[16], fw[16];
+            uint32_t pa[16];
+            bool a_free = i == 0;   // asked for ahead of the second half's arithmetic: a wait takes 75 cycles even where nothing is waited for
 #pragma unroll
-            for (int sub = 0; sub < kCols / 16; ++sub) {
+            for (int sub = 0; sub < 2; ++sub) {
                 uint32_t m[16], n[16];
-                const uint32_t c = part * kCols + sub * 16;
-                tmem_ld16x2_sync(lane_base + colS + c, lane_base + colS + kBI + c, m, n);
-                if (sub == kCols / 16 - 1) {   // S is in registers: the buffer can take the tile after next
+                tmem_ld_16x256b_x4x2_sync(lane_base + kColS + part * 64 + sub * 32, lane_up + kColS + part * 64 + sub * 32, m, n);
+                if (sub == 1) {   // S is in registers: the buffer can take the next tile
                     tc_fence_before();
-                    warp_arrive(bar(DW_SEMPTY + sb));
+                    warp_arrive(bar(DW_SEMPTY));
+                    if (i >= 1) a_free = mbar_test(bar(DW_AEMPTY), (i - 1) & 1);
                 }
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const DwPair x = dw_pair(f2_pack_bits(m[2 * q], m[2 * q + 1]), f2_pack_bits(n[2 * q], n[2 * q + 1]), r2, kc);
-                    fq[sub * 8 + q] = x.q;
-                    fw[sub * 8 + q] = x.w;
-                    pa[sub * 8 + q] = f2_to_bf16x2(x.a);
+                for (int x = 0; x < 4; ++x) {
+                    const float2 r = *reinterpret_cast<const float2 *>(rsrc + slot * kBT + sub * 32 + x * 8);
+#pragma unroll
+                    for (int rr = 0; rr < 2; ++rr) {
+                        const int q = 2 * x + rr, o = sub * 8 + q;
+                        const DwPair d = dw_pair(f2_pack_bits(m[2 * q], m[2 * q + 1]), f2_pack_bits(n[2 * q], n[2 * q + 1]), f2_pack(r.x, r.y), kc);
+                        fq[o] = d.q;
+                        fw[o] = d.w;
+                        pa[o] = f2_to_bf16x2(d.a);
+                    }
                 }
             }
-            if (!mbar_wait(bar(DW_AEMPTY), (i & 1) ^ 1, ctl, W + 8)) { ok = false; break; }
+            warp_arrive(bar(DW_REMPTY + slot));
+            if (!a_free && !mbar_wait(bar(DW_AEMPTY), (i - 1) & 1, ctl, W + 8)) { ok = false; break; }
 #pragma unroll
-            for (int q = 0; q < kCols / 8; ++q)
-                st_shared_v4(sA + sw128_offset(row, part * (kCols / 8) + q), pa[4 * q], pa[4 * q + 1], pa[4 * q + 2], pa[4 * q + 3]);
+            for (int x = 0; x < 8; x += 2)
+                stmatrix_x4(a_row + (((x + a_x) ^ (arow & 7)) << 4), pa[2 * x], pa[2 * x + 1], pa[2 * x + 2], pa[2 * x + 3]);
             fence_async_smem();
             warp_arrive(bar(DW_AFULL));
             // then dM and dN
-            uint32_t da[kCols], pm[kCols / 2], pn[kCols / 2];
+            uint32_t da[32], pm[16], pn[16];
             if (!mbar_wait(bar(DW_DAFULL), i & 1, ctl, W + 11)) { ok = false; break; }
             tc_fence_after();
-            tmem_ld32_sync(lane_base + kColdA + part * kCols, da);
-            tc_fence_before();
-            warp_arrive(bar(DW_DAEMPTY));
+            tmem_ld_16x256b_x8_sync(lane_base + kColdA + part * 64, da);
 #pragma unroll
-            for (int q = 0; q < kCols / 2; ++q) {
+            for (int q = 0; q < 16; ++q) {
                 const f32x2 da2 = f2_pack_bits(da[2 * q], da[2 * q + 1]);
                 pm[q] = f2_to_bf16x2(f2_mul(da2, fw[q]));
                 pn[q] = f2_to_bf16x2(f2_mul(da2, fq[q]));
             }
-            if (!mbar_wait(bar(DW_PEMPTY), (i & 1) ^ 1, ctl, W + 8)) { ok = false; break; }
-#pragma unroll
-            for (int q = 0; q < kCols / 8; ++q) {
-                const uint32_t off = sw128_offset(row, part * (kCols / 8) + q);
-                st_shared_v4(sP + off, pm[4 * q], pm[4 * q + 1], pm[4 * q + 2], pm[4 * q + 3]);
-                st_shared_v4(sP + kTile + off, pn[4 * q], pn[4 * q + 1], pn[4 * q + 2], pn[4 * q + 3]);
-            }
-            fence_async_smem();
+            tmem_st_16x128b_x8(lane_base + kColdA + part * 64, pm);
+            tmem_st_16x128b_x8(lane_up + kColdA + part * 64, pn);
+            tmem_st_wait();
+            tc_fence_before();
             warp_arrive(bar(DW_PFULL));
         }
         if (ok) ok = mbar_wait(bar(DW_ACCFULL), 0, ctl, W + 9);
+        if (ok && ntiles > 0) ok = mbar_wait(bar(DW_AEMPTY), (ntiles - 1) & 1, ctl, W + 16);
         if (ok) {
             tc_fence_after();
             // fp32 partial sums -> workspace[split][which][hk][row][DH], or bf16 results
@@ -805,9 +839,10 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             };
             constexpr int kColsPerHalf = DH / 2;
             const int c0 = part * kColsPerHalf;
-            {   // [dK;dU]: lane = row of the stacked block (0-63 dK, 64-127 dU)
-                float *dst = wsb + (row < kBI ? 0 : plane) + (long long)(row & (kBI - 1)) * DH + c0;
-                __nv_bfloat16 *o16 = out_row(row < kBI ? 0 : 1, row & (kBI - 1)) + c0;
+            {   // [dK;dU]: sixteen lanes of dK, sixteen of dU, ...
+                const int which = lane >> 4, r = quarter * 16 + (lane & 15);
+                float *dst = wsb + which * plane + (long long)r * DH + c0;
+                __nv_bfloat16 *o16 = out_row(which, r) + c0;
 #pragma unroll
                 for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
@@ -1336,7 +1371,10 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         dim3 gw((unsigned)ctas);
         prof_mark(st, kMarkStart);
         if constexpr (DH == 128) {
-            bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, wa);
+            CUtensorMap tmK16, tmU16;
+            if ((rc = encode_weight_map(&tmK16, p.K, d, 16)) != 0) return rc;
+            if ((rc = encode_weight_map(&tmU16, p.U, d, 16)) != 0) return rc;
+            bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK16, tmU16, tmV, wa);
         } else {
             CUtensorMap tmQt, tmdOt;
             if ((rc = encode_act_map(&tmQt, p.Q, d, kTT)) != 0) return rc;
