@@ -78,19 +78,33 @@ int lm_rmsnorm_backward(const void *x, const void *w, bool bf16_w, const void *g
 
 // Launch.  `early`: with programmatic stream serialization, so that the kernel may start before the one ahead of it on the
 // stream has ended (as soon as that one's CTAs have all asked for it, or exited).
+// `cluster`: CTAs (along x) of a thread-block cluster.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_kernel(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+cudaError_t launch_kernel(bool early, int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (early) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)cluster;
+        at[n].val.clusterDim.y = 1;
+        at[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = early ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_kernel(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+    return launch_kernel(early, 1, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 void set_cuda_error(cudaError_t e, const char *where);

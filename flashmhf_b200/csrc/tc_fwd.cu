@@ -23,6 +23,13 @@
 //   * The two MMA chains are issued by different threads (S by two threads, one per S buffer, so that each
 //     sees every phase of the barriers of its buffer; O by a third).
 //
+// Pairs of CTAs (CG = 2).  Every CTA reads all of its head's weights, 48 KB a block at d_h = 128 and as much again as the B operand of its
+// MMAs.  Two CTAs with a token tile each of one head share them: the first loads K and one half of V's columns, the second U and the
+// other half, and one MMA over both (cta_group::2, issued by the first) takes B from both shared memories.  That halves the bytes each
+// SM fetches from L2 and reads from shared memory, which is energy: at the power limit 16 x 2048 tokens of the 370M layer (d_h = 128)
+// 487 -> 471 us, 8192 tokens of the 1.3B layer 453 -> 435, 8 x 2048 tokens of the 128M layer (d_h = 96) 168.6 -> 157.9.  The pair's
+// barriers for its issuing threads lie in the first CTA and take the arrivals of both; its commits go to both.
+//
 // Warp roles: warp 0 TMA producer, warps 1-2 MMA issuers for S (even / odd blocks; warp 1 owns tensor
 // memory), warp 3 MMA issuer for O, then the activation warps (warp % 4 = TMEM lane quarter = 32 token rows).
 //
@@ -47,9 +54,9 @@ constexpr int kBI = 64;   // intermediate rows per block
 // the V ring is asked for again only when the O update that read it is done, so two stages cap the loop at two blocks per
 // (load + update + hand-offs).  At d_h = 64 a block is short and shared memory is plentiful; at 96 and 128 the rings
 // take what the Q tile leaves.
-template <int DH>
+template <int DH, int CG>
 struct FwdRings {
-    static constexpr int kKU = DH == 64 ? 6 : 4, kV = DH == 64 ? 6 : 4;
+    static constexpr int kKU = CG == 2 ? 8 : DH == 64 ? 6 : 4, kV = CG == 2 ? 7 : DH == 64 ? 6 : 4;
     static_assert(kKU % 2 == 0, "each [K;U] stage must belong to one S issuer");
 };
 // Activation teams of eight warps (warp % 4 = lane quarter, next bit = which 32 of a block's 64 columns).  With two
@@ -63,37 +70,39 @@ __host__ __device__ constexpr int threads_for(int dh) { return 128 + teams_for(d
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColO = 0, kColQ = 128, kColA0 = 192, kColAStride = 32, kColS0 = 256, kColSStride = 128;
 
-template <int DH>
+template <int DH, int CG>
 struct FwdSmem {
     static constexpr int kChunks = (DH + 63) / 64;              // 64-column SW128 chunks per row of d_h
     static constexpr uint32_t kQBytes = kChunks * kBT * 128;    // one Q tile (also the O staging tile of its work item)
     static constexpr uint32_t kWChunk = kBI * 128;              // one 64-row x 64-col weight chunk
-    static constexpr uint32_t kKUStage = 2 * kChunks * kWChunk; // per chunk: K rows then U rows = one 128-row K-major tile
-    static constexpr uint32_t kVStage = kChunks * kWChunk;
+    // [K;U]: per chunk K rows then U rows = one 128-row K-major tile; of a pair, the first CTA has the K rows and the second the U rows
+    static constexpr uint32_t kKUChunk = (CG == 2 ? 1 : 2) * kWChunk, kKUStage = kChunks * kKUChunk;
+    static constexpr uint32_t kVStage = CG == 2 ? kWChunk : kChunks * kWChunk;   // of a pair each CTA has half of V's columns
     // offsets from the 1024-aligned base
     // ONE Q tile: an item's Q is copied to tensor memory before the item ahead of it is written out, so the tile is Q first and
     // that item's O staging tile next.  (A second tile would cost the V ring two of its stages.)
     static constexpr uint32_t kOffQ = 0;
     static constexpr uint32_t kOffKU = kOffQ + kQBytes;
-    static constexpr uint32_t kOffV = kOffKU + FwdRings<DH>::kKU * kKUStage;
-    static constexpr uint32_t kOffBar = kOffV + FwdRings<DH>::kV * kVStage;
-    static constexpr uint32_t kTotal = kOffBar + 320 + 1024;  // + barriers/control + alignment slack
+    static constexpr uint32_t kOffV = kOffKU + FwdRings<DH, CG>::kKU * kKUStage;
+    static constexpr uint32_t kOffBar = kOffV + FwdRings<DH, CG>::kV * kVStage;
+    static constexpr uint32_t kTotal = kOffBar + 384 + 1024;  // + barriers/control + alignment slack
 };
 
 // barrier slots (8 bytes each) inside the control area
 // QFULL: an item's Q has landed; QFREE: an item's O, staged over the Q of the item after it, has been read by its TMA store;
 // SFULL[b]: S computed into buffer b; SEMPTY[b]: every warp of the team working on it has its part in registers;
-// AFULL[s]: A written to slot s; AFREE[s]: the O update that read slot s is done; QT: Q copied to tensor memory;
+// AFULL[s]: A written to slot s; AFREE[s]: the O update that read slot s is done; QT: Q copied to tensor memory
+// (QTALL: of a pair, by both CTAs);
 // SLAST: every S of a work item is computed (one commit from each S issuer; two teams only);
 // OFULL: the last O update of a work item is done; OFREE: its accumulator has been read out.
 // A CTA walks several work items (token tiles); blocks are counted through all of them (g), buffer and slot of a block
 // are g % 2, so every barrier has one fixed set of
 // waiters that observes each of its phases and a one-bit phase parity is enough.
-constexpr int kMaxRing = 6;
+constexpr int kMaxRing = 8;
 enum { BAR_QFULL = 0, BAR_QFREE = 1, BAR_QT = 2, BAR_SLAST = 3, BAR_SFULL = 4, BAR_SEMPTY = 6, BAR_AFULL = 8, BAR_AFREE = 10, BAR_OFULL = 12,
-       BAR_OFREE = 13, BAR_KUFULL = 14, BAR_KUEMPTY = BAR_KUFULL + kMaxRing, BAR_VFULL = BAR_KUEMPTY + kMaxRing,
+       BAR_OFREE = 13, BAR_QTALL = 14, BAR_KUFULL = 15, BAR_KUEMPTY = BAR_KUFULL + kMaxRing, BAR_VFULL = BAR_KUEMPTY + kMaxRing,
        BAR_VEMPTY = BAR_VFULL + kMaxRing, BAR_COUNT = BAR_VEMPTY + kMaxRing };
-static_assert(BAR_COUNT * 8 + 8 <= 320, "control area");
+static_assert(BAR_COUNT * 8 + 8 <= 384, "control area");
 
 struct FwdArgs {
     const float *R;
@@ -129,8 +138,21 @@ struct RingPos {
 struct FwdItem {
     int t0, h, b, isplit, j0, nblk;
 };
-__device__ __forceinline__ FwdItem fwd_item(const FwdArgs &a, int item, int nblk_total) {
+// Of a pair: one head and two token tiles, neighbours in the order (sequence, tile); behind the last tile of the last sequence b == B,
+// which reads as zero and is not written.
+template <int CG>
+__device__ __forceinline__ FwdItem fwd_item(const FwdArgs &a, int item, int nblk_total, uint32_t rank) {
     FwdItem w;
+    if (CG == 2) {
+        const int pairs = (a.tiles_per_seq * a.B + 1) >> 1;
+        w.h = item / pairs;
+        const int t = 2 * (item - w.h * pairs) + (int)rank;
+        w.b = t / a.tiles_per_seq;
+        w.t0 = (t - w.b * a.tiles_per_seq) * kBT;
+        w.isplit = w.j0 = 0;
+        w.nblk = nblk_total;
+        return w;
+    }
     w.isplit = item % a.nsplit;
     int t = item / a.nsplit;
     w.t0 = (t % a.tiles_per_seq) * kBT;
@@ -144,13 +166,13 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdArgs &a, int item, int nblk
 
 // Registers: d_h = 128 at most 152, so that a 128-thread CTA of the split reduction (48 registers) fits beside this one on an SM and is
 // resident when it ends; at 154 (allocated as 160) it is not, and a chained 1.3B decode step takes 23.0 instead of 21.9 us.
-template <int DH>
+template <int DH, int CG>
 __global__ void __maxnreg__(DH == 128 ? 152 : 96)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV,
            const __grid_constant__ CUtensorMap tmO, const FwdArgs args) {
-    using L = FwdSmem<DH>;
-    constexpr int kTeams = teams_for(DH), kKURing = FwdRings<DH>::kKU, kVRing = FwdRings<DH>::kV;
+    using L = FwdSmem<DH, CG>;
+    constexpr int kTeams = teams_for(DH), kKURing = FwdRings<DH, CG>::kKU, kVRing = FwdRings<DH, CG>::kV;
     static_assert(kKURing <= kMaxRing && kVRing <= kMaxRing, "barrier slots");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -162,16 +184,28 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     auto bar = [&](int i) { return sBar + 8u * i; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = CG == 2 ? cluster_rank() : 0;
+    const int first_item = blockIdx.x / CG, item_step = gridDim.x / CG;
+    // Barriers that the issuing CTA waits on and the element-wise warps or copies of both CTAs complete lie in the pair's first CTA.
+    const uint32_t sLead = CG == 2 ? cluster_addr(sBar, 0) : sBar;
+    auto lead = [&](int i) { return sLead + 8u * i; };
+    auto arrive_lead = [&](int i) { if (CG == 2) warp_arrive_cluster(lead(i)); else warp_arrive(bar(i)); };
+    auto commit = [&](int i) { if (CG == 2) umma_commit_pair(bar(i)); else umma_commit(bar(i)); };
+    auto mma_ts = [&](uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+        if (CG == 2) umma_ts_pair(d, a, b, id, acc);
+        else umma_ts(d, a, b, id, acc);
+    };
     const int blocks_per_e = args.De / kBI, nblk_total = args.E * blocks_per_e;
     const WaitCtl ctl{abort_flag, args.wait};
     constexpr int W = kKernelFwd * 100;
+    auto wait_lead = [&](int i, uint32_t parity, int code) { return mbar_wait<CG == 2>(bar(i), parity, ctl, code); };
 
     if (threadIdx.x == 0) {
         *abort_flag = launch_aborted(args.wait);  // a CTA of this launch gave up: drain fast
         for (int i = 0; i < 2; ++i) {
             mbar_init(bar(BAR_SFULL + i), 1);
-            mbar_init(bar(BAR_SEMPTY + i), arrivals_of(kTeamThreads));
-            mbar_init(bar(BAR_AFULL + i), arrivals_of(kTeamThreads));
+            mbar_init(bar(BAR_SEMPTY + i), CG * arrivals_of(kTeamThreads));
+            mbar_init(bar(BAR_AFULL + i), CG * arrivals_of(kTeamThreads));
             mbar_init(bar(BAR_AFREE + i), 1);
         }
         for (int i = 0; i < kKURing; ++i) {
@@ -186,16 +220,25 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         mbar_init(bar(BAR_QFREE), 1);
         mbar_init(bar(BAR_SLAST), 2);
         mbar_init(bar(BAR_OFULL), 1);
-        mbar_init(bar(BAR_OFREE), arrivals_of(kTeamThreads));
+        mbar_init(bar(BAR_OFREE), CG * arrivals_of(kTeamThreads));
         mbar_init(bar(BAR_QT), arrivals_of(kTeamThreads));
+        mbar_init(bar(BAR_QTALL), CG * arrivals_of(kTeamThreads));
         fence_mbar_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kTmemCols);
+    if (warp == 1) {
+        if (CG == 2) tmem_alloc_pair(smem_u32(const_cast<uint32_t *>(tmem_slot)), kTmemCols);
+        else tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kTmemCols);
+    }
     tc_fence_before();
     __syncthreads();
+    if (CG == 2) cluster_sync();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const bool dead = *abort_flag != 0;
+    bool dead = *abort_flag != 0;
+    if (CG == 2) {   // both CTAs of a pair give up, or neither
+        dead = dead || ld_shared_cluster(cluster_addr(sBar + BAR_COUNT * 8 + 4, rank ^ 1)) != 0;
+        cluster_sync();
+    }
     // Every launch may start under the end of the kernel before it (a decode step of 8 tokens of the 370M layer 12.3 -> 9.6 us a call);
     // until that kernel has ended only a chained call's producer touches global memory (weight tiles), the others wait below.
 
@@ -213,8 +256,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             RingPos<kVRing> pv;
             bool ok = true;
             int n = 0;  // work items of this CTA so far
-            for (int item = blockIdx.x; ok && item < args.n_items; item += gridDim.x, ++n) {
-                const FwdItem w = fwd_item(args, item, nblk_total);
+            for (int item = first_item; ok && item < args.n_items; item += item_step, ++n) {
+                const FwdItem w = fwd_item<CG>(args, item, nblk_total, rank);
                 const int hk = w.h / args.G;
                 // the tile's last use: Q of item 0 (until it is in tensor memory), then O of item n - 2
                 if (n == 1 && !mbar_wait(bar(BAR_QT), 0, ctl, W + 12)) break;
@@ -232,10 +275,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 for (int j = 0; j < w.nblk + 2; ++j) {
                     if (j < w.nblk) {
                         if (!mbar_wait(bar(BAR_KUEMPTY + pk.slot), pk.lap ^ 1, ctl, W + 1)) { ok = false; break; }
-                        const uint32_t fku = bar(BAR_KUFULL + pk.slot), dku = sKU + pk.slot * L::kKUStage;
-                        mbar_arrive_expect_tx(fku, L::kKUStage);
+                        const uint32_t fku = lead(BAR_KUFULL + pk.slot), dku = sKU + pk.slot * L::kKUStage;
+                        if (rank == 0) mbar_arrive_expect_tx(bar(BAR_KUFULL + pk.slot), CG * L::kKUStage);
 #pragma unroll
                         for (int c = 0; c < L::kChunks; ++c) {
+                            if (CG == 2) {
+                                tma_load_3d_pair(dku + c * L::kKUChunk, rank ? &tmU : &tmK, fku, c * 64, (w.j0 + j) * kBI, hk);
+                                continue;
+                            }
                             tma_load_3d(dku + c * 2 * L::kWChunk, &tmK, fku, c * 64, (w.j0 + j) * kBI, hk);
                             tma_load_3d(dku + c * 2 * L::kWChunk + L::kWChunk, &tmU, fku, c * 64, (w.j0 + j) * kBI, hk);
                         }
@@ -243,10 +290,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
                     if (j >= 2) {
                         if (!mbar_wait(bar(BAR_VEMPTY + pv.slot), pv.lap ^ 1, ctl, W + 2)) { ok = false; break; }
-                        const uint32_t fv = bar(BAR_VFULL + pv.slot), dv = sV + pv.slot * L::kVStage;
-                        mbar_arrive_expect_tx(fv, L::kVStage);
+                        const uint32_t fv = lead(BAR_VFULL + pv.slot), dv = sV + pv.slot * L::kVStage;
+                        if (rank == 0) mbar_arrive_expect_tx(bar(BAR_VFULL + pv.slot), CG * L::kVStage);
+                        if (CG == 2) tma_load_3d_pair(dv, &tmV, fv, (int)rank * (DH / 2), (w.j0 + j - 2) * kBI, hk);
 #pragma unroll
-                        for (int c = 0; c < L::kChunks; ++c)
+                        for (int c = 0; c < (CG == 2 ? 0 : L::kChunks); ++c)
                             tma_load_3d(dv + c * L::kWChunk, &tmV, fv, c * 64, (w.j0 + j - 2) * kBI, hk);
                         pv.advance(1);
                     }
@@ -259,64 +307,64 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         // work items of the CTA): while one is between batches -- barrier polls, commits -- the other keeps the tensor
         // pipe fed.  Q is read from tensor memory.  One thread issues a chain, so its instruction stream is kept
         // minimal: descriptors are built once and advanced by adding constants (the address field counts 16-byte units).
-        if (lane == 0) {
-            constexpr uint32_t idesc1 = umma_idesc(128, 2 * kBI, false, false);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc1 = umma_idesc(CG * 128, 2 * kBI, false, false);
             const uint64_t dKU0 = desc_kmajor(sKU);
             constexpr uint64_t kKUStep = L::kKUStage >> 4;
             const int sb = warp - 1;
             const uint32_t tS = tmem + kColS0 + sb * kColSStride, tQ = tmem + kColQ;
             bool ok = true;
             int g0 = 0, n = 0;   // blocks before this work item; work items so far
-            for (int item = blockIdx.x; ok && item < args.n_items; item += gridDim.x, ++n) {
-                const FwdItem w = fwd_item(args, item, nblk_total);
-                if (!mbar_wait(bar(BAR_QT), n & 1, ctl, W + 3)) break;   // this item's Q is in tensor memory
+            for (int item = first_item; ok && item < args.n_items; item += item_step, ++n) {
+                const FwdItem w = fwd_item<CG>(args, item, nblk_total, rank);
+                if (!wait_lead(CG == 2 ? BAR_QTALL : BAR_QT, n & 1, W + 3)) break;   // this item's Q is in tensor memory
                 for (int j = (g0 + sb) & 1; j < w.nblk; j += 2) {
                     const int g = g0 + j;                                 // g % 2 == sb
                     const int slot = g % kKURing;
                     if (!mbar_wait(bar(BAR_KUFULL + slot), (g / kKURing) & 1, ctl, W + 4)) { ok = false; break; }
                     // the buffer's previous block (g - 2) is in the activation warps' registers
-                    if (g >= 2 && !mbar_wait(bar(BAR_SEMPTY + sb), ((g >> 1) - 1) & 1, ctl, W + 5)) { ok = false; break; }
+                    if (g >= 2 && !wait_lead(BAR_SEMPTY + sb, ((g >> 1) - 1) & 1, W + 5)) { ok = false; break; }
                     tc_fence_after();
                     const uint64_t dku = dKU0 + slot * kKUStep;
 #pragma unroll
                     for (int k = 0; k < DH / 16; ++k) {
                         const int c = k >> 2, kk = k & 3;
-                        umma_ts(tS, tQ + k * 8, dku + ((c * 2 * L::kWChunk + kk * 32) >> 4), idesc1, k > 0 ? 1u : 0u);
+                        mma_ts(tS, tQ + k * 8, dku + ((c * L::kKUChunk + kk * 32) >> 4), idesc1, k > 0 ? 1u : 0u);
                     }
-                    umma_commit(bar(BAR_KUEMPTY + slot));
-                    umma_commit(bar(BAR_SFULL + sb));
+                    commit(BAR_KUEMPTY + slot);
+                    commit(BAR_SFULL + sb);
                 }
-                if (kTeams == 2 && ok) umma_commit(bar(BAR_SLAST));
+                if (kTeams == 2 && ok && item + item_step < args.n_items) commit(BAR_SLAST);   // (read before the next item's Q)
                 g0 += w.nblk;
             }
         }
     } else if (warp == 3) {
         // ------------------------------------------------------------------ MMA issuer 2: O += A V
         // A comes from tensor memory (slot g % 2), V from shared memory as an MN-major operand.
-        if (lane == 0) {
-            constexpr uint32_t idesc2 = umma_idesc(128, DH, false, true);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc2 = umma_idesc(CG * 128, DH, false, true);
             const uint64_t dV0 = desc_mnmajor(sV, L::kWChunk);
             constexpr uint64_t kVStep = L::kVStage >> 4;
             bool ok = true;
             int g0 = 0, n = 0;
-            for (int item = blockIdx.x; ok && item < args.n_items; item += gridDim.x, ++n) {
-                const FwdItem w = fwd_item(args, item, nblk_total);
+            for (int item = first_item; ok && item < args.n_items; item += item_step, ++n) {
+                const FwdItem w = fwd_item<CG>(args, item, nblk_total, rank);
                 // the accumulator of the previous work item has been read out
-                if (n >= 1 && !mbar_wait(bar(BAR_OFREE), (n - 1) & 1, ctl, W + 13)) break;
+                if (n >= 1 && !wait_lead(BAR_OFREE, (n - 1) & 1, W + 13)) break;
                 for (int j = 0; j < w.nblk; ++j) {
                     const int g = g0 + j, slot = g & 1, vs = g % kVRing;
                     if (!mbar_wait(bar(BAR_VFULL + vs), (g / kVRing) & 1, ctl, W + 6)) { ok = false; break; }
-                    if (!mbar_wait(bar(BAR_AFULL + slot), (g >> 1) & 1, ctl, W + 7)) { ok = false; break; }
+                    if (!wait_lead(BAR_AFULL + slot, (g >> 1) & 1, W + 7)) { ok = false; break; }
                     tc_fence_after();
                     const uint64_t dv = dV0 + vs * kVStep;
                     const uint32_t tA = tmem + kColA0 + slot * kColAStride;
 #pragma unroll
                     for (int k = 0; k < kBI / 16; ++k)
-                        umma_ts(tmem + kColO, tA + k * 8, dv + k * 128, idesc2, (j > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(bar(BAR_VEMPTY + vs));
-                    umma_commit(bar(BAR_AFREE + slot));
+                        mma_ts(tmem + kColO, tA + k * 8, dv + k * 128, idesc2, (j > 0 || k > 0) ? 1u : 0u);
+                    commit(BAR_VEMPTY + vs);
+                    commit(BAR_AFREE + slot);
                 }
-                if (ok) umma_commit(bar(BAR_OFULL));
+                if (ok) commit(BAR_OFULL);
                 g0 += w.nblk;
             }
         }
@@ -334,8 +382,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         // must be complete when it starts.  (64 chained tokens of the 1.3B layer 21.5 -> 20.5 us against a trigger before the wait.)
         griddep_launch_dependents();
         if (args.chained) {
-            if (warp == 4 && lane == 0 && blockIdx.x < args.n_items) {   // the first item's Q (q.v. the producer)
-                const FwdItem w = fwd_item(args, blockIdx.x, nblk_total);
+            if (warp == 4 && lane == 0 && first_item < args.n_items) {   // the first item's Q (q.v. the producer)
+                const FwdItem w = fwd_item<CG>(args, first_item, nblk_total, rank);
                 mbar_arrive_expect_tx(bar(BAR_QFULL), L::kQBytes);
                 for (int c = 0; c < L::kChunks; ++c)
                     tma_load_4d(sQ + c * (kBT * 128), &tmQ, bar(BAR_QFULL), c * 64, w.t0, w.h, w.b);
@@ -359,14 +407,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 tmem_st_wait();
             }
             tc_fence_before();
+            if (CG == 2) arrive_lead(BAR_QTALL);
             warp_arrive(bar(BAR_QT));
             return true;
         };
-        if (team == 0 && blockIdx.x < args.n_items) ok = copy_q(0);
-        for (int item = blockIdx.x; ok && item < args.n_items; item += gridDim.x, ++n) {
-            const FwdItem w = fwd_item(args, item, nblk_total);
+        if (team == 0 && first_item < args.n_items) ok = copy_q(0);
+        for (int item = first_item; ok && item < args.n_items; item += item_step, ++n) {
+            const FwdItem w = fwd_item<CG>(args, item, nblk_total, rank);
             const int t = w.t0 + row;
-            const bool in_range = t < args.S;
+            const bool in_range = t < args.S && (CG == 1 || w.b < args.B);
             const float *rrow = args.R + (long long)w.b * args.r_sb + (long long)w.h * args.r_sh + (long long)t * args.r_ss;
             // this team's first block of the item, its sub-network and position inside it; routing weight fetched one ahead
             // (plain loads: the kernel before this one, under which this one may have started, can be the one that wrote R, and a
@@ -393,7 +442,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     else tmem_ld16x2_sync(ts + sub * 16, ts + kBI + sub * 16, m, nn);
                     if (sub == 32 / kPiece - 1) {
                         tc_fence_before();
-                        warp_arrive(bar(BAR_SEMPTY + sb));  // S is in registers: the buffer may take block g + 2
+                        arrive_lead(BAR_SEMPTY + sb);  // S is in registers: the buffer may take block g + 2
                     }
 #pragma unroll
                     for (int i = 0; i < kPiece / 2; ++i)
@@ -406,7 +455,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 tmem_st16(lane_base + kColA0 + sb * kColAStride + group * 16, a);
                 tmem_st_wait();
                 tc_fence_before();
-                warp_arrive(bar(BAR_AFULL + sb));
+                arrive_lead(BAR_AFULL + sb);
 #pragma unroll
                 for (int k = 0; k < kTeams; ++k)
                     if (++in_e == blocks_per_e) {
@@ -421,7 +470,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             // The next item's Q may replace this one's in tensor memory once every S of this item is computed.  One team has read
             // them all by now; of two, team 0 knows of its own blocks only and waits for the others'.  (An issuer begins an item
             // after its Q is there, so it is never a phase ahead of this wait.)
-            if (item + (int)gridDim.x < args.n_items) {
+            if (item + item_step < args.n_items) {
                 if (kTeams == 2) {
                     if (!mbar_wait(bar(BAR_SLAST), n & 1, ctl, W + 14)) { ok = false; break; }
                     tc_fence_after();
@@ -450,7 +499,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
                 }
                 tc_fence_before();
-                warp_arrive(bar(BAR_OFREE));
+                arrive_lead(BAR_OFREE);
             } else {
                 named_bar_sync(2, kTeamThreads);   // the next item's Q has been copied out of the tile by all of the team
 #pragma unroll
@@ -468,11 +517,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
                 }
                 tc_fence_before();
-                warp_arrive(bar(BAR_OFREE));   // the accumulator is in registers / shared memory: the next item may overwrite it
+                arrive_lead(BAR_OFREE);   // the accumulator is in registers / shared memory: the next item may overwrite it
                 fence_async_smem();
                 named_bar_sync(1, kTeamThreads);
                 if (warp == 4 && lane == 0) {
-                    for (int c = 0; c < L::kChunks; ++c) tma_store_4d(&tmO, sO + c * (kBT * 128), c * 64, w.t0, w.h, w.b);
+                    for (int c = 0; c < (CG == 2 && w.b >= args.B ? 0 : L::kChunks); ++c) tma_store_4d(&tmO, sO + c * (kBT * 128), c * 64, w.t0, w.h, w.b);
                     tma_store_commit();
                     tma_store_wait_read();          // the tile has been read: it may take the Q of the item after next
                     mbar_arrive(bar(BAR_QFREE));
@@ -492,9 +541,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     }
     tc_fence_before();
     __syncthreads();
+    if (CG == 2) cluster_sync();   // the other CTA arrives on barriers here, and its MMAs read this one's shared and tensor memory
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, kTmemCols);
+        if (CG == 2) tmem_dealloc_pair(tmem, kTmemCols);
+        else tmem_dealloc(tmem, kTmemCols);
     }
 }
 
@@ -577,9 +628,19 @@ FwdPlan fwd_plan(const flashmhf_dims &d, int num_sms) {
     return p;
 }
 
-template <int DH>
-int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, bool chained) {
-    using L = FwdSmem<DH>;
+// Pairs of token tiles: those of one head in the order (sequence, tile), two by two.
+long long fwd_pairs(const flashmhf_dims &d) { return ((long long)((d.S + kBT - 1) / kBT) * d.B + 1) / 2 * d.H; }
+// In pairs at d_h = 96 and 128 (at 64 the activation paces the kernel: 372 us alone, 375 in pairs, 16384 tokens of 16 x 16 x 192), where
+// they take no more rounds over the SMs than single tiles (an odd number of tiles of a head leaves half a pair empty).
+bool fwd_in_pairs(const flashmhf_dims &d, const FwdPlan &pl, int num_sms) {
+    if (pl.nsplit > 1 || d.Dh == 64) return false;
+    const long long tiles = (long long)((d.S + kBT - 1) / kBT) * d.H * d.B, pairs = num_sms / 2;
+    return (fwd_pairs(d) + pairs - 1) / pairs <= (tiles + num_sms - 1) / num_sms;
+}
+
+template <int DH, int CG>
+int launch_fwd(const flashmhf_fwd_params &p, const FwdPlan &pl, const DeviceCtl *dc, cudaStream_t st, int *n_launch, bool chained) {
+    using L = FwdSmem<DH, CG>;
     CUtensorMap tmQ, tmK, tmU, tmV, tmO;
     int rc;
     if ((rc = encode_act_map(&tmQ, p.Q, p.d, kBT)) != 0) return rc;
@@ -587,17 +648,14 @@ int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, boo
     if ((rc = encode_weight_map(&tmU, p.U, p.d, kBI)) != 0) return rc;
     if ((rc = encode_weight_map(&tmV, p.V, p.d, kBI)) != 0) return rc;
     if ((rc = encode_act_map(&tmO, p.O, p.d, kBT)) != 0) return rc;
-    const DeviceCtl *dc = device_ctl();
-    if (!dc) return FLASHMHF_ERR_CUDA;
     {  // the attributes are per device and per kernel: set once for each pair
         static std::atomic<bool> done[64];
         if (!done[dc->device].load(std::memory_order_acquire)) {
-            cudaError_t e = cudaFuncSetAttribute(fwd_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
+            cudaError_t e = cudaFuncSetAttribute(fwd_kernel<DH, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
             if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(fwd_kernel)"); return FLASHMHF_ERR_CUDA; }
             done[dc->device].store(true, std::memory_order_release);
         }
     }
-    const FwdPlan pl = fwd_plan(p.d, dc->num_sms);
     if (pl.nsplit > 1) {
         if (!p.workspace || p.workspace_bytes < tc_forward_workspace_bytes(p.d) ||
             (reinterpret_cast<uintptr_t>(p.workspace) & 255u))
@@ -609,14 +667,14 @@ int launch_fwd(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, boo
               static_cast<float *>(p.workspace), p.d.H, p.d.B, 0, 0, 0.5f * p.scale.head_scaling,
               p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling, chained ? 1 : 0, wait_args(dc)};
     a.tiles_per_seq = (p.d.S + kBT - 1) / kBT;
-    const long long items = (long long)a.tiles_per_seq * p.d.H * p.d.B * pl.nsplit;
+    const long long items = CG == 2 ? fwd_pairs(p.d) : (long long)a.tiles_per_seq * p.d.H * p.d.B * pl.nsplit;
     if (items > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
     a.n_items = (int)items;
     // one CTA per SM walks the work items round-robin: the next item's Q load, Q copy and first S overlap this item's epilogue
     // (a split call has one item per CTA: tiles * splits <= SMs)
-    const unsigned grid = (unsigned)(items < dc->num_sms ? items : dc->num_sms);
+    const unsigned grid = (unsigned)(CG * (items < dc->num_sms / CG ? items : dc->num_sms / CG));
     prof_mark(st, kMarkStart);
-    cudaError_t e = launch_kernel(true, fwd_kernel<DH>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
+    cudaError_t e = launch_kernel(true, CG, fwd_kernel<DH, CG>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
     prof_mark(st, kMarkFwd);
     *n_launch += 1;
     if (e != cudaSuccess) { set_cuda_error(e, "fwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
@@ -650,11 +708,21 @@ size_t tc_forward_workspace_bytes(const flashmhf_dims &d) {
     return (size_t)pl.nsplit * (size_t)d.B * d.H * d.S * d.Dh * sizeof(float);
 }
 
+template <int DH>
+int forward_of(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, bool chained) {
+    const DeviceCtl *dc = device_ctl();
+    if (!dc) return FLASHMHF_ERR_CUDA;
+    const FwdPlan pl = fwd_plan(p.d, dc->num_sms);
+    if constexpr (DH != 64)
+        if (fwd_in_pairs(p.d, pl, dc->num_sms)) return launch_fwd<DH, 2>(p, pl, dc, st, n_launch, chained);
+    return launch_fwd<DH, 1>(p, pl, dc, st, n_launch, chained);
+}
+
 int tc_forward(const flashmhf_fwd_params &p, cudaStream_t st, int *n_launch, bool chained) {
     switch (p.d.Dh) {
-        case 64: return launch_fwd<64>(p, st, n_launch, chained);
-        case 96: return launch_fwd<96>(p, st, n_launch, chained);
-        case 128: return launch_fwd<128>(p, st, n_launch, chained);
+        case 64: return forward_of<64>(p, st, n_launch, chained);
+        case 96: return forward_of<96>(p, st, n_launch, chained);
+        case 128: return forward_of<128>(p, st, n_launch, chained);
         default: return FLASHMHF_ERR_BAD_SHAPE;
     }
 }
