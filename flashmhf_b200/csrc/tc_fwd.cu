@@ -36,6 +36,7 @@
 // Tensor memory (512 columns): O at [0, d_h), Q (bf16) at [128, 192), A slots at [192, 256), S buffers at
 // [256, 384), [384, 512).
 #include <atomic>
+#include <type_traits>
 
 #include "kernels.h"
 #include "tc_common.cuh"
@@ -115,7 +116,8 @@ struct FwdArgs {
     int H, B;
     int tiles_per_seq, n_items;   // work items = tiles_per_seq * H * B * nsplit, dealt round-robin to the CTAs
     float half_s0;  // 0.5 * head_scaling: tanh argument scale, sigmoid(s0 m) = 0.5 + 0.5 tanh(0.5 s0 m)
-    float c;        // head_scaling * up_scaling * final_scaling, folded into the routing weight
+    float c;        // head_scaling * up_scaling * final_scaling / q.q^2, folded into the routing weight
+    QScale q;
     // Chained call: launched with programmatic stream serialization.  The CTA may start, and stream weight tiles,
     // while the kernel before it on the stream still runs; Q and R are read, and anything written, only after
     // griddep_wait().
@@ -403,6 +405,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
                     qv[4 * c] = v.x; qv[4 * c + 1] = v.y; qv[4 * c + 2] = v.z; qv[4 * c + 3] = v.w;
                 }
+#pragma unroll
+                for (int c = 0; c < 32; ++c) qv[c] = bf16x2_mul(qv[c], args.q.q);
                 tmem_st32(lane_base + kColQ + group * 32, qv);
                 tmem_st_wait();
             }
@@ -444,10 +448,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         tc_fence_before();
                         arrive_lead(BAR_SEMPTY + sb);  // S is in registers: the buffer may take block g + 2
                     }
+                    auto activate = [&](auto pre) {
 #pragma unroll
-                    for (int i = 0; i < kPiece / 2; ++i)
-                        a[sub * 8 + i] = fwd_act_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(nn[2 * i], nn[2 * i + 1]), half_r,
-                                                      half_s0);
+                        for (int i = 0; i < kPiece / 2; ++i)
+                            a[sub * 8 + i] = fwd_act_pair<decltype(pre)::value>(f2_pack_bits(m[2 * i], m[2 * i + 1]),
+                                                                                f2_pack_bits(nn[2 * i], nn[2 * i + 1]), half_r, half_s0);
+                    };
+                    if (args.q.pre) activate(std::true_type{});
+                    else activate(std::false_type{});
                 }
                 // the slot's previous block (g - 2) has been consumed by its O update
                 if (g >= 2 && !mbar_wait(bar(BAR_AFREE + sb), ((g >> 1) - 1) & 1, ctl, W + 9)) { ok = false; break; }
@@ -662,10 +670,11 @@ int launch_fwd(const flashmhf_fwd_params &p, const FwdPlan &pl, const DeviceCtl 
             return FLASHMHF_ERR_WORKSPACE;
         if (p.O.stride[2] % 4 != 0 || p.O.stride[1] % 4 != 0 || p.O.stride[0] % 4 != 0) return FLASHMHF_ERR_BAD_STRIDE;
     }
+    const QScale qs = q_scale(p.scale.head_scaling);
     FwdArgs a{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
               p.d.S, p.d.E, p.d.De, p.d.H / p.d.Hkuv, pl.nsplit, pl.blocks_per_split,
               static_cast<float *>(p.workspace), p.d.H, p.d.B, 0, 0, 0.5f * p.scale.head_scaling,
-              p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling, chained ? 1 : 0, wait_args(dc)};
+              p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling / (qs.q * qs.q), qs, chained ? 1 : 0, wait_args(dc)};
     a.tiles_per_seq = (p.d.S + kBT - 1) / kBT;
     const long long items = CG == 2 ? fwd_pairs(p.d) : (long long)a.tiles_per_seq * p.d.H * p.d.B * pl.nsplit;
     if (items > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
