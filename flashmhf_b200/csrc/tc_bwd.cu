@@ -143,8 +143,9 @@ struct DqArgs {
     // writes an fp32 partial dQ to `part` ([nsplit][B][H][S][DH], added by the split reduction) and dR of its own sub-networks.
     int nsplit, e_per_split, H, B;
     float *part;
-    float s0, c_r, c_dr;  // head_scaling; head_scaling * up_scaling * final_scaling, over q.q for the routing weight, over its square for dR
-    QScale q;
+    float s0, c_r, c_dr;  // head_scaling; head_scaling * up_scaling * final_scaling, over the factor of Q for the routing weight, over its square for dR
+    uint32_t q_scale;     // factor of Q, twice, as bf16
+    int pre;
     WaitArgs wait;
 };
 
@@ -336,7 +337,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 }
                 if (which == 0) {
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) v32[c] = bf16x2_mul(v32[c], args.q.q);
+                    for (int c = 0; c < 32; ++c) v32[c] = bf16x2_mul(v32[c], args.q_scale);
                 }
                 tmem_st32(lane_base + (which ? kColdO : kColQ) + part * 32, v32);
             }
@@ -346,7 +347,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         warp_arrive(bar(DQ_QT));
         float r_cur = 0.f, r_next = in_range ? __ldg(rrow) : 0.f;
         f32x2 dr2 = f2_pack(0.f, 0.f);  // running dR_e of this thread's columns (two interleaved partial sums)
-        const DqConst kc = dq_const(args.s0, args.q.pre != 0);
+        const DqConst kc = dq_const(args.s0, args.pre != 0);
         int in_e = 0, e = 0;  // block index inside the current sub-network; current sub-network
         for (int j = 0; ok && j < nblk; ++j) {
             if (in_e == 0) {
@@ -374,7 +375,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     pn[i] = f2_to_bf16x2(x.dn);
                 }
             };
-            if (args.q.pre) activate(std::true_type{});
+            if (args.pre) activate(std::true_type{});
             else activate(std::false_type{});
             // the dQ update of the previous block has read the [dM|dN] buffer
             if (j >= 1 && !mbar_wait(bar(DQ_PEMPTY), (j - 1) & 1, ctl, W + 8)) { ok = false; break; }
@@ -1413,7 +1414,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         const QScale qs = q_scale(s0);
         const DqArgs qa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
                         static_cast<float *>(p.dR.ptr), p.dR.stride[0], p.dR.stride[1], p.dR.stride[2],
-                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c / qs.q, c / (qs.q * qs.q), qs, wait_args(dc)};
+                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c / qs.q, c / (qs.q * qs.q), qs.packed(), qs.pre, wait_args(dc)};
         const dim3 gq((unsigned)((d.S + kBT - 1) / kBT * ql.nsplit), d.H, d.B);
         prof_mark(st, kMarkStart);
         e = launch_kernel(want_weights, bwd_dq_kernel<DH>, gq, dim3(kThreads), DqSmem<DH>::kTotal, st, tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);

@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "kernels.h"
 
@@ -25,12 +26,17 @@ namespace fmhf {
 
 // The argument of the tanh is (s0 / 2) M (s0: the layer's head scaling).  Where s0 / 2 is 1/4, 1/2 or 1, Q is multiplied by it on its way to
 // tensor memory, which is exact, as is what it does to M and N; that saves the multiplication of every element of M and changes no bit of
-// any result.  At the power limit, 16384 tokens of 16 x 16 x 192 at d_h = 64: forward 368 -> 361.5 us, dQ/dR 682.5 -> 666.5; of the 128M layer
-// (d_h = 96): 155.6 -> 154.1, 277.6 -> 276.1; 32768 of the 370M layer (d_h = 128): 464 -> 464, 803 -> 799.
+// any result.  At the power limit, 16384 tokens of 16 x 16 x 192 at d_h = 64: forward 368 -> 358 us, dQ/dR 682 -> 667; of the 128M layer
+// (d_h = 96): 155.6 -> 154.2, 277.6 -> 276.1; 32768 of the 370M layer (d_h = 128): 464 -> 459, 803 -> 799.
 // (Other factors round, and larger ones could overflow: there Q stays as it is.)
 struct QScale {
     float q;    // factor of Q
     int pre;    // is it s0 / 2?
+    uint32_t packed() const {   // twice, as bf16 (a power of two: the upper half of its fp32 bits)
+        uint32_t b;
+        memcpy(&b, &q, 4);
+        return (b >> 16) | (b & 0xffff0000u);
+    }
 };
 inline QScale q_scale(float s0) {
     const float h = 0.5f * s0;
@@ -485,9 +491,9 @@ __device__ __forceinline__ uint32_t fwd_act_pair(f32x2 m, f32x2 n, f32x2 half_r,
     return f2_to_bf16x2(f2_fma(p, t, p));
 }
 
-// Two bf16 times a factor.
-__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t v, float f) {
-    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&v), __float2bfloat162_rn(f));
+// Two bf16 times two bf16.
+__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t v, uint32_t f) {
+    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&v), *reinterpret_cast<const __nv_bfloat162 *>(&f));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
 
