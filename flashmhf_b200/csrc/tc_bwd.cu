@@ -901,15 +901,14 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // =============================================================================================
 //                        dK / dU / dV kernel, transposed (d_h = 64 and 96)
 // =============================================================================================
-// The kernel above is bound by shared memory: every operand of its four products comes from there, the staged [dM|dN] and A
-// tiles included (ncu at d_h = 64: 142 KB read and 89 KB written per 128-token x 64-row block, 1800 of 2330 clk).  Where the
-// accumulators are narrow enough, the recompute is done transposed instead: a CTA owns 128 weight rows, and
+// A CTA owns 128 weight rows, and the three recomputed products
 //     M^T = K Q^T,  N^T = U Q^T,  dA^T = V dO^T      (128 weight rows x 64 tokens each, lane = weight row)
 // come out such that dM^T, dN^T and A^T, written back to tensor memory as bf16, are the A operands of
 //     dK += dM^T Q,  dU += dN^T Q,  dV += A^T dO     (128 x d_h each).
-// Nothing is staged in shared memory, the accumulating products read only their B operand there, and a token tile serves twice as
-// many weight rows: 112 KB (d_h = 64) instead of 231 KB per block.  Measured against the other form: 16 x 16 x 192 at d_h = 64,
-// 16384 tokens, 0.795 -> 0.697 ms; 128M layer (d_h = 96), 16384 tokens, 0.377 -> 0.342 ms.
+// Nothing is staged in shared memory, and a token tile serves twice as many weight rows as above.  Against the lane = token form, which
+// moved twice the bytes: 16 x 16 x 192 at d_h = 64, 16384 tokens, 0.795 -> 0.697 ms; 128M layer (d_h = 96), 16384 tokens, 0.377 -> 0.342 ms.
+// Against the form above: d_h = 64 754 against 945 us (its element-wise step is longer: loads of sixteen lanes, A through shared memory, and
+// it paces the kernel here), d_h = 96 373.7 against 371.7, at the power limit.
 // Tensor memory: three accumulators of d_h columns; d_h = 64: two buffers of [M^T | N^T] (128 columns), whose columns A^T, dM^T and
 // dN^T later take, and dA^T; d_h = 96: one [M^T | N^T], given back as soon as it is in registers, dA^T, over which dM^T and dN^T
 // are written, and 32 columns for A^T.  (d_h = 128 would need 576 columns.)

@@ -151,7 +151,9 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// One arrival for a whole warp (see warp_arrive) on a barrier of either CTA of the pair, given by its cluster address.
+// One arrival for a whole warp (see warp_arrive) on a barrier of either CTA of the pair, given by its cluster address.  What these barriers
+// guard is tensor memory, which the tcgen05 fences on both sides order; with .release.cluster every arrival is a fence over the cluster
+// besides, and the forward kernel took twice as long.
 __device__ __forceinline__ void warp_arrive_cluster(uint32_t cbar) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cbar) : "memory");
