@@ -25,7 +25,6 @@
 // which half of the columns).
 #include <atomic>
 #include <mutex>
-#include <type_traits>
 
 #include "dw_plan.h"
 #include "kernels.h"
@@ -145,11 +144,10 @@ struct DqArgs {
     float *part;
     float s0, c_r, c_dr;  // head_scaling; head_scaling * up_scaling * final_scaling, over the factor of Q for the routing weight, over its square for dR
     uint32_t q_scale;     // factor of Q, twice, as bf16
-    int pre;
     WaitArgs wait;
 };
 
-template <int DH>
+template <int DH, bool PRE>   // PRE: Q is multiplied by half the head scaling on its way to tensor memory
 __global__ void __maxnreg__(152)
 bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
               const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
@@ -335,7 +333,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
                     v32[4 * c] = v.x; v32[4 * c + 1] = v.y; v32[4 * c + 2] = v.z; v32[4 * c + 3] = v.w;
                 }
-                if (which == 0) {
+                if (PRE && which == 0) {
 #pragma unroll
                     for (int c = 0; c < 32; ++c) v32[c] = bf16x2_mul(v32[c], args.q_scale);
                 }
@@ -347,7 +345,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         warp_arrive(bar(DQ_QT));
         float r_cur = 0.f, r_next = in_range ? __ldg(rrow) : 0.f;
         f32x2 dr2 = f2_pack(0.f, 0.f);  // running dR_e of this thread's columns (two interleaved partial sums)
-        const DqConst kc = dq_const(args.s0, args.pre != 0);
+        const DqConst kc = dq_const(args.s0, PRE);
         int in_e = 0, e = 0;  // block index inside the current sub-network; current sub-network
         for (int j = 0; ok && j < nblk; ++j) {
             if (in_e == 0) {
@@ -365,18 +363,14 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             tmem_ld32x3_sync(tS, tS + kBI, tA, m, n, da);
             tc_fence_before();
             warp_arrive(bar(DQ_SEMPTY));
-            auto activate = [&](auto pre) {
 #pragma unroll
-                for (int i = 0; i < kCols / 2; ++i) {
-                    const DqPair x = dq_pair<decltype(pre)::value>(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
-                                                                   f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
-                    dr2 = f2_fma(x.da, x.sn, dr2);
-                    pm[i] = f2_to_bf16x2(x.dm);
-                    pn[i] = f2_to_bf16x2(x.dn);
-                }
-            };
-            if (args.pre) activate(std::true_type{});
-            else activate(std::false_type{});
+            for (int i = 0; i < kCols / 2; ++i) {
+                const DqPair x = dq_pair<PRE>(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
+                                              f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
+                dr2 = f2_fma(x.da, x.sn, dr2);
+                pm[i] = f2_to_bf16x2(x.dm);
+                pn[i] = f2_to_bf16x2(x.dn);
+            }
             // the dQ update of the previous block has read the [dM|dN] buffer
             if (j >= 1 && !mbar_wait(bar(DQ_PEMPTY), (j - 1) & 1, ctl, W + 8)) { ok = false; break; }
             tc_fence_after();
@@ -1340,7 +1334,9 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
     {  // the attribute is per device and per kernel: set once for each pair
         static std::atomic<bool> done[64];
         if (!done[dc->device].load(std::memory_order_acquire)) {
-            e = cudaFuncSetAttribute(bwd_dq_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DqSmem<DH>::kTotal);
+            e = cudaSuccess;
+            for (const auto k : {bwd_dq_kernel<DH, true>, bwd_dq_kernel<DH, false>})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DqSmem<DH>::kTotal);
             if (e == cudaSuccess)
                 if constexpr (DH == 128)
                     e = cudaFuncSetAttribute(bwd_dw_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DwSmem<DH>::kTotal);
@@ -1413,10 +1409,10 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         const QScale qs = q_scale(s0);
         const DqArgs qa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
                         static_cast<float *>(p.dR.ptr), p.dR.stride[0], p.dR.stride[1], p.dR.stride[2],
-                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c / qs.q, c / (qs.q * qs.q), qs.packed(), qs.pre, wait_args(dc)};
+                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c / qs.q, c / (qs.q * qs.q), qs.packed(), wait_args(dc)};
         const dim3 gq((unsigned)((d.S + kBT - 1) / kBT * ql.nsplit), d.H, d.B);
         prof_mark(st, kMarkStart);
-        e = launch_kernel(want_weights, bwd_dq_kernel<DH>, gq, dim3(kThreads), DqSmem<DH>::kTotal, st, tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);
+        e = launch_kernel(want_weights, qs.pre ? bwd_dq_kernel<DH, true> : bwd_dq_kernel<DH, false>, gq, dim3(kThreads), DqSmem<DH>::kTotal, st, tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);
         prof_mark(st, kMarkBwdDq);
         *n_launch += 1;
         if (e != cudaSuccess) { set_cuda_error(e, "bwd_dq_kernel launch"); return FLASHMHF_ERR_CUDA; }

@@ -26,8 +26,9 @@ namespace fmhf {
 
 // The argument of the tanh is (s0 / 2) M (s0: the layer's head scaling).  Where s0 / 2 is 1/4, 1/2 or 1, Q is multiplied by it on its way to
 // tensor memory, which is exact, as is what it does to M and N; that saves the multiplication of every element of M and changes no bit of
-// any result.  At the power limit, 16384 tokens of 16 x 16 x 192 at d_h = 64: forward 368 -> 358 us, dQ/dR 682 -> 667; of the 128M layer
-// (d_h = 96): 155.6 -> 154.2, 277.6 -> 276.1; 32768 of the 370M layer (d_h = 128): 464 -> 459, 803 -> 799.
+// any result.  Each is a kernel of its own (with a flag in one kernel most of it was lost at d_h = 128).  At the power limit, 16384 tokens of
+// 16 x 16 x 192 at d_h = 64: forward 368 -> 358 us, dQ/dR 682 -> 664; of the 128M layer (d_h = 96): 155.6 -> 154.2, 277.6 -> 274; 32768 of the
+// 370M layer (d_h = 128): 464 -> 459, 803 -> 791.  (dK/dU/dV: nothing at d_h = 128, so not done there.)
 // (Other factors round, and larger ones could overflow: there Q stays as it is.)
 struct QScale {
     float q;    // factor of Q
