@@ -463,15 +463,20 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // =============================================================================================
 // A CTA owns 64 weight rows.  The rows of K and U lie in the 128 lanes of one operand, sixteen of K, sixteen of U and so on, so that
 //     S^T = [K;U] Q^T        (128 lanes x 128 tokens: M in lanes 0-15 of each 32, N of the same weight rows in lanes 16-31)
-//     dA^T = V dO^T          (64 rows x 128 tokens: an M = 64 product fills lanes 0-15 of each 32)
-// put M, N and dA of a weight row under one warp, which reads sixteen lanes at a time, and what it writes back over dA, [dM;dN] as
-// bf16, is the A operand of
+//     dA^T = V dO^T          (64 rows x 128 tokens: an M = 64 product fills sixteen lanes of each 32, here 0-15)
+// put M, N and dA of a weight row under one warp, which reads sixteen lanes at a time, and what it writes back, [dM;dN] as bf16, is
+// the A operand of
 //     [dK;dU] += [dM;dN] Q   (128 x d_h).
-// Only A^T goes through shared memory, as the B operand of dV^T += dO^T A.  [K;U] are copied to tensor memory once.
-// Bound: shared memory (160 KB of operand reads, 64 KB of fills and 16 KB of A a tile: 1875 clk at 128 B/clk) and the tensor pipe
-// (1940 clk) alike, and power.  The other orientation (lane = token) moved 336 KB, since [dM|dN] had to be staged too and S read both its
-// operands there.  370M layer's operator, 32768 tokens, this kernel in a loop at the power limit: 1146 -> 1062 us (2.00 -> 1.70 M cycles);
-// ten passes 1035 -> 926.  Ordering matters as much as traffic: see the issuers.
+// Only A^T goes through shared memory, for dV += A^T dO, an M = 64 product too (lanes 16-31 of dA's columns).  [K;U] are copied to tensor
+// memory once.
+// Tensor memory (512 columns): [dK;dU] 128, [K;U] 64, S 128, dA and dV 128, [dM;dN] 64.  No product writes where another one reads: of two
+// MMAs with different accumulators or shapes, the order in which a thread issues them promises nothing.  As dV^T (M = 128, N = 64) the
+// dV update is half as long on the tensor pipe, but then [dM;dN] must lie over dA, and dA of the next tile must wait for the update that
+// reads them: 1156 us where this form takes 1017 (32768 tokens of the 370M layer's operator, in a loop at the power limit; ten passes
+// 1017 and 891).  [K;U] as an operand in shared memory instead, with dV^T: 1029 to 1039.  dA in two halves of 64 tokens, in lanes 0-15 and
+// 16-31 of 64 columns, with dV^T: 1136, since an M = 64 product takes as long at N = 64 as at 128.
+// Bound: the tensor pipe (2048 clk a tile) and shared memory (160 KB of operand reads, 64 KB of fills and 16 KB of A: 1875 clk at
+// 128 B/clk) of about 2590 clk a tile, and power.
 template <int DH>
 struct DwSmem {
     static constexpr int kChunks = (DH + 63) / 64;
@@ -490,11 +495,11 @@ struct DwSmem {
 };
 
 // Barriers.  Each is waited on by one fixed thread (or all element-wise warps) in every phase, so a one-bit parity is enough.
-//   KUT: [K;U] copied to tensor memory;  SFULL / SEMPTY: S computed / in registers;  DAFULL: dA computed, and with it, because the
-//   same thread issues it behind the [dK;dU] update of the tile before, that update is done, whose operand lies over dA;
-//   AFULL / AEMPTY: A staged / its dV update done;  PFULL: [dM;dN] written;  RFULL, REMPTY: routing weights;  DAISSUED (tile % 2): dA issued.
+//   KUT: [K;U] copied to tensor memory;  SFULL / SEMPTY, DAFULL / DAEMPTY: S, dA computed / in registers;  AFULL / AEMPTY: A staged /
+//   its dV update done;  PFULL / PEMPTY: [dM;dN] written / its update done;  RFULL, REMPTY: routing weights.
 enum { DW_WFULL = 0, DW_KUT = 1, DW_SFULL = 2, DW_SEMPTY = 3, DW_DAFULL = 4, DW_AFULL = 5, DW_AEMPTY = 6, DW_PFULL = 7, DW_ACCFULL = 8,
-       DW_RFULL = 9, DW_REMPTY = 11, DW_DAISSUED = 13, DW_QFULL = 15, DW_QEMPTY = 18, DW_GFULL = 21, DW_GEMPTY = 24, DW_BARS = 27 };
+       DW_RFULL = 9, DW_REMPTY = 11, DW_DAEMPTY = 13, DW_PEMPTY = 14, DW_QFULL = 15, DW_QEMPTY = 18, DW_GFULL = 21, DW_GEMPTY = 24,
+       DW_BARS = 27 };
 static_assert(DW_BARS * 8 + 8 <= 256, "control area");
 
 struct DwArgs {
@@ -576,8 +581,11 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const int ntiles = tile_end - tile_begin;  // >= 1 by construction of the plan
     const WaitCtl ctl{abort_flag, args.wait};
     constexpr int W = kKernelBwdDw * 100;
-    // Columns: [dK;dU] (d_h wide), dV^T (lane = column of dV, 64 wide), [K;U] as bf16 operand, S^T, dA^T (over which [dM;dN] is written).
-    constexpr uint32_t kColKU = 0, kColV = 128, kColW = 192, kColS = 256, kColdA = 384;
+    // Columns.  dA and dV share theirs, in lanes 0-15 and 16-31 of each 32.
+    constexpr uint32_t kColKU = 0, kColW = kColKU + DH, kColS = kColW + DH / 2, kColdA = kColS + kBT, kColV = kColdA,
+                       kColP = kColdA + kBT, kUpper = 16u << 16;
+    static_assert(DH <= kBT, "dV fits under dA");
+    static_assert(kColP + kBT / 2 <= kTmemCols, "tensor memory");
 
     auto tile_coords = [&](int i, int &ts, int &hh, int &bb) {  // token tile i of this CTA -> (seq tile, head, batch)
         const int ti = tile_begin + i;
@@ -589,9 +597,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 
     if (threadIdx.x == 0) {
         *abort_flag = launch_aborted(args.wait);  // a CTA of this launch gave up: drain fast
-        for (int i : {DW_WFULL, DW_SFULL, DW_DAFULL, DW_AEMPTY, DW_ACCFULL}) mbar_init(bar(i), 1);
-        for (int i = 0; i < 2; ++i) mbar_init(bar(DW_DAISSUED + i), 1);
-        for (int i : {DW_KUT, DW_SEMPTY, DW_AFULL, DW_PFULL}) mbar_init(bar(i), arrivals_of(kActThreads));
+        for (int i : {DW_WFULL, DW_SFULL, DW_DAFULL, DW_AEMPTY, DW_PEMPTY, DW_ACCFULL}) mbar_init(bar(i), 1);
+        for (int i : {DW_KUT, DW_SEMPTY, DW_DAEMPTY, DW_AFULL, DW_PFULL}) mbar_init(bar(i), arrivals_of(kActThreads));
         for (int s = 0; s < L::kRSlots; ++s) {
             mbar_init(bar(DW_RFULL + s), arrivals_of(32));
             mbar_init(bar(DW_REMPTY + s), arrivals_of(kActThreads));
@@ -651,24 +658,19 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer 1: S^T of the next tile, dV^T += dO^T A of this one
+        // ------------------------------------------------------------------ MMA issuer 1: S^T of the next tile, dV += A^T dO of this one
         if (lane == 0) {
             constexpr uint32_t idS = umma_idesc(128, kBT, false, false);
-            constexpr uint32_t idV = umma_idesc(128, kBI, true, false);
+            constexpr uint32_t idV = umma_idesc(64, DH, false, true);
             const uint64_t dQ0 = desc_kmajor(sQ), dG0 = desc_mnmajor(sG, kTile), dA0 = desc_kmajor(sA);
             constexpr uint64_t kTokStep = L::kTok >> 4;
             bool ok = mbar_wait(bar(DW_KUT), 0, ctl, W + 3);
             int sq = 0, sg = 0;
-            uint32_t phq = 0;
+            uint32_t phq = 0, phg = 0;
             for (int i = -1; ok && i < ntiles; ++i) {
-                // S of the next tile goes behind dA of this one, which is needed first.  That dA is issued says, too, that dO is there.
                 const bool more = i + 1 < ntiles;
                 if (more && !mbar_wait(bar(DW_QFULL + sq), phq, ctl, W + 4)) break;
                 if (more && i >= 0 && !mbar_wait(bar(DW_SEMPTY), i & 1, ctl, W + 5)) break;
-                // S of the next tile goes behind dA of this one, which is needed first (any order: 1091 instead of 1062 us).  That dA is
-                // issued says, too, that dO is there.  Two barriers in turn: issuer 2 can be one tile ahead of this wait, not two, since
-                // its dA after next needs S of the next tile.
-                if (i >= 0 && !mbar_wait(bar(DW_DAISSUED + (i & 1)), (i >> 1) & 1, ctl, W + 10)) break;
                 if (more) {
                     tc_fence_after();
                     const uint64_t dq = dQ0 + sq * kTokStep;
@@ -681,21 +683,20 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     if (++sq == L::kQStages) { sq = 0; phq ^= 1; }
                 }
                 if (i < 0) continue;
+                if (!mbar_wait(bar(DW_GFULL + sg), phg, ctl, W + 10)) break;   // (A^T does not imply that dO is there)
                 if (!mbar_wait(bar(DW_AFULL), i & 1, ctl, W + 6)) break;
                 tc_fence_after();
                 const uint64_t dg = dG0 + sg * kTokStep;
 #pragma unroll
                 for (int k = 0; k < kBT / 16; ++k)
-                    umma_ss(tmem + kColV, dg + k * 128, dA0 + (((k >> 2) * kWChunk + (k & 3) * 32) >> 4), idV, (i > 0 || k > 0) ? 1u : 0u);
+                    umma_ss(tmem + kUpper + kColV, dA0 + (((k >> 2) * kWChunk + (k & 3) * 32) >> 4), dg + k * 128, idV, (i > 0 || k > 0) ? 1u : 0u);
                 umma_commit(bar(DW_GEMPTY + sg));
                 umma_commit(bar(DW_AEMPTY));
-                if (++sg == L::kGStages) sg = 0;
+                if (++sg == L::kGStages) { sg = 0; phg ^= 1; }
             }
         }
     } else if (warp == 2) {
-        // ------------------------------------------------------------------ MMA issuer 2: dA^T, [dK;dU] += [dM;dN] Q
-        // One thread for both: a tile's dA overwrites the columns that the update of the tile before reads, and MMAs of one thread
-        // execute in order.
+        // ------------------------------------------------------------------ MMA issuer 2: dA^T of the next tile, [dK;dU] += [dM;dN] Q of this one
         if (lane == 0) {
             constexpr uint32_t idA = umma_idesc(64, kBT, false, false);
             constexpr uint32_t idKU = umma_idesc(128, DH, false, true);
@@ -704,33 +705,31 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             bool ok = mbar_wait(bar(DW_WFULL), 0, ctl, W + 3);
             int sq = 0, sg = 0;
             uint32_t phg = 0;
-            // No wait between the update of tile i and dA of tile i + 1: after a batch of MMAs a wait returns only when they have gone
-            // into the pipe, which is then empty.
             for (int i = -1; ok && i < ntiles; ++i) {
-                const bool more = i + 1 < ntiles;
-                if (more && !mbar_wait(bar(DW_GFULL + sg), phg, ctl, W + 4)) { ok = false; break; }
-                if (i >= 0) {
-                    if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
+                if (i + 1 < ntiles) {
+                    if (!mbar_wait(bar(DW_GFULL + sg), phg, ctl, W + 4)) { ok = false; break; }
+                    if (i >= 0 && !mbar_wait(bar(DW_DAEMPTY), i & 1, ctl, W + 18)) { ok = false; break; }
                     tc_fence_after();
-                    const uint64_t dq = dQ0 + sq * kTokStep;
+                    const uint64_t dg = dG0 + sg * kTokStep;
 #pragma unroll
-                    for (int k = 0; k < kBT / 16; ++k)
-                        umma_ts(tmem + kColKU, tmem + kColdA + (k >> 2) * 64 + (k & 3) * 8, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(bar(DW_QEMPTY + sq));
-                    if (++sq == L::kQStages) sq = 0;
+                    for (int k = 0; k < DH / 16; ++k) {
+                        const int c = k >> 2, kk = k & 3;
+                        umma_ss(tmem + kColdA, dV + ((c * kWChunk + kk * 32) >> 4), dg + ((c * kTile + kk * 32) >> 4), idA, k > 0 ? 1u : 0u);
+                    }
+                    umma_commit(bar(DW_DAFULL));
+                    umma_commit(bar(DW_GEMPTY + sg));
+                    if (++sg == L::kGStages) { sg = 0; phg ^= 1; }
                 }
-                if (!more) break;
+                if (i < 0) continue;
+                if (!mbar_wait(bar(DW_PFULL), i & 1, ctl, W + 6)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t dg = dG0 + sg * kTokStep;
+                const uint64_t dq = dQ0 + sq * kTokStep;
 #pragma unroll
-                for (int k = 0; k < DH / 16; ++k) {
-                    const int c = k >> 2, kk = k & 3;
-                    umma_ss(tmem + kColdA, dV + ((c * kWChunk + kk * 32) >> 4), dg + ((c * kTile + kk * 32) >> 4), idA, k > 0 ? 1u : 0u);
-                }
-                umma_commit(bar(DW_DAFULL));
-                umma_commit(bar(DW_GEMPTY + sg));
-                mbar_arrive(bar(DW_DAISSUED + ((i + 1) & 1)));
-                if (++sg == L::kGStages) { sg = 0; phg ^= 1; }
+                for (int k = 0; k < kBT / 16; ++k)
+                    umma_ts(tmem + kColKU, tmem + kColP + k * 8, dq + k * 128, idKU, (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(bar(DW_QEMPTY + sq));
+                umma_commit(bar(DW_PEMPTY));
+                if (++sq == L::kQStages) sq = 0;
             }
             if (ok) umma_commit(bar(DW_ACCFULL));
         }
@@ -758,7 +757,7 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         // and lane / 4 + 8 and of each eight tokens the two at 2 (lane % 4).  Pair 2x + rr: tokens 8x.., row lane / 4 + 8 rr.
         const int quarter = warp & 3, part = (warp - 4) >> 2;
         const int row = quarter * 32 + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), lane_up = lane_base + (16u << 16);
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), lane_up = lane_base + kUpper;
         bool ok = mbar_wait(bar(DW_WFULL), 0, ctl, W + 14);
         if (ok) {   // [K;U]: shared -> tensor memory, once (thread = stacked row; column part p copies columns [64p, 64p + 64) of d_h)
             uint32_t v32[32];
@@ -819,17 +818,23 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             warp_arrive(bar(DW_AFULL));
             // then dM and dN
             uint32_t da[32], pm[16], pn[16];
+            bool p_free = i == 0;
             if (!mbar_wait(bar(DW_DAFULL), i & 1, ctl, W + 11)) { ok = false; break; }
             tc_fence_after();
             tmem_ld_16x256b_x8_sync(lane_base + kColdA + part * 64, da);
+            tc_fence_before();
+            warp_arrive(bar(DW_DAEMPTY));
+            if (i >= 1) p_free = mbar_test(bar(DW_PEMPTY), (i - 1) & 1);
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
                 const f32x2 da2 = f2_pack_bits(da[2 * q], da[2 * q + 1]);
                 pm[q] = f2_to_bf16x2(f2_mul(da2, fw[q]));
                 pn[q] = f2_to_bf16x2(f2_mul(da2, fq[q]));
             }
-            tmem_st_16x128b_x8(lane_base + kColdA + part * 64, pm);
-            tmem_st_16x128b_x8(lane_up + kColdA + part * 64, pn);
+            if (!p_free && !mbar_wait(bar(DW_PEMPTY), (i - 1) & 1, ctl, W + 19)) { ok = false; break; }
+            tc_fence_after();
+            tmem_st_16x128b_x8(lane_base + kColP + part * 32, pm);
+            tmem_st_16x128b_x8(lane_up + kColP + part * 32, pn);
             tmem_st_wait();
             tc_fence_before();
             warp_arrive(bar(DW_PFULL));
@@ -859,20 +864,15 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     dw_store16(direct, dst + g * 16, o16 + g * 16, o);
                 }
             }
-            {   // dV^T: lane = column d of dV, tensor-memory column = row of the block; a warp stores 32 consecutive elements per row
-                float *dst = wsb + 2 * plane + row;
+            {   // dV: lanes 16-31 of each 32
+                const int r = quarter * 16 + (lane & 15);
+                float *dst = wsb + 2 * plane + (long long)r * DH + c0;
+                __nv_bfloat16 *o16 = out_row(2, r) + c0;
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
+                for (int g = 0; g < kColsPerHalf / 16; ++g) {
                     uint32_t o[16];
-                    tmem_ld16_sync(lane_base + kColV + part * 32 + g * 16, o);
-                    const int r0 = part * 32 + g * 16;
-                    if (direct) {
-#pragma unroll
-                        for (int v = 0; v < 16; ++v) out_row(2, r0 + v)[row] = __float2bfloat16(__uint_as_float(o[v]));
-                    } else {
-#pragma unroll
-                        for (int v = 0; v < 16; ++v) dst[(long long)(r0 + v) * DH] = __uint_as_float(o[v]);
-                    }
+                    tmem_ld16_sync(lane_base + kColV + c0 + g * 16, o);
+                    if (lane >= 16) dw_store16(direct, dst + g * 16, o16 + g * 16, o);
                 }
             }
             tc_fence_before();
