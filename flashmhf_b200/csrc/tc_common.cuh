@@ -153,11 +153,12 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
     return r;
 }
 // One arrival for a whole warp (see warp_arrive) on a barrier of either CTA of the pair, given by its cluster address.  What these barriers
-// guard is tensor memory, which the tcgen05 fences on both sides order; with .release.cluster every arrival is a fence over the cluster
-// besides, and the forward kernel took twice as long.
+// guard is tensor memory alone, which the tcgen05 fences on both sides of an execution order put in order, so the arrival has the scope of the
+// cluster but need not release anything: with .release every arrival is a fence over the cluster besides, and the forward kernel took
+// twice as long.  (Not for barriers that guard shared or global memory.)
 __device__ __forceinline__ void warp_arrive_cluster(uint32_t cbar) {
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cbar) : "memory");
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cbar) : "memory");
 }
 __device__ __forceinline__ uint32_t ld_shared_cluster(uint32_t caddr) {
     uint32_t v;
