@@ -49,22 +49,18 @@ constexpr uint32_t kWChunk = kBI * 128;  // one 64-row x 64-col chunk: 8 KB
 // 0.5 + 0.5 t, s = m*sg (so silu(s0 m) = s0 s), silu'(s0 m) = sg + s * s0 (1 - sg).  All three constants
 // fold into the per-row factor r2 = s0 s1 s2 r and into the two constants below, at no cost per element:
 //   dM = dA r2 n silu'(s0 m),  dN = dA r2 s,  A = s n r2,  dR = s0 s1 s2 * sum dA s n.
-// kPre: m and n come multiplied by h = s0 / 2 (see QScale).  Then s h takes the place of s, and what follows from it is put right, exactly, in
-// the row's factors: r2 / h, and dR / h^2.
 struct DqConst {
-    f32x2 half_s0, p_half_s0, n_half_s0;  // (s0/2), (s0/2), (-s0/2): tanh argument scale and s0 (1 - sg) = s0/2 - (s0/2) t (kPre: 1 - t)
+    f32x2 half_s0, p_half_s0, n_half_s0;  // (s0/2), (s0/2), (-s0/2): tanh argument scale and s0 (1 - sg) = s0/2 - (s0/2) t
 };
-__device__ __forceinline__ DqConst dq_const(float s0, bool pre) {
-    const float h = 0.5f * s0, k = pre ? 1.0f : h;
-    return DqConst{f2_pack(h, h), f2_pack(k, k), f2_pack(-k, -k)};
+__device__ __forceinline__ DqConst dq_const(float s0) {
+    return DqConst{f2_pack(0.5f * s0, 0.5f * s0), f2_pack(0.5f * s0, 0.5f * s0), f2_pack(-0.5f * s0, -0.5f * s0)};
 }
 struct DqPair {
     f32x2 dm, dn, sn, da;  // dM, dN, s*N (times r2 gives A, times dA sums to dR / (s0 s1 s2)), dA
 };
-template <bool kPre>
 __device__ __forceinline__ DqPair dq_pair(f32x2 m, f32x2 n, f32x2 da, f32x2 r2, const DqConst &k) {
     const f32x2 half = f2_pack(0.5f, 0.5f);
-    const f32x2 t = f2_tanh(kPre ? m : f2_mul(m, k.half_s0));
+    const f32x2 t = f2_tanh(f2_mul(m, k.half_s0));
     const f32x2 sg = f2_fma(t, half, half);
     const f32x2 omsg = f2_fma(t, k.n_half_s0, k.p_half_s0);
     const f32x2 s = f2_mul(m, sg);
@@ -142,12 +138,11 @@ struct DqArgs {
     // writes an fp32 partial dQ to `part` ([nsplit][B][H][S][DH], added by the split reduction) and dR of its own sub-networks.
     int nsplit, e_per_split, H, B;
     float *part;
-    float s0, c_r, c_dr;  // head_scaling; head_scaling * up_scaling * final_scaling, over the factor of Q for the routing weight, over its square for dR
-    uint32_t q_scale;     // factor of Q, twice, as bf16
+    float s0, c;  // head_scaling; head_scaling * up_scaling * final_scaling
     WaitArgs wait;
 };
 
-template <int DH, bool PRE>   // PRE: Q is multiplied by half the head scaling on its way to tensor memory
+template <int DH>
 __global__ void __maxnreg__(152)
 bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
               const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmU,
@@ -333,10 +328,6 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                     const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
                     v32[4 * c] = v.x; v32[4 * c + 1] = v.y; v32[4 * c + 2] = v.z; v32[4 * c + 3] = v.w;
                 }
-                if (PRE && which == 0) {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) v32[c] = bf16x2_mul(v32[c], args.q_scale);
-                }
                 tmem_st32(lane_base + (which ? kColdO : kColQ) + part * 32, v32);
             }
             tmem_st_wait();
@@ -345,7 +336,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         warp_arrive(bar(DQ_QT));
         float r_cur = 0.f, r_next = in_range ? __ldg(rrow) : 0.f;
         f32x2 dr2 = f2_pack(0.f, 0.f);  // running dR_e of this thread's columns (two interleaved partial sums)
-        const DqConst kc = dq_const(args.s0, PRE);
+        const DqConst kc = dq_const(args.s0);
         int in_e = 0, e = 0;  // block index inside the current sub-network; current sub-network
         for (int j = 0; ok && j < nblk; ++j) {
             if (in_e == 0) {
@@ -357,7 +348,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             tc_fence_after();
             const uint32_t tS = lane_base + kColS + part * kCols, tA = lane_base + kColdA + part * kCols;
             uint32_t pm[kCols / 2], pn[kCols / 2];  // packed bf16 pairs of dM, dN for this thread's columns
-            const f32x2 r2 = f2_pack(args.c_r * r_cur, args.c_r * r_cur);
+            const f32x2 r2 = f2_pack(args.c * r_cur, args.c * r_cur);
             // the whole part at once, so that S and dA are free for the next block before any arithmetic
             uint32_t m[kCols], n[kCols], da[kCols];
             tmem_ld32x3_sync(tS, tS + kBI, tA, m, n, da);
@@ -365,8 +356,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             warp_arrive(bar(DQ_SEMPTY));
 #pragma unroll
             for (int i = 0; i < kCols / 2; ++i) {
-                const DqPair x = dq_pair<PRE>(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
-                                              f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
+                const DqPair x = dq_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(n[2 * i], n[2 * i + 1]),
+                                         f2_pack_bits(da[2 * i], da[2 * i + 1]), r2, kc);
                 dr2 = f2_fma(x.da, x.sn, dr2);
                 pm[i] = f2_to_bf16x2(x.dm);
                 pn[i] = f2_to_bf16x2(x.dn);
@@ -384,7 +375,7 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
                 const int xb = e & 1;
                 float dr_lo, dr_hi;
                 f2_unpack(dr2, dr_lo, dr_hi);
-                const float dr_acc = (dr_lo + dr_hi) * args.c_dr;
+                const float dr_acc = (dr_lo + dr_hi) * args.c;
                 volatile float *xrow = drx + xb * 128 + row;
                 if (part != 0) {
                     // the exchange rows of sub-network e were last used by e - 2: wait until those values have been read
@@ -1334,9 +1325,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
     {  // the attribute is per device and per kernel: set once for each pair
         static std::atomic<bool> done[64];
         if (!done[dc->device].load(std::memory_order_acquire)) {
-            e = cudaSuccess;
-            for (const auto k : {bwd_dq_kernel<DH, true>, bwd_dq_kernel<DH, false>})
-                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DqSmem<DH>::kTotal);
+            e = cudaFuncSetAttribute(bwd_dq_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DqSmem<DH>::kTotal);
             if (e == cudaSuccess)
                 if constexpr (DH == 128)
                     e = cudaFuncSetAttribute(bwd_dw_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DwSmem<DH>::kTotal);
@@ -1406,13 +1395,12 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
             else
                 ql = DqPlan{1, d.E};
         }
-        const QScale qs = q_scale(s0);
         const DqArgs qa{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
                         static_cast<float *>(p.dR.ptr), p.dR.stride[0], p.dR.stride[1], p.dR.stride[2],
-                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c / qs.q, c / (qs.q * qs.q), qs.packed(), wait_args(dc)};
+                        d.S, d.E, d.De, G, ql.nsplit, ql.e_per_split, d.H, d.B, q_part, s0, c, wait_args(dc)};
         const dim3 gq((unsigned)((d.S + kBT - 1) / kBT * ql.nsplit), d.H, d.B);
         prof_mark(st, kMarkStart);
-        e = launch_kernel(want_weights, qs.pre ? bwd_dq_kernel<DH, true> : bwd_dq_kernel<DH, false>, gq, dim3(kThreads), DqSmem<DH>::kTotal, st, tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);
+        e = launch_kernel(want_weights, bwd_dq_kernel<DH>, gq, dim3(kThreads), DqSmem<DH>::kTotal, st, tmQ, tmdO, tmK, tmU, tmV, tmdQ, qa);
         prof_mark(st, kMarkBwdDq);
         *n_launch += 1;
         if (e != cudaSuccess) { set_cuda_error(e, "bwd_dq_kernel launch"); return FLASHMHF_ERR_CUDA; }

@@ -18,31 +18,10 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <string.h>
 
 #include "kernels.h"
 
 namespace fmhf {
-
-// The argument of the tanh is (s0 / 2) M (s0: the layer's head scaling).  Where s0 / 2 is 1/4, 1/2 or 1, Q is multiplied by it on its way to
-// tensor memory, which is exact, as is what it does to M and N; that saves the multiplication of every element of M and changes no bit of
-// any result.  Each is a kernel of its own (with a flag in one kernel most of it was lost at d_h = 128).  At the power limit, 16384 tokens of
-// 16 x 16 x 192 at d_h = 64: forward 368 -> 358 us, dQ/dR 682 -> 664; of the 128M layer (d_h = 96): 155.6 -> 154.2, 277.6 -> 274; 32768 of the
-// 370M layer (d_h = 128): 464 -> 459, 803 -> 791.  (dK/dU/dV: nothing at d_h = 128, so not done there.)
-// (Other factors round, and larger ones could overflow: there Q stays as it is.)
-struct QScale {
-    float q;    // factor of Q
-    int pre;    // is it s0 / 2?
-    uint32_t packed() const {   // twice, as bf16 (a power of two: the upper half of its fp32 bits)
-        uint32_t b;
-        memcpy(&b, &q, 4);
-        return (b >> 16) | (b & 0xffff0000u);
-    }
-};
-inline QScale q_scale(float s0) {
-    const float h = 0.5f * s0;
-    return h == 0.25f || h == 0.5f || h == 1.0f ? QScale{h, 1} : QScale{1.0f, 0};
-}
 
 // Status codes a kernel writes when a bounded wait runs out: kernel id * 100 + wait id.
 constexpr int kKernelFwd = 1, kKernelBwdDq = 2, kKernelBwdDw = 3, kKernelSelfTest = 99;
@@ -486,19 +465,11 @@ __device__ __forceinline__ uint32_t f2_to_bf16x2(f32x2 v) {
 
 // Forward activation for two neighbouring columns: bf16x2 of  silu(s0 m) * (s1 n) * s2 * r  for raw products m, n.
 // With t = tanh(s0 m / 2): the value is p + p*t, p = (m*n) * (s0 s1 s2 r / 2).
-// `half_r` = (s0 s1 s2 r / 2) twice, `half_s0` = (s0 / 2) twice; kPre: m and n come multiplied by s0 / 2 (see QScale), `half_r` divided by
-// its square.
-template <bool kPre>
+// `half_r` = (s0 s1 s2 r / 2) twice, `half_s0` = (s0 / 2) twice.
 __device__ __forceinline__ uint32_t fwd_act_pair(f32x2 m, f32x2 n, f32x2 half_r, f32x2 half_s0) {
-    const f32x2 t = f2_tanh(kPre ? m : f2_mul(m, half_s0));
+    const f32x2 t = f2_tanh(f2_mul(m, half_s0));
     const f32x2 p = f2_mul(f2_mul(m, n), half_r);
     return f2_to_bf16x2(f2_fma(p, t, p));
-}
-
-// Two bf16 times two bf16.
-__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t v, uint32_t f) {
-    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162 *>(&v), *reinterpret_cast<const __nv_bfloat162 *>(&f));
-    return *reinterpret_cast<const uint32_t *>(&r);
 }
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {

@@ -115,8 +115,7 @@ struct FwdArgs {
     int H, B;
     int tiles_per_seq, n_items;   // work items = tiles_per_seq * H * B * nsplit, dealt round-robin to the CTAs
     float half_s0;  // 0.5 * head_scaling: tanh argument scale, sigmoid(s0 m) = 0.5 + 0.5 tanh(0.5 s0 m)
-    float c;        // head_scaling * up_scaling * final_scaling / q_scale^2, folded into the routing weight
-    uint32_t q_scale;   // factor of Q, twice, as bf16
+    float c;        // head_scaling * up_scaling * final_scaling, folded into the routing weight
     // Chained call: launched with programmatic stream serialization.  The CTA may start, and stream weight tiles,
     // while the kernel before it on the stream still runs; Q and R are read, and anything written, only after
     // griddep_wait().
@@ -167,8 +166,7 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdArgs &a, int item, int nblk
 
 // Registers: d_h = 128 at most 152, so that a 128-thread CTA of the split reduction (48 registers) fits beside this one on an SM and is
 // resident when it ends; at 154 (allocated as 160) it is not, and a chained 1.3B decode step takes 23.0 instead of 21.9 us.
-// PRE: Q is multiplied by q_scale on its way (a second kernel, not a flag: short calls wait for their instructions to be fetched).
-template <int DH, int CG, bool PRE>
+template <int DH, int CG>
 __global__ void __maxnreg__(DH == 128 ? 152 : 96)
 fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
            const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV,
@@ -402,10 +400,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 const uint8_t *src = gbase + L::kOffQ + group * (kBT * 128);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
-                    if (PRE)
-                        v = make_uint4(bf16x2_mul(v.x, args.q_scale), bf16x2_mul(v.y, args.q_scale), bf16x2_mul(v.z, args.q_scale),
-                                       bf16x2_mul(v.w, args.q_scale));
+                    const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
                     qv[4 * c] = v.x; qv[4 * c + 1] = v.y; qv[4 * c + 2] = v.z; qv[4 * c + 3] = v.w;
                 }
                 tmem_st32(lane_base + kColQ + group * 32, qv);
@@ -451,8 +446,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
 #pragma unroll
                     for (int i = 0; i < kPiece / 2; ++i)
-                        a[sub * 8 + i] = fwd_act_pair<PRE>(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(nn[2 * i], nn[2 * i + 1]), half_r,
-                                                           half_s0);
+                        a[sub * 8 + i] = fwd_act_pair(f2_pack_bits(m[2 * i], m[2 * i + 1]), f2_pack_bits(nn[2 * i], nn[2 * i + 1]), half_r,
+                                                      half_s0);
                 }
                 // the slot's previous block (g - 2) has been consumed by its O update
                 if (g >= 2 && !mbar_wait(bar(BAR_AFREE + sb), ((g >> 1) - 1) & 1, ctl, W + 9)) { ok = false; break; }
@@ -653,15 +648,10 @@ int launch_fwd(const flashmhf_fwd_params &p, const FwdPlan &pl, const DeviceCtl 
     if ((rc = encode_weight_map(&tmU, p.U, p.d, kBI)) != 0) return rc;
     if ((rc = encode_weight_map(&tmV, p.V, p.d, kBI)) != 0) return rc;
     if ((rc = encode_act_map(&tmO, p.O, p.d, kBT)) != 0) return rc;
-    // (split calls have too few blocks an item to gain by it: 64 tokens of the 128M layer 9.87 us, 9.98 with it)
-    const QScale qs = pl.nsplit == 1 ? q_scale(p.scale.head_scaling) : QScale{1.0f, 0};
-    const auto kernel = qs.pre ? fwd_kernel<DH, CG, true> : fwd_kernel<DH, CG, false>;
     {  // the attributes are per device and per kernel: set once for each pair
         static std::atomic<bool> done[64];
         if (!done[dc->device].load(std::memory_order_acquire)) {
-            cudaError_t e = cudaSuccess;
-            for (const auto k : {fwd_kernel<DH, CG, true>, fwd_kernel<DH, CG, false>})
-                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
+            cudaError_t e = cudaFuncSetAttribute(fwd_kernel<DH, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kTotal);
             if (e != cudaSuccess) { set_cuda_error(e, "cudaFuncSetAttribute(fwd_kernel)"); return FLASHMHF_ERR_CUDA; }
             done[dc->device].store(true, std::memory_order_release);
         }
@@ -675,7 +665,7 @@ int launch_fwd(const flashmhf_fwd_params &p, const FwdPlan &pl, const DeviceCtl 
     FwdArgs a{static_cast<const float *>(p.R.ptr), p.R.stride[0], p.R.stride[1], p.R.stride[2],
               p.d.S, p.d.E, p.d.De, p.d.H / p.d.Hkuv, pl.nsplit, pl.blocks_per_split,
               static_cast<float *>(p.workspace), p.d.H, p.d.B, 0, 0, 0.5f * p.scale.head_scaling,
-              p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling / (qs.q * qs.q), qs.packed(), chained ? 1 : 0, wait_args(dc)};
+              p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling, chained ? 1 : 0, wait_args(dc)};
     a.tiles_per_seq = (p.d.S + kBT - 1) / kBT;
     const long long items = CG == 2 ? fwd_pairs(p.d) : (long long)a.tiles_per_seq * p.d.H * p.d.B * pl.nsplit;
     if (items > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
@@ -684,7 +674,7 @@ int launch_fwd(const flashmhf_fwd_params &p, const FwdPlan &pl, const DeviceCtl 
     // (a split call has one item per CTA: tiles * splits <= SMs)
     const unsigned grid = (unsigned)(CG * (items < dc->num_sms / CG ? items : dc->num_sms / CG));
     prof_mark(st, kMarkStart);
-    cudaError_t e = launch_kernel(true, CG, kernel, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
+    cudaError_t e = launch_kernel(true, CG, fwd_kernel<DH, CG>, dim3(grid), dim3(threads_for(DH)), L::kTotal, st, tmQ, tmK, tmU, tmV, tmO, a);
     prof_mark(st, kMarkFwd);
     *n_launch += 1;
     if (e != cudaSuccess) { set_cuda_error(e, "fwd_kernel launch"); return FLASHMHF_ERR_CUDA; }
