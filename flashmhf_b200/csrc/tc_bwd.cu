@@ -622,10 +622,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
             mbar_arrive_expect_tx(bar(DW_WFULL), L::kChunks * kTile + L::kVBytes);
             const int row = jblk * kBI;
             for (int c = 0; c < L::kChunks; ++c) {
-                for (int g = 0; g < 4; ++g) {   // sixteen rows of K, sixteen of U, ...
-                    tma_load_3d(sKU + c * kTile + g * 32 * 128, &tmK, bar(DW_WFULL), c * 64, row + g * 16, hk);
-                    tma_load_3d(sKU + c * kTile + (g * 32 + 16) * 128, &tmU, bar(DW_WFULL), c * 64, row + g * 16, hk);
-                }
+                tma_load_3d(sKU + c * kTile, &tmK, bar(DW_WFULL), c * 64, row, hk);
+                tma_load_3d(sKU + c * kTile + kWChunk, &tmU, bar(DW_WFULL), c * 64, row, hk);
                 tma_load_3d(sV + c * kWChunk, &tmV, bar(DW_WFULL), c * 64, row, hk);
             }
             int sq = 0, sg = 0;
@@ -747,15 +745,15 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         // A warp has sixteen weight rows (M, dA in lanes 0-15 of its quarter, N in lanes 16-31) and 64 tokens; a thread rows lane / 4
         // and lane / 4 + 8 and of each eight tokens the two at 2 (lane % 4).  Pair 2x + rr: tokens 8x.., row lane / 4 + 8 rr.
         const int quarter = warp & 3, part = (warp - 4) >> 2;
-        const int row = quarter * 32 + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), lane_up = lane_base + kUpper;
         bool ok = mbar_wait(bar(DW_WFULL), 0, ctl, W + 14);
         if (ok) {   // [K;U]: shared -> tensor memory, once (thread = stacked row; column part p copies columns [64p, 64p + 64) of d_h)
             uint32_t v32[32];
+            const int src_row = (lane >> 4) * kBI + quarter * 16 + (lane & 15);   // they arrive as 64 rows of K and 64 of U
             const uint8_t *src = gbase + L::kOffKU + part * kTile;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(row, c));
+                const uint4 v = *reinterpret_cast<const uint4 *>(src + sw128_offset(src_row, c));
                 v32[4 * c] = v.x; v32[4 * c + 1] = v.y; v32[4 * c + 2] = v.z; v32[4 * c + 3] = v.w;
             }
             tmem_st32(lane_base + kColW + part * 32, v32);
@@ -1370,10 +1368,7 @@ int launch_bwd(const flashmhf_bwd_params &p, cudaStream_t st, int *n_launch) {
         dim3 gw((unsigned)ctas);
         prof_mark(st, kMarkStart);
         if constexpr (DH == 128) {
-            CUtensorMap tmK16, tmU16;
-            if ((rc = encode_weight_map(&tmK16, p.K, d, 16)) != 0) return rc;
-            if ((rc = encode_weight_map(&tmU16, p.U, d, 16)) != 0) return rc;
-            bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK16, tmU16, tmV, wa);
+            bwd_dw_kernel<DH><<<gw, kThreads, DwSmem<DH>::kTotal, st>>>(tmQ, tmdO, tmK, tmU, tmV, wa);
         } else {
             CUtensorMap tmQt, tmdOt;
             if ((rc = encode_act_map(&tmQt, p.Q, d, kTT)) != 0) return rc;
