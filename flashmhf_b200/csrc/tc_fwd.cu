@@ -667,8 +667,8 @@ int launch_fwd(const flashmhf_fwd_params &p, const FwdPlan &pl, const DeviceCtl 
               static_cast<float *>(p.workspace), p.d.H, p.d.B, 0, 0, 0.5f * p.scale.head_scaling,
               p.scale.head_scaling * p.scale.up_scaling * p.scale.final_scaling, chained ? 1 : 0, wait_args(dc)};
     a.tiles_per_seq = (p.d.S + kBT - 1) / kBT;
-    const long long items = CG == 2 ? fwd_pairs(p.d) : (long long)a.tiles_per_seq * p.d.H * p.d.B * pl.nsplit;
-    if (items > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;
+    const long long tiles = (long long)a.tiles_per_seq * p.d.H * p.d.B * pl.nsplit, items = CG == 2 ? fwd_pairs(p.d) : tiles;
+    if (tiles > 0x7fffffffLL) return FLASHMHF_ERR_BAD_SHAPE;   // (in pairs, too: the kernel counts a head's tiles in 32 bits)
     a.n_items = (int)items;
     // one CTA per SM walks the work items round-robin: the next item's Q load, Q copy and first S overlap this item's epilogue
     // (a split call has one item per CTA: tiles * splits <= SMs)
