@@ -20,9 +20,9 @@
 //   With more than one split each CTA writes fp32 partial sums to the workspace; dw_reduce_kernel adds the splits in a
 //   fixed order and writes bf16 dK, dU, dV.
 //
-// All use 384 threads: warp 0 TMA producer, warps 1 to 3 MMA issuers (one per MMA chain; warp 1 owns tensor memory; warp 2
-// of bwd_dwt_kernel and warp 3 of bwd_dw_kernel fetch routing weights), warps 4-11 element-wise math (warp % 4 = TMEM lane quarter, (warp-4)/4 =
-// which half of the columns).
+// All use 384 threads: warp 0 TMA producer, warps 1 to 3 MMA issuers (one per chain in bwd_dq_kernel, two chains each in the others, whose
+// third, warp 3 of bwd_dw_kernel and warp 2 of bwd_dwt_kernel, fetches routing weights instead; warp 1 owns tensor memory), warps 4-11
+// element-wise math (warp % 4 = TMEM lane quarter, (warp-4)/4 = which half of the columns).
 #include <atomic>
 #include <mutex>
 
@@ -890,8 +890,8 @@ bwd_dw_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 //     dK += dM^T Q,  dU += dN^T Q,  dV += A^T dO     (128 x d_h each).
 // Nothing is staged in shared memory, and a token tile serves twice as many weight rows as above.  Against the lane = token form, which
 // moved twice the bytes: 16 x 16 x 192 at d_h = 64, 16384 tokens, 0.795 -> 0.697 ms; 128M layer (d_h = 96), 16384 tokens, 0.377 -> 0.342 ms.
-// Against the form above: d_h = 64 754 against 945 us (its element-wise step is longer: loads of sixteen lanes, A through shared memory, and
-// it paces the kernel here), d_h = 96 373.7 against 371.7, at the power limit.
+// Against the form above, when its dV was accumulated transposed: d_h = 64 754 against 945 us (its element-wise step is longer: loads of
+// sixteen lanes, A through shared memory, and it paces the kernel here), d_h = 96 373.7 against 371.7, at the power limit.
 // Tensor memory: three accumulators of d_h columns; d_h = 64: two buffers of [M^T | N^T] (128 columns), whose columns A^T, dM^T and
 // dN^T later take, and dA^T; d_h = 96: one [M^T | N^T], given back as soon as it is in registers, dA^T, over which dM^T and dN^T
 // are written, and 32 columns for A^T.  (d_h = 128 would need 576 columns.)

@@ -154,8 +154,9 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
 }
 
 // ------------------------------------------------------------------------------------ TMA
-// Tile loads into this CTA's shared memory, completion counted in bytes on an mbarrier.  The
-// innermost coordinate is always a multiple of 64 bf16 elements here (128 bytes).
+// Tile loads into this CTA's shared memory, completion counted in bytes on an mbarrier.  The innermost coordinate is a multiple of
+// 64 bf16 elements (128 bytes), but for the second half of V's columns in a pair at d_h = 96: there it is 48 (96 bytes; it must be a
+// multiple of 16 bytes), and the last 16 of the box's 64 columns are out of range and read as zero.
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1,
                                             int c2) {
     asm volatile(

@@ -62,8 +62,8 @@ struct FwdRings {
 // Activation teams of eight warps (warp % 4 = lane quarter, next bit = which 32 of a block's 64 columns).  With two
 // teams, team t owns the blocks j = t (mod 2) and with them S buffer t and A slot t; the two teams are then in
 // different phases of their loop (wait, load, arithmetic, store), which keeps the arithmetic pipes busy.
-// One team at d_h = 128, where the kernel is paced by the arrival of the weight tiles from L2 (48 KB per block at
-// about 50 B/clk per SM) and by the tensor pipe; two teams at d_h = 64 and 96, where it is paced by the activation.
+// Two teams at d_h = 64 and 96, where the activation paces the kernel; one at d_h = 128, where the tensor pipe does and the weight tiles from
+// L2 (48 KB a block and CTA, 24 of a pair): two teams of pairs there take 470.3 us, one 471.5 (32768 tokens of the 370M layer).
 constexpr int kTeamThreads = 256;
 __host__ __device__ constexpr int teams_for(int dh) { return dh == 128 ? 1 : 2; }
 __host__ __device__ constexpr int threads_for(int dh) { return 128 + teams_for(dh) * kTeamThreads; }
@@ -292,6 +292,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         if (!mbar_wait(bar(BAR_VEMPTY + pv.slot), pv.lap ^ 1, ctl, W + 2)) { ok = false; break; }
                         const uint32_t fv = lead(BAR_VFULL + pv.slot), dv = sV + pv.slot * L::kVStage;
                         if (rank == 0) mbar_arrive_expect_tx(bar(BAR_VFULL + pv.slot), CG * L::kVStage);
+                        // (d_h = 96: columns 48 to 111, of which those from 96 on are zero and not read)
                         if (CG == 2) tma_load_3d_pair(dv, &tmV, fv, (int)rank * (DH / 2), (w.j0 + j - 2) * kBI, hk);
 #pragma unroll
                         for (int c = 0; c < (CG == 2 ? 0 : L::kChunks); ++c)
