@@ -18,18 +18,17 @@ struct DwPlan {
     double tiles;               // predicted duration, in token tiles
 };
 
-// How the weight-gradient kernel of a head dimension cuts its work, and what it takes: a token tile; a CTA besides its tiles (weights in,
-// first tile through the pipeline, accumulators out); a split's extra launch (4 us) and a byte of partial sums (written once, read once,
-// about 4 TB/s), all but the first in units of one token tile.  (d_h = 128, one to six full waves of 4 to 128 tiles a CTA: 1.33 us a tile
-// and 9.4 a CTA, at the worst 11 % off.)
+// How the weight-gradient kernel of a head dimension cuts its work, and what a CTA costs besides its token tiles (weights in,
+// first tile through the pipeline, accumulators out: the intercept of kernel time over tiles per CTA, about 7 us), a split's
+// extra launch (4 us) and a byte of partial sums (written once, read once, about 4 TB/s), all in units of one token tile.
 struct DwShape {
     int rows, tokens;
-    double tile_us, cta_us;
-    double fixed() const { return cta_us / tile_us; }
+    double tile_us;
+    double fixed() const { return 7.0 / tile_us; }
     double launch() const { return 4.0 / tile_us; }
     double sums(double bytes) const { return bytes / 4.0e6 / tile_us; }
 };
-inline DwShape dw_shape(int dh) { return dh == 128 ? DwShape{64, 128, 1.33, 9.4} : DwShape{128, 64, dh == 64 ? 0.8 : 1.0, 7.0}; }
+inline DwShape dw_shape(int dh) { return dh == 128 ? DwShape{64, 128, 1.8} : DwShape{128, 64, dh == 64 ? 0.8 : 1.0}; }
 
 // The times at which the SMs become free, as few (time, number of SMs) groups: jobs come in runs of equal length, so a run is dealt
 // out by groups of SMs, and by whole rounds where every SM gets one, instead of job by job.  A run adds one group at most.
@@ -173,9 +172,8 @@ inline DwPlan make_plan(const flashmhf_dims &d, int num_sms, bool followed, size
     best.nsplit = 1;
     best.tiles_per_split = p0.tiles_total;
     double best_cost = (double)((items + num_sms - 1) / num_sms) * (p0.tiles_total + sh.fixed());
-    // The dQ/dR kernel fills the last wave.  (The whole backward of shapes whose plan this factor decides, against none: 1.5 % faster at d_h = 64
-    // and 5.8 % at 96, 16 shapes each, single ones between 7 % slower and 31 % faster; at 128 8.0 %, 78 shapes, between 4 % slower and 1.8
-    // times as fast, and a factor of 0.8 there 4.7 % slower than 0.9.)
+    // The dQ/dR kernel fills the last wave.  (The whole backward of 16 shapes of each head dimension whose plan this factor decides, against
+    // none: 1.5 % faster at d_h = 64, 5.8 % at 96, 3.0 % at 128; single shapes between 7 % slower and 31 % faster.)
     if (followed) best_cost *= 0.9;
     DwPlan rest = p0;
     const double rest_cost = plan_rest(rest, items, num_sms, sh.fixed(), sh.launch(), sums, best_cost, fits);

@@ -31,7 +31,7 @@ def test_plan_does_not_depend_on_the_calls_before(a, b):
 
 # ------------------------------------------------------------------------------------------------ against a job-by-job simulation
 SMS = 148                                                                 # what the library plans for where there is no GPU
-SHAPE = {64: (128, 64, 0.8, 7.0), 96: (128, 64, 1.0, 7.0), 128: (64, 128, 1.33, 9.4)}     # weight rows, tokens and us of a tile, us of a CTA
+SHAPE = {64: (128, 64, 0.8), 96: (128, 64, 1.0), 128: (64, 128, 1.8)}     # weight rows, tokens and us of a tile
 
 
 def _plan(lib, dims, parts):
@@ -55,9 +55,9 @@ class _Search:
 
     def __init__(self, dims, followed):
         B, H, S, dh, Hk, E, de = dims
-        rows, tokens, us, cta = SHAPE[dh]
+        rows, tokens, us = SHAPE[dh]
         self.items, self.T = Hk * -(-E * de // rows), -(-S // tokens) * (H // Hk) * B
-        self.fixed, self.launch, self.sums = cta / us, 4 / us, Hk * E * de * 3 * dh * 4 / 4e6 / us
+        self.fixed, self.launch, self.sums = 7 / us, 4 / us, Hk * E * de * 3 * dh * 4 / 4e6 / us
         self.followed = followed
 
     def _parts(self, n):
