@@ -21,6 +21,9 @@ struct DwPlan {
 // How the weight-gradient kernel of a head dimension cuts its work, and what a CTA costs besides its token tiles (weights in,
 // first tile through the pipeline, accumulators out: the intercept of kernel time over tiles per CTA, about 7 us), a split's
 // extra launch (4 us) and a byte of partial sums (written once, read once, about 4 TB/s), all in units of one token tile.
+// (d_h = 128: measured on the kernel that worked with lane = token.  The present one takes 1.33 us a tile and 9.4 us a CTA besides, over one to
+// six full waves of 4 to 128 tiles a CTA, so these figures split more than is best: with 1.33 and 9.4, 140 of 1495 drawn shapes get another
+// plan, whose whole backward takes 8.4 % less, single ones between 14 % more and 1.6 times less.)
 struct DwShape {
     int rows, tokens;
     double tile_us;
@@ -173,7 +176,8 @@ inline DwPlan make_plan(const flashmhf_dims &d, int num_sms, bool followed, size
     best.tiles_per_split = p0.tiles_total;
     double best_cost = (double)((items + num_sms - 1) / num_sms) * (p0.tiles_total + sh.fixed());
     // The dQ/dR kernel fills the last wave.  (The whole backward of 16 shapes of each head dimension whose plan this factor decides, against
-    // none: 1.5 % faster at d_h = 64, 5.8 % at 96, 3.0 % at 128; single shapes between 7 % slower and 31 % faster.)
+    // none: 1.5 % faster at d_h = 64, 5.8 % at 96, 3.0 % at 128, the latter with the kernel before; single shapes between 7 % slower and 31 %
+    // faster.)
     if (followed) best_cost *= 0.9;
     DwPlan rest = p0;
     const double rest_cost = plan_rest(rest, items, num_sms, sh.fixed(), sh.launch(), sums, best_cost, fits);
