@@ -466,8 +466,8 @@ bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // reads them: 1156 us where this form takes 1017 (32768 tokens of the 370M layer's operator, in a loop at the power limit; ten passes
 // 1017 and 891).  [K;U] as an operand in shared memory instead, with dV^T: 1029 to 1039.  dA in two halves of 64 tokens, in lanes 0-15 and
 // 16-31 of 64 columns, with dV^T: 1136, since an M = 64 product takes as long at N = 64 as at 128.
-// Bound: the tensor pipe (2048 clk a tile) and shared memory (160 KB of operand reads, 64 KB of fills and 16 KB of A: 1875 clk at
-// 128 B/clk) of about 2590 clk a tile, and power.
+// Bound: the tensor pipe (2130 of 2440 clk a tile, 87 %) and with it shared memory, of whose cycles operand reads take 53 % (160 KB a tile),
+// the threads' loads and stores 23 % and the fills about 21 % (64 KB), all by counters; and power.
 template <int DH>
 struct DwSmem {
     static constexpr int kChunks = (DH + 63) / 64;
